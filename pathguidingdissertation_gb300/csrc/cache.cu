@@ -7,14 +7,16 @@
 // the left child receives the used/2 records with the smallest coordinate
 // (std::nth_element at offset + used/2) and the right child the rest.  With
 // distinct coordinates every node holds the same record set as the
-// reference's.  Large nodes are split level by level with a 4-pass radix
-// select on the ordered-int key (byte histograms per 2048-record chunk, then
-// a block-scan partition that also reduces the children's bounds); nodes of
-// at most 256 records are finished by one thread each with an in-place
-// quickselect.
+// reference's.  Nodes of more than kSmall records are split level by level
+// (radix select on the ordered-int key, then a partition that also reduces
+// the children's bounds); the records travel with their positions between two
+// buffers, and since every split is at used/2 the sizes of a level are known
+// on the host, so no level waits for the device.  A subtree of at most kSmall
+// records is finished by one CTA in shared memory (k_psubtree).
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <map>
 #include <vector>
 
 #include "pgx_ctx.h"
@@ -23,11 +25,14 @@
 namespace {
 
 constexpr int kLeafMax = 8;      // MAX_CHILDNODE_RECORDS, Renderer.h:78
-constexpr int kSmall = 256;      // one-thread subtrees at or below this size
-constexpr int kChunk = 2048;
+constexpr int kSmall = 2048;     // one-CTA subtrees at or below this size
+constexpr int kChunk = 2048;     // records per CTA of the level-by-level phase
 constexpr int kThreads = 256;
 constexpr int kPer = kChunk / kThreads;
-constexpr int kStack = 128;
+constexpr int kDigitBits = 11;   // radix select: digits of 11, 11 and 10 bits, from the top
+constexpr int kDigits = 1 << kDigitBits;
+constexpr int kPasses = 3;
+__host__ __device__ constexpr int digit_shift(int pass) { return pass == 0 ? 21 : (pass == 1 ? 10 : 0); }
 
 struct PItem {
     int node;
@@ -37,6 +42,7 @@ struct PItem {
     int k;
     int lcur, rcur, tie;
     int acc[2][6];      // child bounds: min xyz, max xyz (ordered ints)
+    unsigned done;      // chunks of the running pass that have finished
 };
 
 struct PMisc {
@@ -44,14 +50,13 @@ struct PMisc {
     int nitems_next;
     int nsmall;
     int nregions;
-    int nchunks;
     int overflow;
 };
 
 struct CacheState {
-    DevBuf recs_in, recs, pos, idx, idx2, nodes, trav, items, items2, hist, chunks, small, misc, regions, region_of;
+    DevBuf recs_in, recs, pos, pos2, idx, nodes, trav, items, items2, hist, small, misc, regions, region_of;
     DevBuf wts_in, wts;  // flux weight per record (input order, then leaf order)
-    DevBuf uvs;          // quadtree coordinates of each record's wi, leaf order (-1: outside the domain)
+    DevBuf qkey;         // quadtree build: Morton key and weight of each record, two buffers of each
     DevBuf qroot, qnodes, knn_q, knn_i, knn_d, node_region;
     int64_t n_records = 0;
     int64_t n_nodes = 0;
@@ -75,15 +80,31 @@ __device__ __forceinline__ int longest_axis(const pgx_cache_node& n) {
     return ax;
 }
 
-__global__ void k_pos(const pgx_path_vertex* __restrict__ r, int64_t n, float4* __restrict__ pos, int* idx) {
+// Positions of the input records, each with its record index in w (at least
+// one block of 256 threads runs).
+__global__ void k_pos(const pgx_path_vertex* __restrict__ r, int64_t n, float4* __restrict__ pos,
+                      int* __restrict__ acc) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 6) acc[i] = i < 3 ? INT_MAX : INT_MIN;  // for k_root_bounds
     if (i >= n) return;
-    pos[i] = make_float4(r[i].position[0], r[i].position[1], r[i].position[2], 0.f);
-    idx[i] = (int)i;
+    pos[i] = make_float4(r[i].position[0], r[i].position[1], r[i].position[2], __int_as_float((int)i));
 }
 
-__global__ void k_root(const float4* __restrict__ pos, int64_t n, PMisc* misc, pgx_cache_node* nodes, PItem* items,
-                       int* small, int* acc, int region_max) {
+// An item of the level-by-level phase, ready for its first select pass.
+__device__ __forceinline__ void start_item(PItem& it, int node, int offset, int used, const pgx_cache_node& nd) {
+    it.node = node;
+    it.offset = offset;
+    it.used = used;
+    it.axis = longest_axis(nd);
+    it.prefix = 0;
+    it.k = used / 2;
+    it.lcur = it.rcur = it.tie = 0;
+    it.done = 0;
+    for (int s = 0; s < 2; s++)
+        for (int k = 0; k < 6; k++) it.acc[s][k] = k < 3 ? INT_MAX : INT_MIN;
+}
+
+__global__ void k_root(int64_t n, PMisc* misc, pgx_cache_node* nodes, PItem* items, int2* small, int* acc) {
     // acc: 6 ordered ints reduced by k_root_bounds
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     pgx_cache_node& r = nodes[0];
@@ -99,18 +120,12 @@ __global__ void k_root(const float4* __restrict__ pos, int64_t n, PMisc* misc, p
     misc->nsmall = 0;
     misc->nregions = 0;
     misc->overflow = 0;
-    if (n <= region_max) misc->nregions = 1;  // region 0 = the root, written by the host
-    if (n <= kLeafMax) return;
     if (n <= kSmall) {
-        small[0] = 0;
+        small[0] = make_int2(0, 0);
         misc->nsmall = 1;
         return;
     }
-    PItem& it = items[0];
-    it.node = 0;
-    it.offset = 0;
-    it.used = (int)n;
-    misc->nitems_next = 1;
+    start_item(items[0], 0, 0, (int)n, r);
 }
 
 __global__ void k_root_bounds(const float4* __restrict__ pos, int64_t n, int* acc) {
@@ -139,311 +154,458 @@ __global__ void k_root_bounds(const float4* __restrict__ pos, int64_t n, int* ac
     }
 }
 
-__global__ void k_pchunks(PItem* items, int nitems, const pgx_cache_node* nodes, int2* chunks, PMisc* misc) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nitems) return;
-    PItem& it = items[i];
-    it.axis = longest_axis(nodes[it.node]);
-    it.prefix = 0;
-    it.k = it.used / 2;
-    it.lcur = it.rcur = it.tie = 0;
-    for (int s = 0; s < 2; s++)
-        for (int k = 0; k < 6; k++) it.acc[s][k] = k < 3 ? INT_MAX : INT_MIN;
-    int nch = (it.used + kChunk - 1) / kChunk;
-    int base = atomicAdd(&misc->nchunks, nch);
-    for (int c = 0; c < nch; c++) chunks[base + c] = make_int2(i, c * kChunk);
+// True in the block that finishes an item's last chunk: everything the other
+// blocks wrote for the item before their arrival is then visible to it.
+__device__ __forceinline__ bool last_chunk(PItem& it, unsigned nchunks, int* flag) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const bool last = atomicAdd(&it.done, 1u) == nchunks - 1;
+        if (last) it.done = 0;  // ready for the next pass
+        *flag = last ? 1 : 0;
+    }
+    __syncthreads();
+    const bool last = *flag != 0;
+    if (last) __threadfence();
+    return last;
 }
 
-// Histogram of key byte `b` among records whose higher bytes equal the
-// item's selected prefix.
-__global__ void __launch_bounds__(kThreads) k_phist(const PItem* __restrict__ items, const int2* __restrict__ chunks,
-                                                    const PMisc* __restrict__ misc, const int* __restrict__ idx,
-                                                    const float4* __restrict__ pos, int* __restrict__ hist, int b) {
-    __shared__ int sh[256];
-    const int nchunks = misc->nchunks;
-    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        int2 ch = chunks[c];
-        const PItem& it = items[ch.x];
-        sh[threadIdx.x] = 0;
-        __syncthreads();
-        const int end = min(it.used, ch.y + kChunk);
-        const unsigned hi_mask = (b == 3) ? 0u : (0xFFFFFFFFu << (8 * (b + 1)));
-        for (int j = ch.y + threadIdx.x; j < end; j += blockDim.x) {
-            unsigned key = key_of(axis_of(pos[idx[it.offset + j]], it.axis));
-            if ((key & hi_mask) == (it.prefix & hi_mask)) atomicAdd(&sh[(key >> (8 * b)) & 255u], 1);
+// One pass of the radix select, one block per (item, chunk): histogram of the
+// pass's digit among the records whose higher digits equal the item's
+// prefix; the block that finishes the item's last chunk scans the counts,
+// appends the digit holding rank it.k to the prefix and clears the
+// histogram.  Separate one-thread scans (34 us a pass) and 8-bit digits (four
+// passes) were most of this phase: 1.7 of 2.1 ms for 0.9 M records.
+__global__ void __launch_bounds__(kThreads) k_pselect(PItem* __restrict__ items, unsigned per_item,
+                                                      const float4* __restrict__ pos, int* __restrict__ hist,
+                                                      int pass) {
+    __shared__ int sh[kDigits];
+    __shared__ int s_warp[kThreads / 32];
+    __shared__ int s_flag;
+    const unsigned item = blockIdx.x / per_item;
+    PItem& it = items[item];
+    const int begin = (int)(blockIdx.x % per_item) * kChunk;
+    if (begin >= it.used) return;
+    const unsigned nchunks = (unsigned)((it.used + kChunk - 1) / kChunk);
+    const int shift = digit_shift(pass);
+    const unsigned mask = pass == 2 ? 1023u : 2047u;
+    const unsigned hi_mask = pass == 0 ? 0u : (0xFFFFFFFFu << digit_shift(pass - 1));
+    const unsigned prefix = it.prefix;
+    const int axis = it.axis;
+    for (int i = threadIdx.x; i < kDigits; i += kThreads) sh[i] = 0;
+    __syncthreads();
+    const int end = min(it.used, begin + kChunk);
+    for (int j = begin + threadIdx.x; j < end; j += kThreads) {
+        const unsigned key = key_of(axis_of(pos[it.offset + j], axis));
+        if ((key & hi_mask) == prefix) atomicAdd(&sh[(key >> shift) & mask], 1);
+    }
+    __syncthreads();
+    int* h = hist + (size_t)item * kDigits;
+    if (nchunks > 1) {
+        for (int i = threadIdx.x; i < kDigits; i += kThreads)
+            if (sh[i]) atomicAdd(&h[i], sh[i]);
+        if (!last_chunk(it, nchunks, &s_flag)) return;
+        for (int i = threadIdx.x; i < kDigits; i += kThreads) {
+            sh[i] = __ldcg(&h[i]);
+            h[i] = 0;
         }
         __syncthreads();
-        int v = sh[threadIdx.x];
-        if (v) atomicAdd(&hist[(size_t)ch.x * 256 + threadIdx.x], v);
-        __syncthreads();
     }
-}
-
-__global__ void k_pselect(PItem* items, int nitems, int* hist, int b) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nitems) return;
-    PItem& it = items[i];
-    int* h = hist + (size_t)i * 256;
-    int cum = 0;
-    int bucket = 255;
-    for (int v = 0; v < 256; v++) {
-        if (cum + h[v] > it.k) {
-            bucket = v;
-            break;
-        }
-        cum += h[v];
-    }
-    it.prefix |= (unsigned)bucket << (8 * b);
-    it.k -= cum;
-    for (int v = 0; v < 256; v++) h[v] = 0;
-}
-
-// Partition around the selected key: < K left, > K right, == K left while
-// the tie budget (it.k after the select) lasts.
-__global__ void __launch_bounds__(kThreads) k_ppart(PItem* __restrict__ items, const int2* __restrict__ chunks,
-                                                    const PMisc* __restrict__ misc, const int* __restrict__ idx,
-                                                    int* __restrict__ idx2, const float4* __restrict__ pos) {
-    __shared__ int s_wl[kThreads / 32], s_wr[kThreads / 32];
-    __shared__ int s_bl, s_br;
-    __shared__ int s_acc[12];
-    const int nchunks = misc->nchunks;
+    // each thread sums kDigits / kThreads neighbouring digits; a block scan
+    // finds the thread, then the digit, holding rank k
+    constexpr int kSpan = kDigits / kThreads;
+    int sum = 0;
+#pragma unroll
+    for (int i = 0; i < kSpan; i++) sum += sh[threadIdx.x * kSpan + i];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        int2 ch = chunks[c];
-        PItem& it = items[ch.x];
-        if (threadIdx.x < 12) s_acc[threadIdx.x] = (threadIdx.x % 6) < 3 ? INT_MAX : INT_MIN;
-        const int end = min(it.used, ch.y + kChunk);
-        int ids[kPer];
-        unsigned sides = 0;
-        int nl = 0, nr = 0;
-        int acc[12];
-        for (int k = 0; k < 12; k++) acc[k] = (k % 6) < 3 ? INT_MAX : INT_MIN;
-        for (int k = 0; k < kPer; k++) {
-            int j = ch.y + k * kThreads + threadIdx.x;
-            ids[k] = -1;
-            if (j >= end) continue;
-            int id = idx[it.offset + j];
-            ids[k] = id;
-            float4 p = pos[id];
-            unsigned key = key_of(axis_of(p, it.axis));
-            int side;
-            if (key < it.prefix)
-                side = 0;
-            else if (key > it.prefix)
-                side = 1;
-            else
-                side = (atomicAdd(&it.tie, 1) < it.k) ? 0 : 1;
-            sides |= (unsigned)side << k;
-            if (side == 0)
-                nl++;
-            else
-                nr++;
-            int* a = acc + 6 * side;
-            a[0] = min(a[0], f2o(p.x));
-            a[1] = min(a[1], f2o(p.y));
-            a[2] = min(a[2], f2o(p.z));
-            a[3] = max(a[3], f2o(p.x));
-            a[4] = max(a[4], f2o(p.y));
-            a[5] = max(a[5], f2o(p.z));
-        }
-        int il = nl, ir = nr;
-        for (int o = 1; o < 32; o <<= 1) {
-            int tl = __shfl_up_sync(0xFFFFFFFFu, il, o);
-            int tr = __shfl_up_sync(0xFFFFFFFFu, ir, o);
-            if (lane >= o) {
-                il += tl;
-                ir += tr;
+    int inc = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    __syncthreads();
+    for (int w = 0; w < warp; w++) inc += s_warp[w];
+    const int k = it.k;
+    __syncthreads();  // every thread has read k
+    int before = inc - sum;
+    if (before <= k && k < inc) {
+        for (int i = 0; i < kSpan; i++) {
+            const int c = sh[threadIdx.x * kSpan + i];
+            if (k < before + c) {
+                it.prefix = prefix | ((unsigned)(threadIdx.x * kSpan + i) << shift);
+                it.k = k - before;
+                break;
             }
+            before += c;
         }
-        if (lane == 31) {
-            s_wl[warp] = il;
-            s_wr[warp] = ir;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int tl = 0, tr = 0;
-            for (int w = 0; w < kThreads / 32; w++) {
-                int a = s_wl[w], bb = s_wr[w];
-                s_wl[w] = tl;
-                s_wr[w] = tr;
-                tl += a;
-                tr += bb;
-            }
-            s_bl = atomicAdd(&it.lcur, tl);
-            s_br = atomicAdd(&it.rcur, tr);
-        }
-        __syncthreads();
-        int offl = s_bl + s_wl[warp] + il - nl;
-        int offr = s_br + s_wr[warp] + ir - nr;
-        for (int k = 0; k < kPer; k++) {
-            if (ids[k] < 0) continue;
-            if (((sides >> k) & 1u) == 0)
-                idx2[it.offset + (offl++)] = ids[k];
-            else
-                idx2[it.offset + it.used - 1 - (offr++)] = ids[k];
-        }
-        for (int k = 0; k < 12; k++) {
-            int v = acc[k];
-            bool mn = (k % 6) < 3;
-            for (int o = 16; o > 0; o >>= 1) {
-                int w = __shfl_xor_sync(0xFFFFFFFFu, v, o);
-                v = mn ? min(v, w) : max(v, w);
-            }
-            if (lane == 0) {
-                if (mn)
-                    atomicMin(&s_acc[k], v);
-                else
-                    atomicMax(&s_acc[k], v);
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x < 12) {
-            int k = threadIdx.x;
-            int* dst = &it.acc[k / 6][k % 6];
-            if ((k % 6) < 3)
-                atomicMin(dst, s_acc[k]);
-            else
-                atomicMax(dst, s_acc[k]);
-        }
-        __syncthreads();
     }
 }
 
-__global__ void k_pcopy(const PItem* __restrict__ items, const int2* __restrict__ chunks,
-                        const PMisc* __restrict__ misc, int* __restrict__ idx, const int* __restrict__ idx2) {
-    const int nchunks = misc->nchunks;
-    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        int2 ch = chunks[c];
-        const PItem& it = items[ch.x];
-        int end = min(it.used, ch.y + kChunk);
-        for (int j = ch.y + threadIdx.x; j < end; j += blockDim.x) idx[it.offset + j] = idx2[it.offset + j];
+// Partition of every item around its selected key, one block per (item, chunk):
+// < K left, > K right, == K left while the tie budget (it.k after the select)
+// lasts.  The block that finishes the item's last chunk creates its children:
+// a child of more than kSmall records becomes an item of the next level,
+// any other one a subtree of k_psubtree (with the buffer its records are in).
+__global__ void __launch_bounds__(kThreads) k_ppart(PItem* __restrict__ items, unsigned per_item,
+                                                    const float4* __restrict__ pos, float4* __restrict__ out,
+                                                    PItem* __restrict__ next, int next_cap,
+                                                    int2* __restrict__ small, int small_cap, int out_buf,
+                                                    pgx_cache_node* __restrict__ nodes, int2* __restrict__ regions,
+                                                    int* __restrict__ node_region, PMisc* __restrict__ misc,
+                                                    int region_max) {
+    __shared__ int s_wl[kThreads / 32], s_wr[kThreads / 32];
+    __shared__ int s_bl, s_br, s_flag;
+    __shared__ int s_acc[12];
+    const unsigned item = blockIdx.x / per_item;
+    PItem& it = items[item];
+    const int begin = (int)(blockIdx.x % per_item) * kChunk;
+    if (begin >= it.used) return;
+    const unsigned nchunks = (unsigned)((it.used + kChunk - 1) / kChunk);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < 12) s_acc[threadIdx.x] = (threadIdx.x % 6) < 3 ? INT_MAX : INT_MIN;
+    const int end = min(it.used, begin + kChunk);
+    const int axis = it.axis, budget = it.k;
+    const unsigned pivot = it.prefix;
+    float4 p[kPer];
+    unsigned sides = 0, have = 0;
+    int nl = 0, nr = 0;
+    int acc[2][6];
+    for (int s = 0; s < 2; s++)
+        for (int k = 0; k < 6; k++) acc[s][k] = k < 3 ? INT_MAX : INT_MIN;
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const int j = begin + k * kThreads + threadIdx.x;
+        if (j >= end) continue;
+        have |= 1u << k;
+        p[k] = pos[it.offset + j];
+        const unsigned key = key_of(axis_of(p[k], axis));
+        int side = key < pivot ? 0 : 1;
+        if (key == pivot) side = (atomicAdd(&it.tie, 1) < budget) ? 0 : 1;
+        sides |= (unsigned)side << k;
+        nl += 1 - side;
+        nr += side;
+        const int o[3] = {f2o(p[k].x), f2o(p[k].y), f2o(p[k].z)};
+#pragma unroll
+        for (int s = 0; s < 2; s++)
+            if (s == side)
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    acc[s][a] = min(acc[s][a], o[a]);
+                    acc[s][3 + a] = max(acc[s][3 + a], o[a]);
+                }
     }
-}
-
-__global__ void k_pcommit(PItem* items, int nitems, PItem* next, int next_cap, int* small, int small_cap,
-                          pgx_cache_node* nodes, int2* regions, int* node_region, PMisc* misc, int region_max) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nitems) return;
-    PItem& it = items[i];
-    int half = it.used / 2;
-    if (it.lcur != half) atomicExch(&misc->overflow, 3);
-    int c = atomicAdd(&misc->node_count, 2);
+    int il = nl, ir = nr;
+    for (int o = 1; o < 32; o <<= 1) {
+        int tl = __shfl_up_sync(0xFFFFFFFFu, il, o);
+        int tr = __shfl_up_sync(0xFFFFFFFFu, ir, o);
+        if (lane >= o) {
+            il += tl;
+            ir += tr;
+        }
+    }
+    if (lane == 31) {
+        s_wl[warp] = il;
+        s_wr[warp] = ir;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int tl = 0, tr = 0;
+        for (int w = 0; w < kThreads / 32; w++) {
+            int a = s_wl[w], bb = s_wr[w];
+            s_wl[w] = tl;
+            s_wr[w] = tr;
+            tl += a;
+            tr += bb;
+        }
+        s_bl = atomicAdd(&it.lcur, tl);
+        s_br = atomicAdd(&it.rcur, tr);
+    }
+    __syncthreads();
+    int offl = it.offset + s_bl + s_wl[warp] + il - nl;
+    int offr = it.offset + it.used - 1 - (s_br + s_wr[warp] + ir - nr);
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        if (!((have >> k) & 1u)) continue;
+        if (((sides >> k) & 1u) == 0)
+            out[offl++] = p[k];
+        else
+            out[offr--] = p[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+        const bool mn = (k % 6) < 3;
+        const int v = mn ? __reduce_min_sync(0xFFFFFFFFu, acc[k / 6][k % 6]) : __reduce_max_sync(0xFFFFFFFFu, acc[k / 6][k % 6]);
+        if (lane == 0) {
+            if (mn)
+                atomicMin(&s_acc[k], v);
+            else
+                atomicMax(&s_acc[k], v);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 12) {
+        const int k = threadIdx.x;
+        int* dst = &it.acc[k / 6][k % 6];
+        if ((k % 6) < 3)
+            atomicMin(dst, s_acc[k]);
+        else
+            atomicMax(dst, s_acc[k]);
+    }
+    if (!last_chunk(it, nchunks, &s_flag) || threadIdx.x != 0) return;
+    const int half = it.used / 2;
+    if (__ldcg(&it.lcur) != half) atomicExch(&misc->overflow, 3);
+    const int c = atomicAdd(&misc->node_count, 2);
     pgx_cache_node& nd = nodes[it.node];
     nd.left = c;
     nd.right = c + 1;
     nd.used = 0;
     for (int side = 0; side < 2; side++) {
-        pgx_cache_node& ch = nodes[c + side];
-        int cs = side ? it.offset + half : it.offset;
-        int cn = side ? it.used - half : half;
+        pgx_cache_node ch;
         for (int k = 0; k < 3; k++) {
-            ch.bmin[k] = o2f(it.acc[side][k]);
-            ch.bmax[k] = o2f(it.acc[side][3 + k]);
+            ch.bmin[k] = o2f(__ldcg(&it.acc[side][k]));
+            ch.bmax[k] = o2f(__ldcg(&it.acc[side][3 + k]));
         }
         ch.left = ch.right = -1;
-        ch.offset = cs;
-        ch.used = cn;
-        if (cn <= region_max && it.used > region_max) {
-            int r = atomicAdd(&misc->nregions, 1);
-            regions[r] = make_int2(cs, cn);
+        ch.offset = side ? it.offset + half : it.offset;
+        ch.used = side ? it.used - half : half;
+        nodes[c + side] = ch;
+        if (ch.used <= region_max && it.used > region_max) {
+            const int r = atomicAdd(&misc->nregions, 1);
+            regions[r] = make_int2(ch.offset, ch.used);
             node_region[c + side] = r;
         }
-        if (cn <= kLeafMax) continue;
-        if (cn <= kSmall) {
-            int s = atomicAdd(&misc->nsmall, 1);
+        if (ch.used <= kSmall) {
+            const int s = atomicAdd(&misc->nsmall, 1);
             if (s < small_cap)
-                small[s] = c + side;
+                small[s] = make_int2(c + side, out_buf);
             else
                 atomicExch(&misc->overflow, 1);
             continue;
         }
-        int q = atomicAdd(&misc->nitems_next, 1);
+        const int q = atomicAdd(&misc->nitems_next, 1);
         if (q >= next_cap) {
             atomicExch(&misc->overflow, 2);
             continue;
         }
-        next[q].node = c + side;
-        next[q].offset = cs;
-        next[q].used = cn;
+        start_item(next[q], c + side, ch.offset, ch.used, ch);
     }
 }
 
-// In-place quickselect: afterwards idx[lo .. lo+nth) hold the nth smallest
-// keys of idx[lo .. hi) (hi exclusive).
-__device__ void quickselect(int* idx, int lo, int hi, int nth, const float4* pos, int ax) {
-    int left = lo, right = hi - 1;
-    int target = lo + nth;
-    while (right > left) {
-        int mid = left + (right - left) / 2;
-        float a = axis_of(pos[idx[left]], ax), b = axis_of(pos[idx[mid]], ax), c = axis_of(pos[idx[right]], ax);
-        float piv = (a < b) ? ((b < c) ? b : ((a < c) ? c : a)) : ((a < c) ? a : ((b < c) ? c : b));
-        int i = left, j = right;
-        while (i <= j) {
-            while (i <= right && axis_of(pos[idx[i]], ax) < piv) i++;
-            while (j >= left && piv < axis_of(pos[idx[j]], ax)) j--;
-            if (i <= j) {
-                int t = idx[i];
-                idx[i] = idx[j];
-                idx[j] = t;
-                i++;
-                j--;
-            }
-        }
-        if (target <= j)
-            right = j;
-        else if (target >= i)
-            left = i;
-        else
-            break;
-    }
-}
+// One CTA finishes the subtree of a node with at most kSmall records.  Level
+// l of the subtree has 2^l slots of S = P / 2^l record places (P the power of
+// two >= the record count): a slot holds one node, its records first, +inf
+// keys behind them.  Per level every slot is sorted by (coordinate on the
+// node's longest axis, place) with one bitonic network in shared memory; the
+// first used/2 records are the left child and stay, the rest move to the
+// slot's upper half (used - used/2 <= S/2, so both always fit).  A slot whose
+// node is a leaf (at most 8 records) sorts too, which keeps the network
+// uniform, and keeps its records in its lower places.
+//   Bound: the network's shared-memory passes (about 276 compare steps for
+// 2,048 records); one thread per <= 256-record subtree with an in-place
+// quickselect took 5.1 ms for 0.9 M records.
+constexpr int kSubThreads = 512;
+constexpr int kSubSlots = kSmall / 8;  // slots of the deepest level
+constexpr int kSubSmem = kSmall * (int)(sizeof(unsigned long long) + sizeof(float4));
 
-__global__ void k_psmall(const int* __restrict__ small, PMisc* misc, int* idx, const float4* __restrict__ pos,
-                         pgx_cache_node* nodes) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= misc->nsmall) return;
-    int stack[kStack];
-    int sp = 0;
-    stack[sp++] = small[i];
-    while (sp > 0) {
-        int nid = stack[--sp];
-        pgx_cache_node nd = nodes[nid];
-        if (nd.used <= kLeafMax) continue;
-        int ax = longest_axis(nd);
-        int half = nd.used / 2;
-        quickselect(idx, nd.offset, nd.offset + nd.used, half, pos, ax);
-        int c = atomicAdd(&misc->node_count, 2);
-        nodes[nid].left = c;
-        nodes[nid].right = c + 1;
-        nodes[nid].used = 0;
-        for (int side = 0; side < 2; side++) {
-            int cs = side ? nd.offset + half : nd.offset;
-            int cn = side ? nd.used - half : half;
-            float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-            for (int k = 0; k < cn; k++) {
-                float4 p = pos[idx[cs + k]];
-                mn[0] = s_min(mn[0], p.x);
-                mn[1] = s_min(mn[1], p.y);
-                mn[2] = s_min(mn[2], p.z);
-                mx[0] = s_max(mx[0], p.x);
-                mx[1] = s_max(mx[1], p.y);
-                mx[2] = s_max(mx[2], p.z);
-            }
-            pgx_cache_node& ch = nodes[c + side];
-            for (int k = 0; k < 3; k++) {
-                ch.bmin[k] = mn[k];
-                ch.bmax[k] = mx[k];
-            }
-            ch.left = ch.right = -1;
-            ch.offset = cs;
-            ch.used = cn;
+struct SubSlot {
+    int node;   // -1: empty
+    int offset, used;
+    int axis;   // -1: leaf or empty
+};
+
+__global__ void __launch_bounds__(kSubThreads) k_psubtree(const int2* __restrict__ small, PMisc* __restrict__ misc,
+                                                          const float4* __restrict__ pos0,
+                                                          const float4* __restrict__ pos1, int* __restrict__ idx,
+                                                          pgx_cache_node* __restrict__ nodes,
+                                                          int2* __restrict__ regions, int* __restrict__ node_region,
+                                                          int region_max) {
+    extern __shared__ __align__(16) uint8_t s_dyn[];
+    unsigned long long* key = reinterpret_cast<unsigned long long*>(s_dyn);       // [kSmall] (coordinate, place)
+    float4* rec = reinterpret_cast<float4*>(s_dyn + sizeof(unsigned long long) * kSmall);  // [kSmall]
+    __shared__ SubSlot slot[2][kSubSlots];
+    __shared__ int s_acc[kSubSlots][6];
+    __shared__ int s_base, s_nsplit, s_nregion, s_rbase;
+    const int tid = threadIdx.x;
+    const int2 job = small[blockIdx.x];
+    const pgx_cache_node root = nodes[job.x];
+    if (root.used <= kLeafMax) {
+        const float4* src = (job.y ? pos1 : pos0) + root.offset;
+        if (tid < root.used) idx[root.offset + tid] = __float_as_int(src[tid].w);
+        return;
+    }
+    int P = 16;
+    while (P < root.used) P <<= 1;
+    {
+        const float4* src = (job.y ? pos1 : pos0) + root.offset;
+        for (int i = tid; i < P; i += kSubThreads)
+            if (i < root.used) rec[i] = src[i];
+    }
+    if (tid == 0) slot[0][0] = SubSlot{job.x, root.offset, root.used, longest_axis(root)};
+    __syncthreads();
+    int cur = 0;
+    for (int S = P, nslots = 1; S >= 16; S >>= 1, nslots <<= 1) {
+        // Splitting nodes of this level: node ids and region ids for their children.
+        if (tid == 0) {
+            s_nsplit = 0;
+            s_nregion = 0;
         }
-        if (sp + 2 > kStack) {
-            atomicExch(&misc->overflow, 4);
-            continue;
+        __syncthreads();
+        int rank = -1, my_regions = 0, region_rank = 0;
+        if (tid < nslots && slot[cur][tid].axis >= 0) {
+            rank = atomicAdd(&s_nsplit, 1);
+            const int used = slot[cur][tid].used;
+            if (used > region_max) my_regions = (used / 2 <= region_max ? 1 : 0) + (used - used / 2 <= region_max ? 1 : 0);
+            if (my_regions) region_rank = atomicAdd(&s_nregion, my_regions);
         }
-        stack[sp++] = c + 1;
-        stack[sp++] = c;
+        __syncthreads();
+        if (s_nsplit == 0) break;  // only leaves are left
+        if (tid == 0) {
+            s_base = atomicAdd(&misc->node_count, 2 * s_nsplit);
+            s_rbase = s_nregion ? atomicAdd(&misc->nregions, s_nregion) : 0;
+        }
+        // Sort keys of the slots that split; the others keep their order.
+        for (int i = tid; i < P; i += kSubThreads) {
+            const SubSlot& sl = slot[cur][i / S];
+            const int r = i & (S - 1);
+            unsigned k = 0xFFFFFFFFu;
+            if (sl.axis >= 0)
+                k = r < sl.used ? key_of(axis_of(rec[i], sl.axis)) : 0xFFFFFFFFu;
+            else
+                k = 0u;
+            // place breaks ties, and puts records before the empty places
+            key[i] = ((unsigned long long)k << 32) | (unsigned)r;
+        }
+        __syncthreads();
+        bool wide = true;  // whether the previous step crossed warps
+        for (int k2 = 2; k2 <= S; k2 <<= 1) {
+            for (int j = k2 >> 1; j > 0; j >>= 1) {
+                const bool cross = j > 32;
+                if (cross || wide) __syncthreads();
+                else __syncwarp();
+                wide = cross;
+                for (int p = tid; p < (P >> 1); p += kSubThreads) {
+                    const int i = ((p & ~(j - 1)) << 1) | (p & (j - 1));
+                    const unsigned long long a = key[i], b = key[i + j];
+                    // ascending blocks of k2 alternate within a slot; the
+                    // slot-wide merge (k2 == S) always ascends
+                    const bool up = k2 == S || (i & k2) == 0;
+                    if ((a > b) == up) {
+                        key[i] = b;
+                        key[i + j] = a;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        // Children into the slot halves: place q of a half takes the record
+        // ranked q (left) or used/2 + q (right).
+        const int H = S >> 1;
+        float4 moved[kSmall / kSubThreads];
+#pragma unroll
+        for (int m = 0; m < kSmall / kSubThreads; m++) {
+            const int i = tid + m * kSubThreads;
+            if (i >= P) continue;
+            const SubSlot& sl = slot[cur][i / S];
+            const int r = i & (S - 1);
+            int from = -1;
+            if (sl.axis >= 0) {
+                const int half = sl.used / 2;
+                if (r < H)
+                    from = r < half ? r : -1;
+                else
+                    from = r - H < sl.used - half ? half + (r - H) : -1;
+                if (from >= 0) moved[m] = rec[(i & ~(S - 1)) + (int)(unsigned)key[(i & ~(S - 1)) + from]];
+            } else if (r < H) {
+                moved[m] = rec[i];  // a leaf (or an empty slot) stays in the lower half
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < kSmall / kSubThreads; m++) {
+            const int i = tid + m * kSubThreads;
+            if (i < P) rec[i] = moved[m];
+        }
+        for (int i = tid; i < 2 * nslots; i += kSubThreads)
+            for (int k = 0; k < 6; k++) s_acc[i][k] = k < 3 ? INT_MAX : INT_MIN;
+        if (tid < nslots) {
+            const SubSlot sl = slot[cur][tid];
+            SubSlot l = sl, r = SubSlot{-1, 0, 0, -1};
+            if (rank >= 0) {
+                const int half = sl.used / 2;
+                l = SubSlot{s_base + 2 * rank, sl.offset, half, 0};
+                r = SubSlot{s_base + 2 * rank + 1, sl.offset + half, sl.used - half, 0};
+                pgx_cache_node& nd = nodes[sl.node];
+                nd.left = l.node;
+                nd.right = r.node;
+                nd.used = 0;
+                int reg = s_rbase + region_rank;
+                if (sl.used > region_max) {
+                    if (l.used <= region_max) {
+                        regions[reg] = make_int2(l.offset, l.used);
+                        node_region[l.node] = reg++;
+                    }
+                    if (r.used <= region_max) {
+                        regions[reg] = make_int2(r.offset, r.used);
+                        node_region[r.node] = reg;
+                    }
+                }
+            }
+            slot[cur ^ 1][2 * tid] = l;
+            slot[cur ^ 1][2 * tid + 1] = r;
+        }
+        __syncthreads();
+        cur ^= 1;
+        // Bounds of the new nodes: warp reductions over runs of places of one
+        // slot (H >= 8, so a warp covers one slot or 2 or 4 whole ones).
+#pragma unroll
+        for (int m = 0; m < kSmall / kSubThreads; m++) {
+            const int i = tid + m * kSubThreads;
+            if (m * kSubThreads + (tid & ~31) >= P) continue;  // whole warps
+            const int si = i < P ? i / H : 0;
+            const bool in = i < P && slot[cur][si].axis == 0 && (i & (H - 1)) < slot[cur][si].used;
+            int o[6];
+            for (int k = 0; k < 6; k++) o[k] = k < 3 ? INT_MAX : INT_MIN;
+            if (in) {
+                const float4 q = rec[i];
+                o[0] = o[3] = f2o(q.x);
+                o[1] = o[4] = f2o(q.y);
+                o[2] = o[5] = f2o(q.z);
+            }
+            const int width = H < 32 ? H : 32;
+            for (int d = width >> 1; d > 0; d >>= 1)
+                for (int k = 0; k < 6; k++) {
+                    const int w = __shfl_xor_sync(0xFFFFFFFFu, o[k], d);
+                    o[k] = k < 3 ? min(o[k], w) : max(o[k], w);
+                }
+            if ((tid & (width - 1)) == 0 && i < P && slot[cur][si].axis == 0)
+                for (int k = 0; k < 6; k++) {
+                    if (k < 3)
+                        atomicMin(&s_acc[si][k], o[k]);
+                    else
+                        atomicMax(&s_acc[si][k], o[k]);
+                }
+        }
+        __syncthreads();
+        if (tid < 2 * nslots) {
+            SubSlot& sl = slot[cur][tid];
+            if (sl.axis == 0) {  // a node of this level
+                pgx_cache_node ch;
+                for (int k = 0; k < 3; k++) {
+                    ch.bmin[k] = o2f(s_acc[tid][k]);
+                    ch.bmax[k] = o2f(s_acc[tid][3 + k]);
+                }
+                ch.left = ch.right = -1;
+                ch.offset = sl.offset;
+                ch.used = sl.used;
+                nodes[sl.node] = ch;
+                sl.axis = sl.used > kLeafMax ? longest_axis(ch) : -1;
+                // a leaf's records are final: its place in the leaf order
+                if (sl.axis < 0)
+                    for (int q = 0; q < sl.used; q++) idx[sl.offset + q] = __float_as_int(rec[tid * H + q].w);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -457,28 +619,49 @@ __device__ __forceinline__ float record_lum(const pgx_path_vertex& v) {
 }
 
 // Records into leaf order, with their flux weights (the given ones, the
-// renderer's Lum(Li) |cos| / pdf, or Lum(Li); non-finite or negative -> 0)
-// and the quadtree coordinates of their wi: the cylindrical map of the
-// direction, or the diffuse sampler's primary sample (pss; (-1, -1) below
-// the hemisphere, which no cell contains).
+// renderer's Lum(Li) |cos| / pdf, or Lum(Li); non-finite or negative -> 0),
+// their positions, and the Morton key of the quadtree cell their wi falls
+// into at the depth limit: the cylindrical map of the direction, or the
+// diffuse sampler's primary sample (pss; kQtOutside below the hemisphere,
+// which no cell contains).
+constexpr int kQtBits = 2 * PGX_QT_MAX_DEPTH;  // two bits per level
+constexpr unsigned kQtOutside = 1u << 31;
+
+__device__ __forceinline__ unsigned spread_bits(unsigned x) {  // bit i -> bit 2i (16 bits)
+    x = (x | (x << 8)) & 0x00FF00FFu;
+    x = (x | (x << 4)) & 0x0F0F0F0Fu;
+    x = (x | (x << 2)) & 0x33333333u;
+    return (x | (x << 1)) & 0x55555555u;
+}
+
 __global__ void k_gather(const pgx_path_vertex* __restrict__ in, const float* __restrict__ w_in,
                          const int* __restrict__ idx, int64_t n, pgx_path_vertex* __restrict__ out,
-                         float* __restrict__ w_out, float2* __restrict__ uv_out, int pss) {
+                         float* __restrict__ w_out, float4* __restrict__ pos, unsigned* __restrict__ key_out, int pss) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int j = idx[i];
-    const pgx_path_vertex v = in[j];
-    out[i] = v;
+    const float4* src = reinterpret_cast<const float4*>(in + j);  // 48-byte records: 16-byte aligned
+    const float4 a = src[0], b = src[1], c = src[2];
+    float4* dst = reinterpret_cast<float4*>(out + i);
+    dst[0] = a;
+    dst[1] = b;
+    dst[2] = c;
+    pos[i] = make_float4(a.x, a.y, a.z, 0.f);  // w: the region (k_regions)
+    pgx_path_vertex v;
+    v.Li[0] = c.y, v.Li[1] = c.z, v.Li[2] = c.w;
     float w = w_in ? w_in[j] : record_lum(v);
     w_out[i] = (isfinite(w) && w > 0.f) ? w : 0.f;
-    const F3 wi = f3(v.wi[0], v.wi[1], v.wi[2]);
+    const F3 wi = f3(b.z, b.w, c.x);
     float u, vv;
-    if (pss) {
-        if (!pss_uv(f3(v.normal[0], v.normal[1], v.normal[2]), wi, u, vv)) u = vv = -1.f;
-    } else {
+    bool inside = true;
+    if (pss)
+        inside = pss_uv(f3(a.w, b.x, b.y), wi, u, vv);
+    else
         dir_to_uv(wi, u, vv);
-    }
-    uv_out[i] = make_float2(u, vv);
+    // u, v in [0, 1): the product by a power of two and its truncation are
+    // exact, so the key's digits are the comparisons u >= u0 + half of every level
+    const float scale = (float)(1 << PGX_QT_MAX_DEPTH);
+    key_out[i] = inside ? (spread_bits((unsigned)(u * scale)) | (spread_bits((unsigned)(vv * scale)) << 1)) : kQtOutside;
 }
 
 __global__ void k_trav(const pgx_cache_node* __restrict__ nodes, int64_t nn, CacheTravNode* __restrict__ out) {
@@ -492,51 +675,67 @@ __global__ void k_trav(const pgx_cache_node* __restrict__ nodes, int64_t nn, Cac
     out[i] = t;
 }
 
-__global__ void k_regions(const int2* __restrict__ regions, int nreg, const pgx_path_vertex* __restrict__ recs,
-                          float4* __restrict__ pos) {
+__global__ void k_regions(const int2* __restrict__ regions, int nreg, float4* __restrict__ pos) {
     int r = blockIdx.x;
     if (r >= nreg) return;
     int2 g = regions[r];
-    for (int i = threadIdx.x; i < g.y; i += blockDim.x) {
-        const pgx_path_vertex& v = recs[g.x + i];
-        pos[g.x + i] = make_float4(v.position[0], v.position[1], v.position[2], __int_as_float(r));
-    }
+    for (int i = threadIdx.x; i < g.y; i += blockDim.x) pos[g.x + i].w = __int_as_float(r);
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
     return v;
 }
-__device__ __forceinline__ int warp_sum_i(int v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
 
-// One warp builds one region's quadtree (pgx_guide.cuh): the lanes stride
-// over the region's records and reduce with shuffles; lane 0 keeps the BFS
-// queue of cells in shared memory.
-constexpr int kQtWarps = 4;
-
-__global__ void __launch_bounds__(32 * kQtWarps) k_quadtree(const int2* __restrict__ regions, int nreg,
-                                                            const float2* __restrict__ uvs,
-                                                            const float* __restrict__ wts,
-                                                            int* __restrict__ qroot, QuadNode* __restrict__ qnodes,
-                                                            float clamp_median, float refine, float compensate) {
-    __shared__ float s_u[kQtWarps][PGX_QT_MAX_NODES], s_v[kQtWarps][PGX_QT_MAX_NODES],
-        s_s[kQtWarps][PGX_QT_MAX_NODES], s_c[kQtWarps][PGX_QT_MAX_NODES];
-    __shared__ unsigned char s_d[kQtWarps][PGX_QT_MAX_NODES];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.x * kQtWarps + warp;
-    if (r >= nreg) return;  // uniform per warp
-    int2 g = regions[r];
-    const float2* ruv = uvs + g.x;
+// One CTA builds one region's quadtree (pgx_guide.cuh).  The records are
+// sorted once by the Morton key of their cell at the depth limit (four
+// stable 5-bit radix passes), after which every cell of every level is a
+// contiguous range: a level sums each child cell's range with one warp, finds
+// the next level's ranges by binary search and numbers the children that
+// split in breadth-first order.  Work is records x depth; re-reading the
+// region's records for each of up to 256 cells with one warp per region took
+// 9.5 ms for 78 regions of 16,384 records.
+//   Bound: latency (syncs and L2 round trips of one CTA per region).
+// THREADS by region size: the regions' count, not their size, fills the GPU
+// when they are small.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_quadtree(const int2* __restrict__ regions,
+                                                      const unsigned* keys, const float* wts, unsigned* kbuf,
+                                                      float* wbuf, int64_t n_all, int* __restrict__ qroot,
+                                                      QuadNode* __restrict__ qnodes, int pss, float clamp_median, float refine, float compensate) {
+    constexpr int kWarps = THREADS / 32;
+    __shared__ int s_cnt[kWarps][32];
+    __shared__ float s_f[kWarps], s_g[kWarps];
+    __shared__ int s_i[kWarps];
+    __shared__ int s_beg[PGX_QT_MAX_NODES + 1][5];        // a level's cells: child range bounds
+    __shared__ float s_c[PGX_QT_MAX_NODES];
+    __shared__ unsigned short s_first[PGX_QT_MAX_DEPTH + 1];  // first node of each level
+    __shared__ int2 s_range[PGX_QT_MAX_NODES];
+    __shared__ unsigned s_code[PGX_QT_MAX_NODES];         // Morton prefix of each node's cell
+    __shared__ float s_flux[PGX_QT_MAX_NODES][4];
+    __shared__ __align__(4) unsigned char s_want[PGX_QT_MAX_NODES];
+    __shared__ int s_nn;
+    const int r = blockIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const int2 g = regions[r];
+    const int n = g.y;
     const float* rw = wts + g.x;
-    // Median of the positive luminances by bisection on the value (only
-    // needed for the clamp).
+    auto block_sum_i = [&](int v) {
+        v = __reduce_add_sync(0xFFFFFFFFu, v);
+        __syncthreads();
+        if (lane == 0) s_i[warp] = v;
+        __syncthreads();
+        v = 0;
+        for (int w = 0; w < kWarps; w++) v += s_i[w];
+        return v;
+    };
+    // Median of the positive weights by bisection on the value (only needed
+    // for the clamp).
     float lo = FLT_MAX, hi = 0.f;
     int pos = 0;
-    for (int i = lane; i < g.y; i += 32) {
-        float w = rw[i];
+    for (int i = tid; i < n; i += THREADS) {
+        const float w = rw[i];
         if (w > 0.f) {
             lo = fminf(lo, w);
             hi = fmaxf(hi, w);
@@ -547,91 +746,206 @@ __global__ void __launch_bounds__(32 * kQtWarps) k_quadtree(const int2* __restri
         lo = fminf(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
         hi = fmaxf(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
     }
-    pos = warp_sum_i(pos);
+    if (lane == 0) {
+        s_f[warp] = lo;
+        s_g[warp] = hi;
+    }
+    pos = block_sum_i(pos);
+    for (int w = 0; w < kWarps; w++) {
+        lo = fminf(lo, s_f[w]);
+        hi = fmaxf(hi, s_g[w]);
+    }
     if (pos == 0) {
-        if (lane == 0) qroot[r] = -1;
+        if (tid == 0) qroot[r] = -1;
         return;
     }
     const int half_count = (pos + 1) / 2;
     for (int it = 0; it < (clamp_median > 0.f ? 24 : 0); it++) {
-        float mid = 0.5f * (lo + hi);
-        int below = 0;
-        for (int i = lane; i < g.y; i += 32) {
-            float w = rw[i];
-            if (w > 0.f && w <= mid) below++;
+        const float mid = 0.5f * (lo + hi);
+        int cnt = 0;
+        for (int i = tid; i < n; i += THREADS) {
+            const float w = rw[i];
+            if (w > 0.f && w <= mid) cnt++;
         }
-        below = warp_sum_i(below);
-        if (below >= half_count)
+        cnt = block_sum_i(cnt);
+        if (cnt >= half_count)
             hi = mid;
         else
             lo = mid;
     }
     const float clamp = clamp_median > 0.f ? clamp_median * hi : FLT_MAX;
     float total = 0.f;
-    for (int i = lane; i < g.y; i += 32) total += fminf(rw[i], clamp);
+    for (int i = tid; i < n; i += THREADS) total += fminf(rw[i], clamp);
     total = warp_sum(total);
+    __syncthreads();
+    if (lane == 0) s_f[warp] = total;
+    __syncthreads();
+    total = 0.f;
+    for (int w = 0; w < kWarps; w++) total += s_f[w];
     if (!(total > 0.f) || !isfinite(total)) {
-        if (lane == 0) qroot[r] = -1;
+        if (tid == 0) qroot[r] = -1;
         return;
     }
-    QuadNode* out = qnodes + (size_t)r * PGX_QT_MAX_NODES;
-    float* cu = s_u[warp];
-    float* cv = s_v[warp];
-    float* cs = s_s[warp];
-    unsigned char* cd = s_d[warp];
-    if (lane == 0) {
-        cu[0] = 0.f;
-        cv[0] = 0.f;
-        cs[0] = 1.f;
-        cd[0] = 0;
-    }
-    __syncwarp();
-    int nn = 1, head = 0;
-    const float thresh = refine * total;
-    while (head < nn) {
-        int node = head++;
-        float u0 = cu[node], v0 = cv[node], sz = cs[node], half = sz * 0.5f;
-        float flux[4] = {0.f, 0.f, 0.f, 0.f};
-        int cnt[4] = {0, 0, 0, 0};
-        for (int i = lane; i < g.y; i += 32) {
-            float w = fminf(rw[i], clamp);
-            if (!(w > 0.f)) continue;
-            const float2 uv = ruv[i];
-            const float u = uv.x, vv = uv.y;
-            if (u < u0 || u >= u0 + sz || vv < v0 || vv >= v0 + sz) continue;
-            int c = 2 * (vv >= v0 + half ? 1 : 0) + (u >= u0 + half ? 1 : 0);
-            flux[c] += w;
-            cnt[c]++;
-        }
-        QuadNode q;
-        for (int c = 0; c < 4; c++) {
-            q.flux[c] = warp_sum(flux[c]);
-            int cc = warp_sum_i(cnt[c]);
-            q.child[c] = -1;
-            if (q.flux[c] > thresh && cc >= 2 && cd[node] + 1 < PGX_QT_MAX_DEPTH && nn < PGX_QT_MAX_NODES) {
-                int k = nn++;
-                if (lane == 0) {
-                    cu[k] = u0 + half * (float)(c & 1);
-                    cv[k] = v0 + half * (float)(c >> 1);
-                    cs[k] = half;
-                    cd[k] = (unsigned char)(cd[node] + 1);
-                }
-                q.child[c] = k;
+    // Stable LSD radix sort of (key, clamped weight); records outside the
+    // domain sort last.  Every warp owns one contiguous run of a pass's input.
+    const int run = ((n + kWarps - 1) / kWarps + 31) & ~31;
+    const int r0 = min(n, warp * run), r1 = min(n, r0 + run);
+    const unsigned* ksrc = keys + g.x;
+    const float* wsrc = rw;
+    bool raw = true;  // first pass: weights are clamped on the way
+    // Only primary-sample records can lie outside the domain: one more pass
+    // moves those behind the others.
+    const int passes = kQtBits / 5 + (pss ? 1 : 0);
+    for (int pass = 0; pass < passes; pass++) {
+        const int shift = pass < kQtBits / 5 ? 5 * pass : 31;
+        unsigned* kdst = kbuf + (size_t)(pass & 1) * n_all + g.x;
+        float* wdst = wbuf + (size_t)(pass & 1) * n_all + g.x;
+        __syncthreads();
+        s_cnt[warp][lane] = 0;
+        __syncwarp();
+        for (int i = r0 + lane; i < r1; i += 32) atomicAdd(&s_cnt[warp][(ksrc[i] >> shift) & 31u], 1);
+        __syncthreads();
+        if (warp == 0) {  // lane = digit: exclusive offsets, digit-major then warp-major
+            int sum = 0;
+            for (int w = 0; w < kWarps; w++) sum += s_cnt[w][lane];
+            int inc = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                if (lane >= o) inc += t;
+            }
+            int at = inc - sum;
+            for (int w = 0; w < kWarps; w++) {
+                const int c = s_cnt[w][lane];
+                s_cnt[w][lane] = at;
+                at += c;
             }
         }
-        __syncwarp();
-        if (lane == 0) out[node] = q;
+        __syncthreads();
+        for (int b = r0; b < r1; b += 32) {
+            const int i = b + lane;
+            const bool in = i < r1;
+            const unsigned k = in ? ksrc[i] : 0u;
+            const unsigned d = in ? ((k >> shift) & 31u) : 32u;
+            const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
+            int at = 0;
+            if (in) at = s_cnt[warp][d] + __popc(peers & below);
+            __syncwarp();
+            if (in) {
+                if ((peers & below) == 0u) s_cnt[warp][d] += __popc(peers);
+                kdst[at] = k;
+                wdst[at] = raw ? fminf(wsrc[i], clamp) : wsrc[i];
+            }
+            __syncwarp();
+        }
+        __syncthreads();  // the pass's output is visible to the whole block
+        ksrc = kdst;
+        wsrc = wdst;
+        raw = false;
     }
-    if (compensate > 0.f && lane == 0) {
+    // first sorted record whose key is >= bound (records outside the domain have bit 31 set)
+    auto lower = [&](int a, int b, unsigned bound) {
+        while (a < b) {
+            const int m = (a + b) >> 1;
+            if (ksrc[m] < bound)
+                a = m + 1;
+            else
+                b = m;
+        }
+        return a;
+    };
+    QuadNode* out = qnodes + (size_t)r * PGX_QT_MAX_NODES;
+    if (tid == 0) {
+        s_range[0] = make_int2(0, lower(0, n, kQtOutside));
+        s_code[0] = 0u;
+        s_nn = 1;
+        s_first[0] = 0;
+    }
+    __syncthreads();
+    const float thresh = refine * total;
+    int first = 0, nn = 1, depth = 0;
+    while (first < nn) {
+        const int count = nn - first;  // this level's nodes: [first, nn)
+        const int shift = kQtBits - 2 * (depth + 1);
+        for (int i = tid; i < count * 5; i += THREADS) {
+            const int node = first + i / 5, c = i % 5;
+            const int2 rg = s_range[node];
+            s_beg[i / 5][c] = c == 0 ? rg.x : (c == 4 ? rg.y : lower(rg.x, rg.y, ((s_code[node] << 2) | (unsigned)c) << shift));
+        }
+        if (tid < count) s_want[tid] = 0;
+        __syncthreads();
+        for (int i = warp; i < 4 * count; i += kWarps) {
+            const int ni = i >> 2, c = i & 3;
+            const int a = s_beg[ni][c], b = s_beg[ni][c + 1];
+            float f = 0.f;
+            int some = 0;
+            for (int k = a + lane; k < b; k += 32) {
+                const float w = wsrc[k];
+                f += w;
+                some += w > 0.f ? 1 : 0;
+            }
+            f = warp_sum(f);
+            some = __reduce_add_sync(0xFFFFFFFFu, some);
+            if (lane == 0) {
+                s_flux[ni][c] = f;
+                if (f > thresh && some >= 2 && depth + 1 < PGX_QT_MAX_DEPTH) atomicOr(reinterpret_cast<unsigned*>(&s_want[ni & ~3]), 1u << (8 * (ni & 3) + c));
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {  // number the splitting children in order while the node budget lasts
+            int next = nn;
+            for (int b = 0; b < count; b += 32) {
+                const int ni = b + lane;
+                const unsigned want = ni < count ? s_want[ni] : 0u;
+                const int mine = __popc(want);
+                int inc = mine;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                    if (lane >= o) inc += t;
+                }
+                int at = next + inc - mine;
+                if (ni < count) {
+                    QuadNode q;
+                    for (int c = 0; c < 4; c++) {
+                        q.flux[c] = s_flux[ni][c];
+                        q.child[c] = -1;
+                        if ((want >> c) & 1u) {
+                            if (at < PGX_QT_MAX_NODES) {
+                                q.child[c] = at;
+                                s_range[at] = make_int2(s_beg[ni][c], s_beg[ni][c + 1]);
+                                s_code[at] = (s_code[first + ni] << 2) | (unsigned)c;
+                            }
+                            at++;
+                        }
+                    }
+                    out[first + ni] = q;
+                }
+                next += __shfl_sync(0xFFFFFFFFu, inc, 31);
+            }
+            if (lane == 0) {
+                s_nn = min(next, PGX_QT_MAX_NODES);
+                s_first[depth + 1] = (unsigned short)nn;
+            }
+        }
+        __syncthreads();
+        first = nn;
+        nn = s_nn;
+        depth++;
+    }
+    if (compensate > 0.f && tid == 0) {
         // MIS compensation: leaves lose compensate x the mean flux over their
         // area (floored at 0); interior fluxes are the sums of their
         // children, computed leaves-up (reverse breadth-first order).
+        auto depth_of = [&](int node) {
+            int d = 0;
+            while (d + 1 < depth && s_first[d + 1] <= node) d++;
+            return d;
+        };
         const QuadNode root = out[0];
         const float tot = ((root.flux[0] + root.flux[1]) + root.flux[2]) + root.flux[3];
-        float* comp = s_c[warp];
+        float* comp = s_c;
         for (int node = nn - 1; node >= 0; node--) {
             const QuadNode q = out[node];
-            const float sub = compensate * tot * ldexpf(1.f, -2 * (cd[node] + 1));
+            const float sub = compensate * tot * ldexpf(1.f, -2 * (depth_of(node) + 1));
             float sum = 0.f;
             for (int c = 0; c < 4; c++) sum += q.child[c] >= 0 ? comp[q.child[c]] : fmaxf(q.flux[c] - sub, 0.f);
             comp[node] = sum;
@@ -639,29 +953,18 @@ __global__ void __launch_bounds__(32 * kQtWarps) k_quadtree(const int2* __restri
         if (comp[0] >= 0.05f * tot) {
             for (int node = 0; node < nn; node++) {
                 QuadNode q = out[node];
-                const float sub = compensate * tot * ldexpf(1.f, -2 * (cd[node] + 1));
+                const float sub = compensate * tot * ldexpf(1.f, -2 * (depth_of(node) + 1));
                 for (int c = 0; c < 4; c++) q.flux[c] = q.child[c] >= 0 ? comp[q.child[c]] : fmaxf(q.flux[c] - sub, 0.f);
                 out[node] = q;
             }
         }
     }
-    if (lane == 0) qroot[r] = 0;  // region-relative; k_rebase makes it absolute
-}
-
-__global__ void k_rebase(int* qroot, int nreg) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nreg && qroot[r] >= 0) qroot[r] = r * PGX_QT_MAX_NODES;
-}
-
-// Child indices inside a region's quadtree are region-relative; make them
-// absolute.
-__global__ void k_rebase_children(QuadNode* q, const int* qroot, int nreg) {
-    int r = blockIdx.x;
-    if (r >= nreg || qroot[r] < 0) return;
-    for (int i = threadIdx.x; i < PGX_QT_MAX_NODES; i += blockDim.x) {
-        QuadNode& n = q[(size_t)r * PGX_QT_MAX_NODES + i];
-        for (int c = 0; c < 4; c++)
-            if (n.child[c] >= 0) n.child[c] += r * PGX_QT_MAX_NODES;
+    if (tid == 0) qroot[r] = r * PGX_QT_MAX_NODES;
+    // children inside the region's block of nodes: absolute indexes
+    __syncthreads();
+    for (int i = tid; i < nn * 4; i += THREADS) {
+        int& c = out[i >> 2].child[i & 3];
+        if (c >= 0) c += r * PGX_QT_MAX_NODES;
     }
 }
 
@@ -829,37 +1132,63 @@ int cache_build_device(pgx_ctx* ctx, const pgx_path_vertex* d_records, int64_t n
         cs->valid = true;
         return PGX_OK;
     }
-    const int64_t max_nodes = 2 * n;
-    const int64_t item_cap = n / (kSmall / 2) + 64;
-    const int64_t chunk_cap = n / kChunk + item_cap + 64;
-    const int64_t small_cap = n / (kLeafMax / 2) + 64;
-    // Parameters of this build (later pgx_guide_configure calls shape the next one).
+    // Every split is at used/2, so the sizes of the nodes of a level are one
+    // or two neighbouring numbers, and the counts of nodes, of large nodes per
+    // level, of subtrees and of regions follow from n alone.
     const int region_max = ctx->guide.region_records;
+    struct Level {
+        int64_t items, max_used;
+    };
+    std::vector<Level> levels;
+    int64_t nsmall = n <= kSmall ? 1 : 0, total_nodes = 1, nregions = n <= region_max ? 1 : 0;
+    for (std::map<int64_t, int64_t> sizes{{n, 1}}; !sizes.empty();) {
+        std::map<int64_t, int64_t> next;
+        Level lv{0, 0};
+        for (const auto& [used, count] : sizes) {
+            if (used <= kLeafMax) continue;
+            total_nodes += 2 * count;
+            if (used > kSmall) {
+                lv.items += count;
+                lv.max_used = std::max(lv.max_used, used);
+            }
+            for (const int64_t child : {used / 2, used - used / 2}) {
+                next[child] += count;
+                if (used > kSmall && child <= kSmall) nsmall += count;
+                if (used > region_max && child <= region_max) nregions += count;
+            }
+        }
+        if (lv.items) levels.push_back(lv);
+        sizes.swap(next);
+    }
+    int64_t item_cap = 1;
+    for (const Level& lv : levels) item_cap = std::max(item_cap, lv.items);
+    const int64_t max_nodes = total_nodes;
+    // Parameters of this build (later pgx_guide_configure calls shape the next one).
     const float clamp_median = ctx->guide.clamp_median, refine = ctx->guide.refine_fraction;
     const float compensate = ctx->guide.compensate;
-    const int64_t reg_cap = n / (region_max / 4) + 64;
     PGX_CUDA_TRY(ctx, cs->recs_in.reserve(sizeof(pgx_path_vertex) * n));
     PGX_CUDA_TRY(ctx, cs->recs.reserve(sizeof(pgx_path_vertex) * n));
     PGX_CUDA_TRY(ctx, cs->wts.reserve(sizeof(float) * n));
-    PGX_CUDA_TRY(ctx, cs->uvs.reserve(sizeof(float2) * n));
+    PGX_CUDA_TRY(ctx, cs->qkey.reserve(4 * sizeof(float) * n));
     if (d_weights) {
         PGX_CUDA_TRY(ctx, cs->wts_in.reserve(sizeof(float) * n));
         PGX_CUDA_TRY(ctx, cudaMemcpyAsync(cs->wts_in.p, d_weights, sizeof(float) * n, cudaMemcpyDeviceToDevice,
                                           ctx->stream));
     }
     PGX_CUDA_TRY(ctx, cs->pos.reserve(sizeof(float4) * n));
+    PGX_CUDA_TRY(ctx, cs->pos2.reserve(sizeof(float4) * n));
     PGX_CUDA_TRY(ctx, cs->idx.reserve(sizeof(int) * n));
-    PGX_CUDA_TRY(ctx, cs->idx2.reserve(sizeof(int) * n));
     PGX_CUDA_TRY(ctx, cs->nodes.reserve(sizeof(pgx_cache_node) * max_nodes));
     PGX_CUDA_TRY(ctx, cs->trav.reserve(sizeof(CacheTravNode) * max_nodes));
     PGX_CUDA_TRY(ctx, cs->items.reserve(sizeof(PItem) * item_cap));
     PGX_CUDA_TRY(ctx, cs->items2.reserve(sizeof(PItem) * item_cap));
-    PGX_CUDA_TRY(ctx, cs->hist.reserve(sizeof(int) * 256 * item_cap));
-    PGX_CUDA_TRY(ctx, cs->chunks.reserve(sizeof(int2) * chunk_cap));
-    PGX_CUDA_TRY(ctx, cs->small.reserve(sizeof(int) * small_cap));
+    PGX_CUDA_TRY(ctx, cs->hist.reserve(sizeof(int) * kDigits * item_cap));
+    PGX_CUDA_TRY(ctx, cs->small.reserve(sizeof(int2) * std::max<int64_t>(nsmall, 1)));
     PGX_CUDA_TRY(ctx, cs->misc.reserve(sizeof(PMisc) + sizeof(int) * 8));
-    PGX_CUDA_TRY(ctx, cs->regions.reserve(sizeof(int2) * reg_cap));
+    PGX_CUDA_TRY(ctx, cs->regions.reserve(sizeof(int2) * nregions));
     PGX_CUDA_TRY(ctx, cs->node_region.reserve(sizeof(int) * max_nodes));
+    PGX_CUDA_TRY(ctx, cs->qroot.reserve(sizeof(int) * nregions));
+    PGX_CUDA_TRY(ctx, cs->qnodes.reserve(sizeof(QuadNode) * PGX_QT_MAX_NODES * (size_t)nregions));
     // -1 everywhere; region roots get their region index (the root: region 0
     // when the whole cache is one region).
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(cs->node_region.p, 0xFF, sizeof(int) * max_nodes, s));
@@ -868,81 +1197,72 @@ int cache_build_device(pgx_ctx* ctx, const pgx_path_vertex* d_records, int64_t n
         PGX_CUDA_TRY(ctx, cudaMemcpyAsync(cs->recs_in.p, d_records, sizeof(pgx_path_vertex) * n,
                                           cudaMemcpyDeviceToDevice, s));
     float4* pos = cs->pos.as<float4>();
+    float4* pos2 = cs->pos2.as<float4>();
     int* idx = cs->idx.as<int>();
-    int* idx2 = cs->idx2.as<int>();
     pgx_cache_node* nodes = cs->nodes.as<pgx_cache_node>();
     PItem* items = cs->items.as<PItem>();
     PItem* items2 = cs->items2.as<PItem>();
     int* hist = cs->hist.as<int>();
-    int2* chunks = cs->chunks.as<int2>();
-    int* small = cs->small.as<int>();
+    int2* small = cs->small.as<int2>();
     PMisc* misc = cs->misc.as<PMisc>();
     int* acc = reinterpret_cast<int*>(misc + 1);
     int2* regions = cs->regions.as<int2>();
 
-    k_pos<<<blocks_for(n, 256), 256, 0, s>>>(cs->recs_in.as<pgx_path_vertex>(), n, pos, idx);
-    int hacc[8] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN, 0, 0};
-    PGX_CUDA_TRY(ctx, cudaMemcpyAsync(acc, hacc, sizeof(hacc), cudaMemcpyHostToDevice, s));
+    k_pos<<<blocks_for(n, 256), 256, 0, s>>>(cs->recs_in.as<pgx_path_vertex>(), n, pos, acc);
     k_root_bounds<<<std::min<unsigned>(blocks_for(n, 256), 4 * pgx_num_sms()), 256, 0, s>>>(pos, n, acc);
-    k_root<<<1, 32, 0, s>>>(pos, n, misc, nodes, items, small, acc, region_max);
-    PGX_CUDA_TRY(ctx, cudaMemsetAsync(hist, 0, sizeof(int) * 256 * item_cap, s));
+    k_root<<<1, 32, 0, s>>>(n, misc, nodes, items, small, acc);
+    PGX_CUDA_TRY(ctx, cudaMemsetAsync(hist, 0, sizeof(int) * kDigits * item_cap, s));
     PGX_CUDA_TRY(ctx, cudaGetLastError());
-    int nitems = 0;
-    PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&nitems, &misc->nitems_next, sizeof(int), cudaMemcpyDeviceToHost, s));
-    PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-    int levels = 0;
-    while (nitems > 0) {
-        if (++levels > 64) return pgx_fail(ctx, PGX_ERR_OVERFLOW, "cache build: too many levels");
-        PGX_CUDA_TRY(ctx, cudaMemsetAsync(&misc->nchunks, 0, sizeof(int), s));
+    float4 *src = pos, *dst = pos2;
+    int dst_buf = 1;
+    for (const Level& lv : levels) {
+        const int64_t per_item = (lv.max_used + kChunk - 1) / kChunk;
+        if (per_item * lv.items > (int64_t)INT32_MAX) return pgx_fail(ctx, PGX_ERR_OVERFLOW, "cache build: too many records");
+        const unsigned grid = (unsigned)(per_item * lv.items);
         PGX_CUDA_TRY(ctx, cudaMemsetAsync(&misc->nitems_next, 0, sizeof(int), s));
-        k_pchunks<<<blocks_for(nitems, 128), 128, 0, s>>>(items, nitems, nodes, chunks, misc);
-        unsigned grid = (unsigned)std::min<int64_t>(n / kChunk + nitems, 8 * pgx_num_sms());
-        for (int b = 3; b >= 0; b--) {
-            k_phist<<<grid, kThreads, 0, s>>>(items, chunks, misc, idx, pos, hist, b);
-            k_pselect<<<blocks_for(nitems, 64), 64, 0, s>>>(items, nitems, hist, b);
-        }
-        k_ppart<<<grid, kThreads, 0, s>>>(items, chunks, misc, idx, idx2, pos);
-        k_pcopy<<<grid, kThreads, 0, s>>>(items, chunks, misc, idx, idx2);
-        k_pcommit<<<blocks_for(nitems, 128), 128, 0, s>>>(items, nitems, items2, (int)item_cap, small,
-                                                          (int)small_cap, nodes, regions, cs->node_region.as<int>(),
-                                                          misc, region_max);
-        PGX_CUDA_TRY(ctx, cudaGetLastError());
-        PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&nitems, &misc->nitems_next, sizeof(int), cudaMemcpyDeviceToHost, s));
-        PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+        for (int pass = 0; pass < kPasses; pass++)
+            k_pselect<<<grid, kThreads, 0, s>>>(items, (unsigned)per_item, src, hist, pass);
+        k_ppart<<<grid, kThreads, 0, s>>>(items, (unsigned)per_item, src, dst, items2, (int)item_cap, small,
+                                          (int)nsmall, dst_buf, nodes, regions, cs->node_region.as<int>(), misc,
+                                          region_max);
         std::swap(items, items2);
+        std::swap(src, dst);
+        dst_buf ^= 1;
     }
+    PGX_CUDA_TRY(ctx, cudaFuncSetAttribute(k_psubtree, cudaFuncAttributeMaxDynamicSharedMemorySize, kSubSmem));
+    k_psubtree<<<(unsigned)nsmall, kSubThreads, kSubSmem, s>>>(small, misc, pos, pos2, idx, nodes, regions,
+                                                               cs->node_region.as<int>(), region_max);
+    PGX_CUDA_TRY(ctx, cudaGetLastError());
+    cs->n_nodes = total_nodes;
+    cs->n_regions = (int)nregions;
+    if (n <= region_max) {
+        const int2 r0 = make_int2(0, (int)n);
+        PGX_CUDA_TRY(ctx, cudaMemcpyAsync(regions, &r0, sizeof(r0), cudaMemcpyHostToDevice, s));
+    }
+    pgx_path_vertex* recs = cs->recs.as<pgx_path_vertex>();
+    unsigned* qkey = cs->qkey.as<unsigned>();
+    // the keys in leaf order start in the buffer that the sort's second pass
+    // overwrites, once its first pass has read them
+    unsigned* keys = qkey + n;
+    k_gather<<<blocks_for(n, 256), 256, 0, s>>>(cs->recs_in.as<pgx_path_vertex>(),
+                                                d_weights ? cs->wts_in.as<float>() : nullptr, idx, n, recs,
+                                                cs->wts.as<float>(), pos, keys, pss ? 1 : 0);
+    k_trav<<<blocks_for(cs->n_nodes, 256), 256, 0, s>>>(nodes, cs->n_nodes, cs->trav.as<CacheTravNode>());
+    // Records carry their region id; leaves below regions are inside them.
+    k_regions<<<(unsigned)nregions, 128, 0, s>>>(regions, cs->n_regions, pos);
+    float* wbuf = reinterpret_cast<float*>(qkey + 2 * n);
+    // 512 threads keep a region's serial passes short; small regions are many
+    // and need no more than 128 (1,024 records: 8 a thread).
+    auto quad = region_max <= 2048 ? k_quadtree<128> : k_quadtree<512>;
+    quad<<<(unsigned)nregions, region_max <= 2048 ? 128 : 512, 0, s>>>(
+        regions, keys, cs->wts.as<float>(), qkey, wbuf, n, cs->qroot.as<int>(), cs->qnodes.as<QuadNode>(), pss ? 1 : 0,
+        clamp_median, refine, compensate);
+    PGX_CUDA_TRY(ctx, cudaGetLastError());
     PMisc hm{};
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&hm, misc, sizeof(hm), cudaMemcpyDeviceToHost, s));
     PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-    if (hm.nsmall > 0) k_psmall<<<blocks_for(hm.nsmall, 64), 64, 0, s>>>(small, misc, idx, pos, nodes);
-    PGX_CUDA_TRY(ctx, cudaGetLastError());
-    PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&hm, misc, sizeof(hm), cudaMemcpyDeviceToHost, s));
-    PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-    if (hm.overflow) return pgx_fail(ctx, PGX_ERR_OVERFLOW, "cache build: internal overflow (%d)", hm.overflow);
-    cs->n_nodes = hm.node_count;
-    if (n <= region_max) {
-        int2 r0 = make_int2(0, (int)n);
-        PGX_CUDA_TRY(ctx, cudaMemcpyAsync(regions, &r0, sizeof(r0), cudaMemcpyHostToDevice, s));
-        hm.nregions = 1;
-    }
-    cs->n_regions = hm.nregions;
-    pgx_path_vertex* recs = cs->recs.as<pgx_path_vertex>();
-    k_gather<<<blocks_for(n, 256), 256, 0, s>>>(cs->recs_in.as<pgx_path_vertex>(),
-                                                d_weights ? cs->wts_in.as<float>() : nullptr, idx, n, recs,
-                                                cs->wts.as<float>(), cs->uvs.as<float2>(), pss ? 1 : 0);
-    k_trav<<<blocks_for(cs->n_nodes, 256), 256, 0, s>>>(nodes, cs->n_nodes, cs->trav.as<CacheTravNode>());
-    // Records carry their region id; leaves below regions are inside them.
-    k_regions<<<std::max(1, cs->n_regions), 128, 0, s>>>(regions, cs->n_regions, recs, pos);
-    PGX_CUDA_TRY(ctx, cs->qroot.reserve(sizeof(int) * std::max(1, cs->n_regions)));
-    PGX_CUDA_TRY(ctx, cs->qnodes.reserve(sizeof(QuadNode) * PGX_QT_MAX_NODES * (size_t)std::max(1, cs->n_regions)));
-    k_quadtree<<<blocks_for(cs->n_regions, kQtWarps), 32 * kQtWarps, 0, s>>>(
-        regions, cs->n_regions, cs->uvs.as<float2>(), cs->wts.as<float>(), cs->qroot.as<int>(),
-        cs->qnodes.as<QuadNode>(), clamp_median, refine, compensate);
-    k_rebase_children<<<std::max(1, cs->n_regions), 128, 0, s>>>(cs->qnodes.as<QuadNode>(), cs->qroot.as<int>(),
-                                                                   cs->n_regions);
-    k_rebase<<<blocks_for(cs->n_regions, 128), 128, 0, s>>>(cs->qroot.as<int>(), cs->n_regions);
-    PGX_CUDA_TRY(ctx, cudaGetLastError());
-    PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+    if (hm.overflow || hm.node_count != total_nodes || (n > region_max && hm.nregions != nregions))
+        return pgx_fail(ctx, PGX_ERR_OVERFLOW, "cache build: internal overflow (%d)", hm.overflow);
     cs->valid = true;
     cs->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     return PGX_OK;
