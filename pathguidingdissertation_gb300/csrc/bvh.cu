@@ -12,15 +12,18 @@
 // reference; only node numbering and the order of triangles inside a leaf
 // differ (the reference partitions in place by swapping).
 //
-// Phase A (nodes with more than kSmall triangles) runs level by level:
-// CTAs process 2048-triangle chunks of the active nodes — shared-memory
-// binning, a per-node SAH sweep, then a block-scan partition into a second
-// index buffer that also reduces the children's boxes.  Phase B hands each
-// node of at most kSmall triangles to one thread, which finishes its
-// subtree with the reference's sequential algorithm (in-place swap
-// partition) and an explicit stack.
+// Phase A (nodes with more than kSmall triangles) runs level by level with two
+// launches a level and no host round trip: CTAs take 2048-triangle chunks of
+// the active nodes.  k_bin bins a chunk in shared memory, and the block that
+// finishes a node's last chunk sweeps the SAH; k_partition splits the chunk
+// into the other record buffer and reduces the children's boxes, and the
+// node's last block creates its children.  A triangle travels as one 48-byte
+// record (box, centroid, id), so every pass reads and writes runs.  Phase B
+// gives each node of at most kSmall triangles to one warp, which finishes its
+// subtree in shared memory.
 #include <algorithm>
 #include <chrono>
+#include <cstddef>
 #include <vector>
 
 #include "pgx_ctx.h"
@@ -34,29 +37,42 @@ constexpr int kSmall = 128;        // phase-B threshold
 constexpr int kChunk = 2048;       // triangles per CTA chunk in phase A
 constexpr int kThreads = 256;
 constexpr int kPerThread = kChunk / kThreads;
-constexpr int kSmallStack = 256;   // phase-B explicit stack depth
 constexpr int kBinInts = 3 * kBins * 7;
+constexpr int kMaxLevels = 200;
 
 struct BuildItem {
     int node;
     int start, count;
+    int slot;              // global bins of a node of more than one chunk
     int cmin[3], cmax[3];  // centroid bounds, ordered-int encoded
     int axis;
     float pos;
     int split;
     int lcur, rcur;
+    unsigned done;         // chunks of the running pass that have finished
     int acc[2][12];  // per side: tbox min[3], tbox max[3], cent min[3], cent max[3] (ordered ints)
 };
 
 struct BuildMisc {
-    int node_count;
-    int rec_count;
-    int nitems_next;
+    unsigned long long counts;  // nodes in the low word, interior records in the high word
     int nsmall;
-    int nchunks;
     int overflow;
     int root_acc[12];
+    int nitems[kMaxLevels + 1];
+    int nchunks[kMaxLevels + 1];
+    int nslots[kMaxLevels + 1];
 };
+
+// A triangle on its way through the build: vertex bounds, centroid, id.
+struct RecView {
+    float4* lo;  // w = triangle id bits
+    float4* hi;
+    float4* cent;
+};
+
+// Work for phase B: node, and which record buffer holds its triangles; a
+// leaf only has its triangle ids copied.
+constexpr int kSmallBuf = 1, kSmallLeaf = 2;
 
 __device__ __forceinline__ float area_x(float mnx, float mny, float mnz, float mxx, float mxy, float mxz) {
     // AABB::area, Geometry.h:212-215
@@ -64,63 +80,95 @@ __device__ __forceinline__ float area_x(float mnx, float mny, float mnz, float m
     return x_mul(x_add(x_add(x_mul(sx, sy), x_mul(sy, sz)), x_mul(sx, sz)), 2.f);
 }
 
-// Triangle::centre and the triangle's vertex bounds.
-__global__ void k_prep(const pgx_triangle* __restrict__ tris, int64_t n, float4* __restrict__ cent,
-                       float4* __restrict__ tmin, float4* __restrict__ tmax) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const pgx_triangle& t = tris[i];
-    xv3 p0 = mk(t.v[0].p[0], t.v[0].p[1], t.v[0].p[2]);
-    xv3 p1 = mk(t.v[1].p[0], t.v[1].p[1], t.v[1].p[2]);
-    xv3 p2 = mk(t.v[2].p[0], t.v[2].p[1], t.v[2].p[2]);
-    xv3 c = x_scale(x_add(x_add(p0, p1), p2), 0.3333f);
-    cent[i] = make_float4(c.x, c.y, c.z, 0.f);
-    tmin[i] = make_float4(s_min(s_min(p0.x, p1.x), p2.x), s_min(s_min(p0.y, p1.y), p2.y),
-                          s_min(s_min(p0.z, p1.z), p2.z), 0.f);
-    tmax[i] = make_float4(s_max(s_max(p0.x, p1.x), p2.x), s_max(s_max(p0.y, p1.y), p2.y),
-                          s_max(s_max(p0.z, p1.z), p2.z), 0.f);
-}
-
-__device__ __forceinline__ void warp_minmax(int& v, bool is_min) {
-    for (int o = 16; o > 0; o >>= 1) {
-        int w = __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        v = is_min ? min(v, w) : max(v, w);
-    }
-}
-
-// Root bounds: union of triangle boxes and of centroids.
-__global__ void k_root_reduce(const float4* __restrict__ cent, const float4* __restrict__ tmin,
-                              const float4* __restrict__ tmax, int64_t n, BuildMisc* misc) {
+// Box, centroid (Triangle::centre) and id of every triangle, and the root's
+// bounds (one set of 12 atomics per block).
+__global__ void __launch_bounds__(kThreads) k_prep(const pgx_triangle* __restrict__ tris, int64_t n, RecView out,
+                                                   BuildMisc* misc) {
+    __shared__ int s_acc[12];
+    if (threadIdx.x < 12) s_acc[threadIdx.x] = ((threadIdx.x % 6) < 3) ? INT_MAX : INT_MIN;
+    __syncthreads();
     int acc[12];
+#pragma unroll
     for (int k = 0; k < 12; k++) acc[k] = ((k % 6) < 3) ? INT_MAX : INT_MIN;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        float4 a = tmin[i], b = tmax[i], c = cent[i];
-        acc[0] = min(acc[0], f2o(a.x));
-        acc[1] = min(acc[1], f2o(a.y));
-        acc[2] = min(acc[2], f2o(a.z));
-        acc[3] = max(acc[3], f2o(b.x));
-        acc[4] = max(acc[4], f2o(b.y));
-        acc[5] = max(acc[5], f2o(b.z));
-        acc[6] = min(acc[6], f2o(c.x));
-        acc[7] = min(acc[7], f2o(c.y));
-        acc[8] = min(acc[8], f2o(c.z));
-        acc[9] = max(acc[9], f2o(c.x));
-        acc[10] = max(acc[10], f2o(c.y));
-        acc[11] = max(acc[11], f2o(c.z));
+        const pgx_triangle& t = tris[i];
+        xv3 p0 = mk(t.v[0].p[0], t.v[0].p[1], t.v[0].p[2]);
+        xv3 p1 = mk(t.v[1].p[0], t.v[1].p[1], t.v[1].p[2]);
+        xv3 p2 = mk(t.v[2].p[0], t.v[2].p[1], t.v[2].p[2]);
+        xv3 c = x_scale(x_add(x_add(p0, p1), p2), 0.3333f);
+        const float v[9] = {s_min(s_min(p0.x, p1.x), p2.x), s_min(s_min(p0.y, p1.y), p2.y),
+                            s_min(s_min(p0.z, p1.z), p2.z), s_max(s_max(p0.x, p1.x), p2.x),
+                            s_max(s_max(p0.y, p1.y), p2.y), s_max(s_max(p0.z, p1.z), p2.z), c.x, c.y, c.z};
+        out.lo[i] = make_float4(v[0], v[1], v[2], __int_as_float((int)i));
+        out.hi[i] = make_float4(v[3], v[4], v[5], 0.f);
+        out.cent[i] = make_float4(c.x, c.y, c.z, 0.f);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            acc[k] = min(acc[k], f2o(v[k]));
+            acc[3 + k] = max(acc[3 + k], f2o(v[3 + k]));
+            acc[6 + k] = min(acc[6 + k], f2o(v[6 + k]));
+            acc[9 + k] = max(acc[9 + k], f2o(v[6 + k]));
+        }
     }
+#pragma unroll
     for (int k = 0; k < 12; k++) {
-        bool is_min = (k % 6) < 3;
-        warp_minmax(acc[k], is_min);
+        const bool is_min = (k % 6) < 3;
+        const int v = is_min ? __reduce_min_sync(0xFFFFFFFFu, acc[k]) : __reduce_max_sync(0xFFFFFFFFu, acc[k]);
         if ((threadIdx.x & 31) == 0) {
             if (is_min)
-                atomicMin(&misc->root_acc[k], acc[k]);
+                atomicMin(&s_acc[k], v);
             else
-                atomicMax(&misc->root_acc[k], acc[k]);
+                atomicMax(&s_acc[k], v);
         }
+    }
+    __syncthreads();
+    if (threadIdx.x < 12) {
+        if ((threadIdx.x % 6) < 3)
+            atomicMin(&misc->root_acc[threadIdx.x], s_acc[threadIdx.x]);
+        else
+            atomicMax(&misc->root_acc[threadIdx.x], s_acc[threadIdx.x]);
     }
 }
 
-__global__ void k_root_init(pgx_bvh_node* nodes, BuildItem* items, BuildMisc* misc, int64_t n, int* small) {
+// Fills an item and its chunk list; called by one thread.
+__device__ __forceinline__ void add_item(BuildItem* items, int2* chunks, BuildMisc* misc, int level, int item_cap,
+                                         int chunk_cap, int slot_cap, int node, int start, int count, const int* cmin,
+                                         const int* cmax) {
+    const int q = atomicAdd(&misc->nitems[level], 1);
+    const int nch = (count + kChunk - 1) / kChunk;
+    const int base = atomicAdd(&misc->nchunks[level], nch);
+    const int slot = nch > 1 ? atomicAdd(&misc->nslots[level], 1) : 0;
+    if (q >= item_cap || base + nch > chunk_cap || slot >= slot_cap) {
+        atomicExch(&misc->overflow, 1);
+        return;
+    }
+    BuildItem& it = items[q];
+    it.node = node;
+    it.start = start;
+    it.count = count;
+    it.slot = slot;
+    for (int k = 0; k < 3; k++) {
+        it.cmin[k] = cmin[k];
+        it.cmax[k] = cmax[k];
+    }
+    it.split = 0;
+    it.lcur = it.rcur = 0;
+    it.done = 0;
+    for (int s = 0; s < 2; s++)
+        for (int k = 0; k < 12; k++) it.acc[s][k] = ((k % 6) < 3) ? INT_MAX : INT_MIN;
+    for (int c = 0; c < nch; c++) chunks[base + c] = make_int2(q, c * kChunk);
+}
+
+__device__ __forceinline__ void add_small(int2* small, int small_cap, BuildMisc* misc, int node, int flags) {
+    const int s = atomicAdd(&misc->nsmall, 1);
+    if (s < small_cap)
+        small[s] = make_int2(node, flags);
+    else
+        atomicExch(&misc->overflow, 1);
+}
+
+__global__ void k_root_init(pgx_bvh_node* nodes, int* node_rec, BuildItem* items, int2* chunks, int2* small,
+                            BuildMisc* misc, int64_t n, int item_cap, int chunk_cap, int slot_cap, int small_cap) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     pgx_bvh_node& r = nodes[0];
     for (int k = 0; k < 3; k++) {
@@ -129,255 +177,271 @@ __global__ void k_root_init(pgx_bvh_node* nodes, BuildItem* items, BuildMisc* mi
     }
     r.left_first = 0;
     r.used = (int)n;
-    misc->node_count = 1;
-    misc->rec_count = 0;
-    misc->nitems_next = 0;
-    misc->nsmall = 0;
-    misc->overflow = 0;
-    if (n <= kMaxLeaf) return;
-    if (n <= kSmall) {
-        small[0] = 0;
-        misc->nsmall = 1;
-        return;
+    node_rec[0] = -1;
+    misc->counts = 1;
+    if (n <= kSmall)
+        add_small(small, small_cap, misc, 0, 0);
+    else
+        add_item(items, chunks, misc, 0, item_cap, chunk_cap, slot_cap, 0, 0, (int)n, misc->root_acc + 6,
+                 misc->root_acc + 9);
+}
+
+__device__ __forceinline__ void reset_bins(int* b, int i) {
+    const int f = i % 7;
+    b[i] = (f == 0) ? 0 : (f < 4 ? INT_MAX : INT_MIN);
+}
+
+__global__ void k_bins_reset(int* bins, int64_t n) {
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        const int f = (int)(i % kBinInts) % 7;
+        bins[i] = (f == 0) ? 0 : (f < 4 ? INT_MAX : INT_MIN);
     }
-    BuildItem& it = items[0];
-    it.node = 0;
-    it.start = 0;
-    it.count = (int)n;
-    for (int k = 0; k < 3; k++) {
-        it.cmin[k] = misc->root_acc[6 + k];
-        it.cmax[k] = misc->root_acc[9 + k];
-    }
-    misc->nitems_next = 1;
 }
 
-// One chunk descriptor per kChunk triangles of each active node.
-__global__ void k_chunks(BuildItem* items, int nitems, int2* chunks, BuildMisc* misc) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nitems) return;
-    BuildItem& it = items[i];
-    it.split = 0;
-    it.lcur = 0;
-    it.rcur = 0;
-    for (int s = 0; s < 2; s++)
-        for (int k = 0; k < 12; k++) it.acc[s][k] = ((k % 6) < 3) ? INT_MAX : INT_MIN;
-    int nch = (it.count + kChunk - 1) / kChunk;
-    int base = atomicAdd(&misc->nchunks, nch);
-    for (int c = 0; c < nch; c++) chunks[base + c] = make_int2(i, c * kChunk);
-}
-
-__global__ void k_bins_reset(int* bins, int nitems) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nitems * kBinInts) return;
-    int k = (i % kBinInts) % 7;
-    bins[i] = (k == 0) ? 0 : (k < 4 ? INT_MAX : INT_MIN);
-}
-
-// Bin the centroids of each chunk (findBestSplitPlane's binning loop,
-// Geometry.h:313-323) into shared memory, then merge into the node's bins.
-__global__ void __launch_bounds__(kThreads) k_bin(const BuildItem* __restrict__ items, const int2* __restrict__ chunks,
-                                                  const BuildMisc* __restrict__ misc, const int* __restrict__ idx,
-                                                  const float4* __restrict__ cent, const float4* __restrict__ tmin,
-                                                  const float4* __restrict__ tmax, int* __restrict__ gbins) {
-    __shared__ int sb[kBinInts];
-    const int nchunks = misc->nchunks;
-    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        int2 ch = chunks[c];
-        const BuildItem& it = items[ch.x];
-        for (int k = threadIdx.x; k < kBinInts; k += blockDim.x) {
-            int f = k % 7;
-            sb[k] = (f == 0) ? 0 : (f < 4 ? INT_MAX : INT_MIN);
+// Adds one triangle's box to its bin of one axis (findBestSplitPlane's
+// binning loop, Geometry.h:313-323).  Neighbouring triangles usually share a
+// bin; a warp whose lanes all do reduces first and updates the bin once,
+// instead of 32 conflicting updates of each of its 7 fields.  Whole warps;
+// bi < 0: no triangle.
+__device__ __forceinline__ void bin_add(int* bins, int ax, int bi, const int* lo, const int* hi) {
+    int same;
+    __match_all_sync(0xFFFFFFFFu, bi, &same);
+    if (same) {
+        if (bi < 0) return;
+        int* b7 = bins + (ax * kBins + bi) * 7;
+        int v[6];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            v[k] = __reduce_min_sync(0xFFFFFFFFu, lo[k]);
+            v[3 + k] = __reduce_max_sync(0xFFFFFFFFu, hi[k]);
         }
+        const int lane = threadIdx.x & 31;
+        if (lane == 0) {
+            atomicAdd(b7, 32);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                atomicMin(b7 + 1 + k, v[k]);
+                atomicMax(b7 + 4 + k, v[3 + k]);
+            }
+        }
+    } else if (bi >= 0) {
+        int* b7 = bins + (ax * kBins + bi) * 7;
+        atomicAdd(b7, 1);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            atomicMin(b7 + 1 + k, lo[k]);
+            atomicMax(b7 + 4 + k, hi[k]);
+        }
+    }
+}
+
+__device__ __forceinline__ int bin_of(float c, float lo, float scale) {
+    const int bi = (int)x_mul(x_sub(c, lo), scale);
+    return (bi < kBins - 1) ? bi : kBins - 1;
+}
+
+// Sweep of findBestSplitPlane (Geometry.h:325-362) by one warp: 16 lanes per
+// axis hold one bin each (axes 0 and 1 together, then axis 2), prefix and
+// suffix scans give every candidate's sides, and the smallest cost wins, the
+// first one in the reference's order (axis, then plane) on ties.  Returns the
+// axis (-1: none) with its plane and cost.  Minima and maxima commute, so the
+// result is the sequential sweep's.
+__device__ __forceinline__ int warp_sweep(const int* bins, const float* lo, const float* hi, float parent_area,
+                                          float& best, float& pos) {
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, b = lane & 15;
+    int axis = -1;
+    best = FLT_MAX;
+    pos = -FLT_MAX;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+        const int ax = half == 0 ? lane >> 4 : 2;
+        const float l = ax == 0 ? lo[0] : (ax == 1 ? lo[1] : lo[2]);
+        const float h = ax == 0 ? hi[0] : (ax == 1 ? hi[1] : hi[2]);
+        const int* b7 = bins + (ax * kBins + b) * 7;
+        int pc = b7[0], pm[6];
+#pragma unroll
+        for (int k = 0; k < 6; k++) pm[k] = b7[1 + k];
+        int sc = pc, sm[6];
+#pragma unroll
+        for (int k = 0; k < 6; k++) sm[k] = pm[k];
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            int t = __shfl_up_sync(kFull, pc, o, 16);
+            if (b >= o) pc += t;
+            t = __shfl_down_sync(kFull, sc, o, 16);
+            if (b + o < 16) sc += t;
+#pragma unroll
+            for (int k = 0; k < 6; k++) {
+                t = __shfl_up_sync(kFull, pm[k], o, 16);
+                if (b >= o) pm[k] = k < 3 ? min(pm[k], t) : max(pm[k], t);
+                t = __shfl_down_sync(kFull, sm[k], o, 16);
+                if (b + o < 16) sm[k] = k < 3 ? min(sm[k], t) : max(sm[k], t);
+            }
+        }
+        // the right side of plane b starts at bin b + 1
+        sc = __shfl_down_sync(kFull, sc, 1, 16);
+#pragma unroll
+        for (int k = 0; k < 6; k++) sm[k] = __shfl_down_sync(kFull, sm[k], 1, 16);
+        const float la = pc > 0 ? area_x(o2f(pm[0]), o2f(pm[1]), o2f(pm[2]), o2f(pm[3]), o2f(pm[4]), o2f(pm[5])) : 0.f;
+        const float ra = sc > 0 ? area_x(o2f(sm[0]), o2f(sm[1]), o2f(sm[2]), o2f(sm[3]), o2f(sm[4]), o2f(sm[5])) : 0.f;
+        const float cost = x_add(x_add(1.f, x_mul(x_mul(x_div(la, parent_area), (float)pc), 1.5f)),
+                                 x_mul(x_mul(x_div(ra, parent_area), (float)sc), 1.5f));
+        const bool ok = b < kBins - 1 && !(l == h) && (half == 0 || lane < 16) && cost < best;
+        // costs are ordered as ordered ints (a cost that is not below FLT_MAX, or NaN, is no candidate)
+        const int key = ok ? f2o(cost) : INT_MAX;
+        const int mn = __reduce_min_sync(kFull, key);
+        if (mn != INT_MAX) {
+            const int win = __ffs(__ballot_sync(kFull, key == mn)) - 1;
+            const float cand = x_add(l, x_mul(x_div(x_sub(h, l), (float)kBins), (float)(b + 1)));
+            best = __shfl_sync(kFull, cost, win);
+            pos = __shfl_sync(kFull, cand, win);
+            axis = __shfl_sync(kFull, ax, win);
+        }
+    }
+    return axis;
+}
+
+// True in the block that finishes an item's last chunk: everything the other
+// blocks wrote for the item before their arrival is then visible to it.
+__device__ __forceinline__ bool last_chunk(BuildItem& it, unsigned nchunks, int* flag) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const bool last = atomicAdd(&it.done, 1u) == nchunks - 1;
+        if (last) it.done = 0;  // ready for the next pass
+        *flag = last ? 1 : 0;
+    }
+    __syncthreads();
+    const bool last = *flag != 0;
+    if (last) __threadfence();
+    return last;
+}
+
+// Bins of each chunk in shared memory, merged into the node's global bins
+// when it has several chunks; the last chunk's block decides the split
+// (subdivide, Geometry.h:367-381).  A node that stays a leaf goes to phase B
+// for its triangle ids.
+__global__ void __launch_bounds__(kThreads) k_bin(BuildItem* __restrict__ items, const int2* __restrict__ chunks,
+                                                  BuildMisc* __restrict__ misc, int level, RecView rec, int buf,
+                                                  int* __restrict__ gbins, pgx_bvh_node* __restrict__ nodes,
+                                                  int2* __restrict__ small, int small_cap) {
+    __shared__ int sb[kBinInts];
+    __shared__ int s_flag;
+    const int nchunks = misc->nchunks[level];
+    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        const int2 ch = chunks[c];
+        BuildItem& it = items[ch.x];
+        const int start = it.start, count = it.count;
+        for (int k = threadIdx.x; k < kBinInts; k += kThreads) reset_bins(sb, k);
         __syncthreads();
-        float lo[3], scale[3];
-        bool active[3];
+        float lo[3], hi[3], scale[3];
+#pragma unroll
         for (int ax = 0; ax < 3; ax++) {
             lo[ax] = o2f(it.cmin[ax]);
-            float hi = o2f(it.cmax[ax]);
-            active[ax] = !(lo[ax] == hi);
-            scale[ax] = x_div((float)kBins, x_sub(hi, lo[ax]));
+            hi[ax] = o2f(it.cmax[ax]);
+            scale[ax] = x_div((float)kBins, x_sub(hi[ax], lo[ax]));
         }
-        int end = min(it.count, ch.y + kChunk);
-        for (int j = ch.y + threadIdx.x; j < end; j += blockDim.x) {
-            int id = idx[it.start + j];
-            float4 cc = cent[id];
-            float4 a = tmin[id], b = tmax[id];
-            float cv[3] = {cc.x, cc.y, cc.z};
-            for (int ax = 0; ax < 3; ax++) {
-                if (!active[ax]) continue;
-                int bi = (int)x_mul(x_sub(cv[ax], lo[ax]), scale[ax]);
-                bi = (bi < kBins - 1) ? bi : kBins - 1;
-                int* b7 = sb + (ax * kBins + bi) * 7;
-                atomicAdd(b7, 1);
-                atomicMin(b7 + 1, f2o(a.x));
-                atomicMin(b7 + 2, f2o(a.y));
-                atomicMin(b7 + 3, f2o(a.z));
-                atomicMax(b7 + 4, f2o(b.x));
-                atomicMax(b7 + 5, f2o(b.y));
-                atomicMax(b7 + 6, f2o(b.z));
+        const int end = min(count, ch.y + kChunk);
+        for (int b = ch.y; b < end; b += kThreads) {  // whole warps
+            const int j = b + threadIdx.x;
+            const bool in = j < end;
+            float cv[3] = {0.f, 0.f, 0.f};
+            int l[3] = {INT_MAX, INT_MAX, INT_MAX}, h[3] = {INT_MIN, INT_MIN, INT_MIN};
+            if (in) {
+                const float4 a = rec.lo[start + j], bb = rec.hi[start + j], cc = rec.cent[start + j];
+                cv[0] = cc.x, cv[1] = cc.y, cv[2] = cc.z;
+                l[0] = f2o(a.x), l[1] = f2o(a.y), l[2] = f2o(a.z);
+                h[0] = f2o(bb.x), h[1] = f2o(bb.y), h[2] = f2o(bb.z);
             }
+#pragma unroll
+            for (int ax = 0; ax < 3; ax++)
+                if (!(lo[ax] == hi[ax])) bin_add(sb, ax, in ? bin_of(cv[ax], lo[ax], scale[ax]) : -1, l, h);
         }
         __syncthreads();
-        int* g = gbins + (size_t)ch.x * kBinInts;
-        for (int k = threadIdx.x; k < kBinInts; k += blockDim.x) {
-            int bin_base = (k / 7) * 7;
-            if (sb[bin_base] == 0) continue;
-            int f = k % 7;
-            if (f == 0)
-                atomicAdd(g + k, sb[k]);
-            else if (f < 4)
-                atomicMin(g + k, sb[k]);
-            else
-                atomicMax(g + k, sb[k]);
-        }
-        __syncthreads();
-    }
-}
-
-// Sweep of findBestSplitPlane (Geometry.h:325-362) for one axis given its
-// bins; updates best/axis/pos exactly like the reference's loop.
-__device__ void sweep_axis(const int* cnt, const float (*bmn)[3], const float (*bmx)[3], float lo, float hi,
-                           float parent_area, int ax, float& best, int& axis, float& pos) {
-    float left_area[kBins - 1], right_area[kBins - 1];
-    int left_count[kBins - 1], right_count[kBins - 1];
-    int lsum = 0, rsum = 0;
-    float lmn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, lmx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    float rmn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, rmx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (int i = 0; i < kBins - 1; i++) {
-        lsum += cnt[i];
-        left_count[i] = lsum;
-        if (cnt[i] > 0) {
-            for (int k = 0; k < 3; k++) {
-                lmx[k] = s_max(lmx[k], bmn[i][k]);
-                lmn[k] = s_min(lmn[k], bmn[i][k]);
+        const unsigned nch = (unsigned)((count + kChunk - 1) / kChunk);
+        bool decide = true;
+        if (nch > 1) {
+            int* g = gbins + (size_t)it.slot * kBinInts;
+            for (int k = threadIdx.x; k < kBinInts; k += kThreads) {
+                if (sb[(k / 7) * 7] == 0) continue;
+                const int f = k % 7;
+                if (f == 0)
+                    atomicAdd(g + k, sb[k]);
+                else if (f < 4)
+                    atomicMin(g + k, sb[k]);
+                else
+                    atomicMax(g + k, sb[k]);
             }
-            for (int k = 0; k < 3; k++) {
-                lmx[k] = s_max(lmx[k], bmx[i][k]);
-                lmn[k] = s_min(lmn[k], bmx[i][k]);
+            decide = last_chunk(it, nch, &s_flag);
+            if (decide) {
+                for (int k = threadIdx.x; k < kBinInts; k += kThreads) {
+                    sb[k] = __ldcg(g + k);
+                    reset_bins(g, k);  // for the next level's node in this slot
+                }
+                __syncthreads();
             }
         }
-        left_area[i] = (lsum > 0) ? area_x(lmn[0], lmn[1], lmn[2], lmx[0], lmx[1], lmx[2]) : 0.f;
-        int r = kBins - 1 - i;
-        rsum += cnt[r];
-        right_count[kBins - 2 - i] = rsum;
-        if (cnt[r] > 0) {
-            for (int k = 0; k < 3; k++) {
-                rmx[k] = s_max(rmx[k], bmn[r][k]);
-                rmn[k] = s_min(rmn[k], bmn[r][k]);
-            }
-            for (int k = 0; k < 3; k++) {
-                rmx[k] = s_max(rmx[k], bmx[r][k]);
-                rmn[k] = s_min(rmn[k], bmx[r][k]);
-            }
-        }
-        right_area[kBins - 2 - i] = (rsum > 0) ? area_x(rmn[0], rmn[1], rmn[2], rmx[0], rmx[1], rmx[2]) : 0.f;
-    }
-    float scale = x_div(x_sub(hi, lo), (float)kBins);
-    for (int i = 0; i < kBins - 1; i++) {
-        float la = x_div(left_area[i], parent_area);
-        float ra = x_div(right_area[i], parent_area);
-        float cost = x_add(x_add(1.f, x_mul(x_mul(la, (float)left_count[i]), 1.5f)),
-                           x_mul(x_mul(ra, (float)right_count[i]), 1.5f));
-        float cand = x_add(lo, x_mul(scale, (float)(i + 1)));
-        if (cost < best) {
-            pos = cand;
-            axis = ax;
-            best = cost;
-        }
-    }
-}
-
-// SAH decision per active node (subdivide, Geometry.h:367-381).
-__global__ void k_split(BuildItem* items, int nitems, const int* __restrict__ gbins, pgx_bvh_node* nodes) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nitems) return;
-    BuildItem& it = items[i];
-    pgx_bvh_node& nd = nodes[it.node];
-    float parent_area = area_x(nd.bmin[0], nd.bmin[1], nd.bmin[2], nd.bmax[0], nd.bmax[1], nd.bmax[2]);
-    float best = FLT_MAX, pos = -FLT_MAX;
-    int axis = -1;
-    const int* g = gbins + (size_t)i * kBinInts;
-    for (int ax = 0; ax < 3; ax++) {
-        float lo = o2f(it.cmin[ax]), hi = o2f(it.cmax[ax]);
-        if (lo == hi) continue;
-        int cnt[kBins];
-        float bmn[kBins][3], bmx[kBins][3];
-        for (int b = 0; b < kBins; b++) {
-            const int* b7 = g + (ax * kBins + b) * 7;
-            cnt[b] = b7[0];
-            for (int k = 0; k < 3; k++) {
-                bmn[b][k] = o2f(b7[1 + k]);
-                bmx[b][k] = o2f(b7[4 + k]);
+        if (decide && threadIdx.x < 32) {
+            pgx_bvh_node& nd = nodes[it.node];
+            const float parent_area = area_x(nd.bmin[0], nd.bmin[1], nd.bmin[2], nd.bmax[0], nd.bmax[1], nd.bmax[2]);
+            float best, pos;
+            const int axis = warp_sweep(sb, lo, hi, parent_area, best, pos);
+            if (threadIdx.x == 0) {
+                const float no_split = x_mul((float)count, 1.5f);
+                if (best >= no_split || axis == -1) {
+                    it.split = 0;
+                    nd.left_first = start;
+                    nd.used = count;
+                    add_small(small, small_cap, misc, it.node, kSmallLeaf | (buf ? kSmallBuf : 0));
+                } else {
+                    it.split = 1;
+                    it.axis = axis;
+                    it.pos = pos;
+                }
             }
         }
-        sweep_axis(cnt, bmn, bmx, lo, hi, parent_area, ax, best, axis, pos);
+        __syncthreads();  // the shared bins are reused
     }
-    float no_split = x_mul((float)it.count, 1.5f);
-    if (best >= no_split || axis == -1) {
-        it.split = 0;
-        nd.left_first = it.start;
-        nd.used = it.count;
-        return;
-    }
-    it.split = 1;
-    it.axis = axis;
-    it.pos = pos;
 }
 
 // Partition of each chunk by centroid[axis] < pos (Geometry.h:384-391) into
-// the second index buffer, plus the children's box and centroid bounds.
+// the other record buffer, with the children's box and centroid bounds; the
+// node's last chunk's block creates its children (Geometry.h:393-412).
 __global__ void __launch_bounds__(kThreads) k_partition(BuildItem* __restrict__ items, const int2* __restrict__ chunks,
-                                                        const BuildMisc* __restrict__ misc, const int* __restrict__ idx,
-                                                        int* __restrict__ idx2, const float4* __restrict__ cent,
-                                                        const float4* __restrict__ tmin,
-                                                        const float4* __restrict__ tmax) {
+                                                        BuildMisc* __restrict__ misc, int level, RecView rec,
+                                                        RecView out, int out_buf, BuildItem* __restrict__ next,
+                                                        int2* __restrict__ next_chunks, int item_cap, int chunk_cap,
+                                                        int slot_cap, int2* __restrict__ small, int small_cap,
+                                                        pgx_bvh_node* __restrict__ nodes, int* __restrict__ node_rec) {
     __shared__ int s_warp_l[kThreads / 32], s_warp_r[kThreads / 32];
-    __shared__ int s_base_l, s_base_r;
+    __shared__ int s_base_l, s_base_r, s_flag;
     __shared__ int s_acc[24];
-    const int nchunks = misc->nchunks;
+    const int nchunks = misc->nchunks[level];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        int2 ch = chunks[c];
+        const int2 ch = chunks[c];
         BuildItem& it = items[ch.x];
         if (!it.split) continue;  // uniform per block
+        const int start = it.start, count = it.count;
         if (threadIdx.x < 24) s_acc[threadIdx.x] = ((threadIdx.x % 6) < 3) ? INT_MAX : INT_MIN;
         const int axis = it.axis;
         const float pos = it.pos;
-        const int end = min(it.count, ch.y + kChunk);
+        const int end = min(count, ch.y + kChunk);
         // Thread t owns positions ch.y + k*kThreads + t (coalesced reads).
-        int ids[kPerThread];
         unsigned sides = 0;
         int nl = 0, nr = 0;
-        int acc[24];
-        for (int k = 0; k < 24; k++) acc[k] = ((k % 6) < 3) ? INT_MAX : INT_MIN;
+#pragma unroll
         for (int k = 0; k < kPerThread; k++) {
-            int j = ch.y + k * kThreads + threadIdx.x;
-            ids[k] = -1;
+            const int j = ch.y + k * kThreads + threadIdx.x;
             if (j >= end) continue;
-            int id = idx[it.start + j];
-            ids[k] = id;
-            float4 cc = cent[id];
-            float cv = axis == 0 ? cc.x : (axis == 1 ? cc.y : cc.z);
-            int side = (cv < pos) ? 0 : 1;
+            const float4 cc = rec.cent[start + j];
+            const float cv = axis == 0 ? cc.x : (axis == 1 ? cc.y : cc.z);
+            const int side = (cv < pos) ? 0 : 1;
             sides |= (unsigned)side << k;
-            if (side == 0)
-                nl++;
-            else
-                nr++;
-            float4 a = tmin[id], b = tmax[id];
-            int* s = acc + side * 12;
-            s[0] = min(s[0], f2o(a.x));
-            s[1] = min(s[1], f2o(a.y));
-            s[2] = min(s[2], f2o(a.z));
-            s[3] = max(s[3], f2o(b.x));
-            s[4] = max(s[4], f2o(b.y));
-            s[5] = max(s[5], f2o(b.z));
-            s[6] = min(s[6], f2o(cc.x));
-            s[7] = min(s[7], f2o(cc.y));
-            s[8] = min(s[8], f2o(cc.z));
-            s[9] = max(s[9], f2o(cc.x));
-            s[10] = max(s[10], f2o(cc.y));
-            s[11] = max(s[11], f2o(cc.z));
+            nl += 1 - side;
+            nr += side;
         }
         // Exclusive scan of nl / nr across the block.
         int il = nl, ir = nr;
@@ -407,23 +471,43 @@ __global__ void __launch_bounds__(kThreads) k_partition(BuildItem* __restrict__ 
             s_base_r = atomicAdd(&it.rcur, tr);
         }
         __syncthreads();
-        int offl = s_base_l + s_warp_l[warp] + il - nl;
-        int offr = s_base_r + s_warp_r[warp] + ir - nr;
+        int offl = start + s_base_l + s_warp_l[warp] + il - nl;
+        int offr = start + count - 1 - (s_base_r + s_warp_r[warp] + ir - nr);
+        int acc[2][12];
+#pragma unroll
+        for (int k = 0; k < 24; k++) acc[k / 12][k % 12] = ((k % 6) < 3) ? INT_MAX : INT_MIN;
         for (int k = 0; k < kPerThread; k++) {
-            if (ids[k] < 0) continue;
-            if (((sides >> k) & 1u) == 0)
-                idx2[it.start + (offl++)] = ids[k];
-            else
-                idx2[it.start + it.count - 1 - (offr++)] = ids[k];
+            const int j = ch.y + k * kThreads + threadIdx.x;
+            if (j >= end) continue;
+            const float4 a = rec.lo[start + j], b = rec.hi[start + j], cc = rec.cent[start + j];
+            const int side = (sides >> k) & 1;
+            const int to = side ? offr-- : offl++;
+            out.lo[to] = a;
+            out.hi[to] = b;
+            out.cent[to] = cc;
+            const int v[9] = {f2o(a.x), f2o(a.y), f2o(a.z), f2o(b.x), f2o(b.y), f2o(b.z), f2o(cc.x), f2o(cc.y), f2o(cc.z)};
+#pragma unroll
+            for (int s = 0; s < 2; s++)
+                if (s == side) {
+#pragma unroll
+                    for (int x = 0; x < 3; x++) {
+                        acc[s][x] = min(acc[s][x], v[x]);
+                        acc[s][3 + x] = max(acc[s][3 + x], v[3 + x]);
+                        acc[s][6 + x] = min(acc[s][6 + x], v[6 + x]);
+                        acc[s][9 + x] = max(acc[s][9 + x], v[6 + x]);
+                    }
+                }
         }
+#pragma unroll
         for (int k = 0; k < 24; k++) {
-            bool is_min = (k % 6) < 3;
-            warp_minmax(acc[k], is_min);
+            const bool is_min = (k % 6) < 3;
+            const int v = is_min ? __reduce_min_sync(0xFFFFFFFFu, acc[k / 12][k % 12])
+                                 : __reduce_max_sync(0xFFFFFFFFu, acc[k / 12][k % 12]);
             if (lane == 0) {
                 if (is_min)
-                    atomicMin(&s_acc[k], acc[k]);
+                    atomicMin(&s_acc[k], v);
                 else
-                    atomicMax(&s_acc[k], acc[k]);
+                    atomicMax(&s_acc[k], v);
             }
         }
         __syncthreads();
@@ -435,179 +519,263 @@ __global__ void __launch_bounds__(kThreads) k_partition(BuildItem* __restrict__ 
             else
                 atomicMax(dst, s_acc[k]);
         }
+        const unsigned nch = (unsigned)((count + kChunk - 1) / kChunk);
+        if (last_chunk(it, nch, &s_flag) && threadIdx.x == 0) {
+            pgx_bvh_node& nd = nodes[it.node];
+            const int L = __ldcg(&it.lcur);
+            const int from = out_buf ? kSmallBuf : 0;
+            if (L == 0 || L == count) {
+                nd.left_first = start;
+                nd.used = count;
+                add_small(small, small_cap, misc, it.node, kSmallLeaf | from);
+            } else {
+                const unsigned long long at = atomicAdd(&misc->counts, 2ull | (1ull << 32));
+                const int child = (int)(unsigned)at;
+                node_rec[it.node] = (int)(at >> 32);
+                nd.left_first = child;
+                nd.used = 0;
+                for (int side = 0; side < 2; side++) {
+                    const int cs = side ? start + L : start;
+                    const int cn = side ? count - L : L;
+                    int box[12];
+                    for (int k = 0; k < 12; k++) box[k] = __ldcg(&it.acc[side][k]);
+                    pgx_bvh_node& cnd = nodes[child + side];
+                    for (int k = 0; k < 3; k++) {
+                        cnd.bmin[k] = o2f(box[k]);
+                        cnd.bmax[k] = o2f(box[3 + k]);
+                    }
+                    cnd.left_first = cs;
+                    cnd.used = cn;
+                    node_rec[child + side] = -1;
+                    if (cn <= kSmall)
+                        add_small(small, small_cap, misc, child + side, from);
+                    else
+                        add_item(next, next_chunks, misc, level + 1, item_cap, chunk_cap, slot_cap, child + side, cs, cn,
+                                 box + 6, box + 9);
+                }
+            }
+        }
         __syncthreads();
     }
 }
 
-__global__ void k_copyback(const BuildItem* __restrict__ items, const int2* __restrict__ chunks,
-                           const BuildMisc* __restrict__ misc, int* __restrict__ idx, const int* __restrict__ idx2) {
-    const int nchunks = misc->nchunks;
-    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        int2 ch = chunks[c];
-        const BuildItem& it = items[ch.x];
-        if (!it.split) continue;
-        int end = min(it.count, ch.y + kChunk);
-        for (int j = ch.y + threadIdx.x; j < end; j += blockDim.x) idx[it.start + j] = idx2[it.start + j];
-    }
-}
+// Phase B: one warp finishes the subtree of a node of at most kSmall
+// triangles (Geometry.h:274-417), its records in shared memory, depth first.
+// The subtree's nodes go to a scratch block first (a subtree of c triangles
+// needs at most 2c - 2 of them, and those of the position range
+// [first, first + c) are scratch[2 first ...)), so that one atomic reserves a
+// contiguous run of nodes and traversal records per subtree.
+//   Bound: issue of dependent warp steps (about 450 instructions a node).  One
+// thread per subtree, with its bins in local memory and two atomics a node,
+// took 7.4 ms for 2,093,058 triangles.
+constexpr int kSmallWarps = 4;
+struct SmallWarp {
+    float v[9][kSmall];    // box min, box max, centroid
+    int id[kSmall];
+    int bins[kBinInts];
+    int2 stack[kSmall];    // (first | count << 8 | scratch node << 16, parent area)
+    unsigned char perm[kSmall];
+};
 
-// Child creation after the partition (Geometry.h:393-412).
-__global__ void k_commit(BuildItem* items, int nitems, BuildItem* next, int next_cap, int* small, int small_cap,
-                         pgx_bvh_node* nodes, int* node_rec, BuildMisc* misc) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nitems) return;
-    BuildItem& it = items[i];
-    if (!it.split) return;
-    pgx_bvh_node& nd = nodes[it.node];
-    int L = it.lcur;
-    if (L == 0 || L == it.count) {
-        nd.left_first = it.start;
-        nd.used = it.count;
-        return;
-    }
-    int c = atomicAdd(&misc->node_count, 2);
-    node_rec[it.node] = atomicAdd(&misc->rec_count, 1);
-    nd.left_first = c;
-    nd.used = 0;
-    for (int side = 0; side < 2; side++) {
-        int child = c + side;
-        int cs = side ? it.start + L : it.start;
-        int cn = side ? it.count - L : L;
-        pgx_bvh_node& cnd = nodes[child];
-        for (int k = 0; k < 3; k++) {
-            cnd.bmin[k] = o2f(it.acc[side][k]);
-            cnd.bmax[k] = o2f(it.acc[side][3 + k]);
-        }
-        cnd.left_first = cs;
-        cnd.used = cn;
-        if (cn <= kMaxLeaf) continue;
-        if (cn <= kSmall) {
-            int s = atomicAdd(&misc->nsmall, 1);
-            if (s < small_cap)
-                small[s] = child;
-            else
-                atomicExch(&misc->overflow, 1);
+__global__ void __launch_bounds__(32 * kSmallWarps) k_small(const int2* __restrict__ small,
+                                                            BuildMisc* __restrict__ misc, RecView rec0, RecView rec1,
+                                                            int* __restrict__ idx, pgx_bvh_node* __restrict__ nodes,
+                                                            int* __restrict__ node_rec,
+                                                            pgx_bvh_node* __restrict__ scratch) {
+    extern __shared__ __align__(16) uint8_t s_dyn[];
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    SmallWarp& W = reinterpret_cast<SmallWarp*>(s_dyn)[threadIdx.x >> 5];
+    const int nsmall = misc->nsmall;
+    for (int job = blockIdx.x * kSmallWarps + (threadIdx.x >> 5); job < nsmall; job += gridDim.x * kSmallWarps) {
+        const int2 jb = small[job];
+        const pgx_bvh_node root = nodes[jb.x];
+        const int first = root.left_first, total = root.used;
+        const RecView rec = (jb.y & kSmallBuf) ? rec1 : rec0;
+        if ((jb.y & kSmallLeaf) || total <= kMaxLeaf) {
+            for (int k = lane; k < total; k += 32) idx[first + k] = __float_as_int(rec.lo[first + k].w);
             continue;
         }
-        int q = atomicAdd(&misc->nitems_next, 1);
-        if (q >= next_cap) {
-            atomicExch(&misc->overflow, 1);
-            continue;
+        __syncwarp();
+        for (int k = lane; k < total; k += 32) {
+            const float4 a = rec.lo[first + k], b = rec.hi[first + k], c = rec.cent[first + k];
+            W.v[0][k] = a.x, W.v[1][k] = a.y, W.v[2][k] = a.z;
+            W.v[3][k] = b.x, W.v[4][k] = b.y, W.v[5][k] = b.z;
+            W.v[6][k] = c.x, W.v[7][k] = c.y, W.v[8][k] = c.z;
+            W.id[k] = __float_as_int(a.w);
+            W.perm[k] = (unsigned char)k;
         }
-        BuildItem& ni = next[q];
-        ni.node = child;
-        ni.start = cs;
-        ni.count = cn;
-        for (int k = 0; k < 3; k++) {
-            ni.cmin[k] = it.acc[side][6 + k];
-            ni.cmax[k] = it.acc[side][9 + k];
-        }
-    }
-}
-
-// Phase B: one thread finishes the subtree of a small node with the
-// reference's sequential algorithm (Geometry.h:274-417).
-__global__ void k_small(const int* __restrict__ small, const BuildMisc* __restrict__ misc_ro, int* __restrict__ idx,
-                        const float4* __restrict__ cent, const float4* __restrict__ tmin,
-                        const float4* __restrict__ tmax, pgx_bvh_node* nodes, int* node_rec, BuildMisc* misc) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= misc_ro->nsmall) return;
-    int stack[kSmallStack];
-    int sp = 0;
-    stack[sp++] = small[i];
-    while (sp > 0) {
-        int nid = stack[--sp];
-        pgx_bvh_node nd = nodes[nid];
-        int start = nd.left_first, cnt = nd.used;
-        if (cnt <= kMaxLeaf) continue;
-        float parent_area = area_x(nd.bmin[0], nd.bmin[1], nd.bmin[2], nd.bmax[0], nd.bmax[1], nd.bmax[2]);
-        float best = FLT_MAX, pos = -FLT_MAX;
-        int axis = -1;
-        for (int ax = 0; ax < 3; ax++) {
-            float lo = FLT_MAX, hi = -FLT_MAX;
-            for (int k = 0; k < cnt; k++) {
-                float4 c = cent[idx[start + k]];
-                float cv = ax == 0 ? c.x : (ax == 1 ? c.y : c.z);
-                lo = s_min(lo, cv);
-                hi = s_max(hi, cv);
-            }
-            if (lo == hi) continue;
-            int bc[kBins];
-            float bmn[kBins][3], bmx[kBins][3];
-            for (int b = 0; b < kBins; b++) {
-                bc[b] = 0;
-                for (int k = 0; k < 3; k++) {
-                    bmn[b][k] = FLT_MAX;
-                    bmx[b][k] = -FLT_MAX;
+        __syncwarp();
+        pgx_bvh_node* tmp = scratch + 2 * (size_t)first;
+        int nn = 0, ni = 0, sp = 0;    // scratch nodes, interior nodes, stack height
+        int s0 = 0, cnt = total, self = -1;  // current node: [s0, s0 + cnt), its scratch node (-1: the root)
+        float area = area_x(root.bmin[0], root.bmin[1], root.bmin[2], root.bmax[0], root.bmax[1], root.bmax[2]);
+        for (;;) {
+            bool split = cnt > kMaxLeaf;
+            if (split) {
+                const int rounds = (cnt + 31) >> 5;
+                int p[kSmall / 32];
+                float lo[3], hi[3], scale[3];
+                {
+                    int mn[3] = {INT_MAX, INT_MAX, INT_MAX}, mx[3] = {INT_MIN, INT_MIN, INT_MIN};
+#pragma unroll
+                    for (int k = 0; k < kSmall / 32; k++) {
+                        p[k] = -1;
+                        if (k < rounds && k * 32 + lane < cnt) {
+                            p[k] = W.perm[s0 + k * 32 + lane];
+#pragma unroll
+                            for (int x = 0; x < 3; x++) {
+                                const int o = f2o(W.v[6 + x][p[k]]);
+                                mn[x] = min(mn[x], o);
+                                mx[x] = max(mx[x], o);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int x = 0; x < 3; x++) {
+                        lo[x] = o2f(__reduce_min_sync(kFull, mn[x]));
+                        hi[x] = o2f(__reduce_max_sync(kFull, mx[x]));
+                        scale[x] = x_div((float)kBins, x_sub(hi[x], lo[x]));
+                    }
+                }
+                for (int k = lane; k < kBinInts; k += 32) reset_bins(W.bins, k);
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < kSmall / 32; k++) {
+                    if (k >= rounds || p[k] < 0) continue;
+                    int l[3], h[3];
+#pragma unroll
+                    for (int x = 0; x < 3; x++) {
+                        l[x] = f2o(W.v[x][p[k]]);
+                        h[x] = f2o(W.v[3 + x][p[k]]);
+                    }
+#pragma unroll
+                    for (int ax = 0; ax < 3; ax++) {
+                        if (lo[ax] == hi[ax]) continue;
+                        int* b7 = W.bins + (ax * kBins + bin_of(W.v[6 + ax][p[k]], lo[ax], scale[ax])) * 7;
+                        atomicAdd(b7, 1);
+#pragma unroll
+                        for (int x = 0; x < 3; x++) {
+                            atomicMin(b7 + 1 + x, l[x]);
+                            atomicMax(b7 + 4 + x, h[x]);
+                        }
+                    }
+                }
+                __syncwarp();
+                float best, pos;
+                const int axis = warp_sweep(W.bins, lo, hi, area, best, pos);
+                split = !(best >= x_mul((float)cnt, 1.5f) || axis == -1);
+                int L = 0;
+                unsigned left[kSmall / 32];
+                if (split) {
+#pragma unroll
+                    for (int k = 0; k < kSmall / 32; k++) {
+                        left[k] = __ballot_sync(kFull, p[k] >= 0 && W.v[6 + axis][max(p[k], 0)] < pos);
+                        L += __popc(left[k]);
+                    }
+                    split = L != 0 && L != cnt;
+                }
+                if (split) {
+                    int at_l = s0, at_r = s0 + L;
+                    int box[2][6];
+#pragma unroll
+                    for (int k = 0; k < 12; k++) box[k / 6][k % 6] = (k % 6) < 3 ? INT_MAX : INT_MIN;
+#pragma unroll
+                    for (int k = 0; k < kSmall / 32; k++) {
+                        const unsigned have = __ballot_sync(kFull, p[k] >= 0);
+                        const unsigned right = have & ~left[k];
+                        if (p[k] >= 0) {
+                            const bool is_l = (left[k] >> lane) & 1u;
+                            W.perm[is_l ? at_l + __popc(left[k] & below) : at_r + __popc(right & below)] =
+                                (unsigned char)p[k];
+#pragma unroll
+                            for (int s = 0; s < 2; s++)
+                                if ((s == 0) == is_l) {
+#pragma unroll
+                                    for (int x = 0; x < 3; x++) {
+                                        box[s][x] = min(box[s][x], f2o(W.v[x][p[k]]));
+                                        box[s][3 + x] = max(box[s][3 + x], f2o(W.v[3 + x][p[k]]));
+                                    }
+                                }
+                        }
+                        at_l += __popc(left[k]);
+                        at_r += __popc(right);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 12; k++)
+                        box[k / 6][k % 6] = (k % 6) < 3 ? __reduce_min_sync(kFull, box[k / 6][k % 6])
+                                                        : __reduce_max_sync(kFull, box[k / 6][k % 6]);
+                    float ca[2];
+#pragma unroll
+                    for (int s = 0; s < 2; s++) {
+                        const float b[6] = {o2f(box[s][0]), o2f(box[s][1]), o2f(box[s][2]),
+                                            o2f(box[s][3]), o2f(box[s][4]), o2f(box[s][5])};
+                        ca[s] = area_x(b[0], b[1], b[2], b[3], b[4], b[5]);
+                        if (lane == s) {
+                            pgx_bvh_node& ch = tmp[nn + s];
+                            for (int x = 0; x < 3; x++) {
+                                ch.bmin[x] = b[x];
+                                ch.bmax[x] = b[3 + x];
+                            }
+                            ch.left_first = first + (s ? s0 + L : s0);
+                            ch.used = s ? cnt - L : L;
+                        }
+                    }
+                    __syncwarp();
+                    // an interior node: its left child's scratch node and its
+                    // ordinal among the subtree's interior nodes
+                    if (lane == 0) {
+                        if (self >= 0) {
+                            tmp[self].left_first = nn | (ni << 16);
+                            tmp[self].used = 0;
+                        }
+                        W.stack[sp] = make_int2((s0 + L) | ((cnt - L) << 8) | ((nn + 1) << 16), __float_as_int(ca[1]));
+                    }
+                    sp++;
+                    ni++;
+                    self = nn;
+                    cnt = L;
+                    area = ca[0];
+                    nn += 2;
+                    __syncwarp();
+                    continue;
                 }
             }
-            float scale = x_div((float)kBins, x_sub(hi, lo));
-            for (int k = 0; k < cnt; k++) {
-                int id = idx[start + k];
-                float4 c = cent[id];
-                float cv = ax == 0 ? c.x : (ax == 1 ? c.y : c.z);
-                int bi = (int)x_mul(x_sub(cv, lo), scale);
-                bi = (bi < kBins - 1) ? bi : kBins - 1;
-                float4 a = tmin[id], b = tmax[id];
-                bc[bi]++;
-                bmn[bi][0] = s_min(bmn[bi][0], a.x);
-                bmn[bi][1] = s_min(bmn[bi][1], a.y);
-                bmn[bi][2] = s_min(bmn[bi][2], a.z);
-                bmx[bi][0] = s_max(bmx[bi][0], b.x);
-                bmx[bi][1] = s_max(bmx[bi][1], b.y);
-                bmx[bi][2] = s_max(bmx[bi][2], b.z);
-            }
-            sweep_axis(bc, bmn, bmx, lo, hi, parent_area, ax, best, axis, pos);
+            // a leaf: the next node from the stack
+            if (sp == 0) break;
+            sp--;
+            __syncwarp();
+            const int2 e = W.stack[sp];
+            __syncwarp();
+            s0 = e.x & 0xFF;
+            cnt = (e.x >> 8) & 0xFF;
+            self = e.x >> 16;
+            area = __int_as_float(e.y);
         }
-        float no_split = x_mul((float)cnt, 1.5f);
-        if (best >= no_split || axis == -1) continue;
-        int a = start, b = start + cnt - 1;
-        while (a <= b) {
-            float4 c = cent[idx[a]];
-            float cv = axis == 0 ? c.x : (axis == 1 ? c.y : c.z);
-            if (cv < pos) {
-                a++;
-            } else {
-                int t = idx[a];
-                idx[a] = idx[b];
-                idx[b] = t;
-                b--;
+        __syncwarp();
+        for (int k = lane; k < total; k += 32) idx[first + k] = W.id[W.perm[k]];
+        if (nn == 0) continue;  // the root stays a leaf
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(&misc->counts, (unsigned long long)nn | ((unsigned long long)ni << 32));
+        at = __shfl_sync(kFull, at, 0);
+        const int base = (int)(unsigned)at, rbase = (int)(at >> 32);
+        for (int k = lane; k < nn; k += 32) {
+            pgx_bvh_node nd = tmp[k];
+            int r = -1;
+            if (nd.used == 0) {
+                r = rbase + (nd.left_first >> 16);
+                nd.left_first = base + (nd.left_first & 0xFFFF);
             }
+            nodes[base + k] = nd;
+            node_rec[base + k] = r;
         }
-        int L = a - start;
-        if (L == 0 || L == cnt) continue;
-        if (sp + 2 > kSmallStack) {
-            atomicExch(&misc->overflow, 2);
-            continue;
+        if (lane == 0) {
+            nodes[jb.x].left_first = base;
+            nodes[jb.x].used = 0;
+            node_rec[jb.x] = rbase;
         }
-        int c = atomicAdd(&misc->node_count, 2);
-        node_rec[nid] = atomicAdd(&misc->rec_count, 1);
-        nodes[nid].left_first = c;
-        nodes[nid].used = 0;
-        for (int side = 0; side < 2; side++) {
-            int cs = side ? start + L : start;
-            int cn = side ? cnt - L : L;
-            float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-            for (int k = 0; k < cn; k++) {
-                int id = idx[cs + k];
-                float4 ta = tmin[id], tb = tmax[id];
-                mn[0] = s_min(mn[0], ta.x);
-                mn[1] = s_min(mn[1], ta.y);
-                mn[2] = s_min(mn[2], ta.z);
-                mx[0] = s_max(mx[0], tb.x);
-                mx[1] = s_max(mx[1], tb.y);
-                mx[2] = s_max(mx[2], tb.z);
-            }
-            pgx_bvh_node& cnd = nodes[c + side];
-            for (int k = 0; k < 3; k++) {
-                cnd.bmin[k] = mn[k];
-                cnd.bmax[k] = mx[k];
-            }
-            cnd.left_first = cs;
-            cnd.used = cn;
-        }
-        stack[sp++] = c + 1;
-        stack[sp++] = c;
+        __syncwarp();
     }
 }
 
@@ -648,15 +816,6 @@ __global__ void k_reorder(const pgx_triangle* __restrict__ tris, const int* __re
     o.e1 = make_float4(e1.x, e1.y, e1.z, 0.f);
     o.pad = make_float4(0.f, 0.f, 0.f, 0.f);
     out[p] = o;
-}
-
-__global__ void k_fill_int(int* p, int64_t n, int v) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
-}
-__global__ void k_iota(int* p, int64_t n) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = (int)i;
 }
 
 inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -726,81 +885,84 @@ int bvh_build_gpu(pgx_ctx* ctx) {
     }
     if (n > (int64_t)INT32_MAX / 2) return pgx_fail(ctx, PGX_ERR_INVALID_ARG, "too many triangles for a BVH");
     const int64_t max_nodes = 2 * n - 1;
-    const int64_t item_cap = n / (kSmall / 2) + 64;
-    const int64_t small_cap = n / (kMaxLeaf / 2) + 64;
+    const int64_t item_cap = n / kSmall + 64;       // an item has more than kSmall triangles
+    const int64_t slot_cap = n / kChunk + 64;       // a slot's node has more than kChunk
     const int64_t chunk_cap = n / kChunk + item_cap + 64;
-    PGX_CUDA_TRY(ctx, ctx->b_cent.reserve(sizeof(float4) * n));
-    PGX_CUDA_TRY(ctx, ctx->b_tmin.reserve(sizeof(float4) * n));
-    PGX_CUDA_TRY(ctx, ctx->b_tmax.reserve(sizeof(float4) * n));
-    PGX_CUDA_TRY(ctx, ctx->b_idx2.reserve(sizeof(int) * n));
+    const int64_t small_cap = n + 64;               // disjoint, non-empty position ranges
+    PGX_CUDA_TRY(ctx, ctx->b_recs.reserve(3 * sizeof(float4) * n));
+    PGX_CUDA_TRY(ctx, ctx->b_recs2.reserve(3 * sizeof(float4) * n));
+    PGX_CUDA_TRY(ctx, ctx->b_tmp.reserve(2 * sizeof(pgx_bvh_node) * n));
     PGX_CUDA_TRY(ctx, ctx->bvh_idx.reserve(sizeof(int) * n));
     PGX_CUDA_TRY(ctx, ctx->bvh_nodes_ref.reserve(sizeof(pgx_bvh_node) * max_nodes));
     PGX_CUDA_TRY(ctx, ctx->b_noderec.reserve(sizeof(int) * max_nodes));
     PGX_CUDA_TRY(ctx, ctx->b_items.reserve(sizeof(BuildItem) * item_cap));
     PGX_CUDA_TRY(ctx, ctx->b_items2.reserve(sizeof(BuildItem) * item_cap));
-    PGX_CUDA_TRY(ctx, ctx->b_bins.reserve(sizeof(int) * kBinInts * item_cap));
+    PGX_CUDA_TRY(ctx, ctx->b_bins.reserve(sizeof(int) * kBinInts * slot_cap));
     PGX_CUDA_TRY(ctx, ctx->b_chunks.reserve(sizeof(int2) * chunk_cap));
-    PGX_CUDA_TRY(ctx, ctx->b_small.reserve(sizeof(int) * small_cap));
+    PGX_CUDA_TRY(ctx, ctx->b_chunks2.reserve(sizeof(int2) * chunk_cap));
+    PGX_CUDA_TRY(ctx, ctx->b_small.reserve(sizeof(int2) * small_cap));
     PGX_CUDA_TRY(ctx, ctx->b_misc.reserve(sizeof(BuildMisc)));
 
-    float4* cent = ctx->b_cent.as<float4>();
-    float4* tmin = ctx->b_tmin.as<float4>();
-    float4* tmax = ctx->b_tmax.as<float4>();
+    auto view = [n](const DevBuf& b) { return RecView{b.as<float4>(), b.as<float4>() + n, b.as<float4>() + 2 * n}; };
+    const RecView recs[2] = {view(ctx->b_recs), view(ctx->b_recs2)};
     int* idx = ctx->bvh_idx.as<int>();
-    int* idx2 = ctx->b_idx2.as<int>();
     pgx_bvh_node* nodes = ctx->bvh_nodes_ref.as<pgx_bvh_node>();
     int* node_rec = ctx->b_noderec.as<int>();
-    BuildItem* items = ctx->b_items.as<BuildItem>();
-    BuildItem* items2 = ctx->b_items2.as<BuildItem>();
+    BuildItem* items[2] = {ctx->b_items.as<BuildItem>(), ctx->b_items2.as<BuildItem>()};
+    int2* chunks[2] = {ctx->b_chunks.as<int2>(), ctx->b_chunks2.as<int2>()};
     int* bins = ctx->b_bins.as<int>();
-    int2* chunks = ctx->b_chunks.as<int2>();
-    int* small = ctx->b_small.as<int>();
+    int2* small = ctx->b_small.as<int2>();
     BuildMisc* misc = ctx->b_misc.as<BuildMisc>();
 
-    k_prep<<<blocks_for(n, 256), 256, 0, s>>>(ctx->tris_in.as<pgx_triangle>(), n, cent, tmin, tmax);
-    k_iota<<<blocks_for(n, 256), 256, 0, s>>>(idx, n);
-    k_fill_int<<<blocks_for(max_nodes, 256), 256, 0, s>>>(node_rec, max_nodes, -1);
     BuildMisc hm{};
     for (int k = 0; k < 12; k++) hm.root_acc[k] = ((k % 6) < 3) ? INT_MAX : INT_MIN;
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(misc, &hm, sizeof(hm), cudaMemcpyHostToDevice, s));
-    k_root_reduce<<<std::min<unsigned>(blocks_for(n, 256), 4 * pgx_num_sms()), 256, 0, s>>>(cent, tmin, tmax, n, misc);
-    k_root_init<<<1, 32, 0, s>>>(nodes, items, misc, n, small);
-    PGX_CUDA_TRY(ctx, cudaGetLastError());
-
-    int nitems = 0;
-    PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&nitems, &misc->nitems_next, sizeof(int), cudaMemcpyDeviceToHost, s));
-    PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-    int levels = 0;
-    while (nitems > 0) {
-        if (++levels > 200) return pgx_fail(ctx, PGX_ERR_OVERFLOW, "BVH build: too many levels");
-        PGX_CUDA_TRY(ctx, cudaMemsetAsync(&misc->nchunks, 0, sizeof(int), s));
-        PGX_CUDA_TRY(ctx, cudaMemsetAsync(&misc->nitems_next, 0, sizeof(int), s));
-        k_chunks<<<blocks_for(nitems, 128), 128, 0, s>>>(items, nitems, chunks, misc);
-        k_bins_reset<<<blocks_for((int64_t)nitems * kBinInts, 256), 256, 0, s>>>(bins, nitems);
-        unsigned grid = (unsigned)std::min<int64_t>(n / kChunk + nitems, 8 * pgx_num_sms());
-        k_bin<<<grid, kThreads, 0, s>>>(items, chunks, misc, idx, cent, tmin, tmax, bins);
-        k_split<<<blocks_for(nitems, 64), 64, 0, s>>>(items, nitems, bins, nodes);
-        k_partition<<<grid, kThreads, 0, s>>>(items, chunks, misc, idx, idx2, cent, tmin, tmax);
-        k_copyback<<<grid, kThreads, 0, s>>>(items, chunks, misc, idx, idx2);
-        k_commit<<<blocks_for(nitems, 128), 128, 0, s>>>(items, nitems, items2, (int)item_cap, small, (int)small_cap,
-                                                          nodes, node_rec, misc);
+    const unsigned wide = 8 * pgx_num_sms();
+    k_prep<<<std::min<unsigned>(blocks_for(n, kThreads), wide), kThreads, 0, s>>>(ctx->tris_in.as<pgx_triangle>(), n,
+                                                                                  recs[0], misc);
+    k_bins_reset<<<blocks_for(kBinInts * slot_cap, 256), 256, 0, s>>>(bins, kBinInts * slot_cap);
+    k_root_init<<<1, 32, 0, s>>>(nodes, node_rec, items[0], chunks[0], small, misc, n, (int)item_cap, (int)chunk_cap,
+                                 (int)slot_cap, (int)small_cap);
+    // A level's work list is on the device, so levels are enqueued ahead: the
+    // fewest there can be (splits in halves) at once, then two at a time until
+    // the list is empty.
+    int ahead = 0;
+    for (int64_t c = n; c > kSmall; c = (c + 1) / 2) ahead++;
+    const unsigned grid = (unsigned)std::min<int64_t>(chunk_cap, wide);
+    for (int level = 0; n > kSmall;) {
+        for (const int stop = level + ahead; level < stop && level < kMaxLevels; level++) {
+            const int a = level & 1, b = a ^ 1;
+            k_bin<<<grid, kThreads, 0, s>>>(items[a], chunks[a], misc, level, recs[a], a, bins, nodes, small,
+                                            (int)small_cap);
+            k_partition<<<grid, kThreads, 0, s>>>(items[a], chunks[a], misc, level, recs[a], recs[b], b, items[b],
+                                                  chunks[b], (int)item_cap, (int)chunk_cap, (int)slot_cap, small,
+                                                  (int)small_cap, nodes, node_rec);
+        }
         PGX_CUDA_TRY(ctx, cudaGetLastError());
-        PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&nitems, &misc->nitems_next, sizeof(int), cudaMemcpyDeviceToHost, s));
+        int left = 0, bad = 0;
+        PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&left, &misc->nchunks[level], sizeof(int), cudaMemcpyDeviceToHost, s));
+        PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&bad, &misc->overflow, sizeof(int), cudaMemcpyDeviceToHost, s));
         PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-        std::swap(items, items2);
+        if (bad) return pgx_fail(ctx, PGX_ERR_OVERFLOW, "BVH build: work list overflow (%d)", bad);
+        if (left == 0) break;
+        if (level >= kMaxLevels) return pgx_fail(ctx, PGX_ERR_OVERFLOW, "BVH build: too many levels");
+        ahead = 2;
     }
-    int nsmall = 0;
-    PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&nsmall, &misc->nsmall, sizeof(int), cudaMemcpyDeviceToHost, s));
-    PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-    if (nsmall > 0)
-        k_small<<<blocks_for(nsmall, 64), 64, 0, s>>>(small, misc, idx, cent, tmin, tmax, nodes, node_rec, misc);
+    constexpr int kSmallSmem = (int)sizeof(SmallWarp) * kSmallWarps;
+    int per_sm = 0;
+    PGX_CUDA_TRY(ctx, cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem));
+    PGX_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small, 32 * kSmallWarps, kSmallSmem));
+    // about two triangles a leaf at least: no more warps than subtrees of 8 triangles
+    const int64_t small_blocks = std::min<int64_t>(n / (8 * kSmallWarps) + 1, (int64_t)pgx_num_sms() * std::max(per_sm, 1));
+    k_small<<<(unsigned)small_blocks, 32 * kSmallWarps, kSmallSmem, s>>>(small, misc, recs[0], recs[1], idx, nodes,
+                                                                         node_rec, ctx->b_tmp.as<pgx_bvh_node>());
     PGX_CUDA_TRY(ctx, cudaGetLastError());
     BuildMisc fin{};
-    PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&fin, misc, sizeof(fin), cudaMemcpyDeviceToHost, s));
+    PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&fin, misc, offsetof(BuildMisc, root_acc), cudaMemcpyDeviceToHost, s));
     PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
     if (fin.overflow) return pgx_fail(ctx, PGX_ERR_OVERFLOW, "BVH build: work list overflow (%d)", fin.overflow);
-    ctx->n_nodes = fin.node_count;
-    ctx->n_records = fin.rec_count;
+    ctx->n_nodes = (int64_t)(unsigned)fin.counts;
+    ctx->n_records = (int64_t)(fin.counts >> 32);
     PGX_TRY(finish_layout(ctx));
     auto t1 = std::chrono::steady_clock::now();
     ctx->bvh_build_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();

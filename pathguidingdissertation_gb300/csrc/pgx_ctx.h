@@ -166,7 +166,7 @@ struct pgx_ctx {
     unsigned long long last_interior = 0, last_tris = 0;
 
     // ---- build scratch ----
-    DevBuf b_cent, b_tmin, b_tmax, b_idx2, b_items, b_items2, b_bins, b_chunks, b_small, b_misc, b_noderec;
+    DevBuf b_recs, b_recs2, b_tmp, b_items, b_items2, b_bins, b_chunks, b_chunks2, b_small, b_misc, b_noderec;
 
     // ---- film / render ----
     int32_t width = 0, height = 0;
