@@ -779,6 +779,14 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(const int2* __restri
     }
 }
 
+__device__ __forceinline__ TravChild trav_child(const pgx_bvh_node& c, int rec) {
+    TravChild t;
+    t.mnx = c.bmin[0], t.mny = c.bmin[1], t.mnz = c.bmin[2];
+    t.mxx = c.bmax[0], t.mxy = c.bmax[1], t.mxz = c.bmax[2];
+    t.ref = c.used > 0 ? c.left_first : rec;
+    t.count = c.used;
+    return t;
+}
 // Traversal records from the reference-layout tree.
 __global__ void k_layout(const pgx_bvh_node* __restrict__ nodes, int64_t nnodes, const int* __restrict__ node_rec,
                          TravNode* __restrict__ out) {
@@ -790,13 +798,9 @@ __global__ void k_layout(const pgx_bvh_node* __restrict__ nodes, int64_t nnodes,
     if (rec < 0) return;
     const pgx_bvh_node& L = nodes[nd.left_first];
     const pgx_bvh_node& R = nodes[nd.left_first + 1];
-    int lref = L.used > 0 ? L.left_first : node_rec[nd.left_first];
-    int rref = R.used > 0 ? R.left_first : node_rec[nd.left_first + 1];
     TravNode t;
-    t.lmin = make_float4(L.bmin[0], L.bmin[1], L.bmin[2], __int_as_float(lref));
-    t.lmax = make_float4(L.bmax[0], L.bmax[1], L.bmax[2], __int_as_float(L.used));
-    t.rmin = make_float4(R.bmin[0], R.bmin[1], R.bmin[2], __int_as_float(rref));
-    t.rmax = make_float4(R.bmax[0], R.bmax[1], R.bmax[2], __int_as_float(R.used));
+    t.l = trav_child(L, node_rec[nd.left_first]);
+    t.r = trav_child(R, node_rec[nd.left_first + 1]);
     out[rec] = t;
 }
 
@@ -827,8 +831,6 @@ BvhView bvh_view(const pgx_ctx* ctx) {
     v.nodes = ctx->trav_nodes.as<TravNode>();
     v.tris = ctx->trav_tris.as<TravTri>();
     v.root = ctx->root;
-    v.n_records = (int)ctx->n_records;
-    v.n_tris = (int)ctx->ntris;
     if (!ctx->has_bvh) v.root.valid = 0;
     return v;
 }

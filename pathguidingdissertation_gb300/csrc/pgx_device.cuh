@@ -79,25 +79,58 @@ __device__ __forceinline__ bool ray_box(float bminx, float bminy, float bminz, f
     return true;
 }
 
-// Same test for rays whose inverse direction is finite in every component.
-// Then no slab bound is NaN (a finite difference times a finite inverse), so
-// the hardware min/max (which differ from std::min/std::max only for NaN
-// operands and in the sign of a zero result) give the same accept/reject
-// decision; the entry distance may differ from the exact version only in the
-// sign of a zero, which compares equal everywhere it is used.
-__device__ __forceinline__ bool ray_box_finite(float bminx, float bminy, float bminz, float bmaxx, float bmaxy,
-                                               float bmaxz, const xv3& o, const xv3& inv, float& t) {
-    float t0x = x_mul(x_sub(bminx, o.x), inv.x);
-    float t0y = x_mul(x_sub(bminy, o.y), inv.y);
-    float t0z = x_mul(x_sub(bminz, o.z), inv.z);
-    float t1x = x_mul(x_sub(bmaxx, o.x), inv.x);
-    float t1y = x_mul(x_sub(bmaxy, o.y), inv.y);
-    float t1z = x_mul(x_sub(bmaxz, o.z), inv.z);
-    float fen = fmaxf(fmaxf(fminf(t0x, t1x), fminf(t0y, t1y)), fminf(t0z, t1z));
-    float fex = fminf(fminf(fmaxf(t0x, t1x), fmaxf(t0y, t1y)), fmaxf(t0z, t1z));
-    if (fen > fex || fex < 0.f) return false;
-    t = fmaxf(0.f, fen);
-    return true;
+// ---- packed float pairs ---------------------------------------------------
+// Two floats in one 64-bit register; sub2/mul2 are the sm_100 packed
+// instructions, each half rounded like the scalar one.
+struct P2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ P2 pack2(float a, float b) {
+    P2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(P2 p, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v));
+}
+__device__ __forceinline__ P2 sub2(P2 a, P2 b) {
+    P2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ P2 mul2(P2 a, P2 b) {
+    P2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// The slab test for rays whose inverse direction is finite in every
+// component, on a child box packed as (min.xy)(max.xy)(min.z max.z): 6 packed
+// operations instead of 12 scalar ones (the traversal is bound by instruction
+// issue).  No slab bound is NaN then (a finite difference times a finite
+// inverse), so the hardware min/max (which differ from std::min/std::max only
+// for NaN operands and in the sign of a zero result) decide as ray_box does;
+// the entry distance t may differ from its only in the sign of a zero, which
+// compares equal everywhere it is used.
+__device__ __forceinline__ bool slab_packed(P2 mnxy, P2 mxxy, P2 z, P2 oxy, P2 ozz, P2 ixy, P2 izz, float& t) {
+    float t0x, t0y, t1x, t1y, t0z, t1z;
+    unpack2(mul2(sub2(mnxy, oxy), ixy), t0x, t0y);
+    unpack2(mul2(sub2(mxxy, oxy), ixy), t1x, t1y);
+    unpack2(mul2(sub2(z, ozz), izz), t0z, t1z);
+    const float fex = min3(fmaxf(t0x, t1x), fmaxf(t0y, t1y), fmaxf(t0z, t1z));
+    t = fmaxf(max3(fminf(t0x, t1x), fminf(t0y, t1y), fminf(t0z, t1z)), 0.f);
+    // fen <= fex and fex >= 0, with t = max(0, fen)
+    return t <= fex;
 }
 
 // ---- Möller–Trumbore, Triangle::rayIntersect (Geometry.h:101-130), exact --
@@ -108,7 +141,7 @@ __device__ __forceinline__ bool ray_tri(const xv3& v0, const xv3& e0, const xv3&
     xv3 p = x_cross(d, e1);
     float det = x_dot(e0, p);
     if (fabsf(det) < PGX_MT_EPSILON) return false;
-    float inv_det = x_div(1.f, det);
+    float inv_det = __frcp_rn(det);  // the correctly rounded quotient 1 / det
     xv3 T = x_sub(o, v0);
     u = x_mul(x_dot(T, p), inv_det);
     if (u < 0.f || u > 1.f) return false;
@@ -121,13 +154,16 @@ __device__ __forceinline__ bool ray_tri(const xv3& v0, const xv3& e0, const xv3&
 
 // ---- traversal layout ----------------------------------------------------
 // One 64-byte record per interior node of the binary tree, holding both
-// children's boxes so one visit costs four 16-byte loads:
-//   lmin.xyz/lmax.xyz  left child box,  lmin.w = ref, lmax.w = count
-//   rmin.xyz/rmax.xyz  right child box, rmin.w = ref, rmax.w = count
-// count > 0: leaf with `count` triangles at positions [ref, ref+count) of
-// the leaf-ordered triangle array; count == 0: interior, ref = record index.
-struct __align__(16) TravNode {
-    float4 lmin, lmax, rmin, rmax;
+// children: 32 bytes each (one sector, one 256-bit load), the box packed in
+// the pairs the slab test works on and the reference last.  count > 0: leaf
+// with `count` triangles at positions [ref, ref+count) of the leaf-ordered
+// triangle array; count == 0: interior, ref = record index.
+struct __align__(32) TravChild {
+    float mnx, mny, mxx, mxy, mnz, mxz;
+    int ref, count;
+};
+struct __align__(32) TravNode {
+    TravChild l, r;
 };
 // Leaf-ordered triangle: v0 (w = original triangle id bits), e0, e1, padded
 // to 64 bytes so that v0 and e0 arrive in one 32-byte aligned 256-bit load

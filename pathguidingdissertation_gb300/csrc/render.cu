@@ -298,6 +298,7 @@ __global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_extend(Sce
         o = mk(a.x, a.y, a.z);
         d = mk(b.x, b.y, b.z);
         tmax = FLT_MAX;
+        return false;
     };
     auto store = [&](unsigned i, const TraceLane& L) {
         int p = q[i];
@@ -305,10 +306,10 @@ __global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_extend(Sce
         ps.hit[p] = make_float4(__int_as_float(id), L.tmax, L.hu, L.hv);
     };
     if (BATCH)
-        trace_persistent<false, COUNT, decltype(load), decltype(store), BatchRoot, SHORT>(
+        trace_persistent<kTraceClosest, COUNT, decltype(load), decltype(store), BatchRoot, SHORT>(
             sv.bvh, n, &ps.wcount[depth], load, store, ni, nt, status, BatchRoot{binfo, ps.scene, q});
     else
-        trace_persistent<false, COUNT>(sv.bvh, n, &ps.wcount[depth], load, store, ni, nt, status);
+        trace_persistent<kTraceClosest, COUNT>(sv.bvh, n, &ps.wcount[depth], load, store, ni, nt, status);
     if (COUNT) add_counts(&ps.stats[2], ni, nt);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ps.stats[0], (unsigned long long)n);
 }
@@ -326,6 +327,7 @@ __global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_shadow(Sce
         o = mk(a.x, a.y, a.z);
         d = mk(b.x, b.y, b.z);
         tmax = a.w;
+        return true;
     };
     auto store = [&](unsigned i, const TraceLane& L) {
         if (L.hit_id < 0 && !L.status) {
@@ -336,11 +338,11 @@ __global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_shadow(Sce
         }
     };
     if (BATCH)
-        trace_persistent<true, COUNT, decltype(load), decltype(store), BatchRoot, SHORT>(
+        trace_persistent<kTraceAny, COUNT, decltype(load), decltype(store), BatchRoot, SHORT>(
             sv.bvh, n, &ps.wcount[kMaxDepthCap + 2 + depth], load, store, ni, nt, status,
             BatchRoot{binfo, ps.scene, ps.sh_path});
     else
-        trace_persistent<true, COUNT>(sv.bvh, n, &ps.wcount[kMaxDepthCap + 2 + depth], load, store, ni, nt, status);
+        trace_persistent<kTraceAny, COUNT>(sv.bvh, n, &ps.wcount[kMaxDepthCap + 2 + depth], load, store, ni, nt, status);
     if (COUNT) add_counts(&ps.stats[4], ni, nt);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ps.stats[1], (unsigned long long)n);
 }
@@ -1334,9 +1336,7 @@ __device__ bool diff_step(const SceneView& sv, const DiffView& dv, DiffPath& P, 
         int id;
         float t, hu, hv;
         int status;
-        unsigned long long ni = 0, nt = 0;
-        bvh_trace<false, false>(sv.bvh, mk(o.x, o.y, o.z), mk(dir.x, dir.y, dir.z), FLT_MAX, id, t, hu, hv, status,
-                                ni, nt);
+        bvh_trace<false>(sv.bvh, mk(o.x, o.y, o.z), mk(dir.x, dir.y, dir.z), FLT_MAX, id, t, hu, hv, status);
         if (status) id = -1;
         if (id < 0) {
             // Background (k_shade<PLAIN>'s miss branch); decisions on the
@@ -1454,8 +1454,8 @@ __device__ bool diff_step(const SceneView& sv, const DiffView& dv, DiffPath& P, 
                     F3 org = p1 + dvv * PGX_EPSILON;
                     int sid, sst;
                     float st_, su, sv_;
-                    bool occluded = bvh_trace<true, false>(sv.bvh, mk(org.x, org.y, org.z), mk(dvv.x, dvv.y, dvv.z),
-                                                           max_t, sid, st_, su, sv_, sst, ni, nt);
+                    bool occluded = bvh_trace<true>(sv.bvh, mk(org.x, org.y, org.z), mk(dvv.x, dvv.y, dvv.z), max_t,
+                                                    sid, st_, su, sv_, sst);
                     if (!occluded && !sst) {
                         F3 C = T * contrib;
                         L = L + C;
@@ -2441,9 +2441,8 @@ namespace {
 __global__ void k_merge_nodes(TravNode* n, int64_t cnt, int rec_base, int tri_base) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
         TravNode t = n[i];
-        int lc = __float_as_int(t.lmax.w), rc = __float_as_int(t.rmax.w);
-        t.lmin.w = __int_as_float(__float_as_int(t.lmin.w) + (lc > 0 ? tri_base : rec_base));
-        t.rmin.w = __int_as_float(__float_as_int(t.rmin.w) + (rc > 0 ? tri_base : rec_base));
+        t.l.ref += t.l.count > 0 ? tri_base : rec_base;
+        t.r.ref += t.r.count > 0 ? tri_base : rec_base;
         n[i] = t;
     }
 }

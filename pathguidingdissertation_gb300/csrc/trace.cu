@@ -27,6 +27,7 @@ __global__ void __launch_bounds__(kTraceThreads, kPersistentBlocksPerSM)
         o = mk(a.x, a.y, a.z);
         d = mk(b.x, b.y, b.z);
         tmax = a.w;
+        return ANY;
     };
     auto store = [&](unsigned i, const TraceLane& L) {
         if (ANY)
@@ -34,7 +35,7 @@ __global__ void __launch_bounds__(kTraceThreads, kPersistentBlocksPerSM)
         else
             reinterpret_cast<float4*>(hits)[i] = make_float4(__int_as_float(L.hit_id), L.tmax, L.hu, L.hv);
     };
-    trace_persistent<ANY, COUNT>(bvh, (unsigned)n, &counters->next, load, store, ni, nt, status);
+    trace_persistent<ANY ? kTraceAny : kTraceClosest, COUNT>(bvh, (unsigned)n, &counters->next, load, store, ni, nt, status);
     if (COUNT) {
         for (int o = 16; o > 0; o >>= 1) {
             ni += __shfl_xor_sync(0xFFFFFFFFu, ni, o);
@@ -107,7 +108,6 @@ int launch_trace(pgx_ctx* ctx, const pgx_ray* d_rays, int64_t n, pgx_hit* d_hits
     PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
     ctx->last_interior = hc.interior_visits;
     ctx->last_tris = hc.tri_tests;
-    if (hc.overflow & 2u) return pgx_fail(ctx, PGX_ERR_INVALID_ARG, "traversal met a reference outside the BVH");
     if (hc.overflow) return pgx_fail(ctx, PGX_ERR_OVERFLOW, "traversal stack overflow (depth > %d)", PGX_STACK_SIZE);
     return PGX_OK;
 }
@@ -203,7 +203,6 @@ extern "C" int pgx_trace_closest_noalloc(pgx_ctx* ctx, const pgx_ray* rays, int6
     PGX_CUDA_TRY(ctx, cudaStreamSynchronize(s));
     ctx->last_interior = hc.interior_visits;
     ctx->last_tris = hc.tri_tests;
-    if (hc.overflow & 2u) return pgx_fail(ctx, PGX_ERR_INVALID_ARG, "traversal met a reference outside the BVH");
     if (hc.overflow) return pgx_fail(ctx, PGX_ERR_OVERFLOW, "traversal stack overflow (depth > %d)", PGX_STACK_SIZE);
     return PGX_OK;
 }
