@@ -9,14 +9,16 @@
 // One path per (pixel, sample); a wave holds up to 2^25 of them.  The
 // recursion of the reference becomes a loop over depth with queue-per-stage
 // kernels:
-//   camgen -> [extend -> classify -> (guide_infer) -> shade x 6 classes
-//              -> shadow] x (max_depth + 1) -> finalize
+//   camgen -> [trace -> classify -> (guide_infer) -> shade x 6 classes]
+//             x (max_depth + 1) -> trace -> finalize
+// `trace` (k_trace_step) holds the extension rays of a depth and the shadow
+// rays of the depth before it.
 // `classify` bins the depth's paths by surface class and `shade` runs once
 // per class with that class's code compiled in; it compacts surviving paths
 // into the next queue with warp-aggregated atomics (ballot + popc, one
 // atomicAdd per warp) and appends next-event shadow rays to a shadow queue;
-// `shadow` runs the any-hit traversal and adds the stored contribution of
-// unoccluded rays to the path's radiance.  Queue lengths live on the device,
+// their any-hit traversal adds the stored contribution of unoccluded rays to
+// the path's radiance.  Queue lengths live on the device,
 // so a wave needs no host round trip (batches replay their waves from a
 // captured CUDA graph).
 //
@@ -261,12 +263,17 @@ __global__ void __launch_bounds__(kThreads) k_camgen_batch(PathState ps, BatchWa
     if (blockIdx.x == 0 && threadIdx.x == 0) ps.qcount[0] = (unsigned)bw.count;
 }
 
-// Root of a batched path's scene (RootOf of trace_persistent).
+// Root of a batched path's scene (RootOf of trace_persistent): ray i < n_ext
+// is extension ray i of the queue, the others are shadow rays.
 struct BatchRoot {
     const BatchInfo* info;
     const int* scene;
-    const int* path;  // queue entry -> path index
-    __device__ __forceinline__ TravRoot operator()(unsigned i, const BvhView&) const { return info[scene[path[i]]].root; }
+    const int* path;     // extension queue entry -> path index
+    const int* sh_path;  // shadow queue entry -> path index
+    unsigned n_ext;
+    __device__ __forceinline__ TravRoot operator()(unsigned i, const BvhView&) const {
+        return info[scene[i < n_ext ? path[i] : sh_path[i - n_ext]]].root;
+    }
 };
 
 // ---- closest hit for the queue of this depth ----------------------------------
@@ -283,68 +290,118 @@ __device__ __forceinline__ void add_counts(unsigned long long* dst, unsigned lon
 
 constexpr int kPersistentBlocksPerSM = 8;
 
-// Closest hit for the queue of this depth: persistent warps with lane refill
-// (trace_persistent) over qcount[depth] rays.
-template <bool COUNT, bool BATCH = false, int SHORT = kShortStack>
-__global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_extend(SceneView sv, PathState ps, int depth,
-                                                                            const BatchInfo* binfo = nullptr) {
-    const unsigned n = ps.qcount[depth];
-    const int* __restrict__ q = ps.queue[depth & 1];
-    unsigned long long ni = 0, nt = 0;
-    unsigned status = 0;
-    auto load = [&](unsigned i, xv3& o, xv3& d, float& tmax) {
-        int p = q[i];
-        float4 a = ps.o[p], b = ps.d[p];
+// Rays of the wavefront queues: how they are fetched and what becomes of them.
+struct QueueRays {
+    PathState ps;
+    const int* __restrict__ q;  // extension queue of the traced depth
+    __device__ __forceinline__ void load_ext(unsigned i, xv3& o, xv3& d, float& tmax) const {
+        const int p = q[i];
+        const float4 a = ps.o[p], b = ps.d[p];
         o = mk(a.x, a.y, a.z);
         d = mk(b.x, b.y, b.z);
         tmax = FLT_MAX;
+    }
+    __device__ __forceinline__ void store_ext(unsigned i, const TraceLane& L) const {
+        const int p = q[i];
+        const int id = L.status ? -1 : L.hit_id;  // stack overflow: a miss
+        ps.hit[p] = make_float4(__int_as_float(id), L.tmax, L.hu, L.hv);
+    }
+    __device__ __forceinline__ void load_shadow(unsigned i, xv3& o, xv3& d, float& tmax) const {
+        const float4 a = ps.sh_o[i], b = ps.sh_d[i];
+        o = mk(a.x, a.y, a.z);
+        d = mk(b.x, b.y, b.z);
+        tmax = a.w;
+    }
+    // An unoccluded ray adds its contribution to the path's radiance.
+    __device__ __forceinline__ void store_shadow(unsigned i, const TraceLane& L) const {
+        if (L.hit_id < 0 && !L.status) {
+            const int p = ps.sh_path[i];
+            const float4 c = ps.sh_c[i], l = ps.L[p];
+            ps.L[p] = make_float4(l.x + c.x, l.y + c.y, l.z + c.z, 0.f);
+        }
+    }
+};
+
+// Closest hit for the queue of this depth: persistent warps with lane refill
+// (trace_persistent) over qcount[depth] rays.  Waves above kFusedTracePaths
+// and renders with stage times or visit counts; the others trace both kinds
+// of rays in k_trace_step.
+template <bool COUNT>
+__global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_extend(SceneView sv, PathState ps, int depth) {
+    const unsigned n = ps.qcount[depth];
+    const QueueRays rays{ps, ps.queue[depth & 1]};
+    unsigned long long ni = 0, nt = 0;
+    unsigned status = 0;
+    auto load = [&](unsigned i, xv3& o, xv3& d, float& tmax) {
+        rays.load_ext(i, o, d, tmax);
         return false;
     };
-    auto store = [&](unsigned i, const TraceLane& L) {
-        int p = q[i];
-        int id = L.status ? -1 : L.hit_id;  // corrupt tree or stack overflow: a miss
-        ps.hit[p] = make_float4(__int_as_float(id), L.tmax, L.hu, L.hv);
-    };
-    if (BATCH)
-        trace_persistent<kTraceClosest, COUNT, decltype(load), decltype(store), BatchRoot, SHORT>(
-            sv.bvh, n, &ps.wcount[depth], load, store, ni, nt, status, BatchRoot{binfo, ps.scene, q});
-    else
-        trace_persistent<kTraceClosest, COUNT>(sv.bvh, n, &ps.wcount[depth], load, store, ni, nt, status);
+    auto store = [&](unsigned i, const TraceLane& L) { rays.store_ext(i, L); };
+    trace_persistent<kTraceClosest, COUNT>(sv.bvh, n, &ps.wcount[depth], load, store, ni, nt, status);
     if (COUNT) add_counts(&ps.stats[2], ni, nt);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ps.stats[0], (unsigned long long)n);
 }
 
-// Any hit for the shadow queue of this depth; unoccluded rays add their
-// contribution to the path's radiance.
-template <bool COUNT, bool BATCH = false, int SHORT = kShortStack>
-__global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_shadow(SceneView sv, PathState ps, int depth,
-                                                                            const BatchInfo* binfo = nullptr) {
+// Any hit for the shadow queue of this depth.
+template <bool COUNT>
+__global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_shadow(SceneView sv, PathState ps, int depth) {
     const unsigned n = ps.scount[depth];
+    const QueueRays rays{ps, nullptr};
     unsigned long long ni = 0, nt = 0;
     unsigned status = 0;
     auto load = [&](unsigned i, xv3& o, xv3& d, float& tmax) {
-        float4 a = ps.sh_o[i], b = ps.sh_d[i];
-        o = mk(a.x, a.y, a.z);
-        d = mk(b.x, b.y, b.z);
-        tmax = a.w;
+        rays.load_shadow(i, o, d, tmax);
+        return true;
+    };
+    auto store = [&](unsigned i, const TraceLane& L) { rays.store_shadow(i, L); };
+    trace_persistent<kTraceAny, COUNT>(sv.bvh, n, &ps.wcount[kMaxDepthCap + 2 + depth], load, store, ni, nt, status);
+    if (COUNT) add_counts(&ps.stats[4], ni, nt);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ps.stats[1], (unsigned long long)n);
+}
+
+// The extension rays of depth `ext` and the shadow rays of depth `ext - 1` in
+// one launch (with_ext / with_shadow: the first and the last step have one
+// kind only).  Neither kind reads what the other writes, and the shading that
+// follows needs both; together they end in one tail of long rays instead of
+// two (a 1280x720 frame of the interior: 11 + 11 tails of about 100 us were
+// 40 % of its 5.6 ms; fused 4.64 -> 4.08 ms), and the short shadow rays, last
+// in the counter's order, fill the extension rays' tail.  A wave of 29.5 M
+// paths has nothing to gain from the tails and loses by warps that hold both
+// kinds (76.0 against 77.2 ms), a batch of 10.8 M gains (16.6 -> 16.2 ms).
+constexpr int64_t kFusedTracePaths = 1 << 24;
+template <bool BATCH, int SHORT = kShortStack>
+__global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_trace_step(SceneView sv, PathState ps, int ext,
+                                                                                bool with_ext, bool with_shadow,
+                                                                                const BatchInfo* binfo = nullptr) {
+    const unsigned n_ext = with_ext ? ps.qcount[ext] : 0u;
+    const unsigned n_sh = with_shadow ? ps.scount[ext - 1] : 0u;
+    const QueueRays rays{ps, ps.queue[ext & 1]};
+    unsigned long long ni = 0, nt = 0;
+    unsigned status = 0;
+    auto load = [&](unsigned i, xv3& o, xv3& d, float& tmax) {
+        if (i < n_ext) {
+            rays.load_ext(i, o, d, tmax);
+            return false;
+        }
+        rays.load_shadow(i - n_ext, o, d, tmax);
         return true;
     };
     auto store = [&](unsigned i, const TraceLane& L) {
-        if (L.hit_id < 0 && !L.status) {
-            int p = ps.sh_path[i];
-            float4 c = ps.sh_c[i];
-            float4 l = ps.L[p];
-            ps.L[p] = make_float4(l.x + c.x, l.y + c.y, l.z + c.z, 0.f);
-        }
+        if (i < n_ext)
+            rays.store_ext(i, L);
+        else
+            rays.store_shadow(i - n_ext, L);
     };
     if (BATCH)
-        trace_persistent<kTraceAny, COUNT, decltype(load), decltype(store), BatchRoot, SHORT>(
-            sv.bvh, n, &ps.wcount[kMaxDepthCap + 2 + depth], load, store, ni, nt, status,
-            BatchRoot{binfo, ps.scene, ps.sh_path});
+        trace_persistent<kTraceMixed, false, decltype(load), decltype(store), BatchRoot, SHORT>(
+            sv.bvh, n_ext + n_sh, &ps.wcount[ext], load, store, ni, nt, status,
+            BatchRoot{binfo, ps.scene, rays.q, ps.sh_path, n_ext});
     else
-        trace_persistent<kTraceAny, COUNT>(sv.bvh, n, &ps.wcount[kMaxDepthCap + 2 + depth], load, store, ni, nt, status);
-    if (COUNT) add_counts(&ps.stats[4], ni, nt);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ps.stats[1], (unsigned long long)n);
+        trace_persistent<kTraceMixed, false>(sv.bvh, n_ext + n_sh, &ps.wcount[ext], load, store, ni, nt, status);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        atomicAdd(&ps.stats[0], (unsigned long long)n_ext);
+        atomicAdd(&ps.stats[1], (unsigned long long)n_sh);
+    }
 }
 
 inline unsigned persistent_grid(int64_t n) {
@@ -1936,13 +1993,17 @@ int enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, cudaStre
     cudaMemsetAsync(ps.ccount, 0, sizeof(unsigned) * kShadeClasses * (kMaxDepthCap + 2), s);
     k_camgen<<<g, kThreads, 0, s>>>(sv, ps, fp);
     launches++;
+    const unsigned pg = persistent_grid(n);
+    const bool shadows = fp.mode != PGX_MODE_GUIDED_LI;
+    const bool fused = !prof && n <= kFusedTracePaths;
     for (int depth = 0; depth <= fp.max_depth; depth++) {
         if (prof) cudaEventRecord(rs->prof[4 * depth + 0], s);
-        const unsigned pg = persistent_grid(n);
         if (cnt)
             k_extend<true><<<pg, kThreads, 0, s>>>(sv, ps, depth);
-        else
+        else if (!fused)
             k_extend<false><<<pg, kThreads, 0, s>>>(sv, ps, depth);
+        else
+            k_trace_step<false><<<pg, kThreads, 0, s>>>(sv, ps, depth, true, shadows && depth > 0);
         if (prof) cudaEventRecord(rs->prof[4 * depth + 1], s);
         k_classify<<<grid_for((n + kClassifyItems - 1) / kClassifyItems), kThreads, 0, s>>>(sv, ps, depth);
         if (fp.mode == PGX_MODE_GUIDED_MLP && depth < fp.guide_depth) {
@@ -1974,7 +2035,7 @@ int enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, cudaStre
         }
         launches += 2 + kShadeClasses;
         if (prof) cudaEventRecord(rs->prof[4 * depth + 2], s);
-        if (fp.mode != PGX_MODE_GUIDED_LI) {
+        if (!fused && shadows) {
             if (cnt)
                 k_shadow<true><<<pg, kThreads, 0, s>>>(sv, ps, depth);
             else
@@ -1982,6 +2043,10 @@ int enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, cudaStre
             launches++;
         }
         if (prof) cudaEventRecord(rs->prof[4 * depth + 3], s);
+    }
+    if (fused && shadows) {
+        k_trace_step<false><<<pg, kThreads, 0, s>>>(sv, ps, fp.max_depth + 1, false, true);
+        launches++;
     }
     float* film = ctx->film.as<float>();
     float* film2 = ctx->film2.as<float>();
@@ -2545,21 +2610,20 @@ int batch_enqueue(pgx_batch* b, int64_t total, int depth, const pgx_batch_tuning
         cudaMemsetAsync(ps.qcount, 0, sizeof(unsigned) * 4 * (kMaxDepthCap + 2), s);
         cudaMemsetAsync(ps.ccount, 0, sizeof(unsigned) * kShadeClasses * (kMaxDepthCap + 2), s);
         k_camgen_batch<<<sg, kThreads, 0, s>>>(ps, bw);
-        for (int d = 0; d <= depth; d++) {
+        auto trace = [&](int ext, bool with_ext, bool with_shadow) {
             switch (tu.stack_shared) {
-                case 4: k_extend<false, true, 4><<<tg, kThreads, 0, s>>>(sv, ps, d, info); break;
-                case 16: k_extend<false, true, 16><<<tg, kThreads, 0, s>>>(sv, ps, d, info); break;
-                default: k_extend<false, true, 8><<<tg, kThreads, 0, s>>>(sv, ps, d, info); break;
+                case 4: k_trace_step<true, 4><<<tg, kThreads, 0, s>>>(sv, ps, ext, with_ext, with_shadow, info); break;
+                case 16: k_trace_step<true, 16><<<tg, kThreads, 0, s>>>(sv, ps, ext, with_ext, with_shadow, info); break;
+                default: k_trace_step<true, 8><<<tg, kThreads, 0, s>>>(sv, ps, ext, with_ext, with_shadow, info); break;
             }
+        };
+        for (int d = 0; d <= depth; d++) {
+            trace(d, true, d > 0);
             k_classify<<<grid_for((bw.count + kClassifyItems - 1) / kClassifyItems), kThreads, 0, s>>>(sv, ps, d);
             for (int c = 0; c < kShadeClasses; c++)
                 launch_shade_class<PGX_MODE_PLAIN, true>(c, sg, s, sv, ps, fp, d, gv, info);
-            switch (tu.stack_shared) {
-                case 4: k_shadow<false, true, 4><<<tg, kThreads, 0, s>>>(sv, ps, d, info); break;
-                case 16: k_shadow<false, true, 16><<<tg, kThreads, 0, s>>>(sv, ps, d, info); break;
-                default: k_shadow<false, true, 8><<<tg, kThreads, 0, s>>>(sv, ps, d, info); break;
-            }
         }
+        trace(depth + 1, false, true);
         k_finalize_batch<<<sg, kThreads, 0, s>>>(ps, bw);
     }
     PGX_CUDA_TRY(h, cudaGetLastError());
