@@ -751,269 +751,303 @@ __global__ void __launch_bounds__(kThreads) k_classify(SceneView sv, PathState p
 // at 5-7 blocks per SM without spills or at 10-12 with more spills.
 constexpr int kShadeBlocksPerSM = 8;
 
-// CLS >= 0 shades the bin of that surface class with everything the class
-// implies known at compile time (0: misses only; 1: emitters, which end the
-// path; 2, 3, 4: diffuse, conductor, glass BSDFs inlined); CLS < 0 takes the
-// class from `cls` at run time (cls < 0: the whole queue of this depth).
-template <int MODE, bool BATCH = false, int CLS = -1>
-__global__ void __launch_bounds__(kThreads, kShadeBlocksPerSM) k_shade(SceneView sv0, PathState ps, FrameParams fp, int depth,
-                                                    GuideView gv, const BatchInfo* binfo = nullptr, int cls = -1) {
+// One path vertex: shades path p of this depth (whole warps; inactive lanes
+// pass active = false).  CLS >= 0 says what surface class the path hit, and
+// everything the class implies is known at compile time (0: misses only; 1:
+// emitters, which end the path; 2, 3, 4: diffuse, conductor, glass BSDFs
+// inlined); CLS < 0 finds out from the hit.
+template <int MODE, bool BATCH, int CLS>
+__device__ __forceinline__ void shade_path(const SceneView& sv0, PathState& ps, const FrameParams& fp, int depth,
+                                           const GuideView& gv, const BatchInfo* binfo, int p, bool active) {
     constexpr int KIND = CLS == 2 ? PGX_BSDF_DIFFUSE
                        : CLS == 3 ? PGX_BSDF_CONDUCTOR
                        : CLS == 4 ? PGX_BSDF_GLASS
                                   : -1;
     constexpr bool INL = CLS >= 0 && CLS <= 4;
-    if (CLS >= 0) cls = CLS;
-    const unsigned n = cls < 0 ? ps.qcount[depth] : ps.ccount[depth * kShadeClasses + cls];
-    const int* __restrict__ q = cls < 0 ? ps.queue[depth & 1] : ps.cqueue + (size_t)cls * ps.capacity;
     int* __restrict__ qn = ps.queue[(depth + 1) & 1];
     const int64_t cap = ps.capacity;
-    // Uniform trip count per warp so the warp-aggregated appends see whole warps.
-    const unsigned stride = gridDim.x * blockDim.x;
-    const unsigned first = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned rounds = (n + stride - 1) / stride;
-    for (unsigned r = 0; r < rounds; r++) {
-        unsigned i = first + r * stride;
-        bool active = i < n;
-        bool cont = false, want_shadow = false;
-        float4 so = make_float4(0.f, 0.f, 0.f, 0.f), sdir = so;
-        F3 sc = zero3();
-        int p = active ? q[i] : 0;
-        SceneView svb;
-        if (BATCH) {
-            // the path's scene: its lights and bounds in the merged arrays
-            svb = sv0;
-            if (active) {
-                const BatchInfo& bi = binfo[ps.scene[p]];
-                svb.lights = sv0.lights + bi.light_base;
-                svb.nlights = bi.n_lights + bi.has_env_light;
-                svb.n_area_lights = bi.n_lights;
-                svb.env = bi.env;
-                svb.has_env_light = bi.has_env_light;
-                svb.bounds = bi.bounds;
-                svb.width = bi.width;
-                svb.height = bi.height;
-            }
-        }
-        const SceneView& sv = BATCH ? svb : sv0;
-        // Recording for the cache outside guided-Li: the radiance the path has
-        // gathered up to here (after the previous vertex's NEE) is the
-        // baseline from which k_finalize recovers that vertex's incident Li.
-        const int sample_of_p = fp.spp0 + (int)(p / ((int64_t)sv.width * sv.height));
-        const bool rec_on = MODE != PGX_MODE_GUIDED_LI && active && sample_of_p >= fp.collect_lo &&
-                            sample_of_p < fp.collect_hi;
-        // (written below, after this vertex's emission is known)
+    bool cont = false, want_shadow = false;
+    float4 so = make_float4(0.f, 0.f, 0.f, 0.f), sdir = so;
+    F3 sc = zero3();
+    SceneView svb;
+    if (BATCH) {
+        // the path's scene: its lights and bounds in the merged arrays
+        svb = sv0;
         if (active) {
-            float4 o = ps.o[p], d = ps.d[p], h = ps.hit[p], Tw = ps.T[p];
-            uint64_t rng = ps.rng[p];
-            int flags = ps.flags[p];
-            bool prev_spec = flags & 1;
-            float prev_pdf = Tw.w;
-            F3 T = f3(Tw);
-            F3 add = zero3();
-            F3 dir = f3(d);
-            int id = __float_as_int(h.x);
-            // guided-Li record of this vertex (Renderer.h:419-427)
-            F3 r_pos = zero3(), r_nrm = zero3(), r_wi = zero3(), r_w = zero3(), r_e = zero3();
-            F3 r_wo = zero3(), r_f = zero3();
-            float r_pdf = 0.f;  // solid-angle pdf the continuation was sampled with
-            bool r_store = false;
-            if (CLS != 0 && id >= 0) {
-                Shading sd;
-                DevMaterial m;
-                F3 tri_gn;
-                float tri_area;
-                shading_data(sv, o, d, h, sd, m, tri_gn, tri_area);
-                r_pos = sd.x;
-                r_nrm = sd.sn;
-                r_wo = sd.wo;
-                const bool is_light = CLS < 0 ? (bool)m.is_light : CLS == 1;
-                if (is_light) {
-                    F3 em = f3(m.emission[0], m.emission[1], m.emission[2]);
-                    if (MODE == PGX_MODE_GUIDED_LI) {
-                        r_e = em;
-                    } else if (depth == 0 || prev_spec) {
-                        add = T * em;
-                    } else {
-                        float pmf = 1.f / (float)sv.nlights;
-                        float pdf_light = 1.f / tri_area;
-                        float cos_tp = s_max(dot(-dir, tri_gn), 0.f);
-                        float d2 = sd.t * sd.t;
-                        if (cos_tp > 0.f && !(d2 < PGX_EPSILON)) {
-                            float pal = pdf_light * pmf;
-                            float pab = (prev_pdf * cos_tp) / d2;
-                            float wind = power_heuristic(pab, pal);
-                            add = (T * em) * wind;
-                        }
-                    }
-                } else {
-                    int qroot = -1;
-                    const bool spec = bsdf_pure_specular_k<KIND>(m);
-                    if (MODE == PGX_MODE_GUIDED_QUADTREE && depth < fp.guide_depth && !spec && !gv.pss &&
-                        qt_guided_surface<KIND>(gv, m))
-                        qroot = guide_region_root(gv, sd.x);
-                    if (MODE == PGX_MODE_GUIDED_PSS && depth < fp.guide_depth && gv.pss && pss_surface<KIND>(m))
-                        qroot = guide_region_root(gv, sd.x);
-                    bool use_mix =
-                        MODE == PGX_MODE_GUIDED_MLP && depth < fp.guide_depth && mlp_guided_surface<KIND>(m);
-                    if (MODE == PGX_MODE_GUIDED_MLP && use_mix) {
-                        // the region's quadtree stands in for an untrained network
-                        const int fb = ps.fallback[p];
-                        if (fb != -1) {
-                            qroot = fb >= 0 ? fb : -1;
-                            use_mix = false;
-                        }
-                    }
-                    const float4* mix = use_mix ? ps.guide + (size_t)p * mlp::kPacked : nullptr;
-                    if (MODE == PGX_MODE_GUIDED_LI) {
-                        next_event_draws(sv, m, rng);
-                    } else {
-                        F3 c;
-                        if constexpr (INL) {
-                            want_shadow =
-                                next_event_t<KIND, true>(sv, m, sd, rng, so, sdir, c, gv, qroot, fp.guide_fraction, mix);
-                            // queued here so the shadow ray is not held through sampling
-                            push_shadow(ps, depth, p, so, sdir, T * c, want_shadow);
-                        } else {
-                            want_shadow = next_event(sv, m, sd, rng, so, sdir, c, gv, qroot, fp.guide_fraction, mix);
-                            sc = T * c;
-                        }
-                    }
-                    bool alive = true;
-                    float rrp_rec = 1.f;
-                    if (depth > 3) {
-                        if (MODE == PGX_MODE_GUIDED_LI) {
-                            if (pgx_rng_next(rng) < 0.7f)
-                                rrp_rec = 0.7f;
-                            else
-                                alive = false;
-                        } else {
-                            float rrp = s_min(s_max(PGX_EPSILON, lum(T)), 1.f);
-                            if (pgx_rng_next(rng) < rrp)
-                                T = divs(T, rrp);
-                            else
-                                alive = false;
-                        }
-                    }
-                    if (alive && depth == fp.max_depth) alive = false;
-                    if (alive) {
-                        // The diffuse light sampling above reads only the frame's
-                        // normal: rebuilding the frame (same input, same bits) here
-                        // keeps its tangents out of registers during it.
-                        if constexpr (KIND == PGX_BSDF_DIFFUSE) sd.frame = frame_from(sd.sn);
-                        F3 f;
-                        float pdf;
-                        F3 wi;
-                        if (MODE == PGX_MODE_GUIDED_QUADTREE || (MODE == PGX_MODE_GUIDED_MLP && qroot >= 0))
-                            wi = guided_sample<KIND>(gv, fp.guide_fraction, m, sv.tex, sd, rng, f, pdf, qroot);
-                        else if (MODE == PGX_MODE_GUIDED_PSS)
-                            wi = pss_guided_sample<KIND>(gv, fp.guide_fraction, m, sv.tex, sd, rng, f, pdf, qroot);
-                        else if (MODE == PGX_MODE_GUIDED_MLP && use_mix && INL)
-                            wi = mlp_guided_sample_t<KIND>(mix, fp.guide_fraction, m, sv.tex, sd, rng, f, pdf);
-                        else if (MODE == PGX_MODE_GUIDED_MLP && use_mix)
-                            wi = mlp_guided_sample(mix, fp.guide_fraction, m, sv.tex, sd, rng, f, pdf);
-                        else
-                            wi = bsdf_sample_k<KIND>(m, sv.tex, sd, rng, f, pdf);
-                        float cos_t = fabsf(dot(wi, sd.sn));
-                        if (MODE == PGX_MODE_GUIDED_LI) {
-                            if (pdf <= 0.f || cos_t <= 0.f) {
-                                alive = false;
-                            } else {
-                                r_wi = wi;
-                                r_w = divs(f * cos_t, pdf * rrp_rec);
-                                r_store = !spec;
-                            }
-                        } else {
-                            if (pdf <= 0.f || cos_t <= 0.f) {
-                                alive = false;
-                            } else {
-                                r_f = divs(f * cos_t, pdf);
-                                T = divs(T * f * cos_t, pdf);
-                                if (lum(T) <= 0.f) alive = false;
-                                if (isnan(T.x) || isnan(T.y) || isnan(T.z)) alive = false;
-                                if (isinf(T.x) || isinf(T.y) || isinf(T.z)) alive = false;
-                                if (T.x < 0.f || T.y < 0.f || T.z < 0.f) alive = false;
-                            }
-                        }
-                        if (alive) {
-                            if (rec_on) {
-                                // Primary-sample guides are built over the
-                                // cosine sampler's inverse: record only the
-                                // surfaces that sample through it.
-                                r_store = !spec && (MODE != PGX_MODE_GUIDED_PSS || pss_surface<KIND>(m));
-                                r_wi = wi;
-                                r_pdf = pdf;
-                                r_w = T;  // throughput after this vertex
-                            }
-                            float sgn = (dot(wi, sd.gn) >= 0.f) ? 1.f : -1.f;
-                            F3 org = sd.x + sd.gn * (PGX_EPSILON * sgn);
-                            ps.o[p] = make_float4(org.x, org.y, org.z, 0.f);
-                            ps.d[p] = make_float4(wi.x, wi.y, wi.z, 0.f);
-                            ps.T[p] = make_float4(T.x, T.y, T.z, pdf);
-                            ps.flags[p] = spec ? 1 : 0;
-                            cont = true;
-                        }
-                    }
-                }
-            } else if (CLS <= 0) {
-                // Miss: background (Renderer.h:501-527, 596-612).
-                F3 bg = env_eval(sv.env, dir);
-                if (MODE == PGX_MODE_GUIDED_LI) {
-                    r_e = bg;
-                } else if (depth == 0 || prev_spec) {
-                    add = T * bg;
-                } else if (!(lum(bg) < 1e-8f)) {
-                    float pmf = 1.f / (float)sv.nlights;
-                    float pdf_light = INL ? env_pdf_i(sv.env, dir) : env_pdf(sv.env, dir);
-                    if (pmf > 0.f && pdf_light > 0.f) {
-                        float pal = pmf * pdf_light;
-                        float wind = power_heuristic(prev_pdf, pal);
-                        add = (T * bg) * wind;
-                    }
-                }
-            }
-            if (MODE == PGX_MODE_GUIDED_LI) {
-                size_t ri = (size_t)depth * cap + p;
-                ps.rec_pos[ri] = make_float4(r_pos.x, r_pos.y, r_pos.z, r_store ? 1.f : 0.f);
-                ps.rec_nrm[ri] = make_float4(r_nrm.x, r_nrm.y, r_nrm.z, 0.f);
-                ps.rec_wi[ri] = make_float4(r_wi.x, r_wi.y, r_wi.z, 0.f);
-                ps.rec_w[ri] = make_float4(r_w.x, r_w.y, r_w.z, 0.f);
-                ps.rec_e[ri] = make_float4(r_e.x, r_e.y, r_e.z, 0.f);
-                ps.nrec[p] = depth + 1;
-            } else {
-                const bool adds = add.x != 0.f || add.y != 0.f || add.z != 0.f || !valid(add);
-                const bool snap = rec_on && depth > 0;
-                if (adds || snap) {
-                    float4 l = ps.L[p];
-                    // Baseline of the previous vertex's incident radiance: the
-                    // full Li is what the path gathers from this vertex's
-                    // emission on (snapshot before it); the indirect-only
-                    // target of the learned guide starts after it.
-                    if (snap)
-                        ps.rec_e[(size_t)(depth - 1) * cap + p] =
-                            fp.train == 1 ? make_float4(l.x + add.x, l.y + add.y, l.z + add.z, 0.f) : l;
-                    if (adds) ps.L[p] = make_float4(l.x + add.x, l.y + add.y, l.z + add.z, 0.f);
-                }
-                if (rec_on) {
-                    size_t ri = (size_t)depth * cap + p;
-                    ps.rec_pos[ri] = make_float4(r_pos.x, r_pos.y, r_pos.z, (cont && r_store) ? 1.f : 0.f);
-                    if (cont && r_store) {
-                        ps.rec_nrm[ri] = make_float4(r_nrm.x, r_nrm.y, r_nrm.z, 0.f);
-                        ps.rec_wi[ri] = make_float4(r_wi.x, r_wi.y, r_wi.z, r_pdf);
-                        ps.rec_w[ri] = make_float4(r_w.x, r_w.y, r_w.z, 0.f);
-                        if (MODE == PGX_MODE_GUIDED_MLP && fp.train) {
-                            ps.rec_wo[ri] = make_float4(r_wo.x, r_wo.y, r_wo.z, 0.f);
-                            ps.rec_f[ri] = make_float4(r_f.x, r_f.y, r_f.z, 0.f);
-                        }
-                    }
-                    ps.nrec[p] = depth + 1;
-                }
-            }
-            ps.rng[p] = rng;
+            const BatchInfo& bi = binfo[ps.scene[p]];
+            svb.lights = sv0.lights + bi.light_base;
+            svb.nlights = bi.n_lights + bi.has_env_light;
+            svb.n_area_lights = bi.n_lights;
+            svb.env = bi.env;
+            svb.has_env_light = bi.has_env_light;
+            svb.bounds = bi.bounds;
+            svb.width = bi.width;
+            svb.height = bi.height;
         }
-        if (MODE != PGX_MODE_GUIDED_LI && !INL) push_shadow(ps, depth, p, so, sdir, sc, active && want_shadow);
-        unsigned slot = warp_aggregated_add(&ps.qcount[depth + 1], active && cont);
-        if (active && cont) qn[slot] = p;
+    }
+    const SceneView& sv = BATCH ? svb : sv0;
+    // Recording for the cache outside guided-Li: the radiance the path has
+    // gathered up to here (after the previous vertex's NEE) is the
+    // baseline from which k_finalize recovers that vertex's incident Li.
+    const int sample_of_p = fp.spp0 + (int)(p / ((int64_t)sv.width * sv.height));
+    const bool rec_on = MODE != PGX_MODE_GUIDED_LI && active && sample_of_p >= fp.collect_lo &&
+                        sample_of_p < fp.collect_hi;
+    // (written below, after this vertex's emission is known)
+    if (active) {
+        float4 o = ps.o[p], d = ps.d[p], h = ps.hit[p], Tw = ps.T[p];
+        uint64_t rng = ps.rng[p];
+        int flags = ps.flags[p];
+        bool prev_spec = flags & 1;
+        float prev_pdf = Tw.w;
+        F3 T = f3(Tw);
+        F3 add = zero3();
+        F3 dir = f3(d);
+        int id = __float_as_int(h.x);
+        // guided-Li record of this vertex (Renderer.h:419-427)
+        F3 r_pos = zero3(), r_nrm = zero3(), r_wi = zero3(), r_w = zero3(), r_e = zero3();
+        F3 r_wo = zero3(), r_f = zero3();
+        float r_pdf = 0.f;  // solid-angle pdf the continuation was sampled with
+        bool r_store = false;
+        if (CLS != 0 && id >= 0) {
+            Shading sd;
+            DevMaterial m;
+            F3 tri_gn;
+            float tri_area;
+            shading_data(sv, o, d, h, sd, m, tri_gn, tri_area);
+            r_pos = sd.x;
+            r_nrm = sd.sn;
+            r_wo = sd.wo;
+            const bool is_light = CLS < 0 ? (bool)m.is_light : CLS == 1;
+            if (is_light) {
+                F3 em = f3(m.emission[0], m.emission[1], m.emission[2]);
+                if (MODE == PGX_MODE_GUIDED_LI) {
+                    r_e = em;
+                } else if (depth == 0 || prev_spec) {
+                    add = T * em;
+                } else {
+                    float pmf = 1.f / (float)sv.nlights;
+                    float pdf_light = 1.f / tri_area;
+                    float cos_tp = s_max(dot(-dir, tri_gn), 0.f);
+                    float d2 = sd.t * sd.t;
+                    if (cos_tp > 0.f && !(d2 < PGX_EPSILON)) {
+                        float pal = pdf_light * pmf;
+                        float pab = (prev_pdf * cos_tp) / d2;
+                        float wind = power_heuristic(pab, pal);
+                        add = (T * em) * wind;
+                    }
+                }
+            } else {
+                int qroot = -1;
+                const bool spec = bsdf_pure_specular_k<KIND>(m);
+                if (MODE == PGX_MODE_GUIDED_QUADTREE && depth < fp.guide_depth && !spec && !gv.pss &&
+                    qt_guided_surface<KIND>(gv, m))
+                    qroot = guide_region_root(gv, sd.x);
+                if (MODE == PGX_MODE_GUIDED_PSS && depth < fp.guide_depth && gv.pss && pss_surface<KIND>(m))
+                    qroot = guide_region_root(gv, sd.x);
+                bool use_mix =
+                    MODE == PGX_MODE_GUIDED_MLP && depth < fp.guide_depth && mlp_guided_surface<KIND>(m);
+                if (MODE == PGX_MODE_GUIDED_MLP && use_mix) {
+                    // the region's quadtree stands in for an untrained network
+                    const int fb = ps.fallback[p];
+                    if (fb != -1) {
+                        qroot = fb >= 0 ? fb : -1;
+                        use_mix = false;
+                    }
+                }
+                const float4* mix = use_mix ? ps.guide + (size_t)p * mlp::kPacked : nullptr;
+                if (MODE == PGX_MODE_GUIDED_LI) {
+                    next_event_draws(sv, m, rng);
+                } else {
+                    F3 c;
+                    if constexpr (INL) {
+                        want_shadow =
+                            next_event_t<KIND, true>(sv, m, sd, rng, so, sdir, c, gv, qroot, fp.guide_fraction, mix);
+                        // queued here so the shadow ray is not held through sampling
+                        push_shadow(ps, depth, p, so, sdir, T * c, want_shadow);
+                    } else {
+                        want_shadow = next_event(sv, m, sd, rng, so, sdir, c, gv, qroot, fp.guide_fraction, mix);
+                        sc = T * c;
+                    }
+                }
+                bool alive = true;
+                float rrp_rec = 1.f;
+                if (depth > 3) {
+                    if (MODE == PGX_MODE_GUIDED_LI) {
+                        if (pgx_rng_next(rng) < 0.7f)
+                            rrp_rec = 0.7f;
+                        else
+                            alive = false;
+                    } else {
+                        float rrp = s_min(s_max(PGX_EPSILON, lum(T)), 1.f);
+                        if (pgx_rng_next(rng) < rrp)
+                            T = divs(T, rrp);
+                        else
+                            alive = false;
+                    }
+                }
+                if (alive && depth == fp.max_depth) alive = false;
+                if (alive) {
+                    // The diffuse light sampling above reads only the frame's
+                    // normal: rebuilding the frame (same input, same bits) here
+                    // keeps its tangents out of registers during it.
+                    if constexpr (KIND == PGX_BSDF_DIFFUSE) sd.frame = frame_from(sd.sn);
+                    F3 f;
+                    float pdf;
+                    F3 wi;
+                    if (MODE == PGX_MODE_GUIDED_QUADTREE || (MODE == PGX_MODE_GUIDED_MLP && qroot >= 0))
+                        wi = guided_sample<KIND>(gv, fp.guide_fraction, m, sv.tex, sd, rng, f, pdf, qroot);
+                    else if (MODE == PGX_MODE_GUIDED_PSS)
+                        wi = pss_guided_sample<KIND>(gv, fp.guide_fraction, m, sv.tex, sd, rng, f, pdf, qroot);
+                    else if (MODE == PGX_MODE_GUIDED_MLP && use_mix && INL)
+                        wi = mlp_guided_sample_t<KIND>(mix, fp.guide_fraction, m, sv.tex, sd, rng, f, pdf);
+                    else if (MODE == PGX_MODE_GUIDED_MLP && use_mix)
+                        wi = mlp_guided_sample(mix, fp.guide_fraction, m, sv.tex, sd, rng, f, pdf);
+                    else
+                        wi = bsdf_sample_k<KIND>(m, sv.tex, sd, rng, f, pdf);
+                    float cos_t = fabsf(dot(wi, sd.sn));
+                    if (MODE == PGX_MODE_GUIDED_LI) {
+                        if (pdf <= 0.f || cos_t <= 0.f) {
+                            alive = false;
+                        } else {
+                            r_wi = wi;
+                            r_w = divs(f * cos_t, pdf * rrp_rec);
+                            r_store = !spec;
+                        }
+                    } else {
+                        if (pdf <= 0.f || cos_t <= 0.f) {
+                            alive = false;
+                        } else {
+                            r_f = divs(f * cos_t, pdf);
+                            T = divs(T * f * cos_t, pdf);
+                            if (lum(T) <= 0.f) alive = false;
+                            if (isnan(T.x) || isnan(T.y) || isnan(T.z)) alive = false;
+                            if (isinf(T.x) || isinf(T.y) || isinf(T.z)) alive = false;
+                            if (T.x < 0.f || T.y < 0.f || T.z < 0.f) alive = false;
+                        }
+                    }
+                    if (alive) {
+                        if (rec_on) {
+                            // Primary-sample guides are built over the
+                            // cosine sampler's inverse: record only the
+                            // surfaces that sample through it.
+                            r_store = !spec && (MODE != PGX_MODE_GUIDED_PSS || pss_surface<KIND>(m));
+                            r_wi = wi;
+                            r_pdf = pdf;
+                            r_w = T;  // throughput after this vertex
+                        }
+                        float sgn = (dot(wi, sd.gn) >= 0.f) ? 1.f : -1.f;
+                        F3 org = sd.x + sd.gn * (PGX_EPSILON * sgn);
+                        ps.o[p] = make_float4(org.x, org.y, org.z, 0.f);
+                        ps.d[p] = make_float4(wi.x, wi.y, wi.z, 0.f);
+                        ps.T[p] = make_float4(T.x, T.y, T.z, pdf);
+                        ps.flags[p] = spec ? 1 : 0;
+                        cont = true;
+                    }
+                }
+            }
+        } else if (CLS <= 0) {
+            // Miss: background (Renderer.h:501-527, 596-612).
+            F3 bg = env_eval(sv.env, dir);
+            if (MODE == PGX_MODE_GUIDED_LI) {
+                r_e = bg;
+            } else if (depth == 0 || prev_spec) {
+                add = T * bg;
+            } else if (!(lum(bg) < 1e-8f)) {
+                float pmf = 1.f / (float)sv.nlights;
+                float pdf_light = INL ? env_pdf_i(sv.env, dir) : env_pdf(sv.env, dir);
+                if (pmf > 0.f && pdf_light > 0.f) {
+                    float pal = pmf * pdf_light;
+                    float wind = power_heuristic(prev_pdf, pal);
+                    add = (T * bg) * wind;
+                }
+            }
+        }
+        if (MODE == PGX_MODE_GUIDED_LI) {
+            size_t ri = (size_t)depth * cap + p;
+            ps.rec_pos[ri] = make_float4(r_pos.x, r_pos.y, r_pos.z, r_store ? 1.f : 0.f);
+            ps.rec_nrm[ri] = make_float4(r_nrm.x, r_nrm.y, r_nrm.z, 0.f);
+            ps.rec_wi[ri] = make_float4(r_wi.x, r_wi.y, r_wi.z, 0.f);
+            ps.rec_w[ri] = make_float4(r_w.x, r_w.y, r_w.z, 0.f);
+            ps.rec_e[ri] = make_float4(r_e.x, r_e.y, r_e.z, 0.f);
+            ps.nrec[p] = depth + 1;
+        } else {
+            const bool adds = add.x != 0.f || add.y != 0.f || add.z != 0.f || !valid(add);
+            const bool snap = rec_on && depth > 0;
+            if (adds || snap) {
+                float4 l = ps.L[p];
+                // Baseline of the previous vertex's incident radiance: the
+                // full Li is what the path gathers from this vertex's
+                // emission on (snapshot before it); the indirect-only
+                // target of the learned guide starts after it.
+                if (snap)
+                    ps.rec_e[(size_t)(depth - 1) * cap + p] =
+                        fp.train == 1 ? make_float4(l.x + add.x, l.y + add.y, l.z + add.z, 0.f) : l;
+                if (adds) ps.L[p] = make_float4(l.x + add.x, l.y + add.y, l.z + add.z, 0.f);
+            }
+            if (rec_on) {
+                size_t ri = (size_t)depth * cap + p;
+                ps.rec_pos[ri] = make_float4(r_pos.x, r_pos.y, r_pos.z, (cont && r_store) ? 1.f : 0.f);
+                if (cont && r_store) {
+                    ps.rec_nrm[ri] = make_float4(r_nrm.x, r_nrm.y, r_nrm.z, 0.f);
+                    ps.rec_wi[ri] = make_float4(r_wi.x, r_wi.y, r_wi.z, r_pdf);
+                    ps.rec_w[ri] = make_float4(r_w.x, r_w.y, r_w.z, 0.f);
+                    if (MODE == PGX_MODE_GUIDED_MLP && fp.train) {
+                        ps.rec_wo[ri] = make_float4(r_wo.x, r_wo.y, r_wo.z, 0.f);
+                        ps.rec_f[ri] = make_float4(r_f.x, r_f.y, r_f.z, 0.f);
+                    }
+                }
+                ps.nrec[p] = depth + 1;
+            }
+        }
+        ps.rng[p] = rng;
+    }
+    if (MODE != PGX_MODE_GUIDED_LI && !INL) push_shadow(ps, depth, p, so, sdir, sc, active && want_shadow);
+    unsigned slot = warp_aggregated_add(&ps.qcount[depth + 1], active && cont);
+    if (active && cont) qn[slot] = p;
+}
+
+// Shades the paths of this depth, binned by surface class (k_classify), in one
+// launch: blocks take 128-path tiles, class after class, the costly classes
+// first, so at any time most SMs run one class's code, a tile is never mixed,
+// and the cheap classes fill the tail.  A launch per class cost a gap and a
+// tail each: five of six bins of a depth are often empty or small (empty
+// launches alone were 20-25 us a depth).
+template <int MODE, bool BATCH>
+__global__ void __launch_bounds__(kThreads, kShadeBlocksPerSM) k_shade(SceneView sv, PathState ps, FrameParams fp, int depth,
+                                                                       GuideView gv, const BatchInfo* binfo = nullptr) {
+    constexpr int kOrder[kShadeClasses] = {2, 3, 5, 4, 0, 1};
+    const unsigned* cc = ps.ccount + depth * kShadeClasses;
+    unsigned count[kShadeClasses];
+#pragma unroll
+    for (int j = 0; j < kShadeClasses; j++) count[j] = cc[kOrder[j]];
+    for (unsigned tile = blockIdx.x;; tile += gridDim.x) {
+        unsigned first = tile;  // tile index within the class
+        int cls = -1;
+        unsigned n = 0;
+#pragma unroll
+        for (int j = 0; j < kShadeClasses; j++) {
+            const unsigned tiles = (count[j] + kThreads - 1) / kThreads;
+            if (cls < 0) {
+                if (first < tiles) {
+                    cls = kOrder[j];
+                    n = count[j];
+                } else {
+                    first -= tiles;
+                }
+            }
+        }
+        if (cls < 0) break;  // uniform per block
+        const unsigned i = first * kThreads + threadIdx.x;
+        const bool active = i < n;
+        const int p = active ? ps.cqueue[(size_t)cls * ps.capacity + i] : 0;
+        switch (cls) {
+            case 0: shade_path<MODE, BATCH, 0>(sv, ps, fp, depth, gv, binfo, p, active); break;
+            case 1: shade_path<MODE, BATCH, 1>(sv, ps, fp, depth, gv, binfo, p, active); break;
+            case 2: shade_path<MODE, BATCH, 2>(sv, ps, fp, depth, gv, binfo, p, active); break;
+            case 3: shade_path<MODE, BATCH, 3>(sv, ps, fp, depth, gv, binfo, p, active); break;
+            case 4: shade_path<MODE, BATCH, 4>(sv, ps, fp, depth, gv, binfo, p, active); break;
+            default: shade_path<MODE, BATCH, 5>(sv, ps, fp, depth, gv, binfo, p, active); break;
+        }
     }
 }
 
@@ -1817,20 +1851,6 @@ __global__ void __launch_bounds__(kThreads) k_finalize_batch(PathState ps, Batch
     }
 }
 
-// One surface class's bin shaded by estimator MODE, with the class compiled in.
-template <int MODE, bool BATCH>
-void launch_shade_class(int c, unsigned grid, cudaStream_t s, const SceneView& sv, const PathState& ps,
-                        const FrameParams& fp, int depth, const GuideView& gv, const BatchInfo* info) {
-    switch (c) {
-        case 0: k_shade<MODE, BATCH, 0><<<grid, kThreads, 0, s>>>(sv, ps, fp, depth, gv, info); break;
-        case 1: k_shade<MODE, BATCH, 1><<<grid, kThreads, 0, s>>>(sv, ps, fp, depth, gv, info); break;
-        case 2: k_shade<MODE, BATCH, 2><<<grid, kThreads, 0, s>>>(sv, ps, fp, depth, gv, info); break;
-        case 3: k_shade<MODE, BATCH, 3><<<grid, kThreads, 0, s>>>(sv, ps, fp, depth, gv, info); break;
-        case 4: k_shade<MODE, BATCH, 4><<<grid, kThreads, 0, s>>>(sv, ps, fp, depth, gv, info); break;
-        default: k_shade<MODE, BATCH, 5><<<grid, kThreads, 0, s>>>(sv, ps, fp, depth, gv, info); break;
-    }
-}
-
 inline unsigned grid_for(int64_t n) {
     int64_t b = (n + kThreads - 1) / kThreads;
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, (int64_t)pgx_num_sms() * 16));
@@ -2014,26 +2034,20 @@ int enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, cudaStre
                                                                       fb_min);
             launches++;
         }
-        for (int c = 0; c < kShadeClasses; c++) {
-            switch (fp.mode) {
-                case PGX_MODE_GUIDED_LI:
-                    launch_shade_class<PGX_MODE_GUIDED_LI, false>(c, g, s, sv, ps, fp, depth, gv, nullptr);
-                    break;
-                case PGX_MODE_GUIDED_QUADTREE:
-                    launch_shade_class<PGX_MODE_GUIDED_QUADTREE, false>(c, g, s, sv, ps, fp, depth, gv, nullptr);
-                    break;
-                case PGX_MODE_GUIDED_PSS:
-                    launch_shade_class<PGX_MODE_GUIDED_PSS, false>(c, g, s, sv, ps, fp, depth, gv, nullptr);
-                    break;
-                case PGX_MODE_GUIDED_MLP:
-                    launch_shade_class<PGX_MODE_GUIDED_MLP, false>(c, g, s, sv, ps, fp, depth, gv, nullptr);
-                    break;
-                default:
-                    launch_shade_class<PGX_MODE_PLAIN, false>(c, g, s, sv, ps, fp, depth, gv, nullptr);
-                    break;
-            }
+        switch (fp.mode) {
+            case PGX_MODE_GUIDED_LI: k_shade<PGX_MODE_GUIDED_LI, false><<<g, kThreads, 0, s>>>(sv, ps, fp, depth, gv); break;
+            case PGX_MODE_GUIDED_QUADTREE:
+                k_shade<PGX_MODE_GUIDED_QUADTREE, false><<<g, kThreads, 0, s>>>(sv, ps, fp, depth, gv);
+                break;
+            case PGX_MODE_GUIDED_PSS:
+                k_shade<PGX_MODE_GUIDED_PSS, false><<<g, kThreads, 0, s>>>(sv, ps, fp, depth, gv);
+                break;
+            case PGX_MODE_GUIDED_MLP:
+                k_shade<PGX_MODE_GUIDED_MLP, false><<<g, kThreads, 0, s>>>(sv, ps, fp, depth, gv);
+                break;
+            default: k_shade<PGX_MODE_PLAIN, false><<<g, kThreads, 0, s>>>(sv, ps, fp, depth, gv); break;
         }
-        launches += 2 + kShadeClasses;
+        launches += 3;
         if (prof) cudaEventRecord(rs->prof[4 * depth + 2], s);
         if (!fused && shadows) {
             if (cnt)
@@ -2620,8 +2634,7 @@ int batch_enqueue(pgx_batch* b, int64_t total, int depth, const pgx_batch_tuning
         for (int d = 0; d <= depth; d++) {
             trace(d, true, d > 0);
             k_classify<<<grid_for((bw.count + kClassifyItems - 1) / kClassifyItems), kThreads, 0, s>>>(sv, ps, d);
-            for (int c = 0; c < kShadeClasses; c++)
-                launch_shade_class<PGX_MODE_PLAIN, true>(c, sg, s, sv, ps, fp, d, gv, info);
+            k_shade<PGX_MODE_PLAIN, true><<<sg, kThreads, 0, s>>>(sv, ps, fp, d, gv, info);
         }
         trace(depth + 1, false, true);
         k_finalize_batch<<<sg, kThreads, 0, s>>>(ps, bw);
