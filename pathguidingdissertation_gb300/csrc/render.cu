@@ -208,26 +208,31 @@ __device__ __forceinline__ F3 camera_dir(const DevCamera& cam, float px, float p
 }
 
 // ---- camera rays (Camera::generateRay, Scene.h:253-265; jitter Renderer.h:679-681)
+__device__ __forceinline__ void camgen_path(const SceneView& sv, const PathState& ps, const FrameParams& fp, int64_t npix,
+                                            int64_t i) {
+    int64_t pixel = i % npix;
+    int s = (int)(i / npix);
+    int xpix = (int)(pixel % sv.width), ypix = (int)(pixel / sv.width);
+    uint64_t rng = pgx_rng_init(fp.seed, (uint64_t)pixel, (uint64_t)(fp.spp0 + s));
+    float px = (float)xpix + pgx_rng_next(rng);
+    float py = (float)ypix + pgx_rng_next(rng);
+    const DevCamera& cam = sv.cam;
+    F3 dir = camera_dir(cam, px, py);
+    ps.o[i] = make_float4(cam.origin[0], cam.origin[1], cam.origin[2], 0.f);
+    ps.d[i] = make_float4(dir.x, dir.y, dir.z, 0.f);
+    ps.T[i] = make_float4(1.f, 1.f, 1.f, 0.f);
+    ps.L[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    ps.pix[i] = make_float2(px, py);
+    ps.rng[i] = rng;
+    ps.flags[i] = 0;
+    ps.nrec[i] = 0;
+}
+
 __global__ void __launch_bounds__(kThreads) k_camgen(SceneView sv, PathState ps, FrameParams fp) {
     const int64_t npix = (int64_t)sv.width * sv.height;
     const int64_t n = npix * fp.batch;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        int64_t pixel = i % npix;
-        int s = (int)(i / npix);
-        int xpix = (int)(pixel % sv.width), ypix = (int)(pixel / sv.width);
-        uint64_t rng = pgx_rng_init(fp.seed, (uint64_t)pixel, (uint64_t)(fp.spp0 + s));
-        float px = (float)xpix + pgx_rng_next(rng);
-        float py = (float)ypix + pgx_rng_next(rng);
-        const DevCamera& cam = sv.cam;
-        F3 dir = camera_dir(cam, px, py);
-        ps.o[i] = make_float4(cam.origin[0], cam.origin[1], cam.origin[2], 0.f);
-        ps.d[i] = make_float4(dir.x, dir.y, dir.z, 0.f);
-        ps.T[i] = make_float4(1.f, 1.f, 1.f, 0.f);
-        ps.L[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        ps.pix[i] = make_float2(px, py);
-        ps.rng[i] = rng;
-        ps.flags[i] = 0;
-        ps.nrec[i] = 0;
+        camgen_path(sv, ps, fp, npix, i);
         ps.queue[0][i] = (int)i;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) ps.qcount[0] = (unsigned)n;
@@ -755,10 +760,18 @@ constexpr int kShadeBlocksPerSM = 8;
 // pass active = false).  CLS >= 0 says what surface class the path hit, and
 // everything the class implies is known at compile time (0: misses only; 1:
 // emitters, which end the path; 2, 3, 4: diffuse, conductor, glass BSDFs
-// inlined); CLS < 0 finds out from the hit.
-template <int MODE, bool BATCH, int CLS>
+// inlined); CLS < 0 finds out from the hit.  With `next`, the continuation and
+// the shadow ray are returned there instead of being queued (generic class).
+struct NextRays {
+    bool cont, shadow;
+    float4 so, sdir;
+    F3 c;
+};
+template <int MODE, bool BATCH, int CLS, bool QUEUED = true>
 __device__ __forceinline__ void shade_path(const SceneView& sv0, PathState& ps, const FrameParams& fp, int depth,
-                                           const GuideView& gv, const BatchInfo* binfo, int p, bool active) {
+                                           const GuideView& gv, const BatchInfo* binfo, int p, bool active,
+                                           NextRays* next = nullptr) {
+    static_assert(QUEUED || CLS < 0, "the class cores queue their shadow rays themselves");
     constexpr int KIND = CLS == 2 ? PGX_BSDF_DIFFUSE
                        : CLS == 3 ? PGX_BSDF_CONDUCTOR
                        : CLS == 4 ? PGX_BSDF_GLASS
@@ -1001,6 +1014,10 @@ __device__ __forceinline__ void shade_path(const SceneView& sv0, PathState& ps, 
         }
         ps.rng[p] = rng;
     }
+    if (!QUEUED) {
+        *next = NextRays{cont, want_shadow, so, sdir, sc};
+        return;
+    }
     if (MODE != PGX_MODE_GUIDED_LI && !INL) push_shadow(ps, depth, p, so, sdir, sc, active && want_shadow);
     unsigned slot = warp_aggregated_add(&ps.qcount[depth + 1], active && cont);
     if (active && cont) qn[slot] = p;
@@ -1138,80 +1155,20 @@ __global__ void k_tonemap(const float* __restrict__ film, int64_t npix, int spp,
 // End of frame: guided-Li back-propagation (Renderer.h:376-393), NaN/Inf
 // drop (Renderer.h:697-700) and the film splat.
 template <int MODE>
-__global__ void __launch_bounds__(kThreads) k_finalize(SceneView sv, PathState ps, FrameParams fp, float* film,
-                                                       float* film2) {
-    const int64_t npix = (int64_t)sv.width * sv.height;
-    const int64_t n = npix * fp.batch;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
-        F3 col;
-        const int sample_of_p = fp.spp0 + (int)(p / npix);
-        const bool collect = sample_of_p >= fp.collect_lo && sample_of_p < fp.collect_hi;
-        if (MODE == PGX_MODE_GUIDED_LI) {
-            int nr = ps.nrec[p];
-            F3 li = zero3();
-            for (int i = nr - 1; i >= 0; i--) {
-                size_t ri = (size_t)i * ps.capacity + p;
-                float4 pos = ps.rec_pos[ri];
-                if (collect && pos.w != 0.f && valid(li) && lum(li) > 0.f) {
-                    unsigned slot = atomicAdd(ps.nvertices, 1u);
-                    if (slot < (unsigned)ps.vcapacity) {
-                        float4 nr4 = ps.rec_nrm[ri], wi = ps.rec_wi[ri];
-                        pgx_path_vertex v;
-                        v.position[0] = pos.x;
-                        v.position[1] = pos.y;
-                        v.position[2] = pos.z;
-                        v.normal[0] = nr4.x;
-                        v.normal[1] = nr4.y;
-                        v.normal[2] = nr4.z;
-                        v.wi[0] = wi.x;
-                        v.wi[1] = wi.y;
-                        v.wi[2] = wi.z;
-                        v.Li[0] = li.x;
-                        v.Li[1] = li.y;
-                        v.Li[2] = li.z;
-                        ps.vertices[slot] = v;
-                    }
-                }
-                li = f3(ps.rec_e[ri]) + (f3(ps.rec_w[ri]) * li);
-            }
-            col = li;
-        } else {
-            col = f3(ps.L[p]);
-            if (collect && valid(col)) {
-                // Incident radiance along each recorded wi: what the path gathered
-                // after that vertex, divided by the throughput it carried.
-                int nr = ps.nrec[p];
-                for (int i = 0; i < nr; i++) {
-                    size_t ri = (size_t)i * ps.capacity + p;
-                    float4 pos = ps.rec_pos[ri];
-                    if (pos.w == 0.f) continue;
-                    F3 tn = f3(ps.rec_w[ri]);
-                    F3 dl = col - f3(ps.rec_e[ri]);
-                    F3 li = f3(tn.x > 0.f ? dl.x / tn.x : 0.f, tn.y > 0.f ? dl.y / tn.y : 0.f,
-                               tn.z > 0.f ? dl.z / tn.z : 0.f);
-                    if (!(valid(li) && lum(li) > 0.f)) continue;
-                    if (fp.train) {
-                        // radiance sample for the learned guide, weight
-                        // Lum(Li f |cos| / pdf); a hash of (path, vertex,
-                        // batch) keeps a uniform share fp.train_keep of them
-                        uint64_t hsh = pgx_splitmix64(((uint64_t)p << 5) ^ (uint64_t)i ^ ((uint64_t)fp.spp0 << 40));
-                        float u = (float)(hsh >> 40) * (1.f / 16777216.f);
-                        if (u >= fp.train_keep) continue;
-                        float wgt = lum(li * f3(ps.rec_f[ri]));
-                        if (!(wgt > 0.f) || isinf(wgt)) continue;
-                        unsigned slot = atomicAdd(ps.ntrain, 1u);
-                        if (slot >= (unsigned)ps.tcapacity) continue;
-                        float4 nr4 = ps.rec_nrm[ri], wi = ps.rec_wi[ri], wo = ps.rec_wo[ri];
-                        float* o = ps.train + (size_t)slot * 13;
-                        o[0] = pos.x, o[1] = pos.y, o[2] = pos.z;
-                        o[3] = nr4.x, o[4] = nr4.y, o[5] = nr4.z;
-                        o[6] = wo.x, o[7] = wo.y, o[8] = wo.z;
-                        o[9] = wi.x, o[10] = wi.y, o[11] = wi.z;
-                        o[12] = wgt;
-                        continue;
-                    }
-                    unsigned slot = atomicAdd(ps.nvertices, 1u);
-                    if (slot >= (unsigned)ps.vcapacity) continue;
+__device__ __forceinline__ void finalize_path(const SceneView& sv, const PathState& ps, const FrameParams& fp, int64_t npix,
+                                              int64_t p, float* film, float* film2) {
+    F3 col;
+    const int sample_of_p = fp.spp0 + (int)(p / npix);
+    const bool collect = sample_of_p >= fp.collect_lo && sample_of_p < fp.collect_hi;
+    if (MODE == PGX_MODE_GUIDED_LI) {
+        int nr = ps.nrec[p];
+        F3 li = zero3();
+        for (int i = nr - 1; i >= 0; i--) {
+            size_t ri = (size_t)i * ps.capacity + p;
+            float4 pos = ps.rec_pos[ri];
+            if (collect && pos.w != 0.f && valid(li) && lum(li) > 0.f) {
+                unsigned slot = atomicAdd(ps.nvertices, 1u);
+                if (slot < (unsigned)ps.vcapacity) {
                     float4 nr4 = ps.rec_nrm[ri], wi = ps.rec_wi[ri];
                     pgx_path_vertex v;
                     v.position[0] = pos.x;
@@ -1227,20 +1184,133 @@ __global__ void __launch_bounds__(kThreads) k_finalize(SceneView sv, PathState p
                     v.Li[1] = li.y;
                     v.Li[2] = li.z;
                     ps.vertices[slot] = v;
-                    // Flux weight for the QuadTree guide: Lum(Li) |cos| / pdf
-                    // (Mueller et al. 2017 divide by the sampling pdf).  Over
-                    // directions its expected density is Li |cos|, over the
-                    // cosine sampler's primary samples pi Li, whichever
-                    // distribution sampled wi, so training on guided paths
-                    // does not compound the previous guide.
-                    const float cos_n = fabsf(nr4.x * wi.x + nr4.y * wi.y + nr4.z * wi.z);
-                    ps.vweight[slot] = wi.w > 0.f ? lum(li) * cos_n / wi.w : 0.f;
                 }
             }
+            li = f3(ps.rec_e[ri]) + (f3(ps.rec_w[ri]) * li);
         }
-        if (!valid(col)) continue;
-        float2 xy = ps.pix[p];
-        splat(film, film2, sv.width, sv.height, xy.x, xy.y, col, fp.mitchell != 0);
+        col = li;
+    } else {
+        col = f3(ps.L[p]);
+        if (collect && valid(col)) {
+            // Incident radiance along each recorded wi: what the path gathered
+            // after that vertex, divided by the throughput it carried.
+            int nr = ps.nrec[p];
+            for (int i = 0; i < nr; i++) {
+                size_t ri = (size_t)i * ps.capacity + p;
+                float4 pos = ps.rec_pos[ri];
+                if (pos.w == 0.f) continue;
+                F3 tn = f3(ps.rec_w[ri]);
+                F3 dl = col - f3(ps.rec_e[ri]);
+                F3 li = f3(tn.x > 0.f ? dl.x / tn.x : 0.f, tn.y > 0.f ? dl.y / tn.y : 0.f,
+                           tn.z > 0.f ? dl.z / tn.z : 0.f);
+                if (!(valid(li) && lum(li) > 0.f)) continue;
+                if (fp.train) {
+                    // radiance sample for the learned guide, weight
+                    // Lum(Li f |cos| / pdf); a hash of (path, vertex,
+                    // batch) keeps a uniform share fp.train_keep of them
+                    uint64_t hsh = pgx_splitmix64(((uint64_t)p << 5) ^ (uint64_t)i ^ ((uint64_t)fp.spp0 << 40));
+                    float u = (float)(hsh >> 40) * (1.f / 16777216.f);
+                    if (u >= fp.train_keep) continue;
+                    float wgt = lum(li * f3(ps.rec_f[ri]));
+                    if (!(wgt > 0.f) || isinf(wgt)) continue;
+                    unsigned slot = atomicAdd(ps.ntrain, 1u);
+                    if (slot >= (unsigned)ps.tcapacity) continue;
+                    float4 nr4 = ps.rec_nrm[ri], wi = ps.rec_wi[ri], wo = ps.rec_wo[ri];
+                    float* o = ps.train + (size_t)slot * 13;
+                    o[0] = pos.x, o[1] = pos.y, o[2] = pos.z;
+                    o[3] = nr4.x, o[4] = nr4.y, o[5] = nr4.z;
+                    o[6] = wo.x, o[7] = wo.y, o[8] = wo.z;
+                    o[9] = wi.x, o[10] = wi.y, o[11] = wi.z;
+                    o[12] = wgt;
+                    continue;
+                }
+                unsigned slot = atomicAdd(ps.nvertices, 1u);
+                if (slot >= (unsigned)ps.vcapacity) continue;
+                float4 nr4 = ps.rec_nrm[ri], wi = ps.rec_wi[ri];
+                pgx_path_vertex v;
+                v.position[0] = pos.x;
+                v.position[1] = pos.y;
+                v.position[2] = pos.z;
+                v.normal[0] = nr4.x;
+                v.normal[1] = nr4.y;
+                v.normal[2] = nr4.z;
+                v.wi[0] = wi.x;
+                v.wi[1] = wi.y;
+                v.wi[2] = wi.z;
+                v.Li[0] = li.x;
+                v.Li[1] = li.y;
+                v.Li[2] = li.z;
+                ps.vertices[slot] = v;
+                // Flux weight for the QuadTree guide: Lum(Li) |cos| / pdf
+                // (Mueller et al. 2017 divide by the sampling pdf).  Over
+                // directions its expected density is Li |cos|, over the
+                // cosine sampler's primary samples pi Li, whichever
+                // distribution sampled wi, so training on guided paths
+                // does not compound the previous guide.
+                const float cos_n = fabsf(nr4.x * wi.x + nr4.y * wi.y + nr4.z * wi.z);
+                ps.vweight[slot] = wi.w > 0.f ? lum(li) * cos_n / wi.w : 0.f;
+            }
+        }
+    }
+    if (!valid(col)) return;
+    float2 xy = ps.pix[p];
+    splat(film, film2, sv.width, sv.height, xy.x, xy.y, col, fp.mitchell != 0);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreads) k_finalize(SceneView sv, PathState ps, FrameParams fp, float* film,
+                                                       float* film2) {
+    const int64_t npix = (int64_t)sv.width * sv.height;
+    const int64_t n = npix * fp.batch;
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x)
+        finalize_path<MODE>(sv, ps, fp, npix, p, film, film2);
+}
+
+// Small waves: one thread takes a path from the camera ray to the film in one
+// launch.  The wavefront's three launches a depth cost a gap and a latency
+// tail each, whatever the wave's size; below kPathWave paths the GPU is not
+// full and the tails are all there is (64x64 frame: 30 launches, 0.64 ms).
+// A block is one warp holding `lanes` paths: while there are fewer paths than
+// lanes on the GPU, spreading them over more warps keeps divergent paths from
+// waiting for each other.  The vertices are shade_path's generic ones, on the
+// same state, so a path's draws, decisions and sums are the wavefront's.
+template <int MODE>
+__global__ void __launch_bounds__(32) k_path(SceneView sv, PathState ps, FrameParams fp, GuideView gv, int lanes, float* film,
+                                             float* film2) {
+    const int64_t npix = (int64_t)sv.width * sv.height;
+    const int64_t n = npix * fp.batch;
+    const int64_t p = (int64_t)blockIdx.x * lanes + threadIdx.x;
+    unsigned n_ext = 0, n_sh = 0;
+    if (threadIdx.x < lanes && p < n) {
+        camgen_path(sv, ps, fp, npix, p);
+        for (int depth = 0; depth <= fp.max_depth; depth++) {
+            const float4 o = ps.o[p], d = ps.d[p];
+            int id, status;
+            float t, u, v;
+            bvh_trace<false>(sv.bvh, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), FLT_MAX, id, t, u, v, status);
+            ps.hit[p] = make_float4(__int_as_float(status ? -1 : id), t, u, v);
+            n_ext++;
+            NextRays next;
+            shade_path<MODE, false, -1, false>(sv, ps, fp, depth, gv, nullptr, (int)p, true, &next);
+            if (MODE != PGX_MODE_GUIDED_LI && next.shadow) {
+                n_sh++;
+                const bool occluded =
+                    bvh_trace<true>(sv.bvh, mk(next.so.x, next.so.y, next.so.z), mk(next.sdir.x, next.sdir.y, next.sdir.z),
+                                    next.so.w, id, t, u, v, status);
+                if (!occluded && !status) {
+                    const float4 l = ps.L[p];
+                    ps.L[p] = make_float4(l.x + next.c.x, l.y + next.c.y, l.z + next.c.z, 0.f);
+                }
+            }
+            if (!next.cont) break;
+        }
+        finalize_path<MODE == PGX_MODE_GUIDED_LI ? PGX_MODE_GUIDED_LI : PGX_MODE_PLAIN>(sv, ps, fp, npix, p, film, film2);
+    }
+    n_ext = __reduce_add_sync(0xFFFFFFFFu, n_ext);
+    n_sh = __reduce_add_sync(0xFFFFFFFFu, n_sh);
+    if (threadIdx.x == 0) {
+        atomicAdd(&ps.stats[0], (unsigned long long)n_ext);
+        atomicAdd(&ps.stats[1], (unsigned long long)n_sh);
     }
 }
 
@@ -1989,15 +2059,27 @@ SceneView scene_view(pgx_ctx* ctx) {
     return sv;
 }
 
+// Waves of at most this many paths run in k_path.  us per call (wavefront /
+// k_path), clear and film read included: material zoo 64x64 625 / 268, 181x97
+// 663 / 355, 256x256 801 / 690, 512x384 948 / 1315; box 256x256 483 / 305,
+// 512x400 586 / 617; interior 64x64 1230 / 497, 256x256 1525 / 1264, 512x400
+// 1843 / 3118.
+constexpr int64_t kPathWave = 1 << 16;
+
 // Stage times of one profiled batch (milliseconds).
 struct StageTimes {
     double extend = 0, shade = 0, shadow = 0;
 };
 
+// Kernels of one batch: all of them, and those that trace extension rays.
+struct LaunchCount {
+    int all, extend;
+};
+
 // Enqueues one batch (fp.batch samples per pixel) on stream s; returns the
-// number of kernels launched.  With fp.profile, events bracket every stage
+// kernels launched.  With fp.profile, events bracket every stage
 // (read back by stage_times after the stream is synchronised).
-int enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, cudaStream_t s, int* mlp_status) {
+LaunchCount enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, cudaStream_t s, int* mlp_status) {
     SceneView sv = scene_view(ctx);
     PathState ps = path_view(rs);
     GuideView gv = guide_view(ctx);
@@ -2009,6 +2091,22 @@ int enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, cudaStre
     const bool prof = fp.profile != 0;  // stage events
     const bool cnt = fp.profile > 1;    // counting traversal kernels
     int launches = 0;
+    if (!prof && n <= kPathWave && fp.mode != PGX_MODE_GUIDED_MLP) {
+        const int64_t warps = (int64_t)pgx_num_sms() * 8;  // two a scheduler (4 and 16: within 3 %, 32: up to 1.3x slower)
+        int lanes = 8;                                      // at least (4: 5 % slower, 1: 15 %)
+        while (lanes < 32 && lanes * warps < n) lanes *= 2;
+        const unsigned pb = (unsigned)((n + lanes - 1) / lanes);
+        float *f1 = ctx->film.as<float>(), *f2 = ctx->film2.as<float>();
+        switch (fp.mode) {
+            case PGX_MODE_GUIDED_LI: k_path<PGX_MODE_GUIDED_LI><<<pb, 32, 0, s>>>(sv, ps, fp, gv, lanes, f1, f2); break;
+            case PGX_MODE_GUIDED_QUADTREE:
+                k_path<PGX_MODE_GUIDED_QUADTREE><<<pb, 32, 0, s>>>(sv, ps, fp, gv, lanes, f1, f2);
+                break;
+            case PGX_MODE_GUIDED_PSS: k_path<PGX_MODE_GUIDED_PSS><<<pb, 32, 0, s>>>(sv, ps, fp, gv, lanes, f1, f2); break;
+            default: k_path<PGX_MODE_PLAIN><<<pb, 32, 0, s>>>(sv, ps, fp, gv, lanes, f1, f2); break;
+        }
+        return {1, 1};
+    }
     cudaMemsetAsync(ps.qcount, 0, sizeof(unsigned) * 4 * (kMaxDepthCap + 2), s);
     cudaMemsetAsync(ps.ccount, 0, sizeof(unsigned) * kShadeClasses * (kMaxDepthCap + 2), s);
     k_camgen<<<g, kThreads, 0, s>>>(sv, ps, fp);
@@ -2068,7 +2166,7 @@ int enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, cudaStre
         k_finalize<PGX_MODE_GUIDED_LI><<<g, kThreads, 0, s>>>(sv, ps, fp, film, film2);
     else
         k_finalize<PGX_MODE_PLAIN><<<g, kThreads, 0, s>>>(sv, ps, fp, film, film2);
-    return launches + 1;
+    return {launches + 1, fp.max_depth + 1};
 }
 
 void stage_times(RenderState* rs, int max_depth, StageTimes& t) {
@@ -2197,7 +2295,7 @@ extern "C" int pgx_render(pgx_ctx* ctx, const pgx_render_config* cfg, int32_t fr
     const bool count = (cfg->flags & PGX_RENDER_PROFILE) != 0;
     const bool prof = count || (cfg->flags & PGX_RENDER_TIMING) != 0;
     StageTimes times;
-    int64_t launches = 0, batches = 0;
+    int64_t launches = 0, extend_launches = 0;
     PGX_CUDA_TRY(ctx, cudaEventRecord(rs->ev0, s));
     int done = 0;
     while (done < frames) {
@@ -2218,8 +2316,9 @@ extern "C" int pgx_render(pgx_ctx* ctx, const pgx_render_config* cfg, int32_t fr
         if (train && rs->train_last > 0)
             fp.train_keep = (float)std::min(1.0, (double)tcap / (1.25 * (double)rs->train_last * fp.batch));
         if (train) PGX_CUDA_TRY(ctx, cudaMemsetAsync(ps.ntrain, 0, sizeof(unsigned), s));
-        launches += enqueue_frame(ctx, rs, fp, s, mlp_status);
-        batches++;
+        const LaunchCount lc = enqueue_frame(ctx, rs, fp, s, mlp_status);
+        launches += lc.all;
+        extend_launches += lc.extend;
         PGX_CUDA_TRY(ctx, cudaGetLastError());
         if (train) {
             // one Adam step on this batch's radiance samples
@@ -2259,7 +2358,7 @@ extern "C" int pgx_render(pgx_ctx* ctx, const pgx_render_config* cfg, int32_t fr
     rst.shadow_tri_tests = (int64_t)st[5];
     rst.guide_fallbacks = (int64_t)st[6];
     rst.kernel_launches = launches;
-    rst.extend_launches = batches * (cfg->max_depth + 1);
+    rst.extend_launches = extend_launches;
     rst.ms_total = ms;
     rst.ms_extend = times.extend;
     rst.ms_shade = times.shade;
