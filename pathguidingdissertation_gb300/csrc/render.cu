@@ -118,7 +118,7 @@ struct RenderState {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t prof[kProfEvents] = {};
     // differentiable rendering: evaluation parameters and scratch
-    DevBuf d_mats, d_env, d_partial, d_img, d_dimg, d_genv, d_galb, d_grough, d_next, d_samples;
+    DevBuf d_mats, d_env, d_partial, d_img, d_dimg, d_genv, d_galb, d_grough, d_samples, d_ts, d_rec;
     bool d_params = false;
 };
 
@@ -295,6 +295,9 @@ __device__ __forceinline__ void add_counts(unsigned long long* dst, unsigned lon
 
 constexpr int kPersistentBlocksPerSM = 8;
 
+// Set in a vertex's record flags when its light sample was visible.
+constexpr int kDiffSeen = 32;
+
 // Rays of the wavefront queues: how they are fetched and what becomes of them.
 struct QueueRays {
     PathState ps;
@@ -317,10 +320,12 @@ struct QueueRays {
         d = mk(b.x, b.y, b.z);
         tmax = a.w;
     }
-    // An unoccluded ray adds its contribution to the path's radiance.
-    __device__ __forceinline__ void store_shadow(unsigned i, const TraceLane& L) const {
+    // An unoccluded ray adds its contribution to the path's radiance.  seen:
+    // the flags of the path's vertex, told about it (differentiable renders).
+    __device__ __forceinline__ void store_shadow(unsigned i, const TraceLane& L, float4* seen = nullptr) const {
         if (L.hit_id < 0 && !L.status) {
             const int p = ps.sh_path[i];
+            if (seen) reinterpret_cast<int*>(seen + p)[3] |= kDiffSeen;
             const float4 c = ps.sh_c[i], l = ps.L[p];
             ps.L[p] = make_float4(l.x + c.x, l.y + c.y, l.z + c.z, 0.f);
         }
@@ -377,7 +382,8 @@ constexpr int64_t kFusedTracePaths = 1 << 24;
 template <bool BATCH, int SHORT = kShortStack>
 __global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_trace_step(SceneView sv, PathState ps, int ext,
                                                                                 bool with_ext, bool with_shadow,
-                                                                                const BatchInfo* binfo = nullptr) {
+                                                                                const BatchInfo* binfo = nullptr,
+                                                                                float4* seen = nullptr) {
     const unsigned n_ext = with_ext ? ps.qcount[ext] : 0u;
     const unsigned n_sh = with_shadow ? ps.scount[ext - 1] : 0u;
     const QueueRays rays{ps, ps.queue[ext & 1]};
@@ -395,7 +401,7 @@ __global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_trace_step
         if (i < n_ext)
             rays.store_ext(i, L);
         else
-            rays.store_shadow(i - n_ext, L);
+            rays.store_shadow(i - n_ext, L, seen);
     };
     if (BATCH)
         trace_persistent<kTraceMixed, false, decltype(load), decltype(store), BatchRoot, SHORT>(
@@ -1023,38 +1029,51 @@ __device__ __forceinline__ void shade_path(const SceneView& sv0, PathState& ps, 
     if (active && cont) qn[slot] = p;
 }
 
-// Shades the paths of this depth, binned by surface class (k_classify), in one
-// launch: blocks take 128-path tiles, class after class, the costly classes
-// first, so at any time most SMs run one class's code, a tile is never mixed,
-// and the cheap classes fill the tail.  A launch per class cost a gap and a
-// tail each: five of six bins of a depth are often empty or small (empty
-// launches alone were 20-25 us a depth).
-template <int MODE, bool BATCH>
-__global__ void __launch_bounds__(kThreads, kShadeBlocksPerSM) k_shade(SceneView sv, PathState ps, FrameParams fp, int depth,
-                                                                       GuideView gv, const BatchInfo* binfo = nullptr) {
-    constexpr int kOrder[kShadeClasses] = {2, 3, 5, 4, 0, 1};
-    const unsigned* cc = ps.ccount + depth * kShadeClasses;
+// The 128-path tiles of a depth's class bins (k_classify), class after class,
+// the costly classes first: blocks that take them in order run one class's
+// code on most SMs at any time, a tile is never mixed, and the cheap classes
+// fill the tail.
+struct ClassTiles {
     unsigned count[kShadeClasses];
+    __device__ __forceinline__ static constexpr int cls_at(int j) {
+        constexpr int order[kShadeClasses] = {2, 3, 5, 4, 0, 1};
+        return order[j];
+    }
+    __device__ __forceinline__ ClassTiles(const PathState& ps, int depth) {
 #pragma unroll
-    for (int j = 0; j < kShadeClasses; j++) count[j] = cc[kOrder[j]];
-    for (unsigned tile = blockIdx.x;; tile += gridDim.x) {
-        unsigned first = tile;  // tile index within the class
-        int cls = -1;
-        unsigned n = 0;
+        for (int j = 0; j < kShadeClasses; j++) count[j] = ps.ccount[depth * kShadeClasses + cls_at(j)];
+    }
+    // Class of tile t, this thread's entry i of its bin and the bin's length;
+    // false past the last tile.
+    __device__ __forceinline__ bool find(unsigned t, int& cls, unsigned& i, unsigned& n) const {
+        cls = -1;
 #pragma unroll
         for (int j = 0; j < kShadeClasses; j++) {
             const unsigned tiles = (count[j] + kThreads - 1) / kThreads;
             if (cls < 0) {
-                if (first < tiles) {
-                    cls = kOrder[j];
+                if (t < tiles) {
+                    cls = cls_at(j);
                     n = count[j];
                 } else {
-                    first -= tiles;
+                    t -= tiles;
                 }
             }
         }
-        if (cls < 0) break;  // uniform per block
-        const unsigned i = first * kThreads + threadIdx.x;
+        i = t * kThreads + threadIdx.x;
+        return cls >= 0;
+    }
+};
+
+// Shades the paths of this depth in one launch.  A launch per class cost a gap
+// and a tail each: five of six bins of a depth are often empty or small (empty
+// launches alone were 20-25 us a depth).
+template <int MODE, bool BATCH>
+__global__ void __launch_bounds__(kThreads, kShadeBlocksPerSM) k_shade(SceneView sv, PathState ps, FrameParams fp, int depth,
+                                                                       GuideView gv, const BatchInfo* binfo = nullptr) {
+    const ClassTiles tiles(ps, depth);
+    int cls;
+    unsigned i, n;
+    for (unsigned tile = blockIdx.x; tiles.find(tile, cls, i, n); tile += gridDim.x) {
         const bool active = i < n;
         const int p = active ? ps.cqueue[(size_t)cls * ps.capacity + i] : 0;
         switch (cls) {
@@ -1316,7 +1335,7 @@ __global__ void __launch_bounds__(32) k_path(SceneView sv, PathState ps, FramePa
 
 // ---- differentiable rendering ---------------------------------------------------------
 // Plain path tracing with NEE + MIS (the estimator of k_shade<PLAIN>), in
-// two flavours sharing diff_path:
+// two flavours sharing diff_shade:
 //  * primal: sampling decisions (directions, pdfs, MIS weights, Russian
 //    roulette, the environment's sampling tables) use the uploaded scene,
 //    while radiance is evaluated with the "evaluation" parameters -- the
@@ -1325,10 +1344,9 @@ __global__ void __launch_bounds__(32) k_path(SceneView sv, PathState ps, FramePa
 //    and a gather kernel adds the 4 neighbours' partial sums in a fixed
 //    order, so the image is deterministic and a finite difference between
 //    two parameter sets differs only through the samples a parameter touches;
-//  * adjoint: with evaluation = uploaded parameters, one thread per sample
-//    traces the path once from its seed; every vertex j keeps (in the
-//    thread's registers and local memory, never in global memory) what its
-//    terms need, and once the path's radiance L is known the thread adds
+//  * adjoint: with evaluation = uploaded parameters, every path is traced once
+//    from its seed; every vertex j leaves a record of what its terms need, and
+//    once the path's radiance L is known k_diff_emit adds
 //      d/dtheta of the terms added at j (NEE: albedo, roughness, the
 //      environment texels under the light direction; escaped rays: the
 //      texels under the ray), and
@@ -1338,6 +1356,11 @@ __global__ void __launch_bounds__(32) k_path(SceneView sv, PathState ps, FramePa
 //      replace), with pdf detached,
 //    each weighted by dLoss/dImage at the sample's pixel / spp, into double
 //    accumulators (material terms per block in shared memory).
+// Both run on the wavefront's own kernels (k_trace_step, k_classify) with a
+// shading kernel over the class bins, in waves bounded by memory.  One thread
+// tracing and shading its path had 5.8 lanes busy per instruction: a 256x256 x
+// 16 spp step on 522,242 triangles took 4.7 ms (primal) and 7.5 ms (adjoint);
+// the waves take 1.6 and 2.1 ms, of which 2.3 are traversal.
 struct DiffView {
     const DevMaterial* __restrict__ mats_e;  // evaluation materials
     DevEnv env_e;                            // evaluation environment (sampling tables of sv.env)
@@ -1348,9 +1371,12 @@ struct DiffView {
     double* g_env;            // [env W*H*3]
     double* g_alb;            // [nmats*3]
     double* g_rough;          // [nmats]
-    unsigned long long* next; // next sample to take (zeroed before each launch)
     float4* samples;          // primal: values of the chunk's samples
-    int s0, ns;               // primal: the chunk's samples [s0, s0 + ns)
+    float4* Ts;               // sampling throughput of each path of the wave
+    int64_t first;            // the wave's first sample (item = sample index x pixels + pixel)
+    int64_t count;            // samples in the wave, path i = item first + i
+    int64_t chunk0;           // primal: item of samples[0]
+    int64_t stride;           // adjoint: paths between the depths of the record arrays
     int nmats;
 };
 
@@ -1429,56 +1455,52 @@ __device__ __forceinline__ void add_alb(const DiffAcc& acc, int mat, F3 g) {
 // known: the NEE contribution and its log-derivative factors, the radiance
 // collected up to the vertex (the continuation's term is delta x (L_total -
 // L_snap) x d log beta / d theta), and the environment lookup of an
-// environment light sample.
+// environment light sample or of the escaped ray.  Kept in the wave's record
+// arrays at [depth][path], five float4 of which only the used ones are
+// written: C + dr_nee, 1/albedo + dr_cont, L_snap + material, T x weight +
+// flags, direction.
 struct DiffVertex {
     F3 ia;        // 1 / albedo (per channel) when the material is albedo-linear, else 0
-    F3 C;         // NEE contribution T * emitted * weight (0 without one)
-    F3 tcw;       // environment NEE: T * radiance weight of the sample
-    F3 wi;        // environment NEE direction
-    F3 l_snap;    // radiance collected up to and including this vertex's NEE
+    F3 C;         // NEE contribution T * emitted * weight
+    F3 tcw;       // environment: T * radiance weight
+    F3 wi;        // environment: direction
     float dr_nee, dr_cont;
     int mat;
-    int flags;    // 1: NEE term, 2: environment NEE, 4: continuation term
+    int flags;    // kDiff* bits
 };
 
 __device__ __forceinline__ F3 safe_div3(F3 a, F3 b) {
     return f3(a.x / fmaxf(b.x, 1e-6f), a.y / fmaxf(b.y, 1e-6f), a.z / fmaxf(b.z, 1e-6f));
 }
 
-// State of one path of the differentiable estimator between bounces.
+// State of one path of the differentiable estimator at a vertex.
 struct DiffPath {
     F3 o, dir;
     F3 T, Ts, L;          // evaluation and sampling throughput, radiance so far
-    F3 delta;             // adjoint of the sample's value (gradient pass)
-    F3 esc_dir, esc_w;    // escaped ray: direction, T x MIS weight
+    F3 nee;               // light sample waiting for its shadow ray: T x contribution
     uint64_t rng;
     float prev_pdf;
-    int depth, nvtx;
-    bool prev_spec, escaped;
+    bool prev_spec;
 };
 
-__device__ __forceinline__ void diff_begin(DiffPath& P, uint64_t rng, F3 o, F3 dir, F3 delta) {
-    P.o = o;
-    P.dir = dir;
-    P.T = f3(1.f, 1.f, 1.f);
-    P.Ts = P.T;
-    P.L = zero3();
-    P.delta = delta;
-    P.esc_dir = zero3();
-    P.esc_w = zero3();
-    P.rng = rng;
-    P.prev_pdf = 0.f;
-    P.depth = 0;
-    P.nvtx = 0;
-    P.prev_spec = false;
-    P.escaped = false;
-}
+// What a shaded vertex leaves behind (bits).
+constexpr int kDiffShadow = 1;     // a shadow ray decides P.nee (the NEE term exists)
+constexpr int kDiffEnvLight = 2;   // ... of an environment light sample
+constexpr int kDiffWeight = 4;     // the continuation has a weight (its term exists if the path goes on)
+constexpr int kDiffContinue = 8;   // the path goes on with (P.o, P.dir)
+constexpr int kDiffEscape = 16;    // the ray left the scene with weight V.tcw
 
-// One bounce of the path: trace, background or emitter, NEE, Russian
-// roulette, continuation.  Returns true when the path has ended.  GRAD: the
-// vertex keeps what its gradient terms need (DiffVertex) in vtx[P.nvtx].
-template <bool GRAD>
-__device__ bool diff_step(const SceneView& sv, const DiffView& dv, DiffPath& P, DiffVertex* vtx) {
+// One vertex of the path, given its extension ray's hit: background or
+// emitter, NEE, Russian roulette, continuation.  Returns kDiff* bits; the
+// shadow ray is (so, sdir) with its limit in so.w.  GRAD: the vertex keeps
+// what its gradient terms need in V.  CLS as in shade_path.
+template <bool GRAD, int CLS>
+__device__ __forceinline__ int diff_shade(const SceneView& sv, const DiffView& dv, DiffPath& P, DiffVertex& V, int depth,
+                                          const float4& hit, float4& so, F3& sdir) {
+    constexpr int KIND = CLS == 2 ? PGX_BSDF_DIFFUSE
+                       : CLS == 3 ? PGX_BSDF_CONDUCTOR
+                       : CLS == 4 ? PGX_BSDF_GLASS
+                                  : -1;
     F3& o = P.o;
     F3& dir = P.dir;
     F3& T = P.T;
@@ -1487,247 +1509,177 @@ __device__ bool diff_step(const SceneView& sv, const DiffView& dv, DiffPath& P, 
     uint64_t& rng = P.rng;
     bool& prev_spec = P.prev_spec;
     float& prev_pdf = P.prev_pdf;
-    int& nvtx = P.nvtx;
-    bool& escaped = P.escaped;
-    F3& esc_dir = P.esc_dir;
-    F3& esc_w = P.esc_w;
-    const int depth = P.depth;
-    {
-
-        int id;
-        float t, hu, hv;
-        int status;
-        bvh_trace<false>(sv.bvh, mk(o.x, o.y, o.z), mk(dir.x, dir.y, dir.z), FLT_MAX, id, t, hu, hv, status);
-        if (status) id = -1;
-        if (id < 0) {
-            // Background (k_shade<PLAIN>'s miss branch); decisions on the
-            // sampling environment, radiance from the evaluation one.
-            F3 bg_s = env_eval(sv.env, dir);
-            F3 bg = env_eval(dv.env_e, dir);
-            float w = 0.f;
-            if (depth == 0 || prev_spec) {
-                w = 1.f;
-            } else if (!(lum(bg_s) < 1e-8f)) {
-                float pmf = 1.f / (float)sv.nlights;
-                float pdf_light = env_pdf(sv.env, dir);
-                if (pmf > 0.f && pdf_light > 0.f) w = power_heuristic(prev_pdf, pmf * pdf_light);
-            }
-            if (w > 0.f) {
-                L = L + (T * bg) * w;
-                if (GRAD) {
-                    escaped = true;
-                    esc_dir = dir;
-                    esc_w = T * w;
-                }
-            }
-            return true;
-        }
-        Shading sd;
-        DevMaterial ms;
-        F3 tri_gn;
-        float tri_area;
-        shading_data(sv, make_float4(o.x, o.y, o.z, 0.f), make_float4(dir.x, dir.y, dir.z, 0.f),
-                     make_float4(__int_as_float(id), t, hu, hv), sd, ms, tri_gn, tri_area);
-        const DevMaterial me = dv.mats_e[sd.mat];
-        DiffVertex* V = GRAD ? &vtx[nvtx] : nullptr;
-        if (GRAD) {
-            nvtx++;
-            V->flags = 0;
-            V->mat = sd.mat;
-            V->ia = albedo_linear(me) ? safe_div3(f3(1.f, 1.f, 1.f), albedo_of(sv.tex, me, sd)) : zero3();
-        }
-        if (ms.is_light) {
-            F3 em = f3(ms.emission[0], ms.emission[1], ms.emission[2]);
-            if (depth == 0 || prev_spec) {
-                L = L + T * em;
-            } else {
-                float pmf = 1.f / (float)sv.nlights;
-                float cos_tp = s_max(dot(-dir, tri_gn), 0.f);
-                float d2 = sd.t * sd.t;
-                if (cos_tp > 0.f && !(d2 < PGX_EPSILON)) {
-                    float pab = (prev_pdf * cos_tp) / d2;
-                    L = L + (T * em) * power_heuristic(pab, (1.f / tri_area) * pmf);
-                }
-            }
-            return true;
-        }
-        // ---- next-event estimation (next_event with detached pdfs) ----
-        if (!bsdf_pure_specular(ms) && sv.nlights > 0) {
+    int out = 0;
+    if (CLS == 0) {
+        // Background (k_shade<PLAIN>'s miss branch); decisions on the
+        // sampling environment, radiance from the evaluation one.
+        F3 bg_s = env_eval(sv.env, dir);
+        F3 bg = env_eval(dv.env_e, dir);
+        float w = 0.f;
+        if (depth == 0 || prev_spec) {
+            w = 1.f;
+        } else if (!(lum(bg_s) < 1e-8f)) {
             float pmf = 1.f / (float)sv.nlights;
-            unsigned nl = (unsigned)sv.nlights;
-            unsigned idx = (unsigned)floorf(pgx_rng_next(rng) * (float)nl);
-            idx = (nl - 1u < idx) ? nl - 1u : idx;
-            F3 target, wi, emitted;
-            float pal = 0.f, wd = 0.f, geo = 0.f;
-            bool ok = false, env_light = false;
-            if (sv.has_env_light && idx == 0) {
-                F3 col_s;
-                float pdf_light;
-                F3 d0 = env_sample(sv.env, rng, col_s, pdf_light);
-                if (pdf_light > 0.f) {
-                    wi = normalize(d0);
-                    float cos_t = s_max(dot(wi, sd.sn), 0.f);
-                    if (cos_t > 0.f) {
-                        emitted = env_eval(dv.env_e, wi);
-                        pal = pdf_light * pmf;
-                        wd = power_heuristic(pal, bsdf_pdf(ms, sv.tex, sd, wi));
-                        geo = cos_t;
-                        target = f3(sv.bounds.centre[0], sv.bounds.centre[1], sv.bounds.centre[2]) +
-                                 wi * sv.bounds.radius;
-                        ok = true;
-                        env_light = true;
-                    }
-                }
-            } else {
-                const DevAreaLight& Lt = sv.lights[idx - (unsigned)sv.has_env_light];
-                float r1 = pgx_rng_next(rng);
-                float r2 = pgx_rng_next(rng);
-                float sq = sqrtf(r1);
-                float a = 1.f - sq, b = r2 * sq, c = (1.f - a) - b;
-                float pdf_light = 1.f / Lt.p0.w;
-                target = ((f3(Lt.p0) * a) + (f3(Lt.p1) * b)) + (f3(Lt.p2) * c);
-                emitted = f3(Lt.emission);
-                if (pdf_light > 0.f) {
-                    F3 stl = target - sd.x;
-                    wi = normalize(stl);
-                    float den = length_sq(stl);
-                    if (!(den < PGX_EPSILON)) {
-                        float cos_t = s_max(dot(wi, sd.sn), 0.f);
-                        float cos_tp = s_max(dot(-wi, f3(Lt.gn)), 0.f);
-                        geo = (cos_t * cos_tp) / den;
-                        pal = pdf_light * pmf;
-                        float pab = (bsdf_pdf(ms, sv.tex, sd, wi) * cos_tp) / den;
-                        wd = power_heuristic(pal, pab);
-                        ok = geo > 0.f;
-                    }
-                }
-            }
-            if (ok) {
-                F3 fe = bsdf_eval(me, sv.tex, sd, wi);
-                F3 cw = divs(fe * (geo * wd), pal);  // radiance weight of the light sample
-                F3 contrib = emitted * cw;
-                if (contrib.x != 0.f || contrib.y != 0.f || contrib.z != 0.f) {
-                    float sgn = (dot(wi, sd.gn) >= 0.f) ? 1.f : -1.f;
-                    F3 p1 = sd.x + sd.gn * (PGX_EPSILON * sgn);
-                    F3 dvv = target - p1;
-                    float max_t = length(dvv) - (2.f * PGX_EPSILON);
-                    dvv = normalize(dvv);
-                    F3 org = p1 + dvv * PGX_EPSILON;
-                    int sid, sst;
-                    float st_, su, sv_;
-                    bool occluded = bvh_trace<true>(sv.bvh, mk(org.x, org.y, org.z), mk(dvv.x, dvv.y, dvv.z), max_t,
-                                                    sid, st_, su, sv_, sst);
-                    if (!occluded && !sst) {
-                        F3 C = T * contrib;
-                        L = L + C;
-                        if (GRAD) {
-                            V->flags |= 1;
-                            V->C = C;
-                            V->dr_nee = conductor_dlogf_drough(me, to_local(sd.frame, wi), to_local(sd.frame, sd.wo));
-                            if (env_light) {
-                                V->flags |= 2;
-                                V->wi = wi;
-                                V->tcw = T * cw;
-                            }
-                        }
-                    }
-                }
+            float pdf_light = env_pdf(sv.env, dir);
+            if (pmf > 0.f && pdf_light > 0.f) w = power_heuristic(prev_pdf, pmf * pdf_light);
+        }
+        if (w > 0.f) {
+            L = L + (T * bg) * w;
+            if (GRAD) {
+                V.wi = dir;
+                V.tcw = T * w;
+                out = kDiffEscape;
             }
         }
-        // ---- Russian roulette on the sampling throughput ----
-        if (depth > 3) {
-            float q = s_min(s_max(PGX_EPSILON, lum(Ts)), 1.f);
-            if (pgx_rng_next(rng) < q) {
-                T = divs(T, q);
-                Ts = divs(Ts, q);
-            } else {
-                return true;
-            }
-        }
-        if (depth == dv.max_depth) return true;
-        // ---- continuation: sampled with the sampling material ----
-        const bool spec = bsdf_pure_specular(ms);
-        uint64_t rng0 = rng;
-        F3 fs;
-        float pdf;
-        F3 wi = bsdf_sample(ms, sv.tex, sd, rng, fs, pdf);
-        float cos_t = fabsf(dot(wi, sd.sn));
-        if (pdf <= 0.f || cos_t <= 0.f) return true;
-        F3 fe;
-        if (spec) {
-            // deterministic directions: the evaluation material's own sample
-            float pe;
-            uint64_t r2 = rng0;
-            bsdf_sample(me, sv.tex, sd, r2, fe, pe);
+        return out;
+    }
+    Shading sd;
+    DevMaterial ms;
+    F3 tri_gn;
+    float tri_area;
+    shading_data(sv, make_float4(o.x, o.y, o.z, 0.f), make_float4(dir.x, dir.y, dir.z, 0.f),
+                 hit, sd, ms, tri_gn, tri_area);
+    const DevMaterial me = dv.mats_e[sd.mat];
+    if (GRAD) {
+        V.mat = sd.mat;
+        V.ia = albedo_linear(me) ? safe_div3(f3(1.f, 1.f, 1.f), albedo_of(sv.tex, me, sd)) : zero3();
+    }
+    if (CLS == 1) {
+        F3 em = f3(ms.emission[0], ms.emission[1], ms.emission[2]);
+        if (depth == 0 || prev_spec) {
+            L = L + T * em;
         } else {
-            fe = bsdf_eval(me, sv.tex, sd, wi);
-        }
-        if (GRAD) {
-            V->flags |= 4;
-            V->l_snap = L;
-            V->dr_cont = spec ? 0.f : conductor_dlogf_drough(me, to_local(sd.frame, wi), to_local(sd.frame, sd.wo));
-        }
-        T = divs(T * fe * cos_t, pdf);
-        Ts = divs(Ts * fs * cos_t, pdf);
-        if (lum(Ts) <= 0.f) return true;
-        if (isnan(Ts.x) || isnan(Ts.y) || isnan(Ts.z)) return true;
-        if (isinf(Ts.x) || isinf(Ts.y) || isinf(Ts.z)) return true;
-        if (Ts.x < 0.f || Ts.y < 0.f || Ts.z < 0.f) return true;
-        float sgn = (dot(wi, sd.gn) >= 0.f) ? 1.f : -1.f;
-        o = sd.x + sd.gn * (PGX_EPSILON * sgn);
-        dir = wi;
-        prev_spec = spec;
-        prev_pdf = pdf;
-    
-    }
-    return ++P.depth > dv.max_depth;
-}
-
-// The gradient terms of a finished path: emitted once its radiance L is
-// known, and only when L is finite (the film drops the other samples).
-template <bool GRAD>
-__device__ void diff_finish(const DiffView& dv, const DiffPath& P, const DiffVertex* vtx, const DiffAcc& acc) {
-    const F3 L = P.L, delta = P.delta;
-    const int nvtx = P.nvtx;
-    const bool escaped = P.escaped;
-    const F3 esc_dir = P.esc_dir, esc_w = P.esc_w;
-    if (GRAD && valid(L)) {  // the film drops non-finite samples: no gradient from them
-        for (int j = 0; j < nvtx; j++) {
-            const DiffVertex& v = vtx[j];
-            const bool alb = v.ia.x != 0.f || v.ia.y != 0.f || v.ia.z != 0.f;
-            if (v.flags & 1) {
-                F3 g = delta * v.C;
-                if (alb) add_alb(acc, v.mat, g * v.ia);
-                if (v.dr_nee != 0.f) atomicAdd(acc.rough + v.mat, (double)((g.x + g.y + g.z) * v.dr_nee));
-                if (v.flags & 2) env_scatter(dv.env_e, v.wi, delta * v.tcw, dv.g_env);
-            }
-            if (v.flags & 4) {
-                F3 g = delta * (L - v.l_snap);  // radiance collected after this vertex
-                if (alb) add_alb(acc, v.mat, g * v.ia);
-                if (v.dr_cont != 0.f) atomicAdd(acc.rough + v.mat, (double)((g.x + g.y + g.z) * v.dr_cont));
+            float pmf = 1.f / (float)sv.nlights;
+            float cos_tp = s_max(dot(-dir, tri_gn), 0.f);
+            float d2 = sd.t * sd.t;
+            if (cos_tp > 0.f && !(d2 < PGX_EPSILON)) {
+                float pab = (prev_pdf * cos_tp) / d2;
+                L = L + (T * em) * power_heuristic(pab, (1.f / tri_area) * pmf);
             }
         }
-        if (escaped) env_scatter(dv.env_e, esc_dir, delta * esc_w, dv.g_env);
+        return out;
     }
-}
-
-// One path from its seed.  Returns the path's radiance.  GRAD: delta is the
-// adjoint of the sample's value; each vertex keeps what its gradient terms
-// need (DiffVertex) and the terms are emitted after the last vertex, when
-// the path's total radiance is known and the sample is known to be kept by
-// the film (finite) — one traversal per sample (path replay
-// backpropagation, Vicini et al. 2021, with the replay's second pass folded
-// into per-vertex records held by the thread).
-template <bool GRAD>
-__device__ F3 diff_path(const SceneView& sv, const DiffView& dv, uint64_t rng, F3 o, F3 dir, F3 delta,
-                        const DiffAcc& acc) {
-    DiffPath P;
-    DiffVertex vtx[GRAD ? kMaxDepthCap + 1 : 1];
-    diff_begin(P, rng, o, dir, delta);
-    while (!diff_step<GRAD>(sv, dv, P, vtx)) {
+    // ---- next-event estimation (next_event with detached pdfs) ----
+    if (!bsdf_pure_specular_k<KIND>(ms) && sv.nlights > 0) {
+        float pmf = 1.f / (float)sv.nlights;
+        unsigned nl = (unsigned)sv.nlights;
+        unsigned idx = (unsigned)floorf(pgx_rng_next(rng) * (float)nl);
+        idx = (nl - 1u < idx) ? nl - 1u : idx;
+        F3 target, wi, emitted;
+        float pal = 0.f, wd = 0.f, geo = 0.f;
+        bool ok = false, env_light = false;
+        if (sv.has_env_light && idx == 0) {
+            F3 col_s;
+            float pdf_light;
+            F3 d0 = env_sample(sv.env, rng, col_s, pdf_light);
+            if (pdf_light > 0.f) {
+                wi = normalize(d0);
+                float cos_t = s_max(dot(wi, sd.sn), 0.f);
+                if (cos_t > 0.f) {
+                    emitted = env_eval(dv.env_e, wi);
+                    pal = pdf_light * pmf;
+                    wd = power_heuristic(pal, bsdf_pdf_k<KIND>(ms, sv.tex, sd, wi));
+                    geo = cos_t;
+                    target = f3(sv.bounds.centre[0], sv.bounds.centre[1], sv.bounds.centre[2]) +
+                             wi * sv.bounds.radius;
+                    ok = true;
+                    env_light = true;
+                }
+            }
+        } else {
+            const DevAreaLight& Lt = sv.lights[idx - (unsigned)sv.has_env_light];
+            float r1 = pgx_rng_next(rng);
+            float r2 = pgx_rng_next(rng);
+            float sq = sqrtf(r1);
+            float a = 1.f - sq, b = r2 * sq, c = (1.f - a) - b;
+            float pdf_light = 1.f / Lt.p0.w;
+            target = ((f3(Lt.p0) * a) + (f3(Lt.p1) * b)) + (f3(Lt.p2) * c);
+            emitted = f3(Lt.emission);
+            if (pdf_light > 0.f) {
+                F3 stl = target - sd.x;
+                wi = normalize(stl);
+                float den = length_sq(stl);
+                if (!(den < PGX_EPSILON)) {
+                    float cos_t = s_max(dot(wi, sd.sn), 0.f);
+                    float cos_tp = s_max(dot(-wi, f3(Lt.gn)), 0.f);
+                    geo = (cos_t * cos_tp) / den;
+                    pal = pdf_light * pmf;
+                    float pab = (bsdf_pdf_k<KIND>(ms, sv.tex, sd, wi) * cos_tp) / den;
+                    wd = power_heuristic(pal, pab);
+                    ok = geo > 0.f;
+                }
+            }
+        }
+        if (ok) {
+            F3 fe = bsdf_eval_k<KIND>(me, sv.tex, sd, wi);
+            F3 cw = divs(fe * (geo * wd), pal);  // radiance weight of the light sample
+            F3 contrib = emitted * cw;
+            if (contrib.x != 0.f || contrib.y != 0.f || contrib.z != 0.f) {
+                float sgn = (dot(wi, sd.gn) >= 0.f) ? 1.f : -1.f;
+                F3 p1 = sd.x + sd.gn * (PGX_EPSILON * sgn);
+                F3 dvv = target - p1;
+                float max_t = length(dvv) - (2.f * PGX_EPSILON);
+                dvv = normalize(dvv);
+                F3 org = p1 + dvv * PGX_EPSILON;
+                out |= kDiffShadow | (env_light ? kDiffEnvLight : 0);
+                so = make_float4(org.x, org.y, org.z, max_t);
+                sdir = dvv;
+                P.nee = T * contrib;
+                if (GRAD) {
+                    V.C = P.nee;
+                    V.dr_nee = conductor_dlogf_drough(me, to_local(sd.frame, wi), to_local(sd.frame, sd.wo));
+                    if (env_light) {
+                        V.wi = wi;
+                        V.tcw = T * cw;
+                    }
+                }
+            }
+        }
     }
-    diff_finish<GRAD>(dv, P, vtx, acc);
-    return P.L;
+    // ---- Russian roulette on the sampling throughput ----
+    if (depth > 3) {
+        float q = s_min(s_max(PGX_EPSILON, lum(Ts)), 1.f);
+        if (pgx_rng_next(rng) < q) {
+            T = divs(T, q);
+            Ts = divs(Ts, q);
+        } else {
+            return out;
+        }
+    }
+    if (depth == dv.max_depth) return out;
+    // ---- continuation: sampled with the sampling material ----
+    const bool spec = bsdf_pure_specular_k<KIND>(ms);
+    uint64_t rng0 = rng;
+    F3 fs;
+    float pdf;
+    F3 wi = bsdf_sample_k<KIND>(ms, sv.tex, sd, rng, fs, pdf);
+    float cos_t = fabsf(dot(wi, sd.sn));
+    if (pdf <= 0.f || cos_t <= 0.f) return out;
+    F3 fe;
+    if (spec) {
+        // deterministic directions: the evaluation material's own sample
+        float pe;
+        uint64_t r2 = rng0;
+        bsdf_sample_k<KIND>(me, sv.tex, sd, r2, fe, pe);
+    } else {
+        fe = bsdf_eval_k<KIND>(me, sv.tex, sd, wi);
+    }
+    out |= kDiffWeight;
+    if (GRAD) {
+        V.dr_cont = spec ? 0.f : conductor_dlogf_drough(me, to_local(sd.frame, wi), to_local(sd.frame, sd.wo));
+    }
+    T = divs(T * fe * cos_t, pdf);
+    Ts = divs(Ts * fs * cos_t, pdf);
+    if (lum(Ts) <= 0.f) return out;
+    if (isnan(Ts.x) || isnan(Ts.y) || isnan(Ts.z)) return out;
+    if (isinf(Ts.x) || isinf(Ts.y) || isinf(Ts.z)) return out;
+    if (Ts.x < 0.f || Ts.y < 0.f || Ts.z < 0.f) return out;
+    float sgn = (dot(wi, sd.gn) >= 0.f) ? 1.f : -1.f;
+    o = sd.x + sd.gn * (PGX_EPSILON * sgn);
+    dir = wi;
+    prev_spec = spec;
+    prev_pdf = pdf;
+    return out | kDiffContinue;
 }
 
 // Sample s of pixel (x, y): jitter, camera ray, target pixel of the box
@@ -1745,53 +1697,188 @@ __device__ __forceinline__ int diff_camera(const SceneView& sv, const DiffView& 
     return (by - y) * 2 + (bx - x);  // 0..3: which neighbour (right, down)
 }
 
-// Primal samples [s0, s0 + ns) on persistent warps with lane refill (as the
-// adjoint): sample i of the chunk (pixel-major) stores its value and the box
-// filter's target neighbour k in samples[i] (w = -1 when the film drops it).
-// The per-pixel sums happen afterwards in sample order (k_diff_accumulate),
-// so the image does not depend on which lane traced which sample.
-__global__ void __launch_bounds__(kThreads) k_diff_primal(SceneView sv, DiffView dv) {
-    constexpr unsigned kFull = 0xFFFFFFFFu;
+// Camera rays of one wave of differentiable samples.  The target neighbour of
+// the box filter (diff_camera; -1: outside) is kept with the path; the adjoint
+// traces only samples with a target and a non-zero adjoint there.
+template <bool GRAD>
+__global__ void __launch_bounds__(kThreads) k_diff_camgen(SceneView sv, PathState ps, DiffView dv) {
     const int64_t npix = (int64_t)sv.width * sv.height;
-    const unsigned long long items = (unsigned long long)npix * (unsigned long long)dv.ns;
-    const F3 origin = f3(sv.cam.origin[0], sv.cam.origin[1], sv.cam.origin[2]);
-    const int lane = threadIdx.x & 31;
-    DiffAcc none{nullptr, nullptr};
-    DiffPath P;
-    DiffVertex vtx[1];
-    bool active = false, exhausted = false;
-    unsigned long long mine = 0;
-    int k = -1;
-    for (;;) {
-        const bool need = !active && !exhausted;
-        const unsigned m = __ballot_sync(kFull, need);
-        if (m) {
-            const int leader = __ffs(m) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(dv.next, (unsigned long long)__popc(m));
-            base = __shfl_sync(kFull, base, leader);
-            if (need) {
-                mine = base + (unsigned long long)__popc(m & ((1u << lane) - 1u));
-                if (mine < items) {
-                    const int64_t pixel = (int64_t)(mine % (unsigned long long)npix);
-                    const int smp = dv.s0 + (int)(mine / (unsigned long long)npix);
-                    uint64_t rng;
-                    F3 dir;
-                    k = diff_camera(sv, dv, pixel, smp, rng, dir);
-                    diff_begin(P, rng, origin, dir, zero3());
-                    active = true;
-                } else {
-                    exhausted = true;
+    const int64_t rounds = (dv.count + (int64_t)gridDim.x * blockDim.x - 1) / ((int64_t)gridDim.x * blockDim.x);
+    for (int64_t r = 0; r < rounds; r++) {  // whole warps reach the append
+        const int64_t i = (r * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+        bool trace = false;
+        if (i < dv.count) {
+            const int64_t item = dv.first + i;
+            const int64_t pixel = item % npix;
+            uint64_t rng;
+            F3 dir;
+            const int k = diff_camera(sv, dv, pixel, (int)(item / npix), rng, dir);
+            trace = true;
+            if (GRAD) {
+                trace = false;
+                if (k >= 0) {
+                    const int64_t tp = (pixel / sv.width + k / 2) * sv.width + (pixel % sv.width + k % 2);
+                    trace = dv.dimg[3 * tp] != 0.f || dv.dimg[3 * tp + 1] != 0.f || dv.dimg[3 * tp + 2] != 0.f;
                 }
             }
+            ps.o[i] = make_float4(sv.cam.origin[0], sv.cam.origin[1], sv.cam.origin[2], 0.f);
+            ps.d[i] = make_float4(dir.x, dir.y, dir.z, 0.f);
+            ps.T[i] = make_float4(1.f, 1.f, 1.f, 0.f);
+            dv.Ts[i] = make_float4(1.f, 1.f, 1.f, 0.f);
+            ps.L[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            ps.pix[i] = make_float2((float)k, 0.f);
+            ps.rng[i] = rng;
+            ps.flags[i] = 0;
+            ps.nrec[i] = 0;
         }
-        if (__all_sync(kFull, !active && exhausted)) break;
-        if (active && diff_step<false>(sv, dv, P, vtx)) {
-            const F3 c = P.L;
-            const bool keep = k >= 0 && valid(c);
-            dv.samples[mine] = make_float4(c.x, c.y, c.z, keep ? (float)k : -1.f);
-            active = false;
+        const unsigned slot = warp_aggregated_add(&ps.qcount[0], trace);
+        if (trace) ps.queue[0][slot] = (int)i;
+    }
+}
+
+// One path's vertex at this depth: state in, diff_shade, state, record, queues out.
+template <bool GRAD, int CLS>
+__device__ __forceinline__ void diff_vertex(const SceneView& sv, const DiffView& dv, PathState& ps, int depth, int p,
+                                            bool active) {
+    DiffPath P;
+    DiffVertex V;
+    int out = 0;
+    float4 so = make_float4(0.f, 0.f, 0.f, 0.f);
+    F3 sdir = zero3();
+    if (active) {
+        const float4 o = ps.o[p], d = ps.d[p], Tw = ps.T[p], ts = dv.Ts[p], l = ps.L[p], hit = ps.hit[p];
+        P.o = f3(o);
+        P.dir = f3(d);
+        P.T = f3(Tw);
+        P.Ts = f3(ts);
+        P.L = f3(l);
+        P.rng = ps.rng[p];
+        P.prev_pdf = Tw.w;
+        P.prev_spec = ps.flags[p] & 1;
+        const size_t at = (size_t)depth * dv.stride + p;
+        // the light sample of the vertex before has been settled: the
+        // radiance up to there, its material kept in w
+        if (GRAD && depth > 0) {
+            float* snap = reinterpret_cast<float*>(ps.rec_wi + (at - dv.stride));
+            snap[0] = l.x, snap[1] = l.y, snap[2] = l.z;
         }
+        out = diff_shade<GRAD, CLS>(sv, dv, P, V, depth, hit, so, sdir);
+        if (GRAD) {
+            if (out & kDiffShadow) ps.rec_pos[at] = make_float4(V.C.x, V.C.y, V.C.z, V.dr_nee);
+            if (CLS != 0) {
+                ps.rec_nrm[at] = make_float4(V.ia.x, V.ia.y, V.ia.z, (out & kDiffWeight) ? V.dr_cont : 0.f);
+                reinterpret_cast<float*>(ps.rec_wi + at)[3] = __int_as_float(V.mat);
+            }
+            const bool env = (out & (kDiffEnvLight | kDiffEscape)) != 0;
+            ps.rec_w[at] = make_float4(env ? V.tcw.x : 0.f, env ? V.tcw.y : 0.f, env ? V.tcw.z : 0.f, __int_as_float(out));
+            if (env) ps.rec_e[at] = make_float4(V.wi.x, V.wi.y, V.wi.z, 0.f);
+            ps.nrec[p] = depth + 1;
+        }
+        if (CLS <= 1) {
+            ps.L[p] = make_float4(P.L.x, P.L.y, P.L.z, 0.f);
+        } else if (out & kDiffContinue) {
+            ps.o[p] = make_float4(P.o.x, P.o.y, P.o.z, 0.f);
+            ps.d[p] = make_float4(P.dir.x, P.dir.y, P.dir.z, 0.f);
+            ps.T[p] = make_float4(P.T.x, P.T.y, P.T.z, P.prev_pdf);
+            dv.Ts[p] = make_float4(P.Ts.x, P.Ts.y, P.Ts.z, 0.f);
+            ps.rng[p] = P.rng;
+            ps.flags[p] = P.prev_spec ? 1 : 0;
+        }
+    }
+    if (CLS > 1) {
+        push_shadow(ps, depth, p, so, make_float4(sdir.x, sdir.y, sdir.z, 0.f), P.nee, active && (out & kDiffShadow));
+        const bool cont = active && (out & kDiffContinue);
+        const unsigned slot = warp_aggregated_add(&ps.qcount[depth + 1], cont);
+        if (cont) ps.queue[(depth + 1) & 1][slot] = p;
+    }
+}
+
+// Vertices of this depth, binned by surface class (the tiles of k_shade).
+template <bool GRAD>
+__global__ void __launch_bounds__(kThreads, kShadeBlocksPerSM) k_diff_shade(SceneView sv, PathState ps, DiffView dv, int depth) {
+    const ClassTiles tiles(ps, depth);
+    int cls;
+    unsigned i, n;
+    for (unsigned tile = blockIdx.x; tiles.find(tile, cls, i, n); tile += gridDim.x) {
+        const bool active = i < n;
+        const int p = active ? ps.cqueue[(size_t)cls * ps.capacity + i] : 0;
+        switch (cls) {
+            case 0: diff_vertex<GRAD, 0>(sv, dv, ps, depth, p, active); break;
+            case 1: diff_vertex<GRAD, 1>(sv, dv, ps, depth, p, active); break;
+            case 2: diff_vertex<GRAD, 2>(sv, dv, ps, depth, p, active); break;
+            case 3: diff_vertex<GRAD, 3>(sv, dv, ps, depth, p, active); break;
+            case 4: diff_vertex<GRAD, 4>(sv, dv, ps, depth, p, active); break;
+            default: diff_vertex<GRAD, 5>(sv, dv, ps, depth, p, active); break;
+        }
+    }
+}
+
+// Primal: the wave's sample values with their target neighbour (w = -1 when
+// the film drops the sample).  The per-pixel sums happen afterwards in sample
+// order (k_diff_accumulate), so the image is deterministic.
+__global__ void __launch_bounds__(kThreads) k_diff_store(PathState ps, DiffView dv) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dv.count; i += (int64_t)gridDim.x * blockDim.x) {
+        const F3 c = f3(ps.L[i]);
+        const float k = ps.pix[i].x;
+        dv.samples[dv.first - dv.chunk0 + i] = make_float4(c.x, c.y, c.z, k >= 0.f && valid(c) ? k : -1.f);
+    }
+}
+
+// Adjoint: the gradient terms of the wave's finished paths, from their vertex
+// records, once the radiance L is known, and only when it is finite (the film
+// drops the other samples).
+__global__ void __launch_bounds__(kThreads) k_diff_emit(SceneView sv, PathState ps, DiffView dv) {
+    extern __shared__ double sacc[];  // [nmats*3 + nmats] when it fits
+    const bool shared_acc = dv.nmats * 4 * (int)sizeof(double) <= 32 * 1024;
+    DiffAcc acc{dv.g_alb, dv.g_rough};
+    if (shared_acc) {
+        for (int i = threadIdx.x; i < dv.nmats * 4; i += blockDim.x) sacc[i] = 0.0;
+        __syncthreads();
+        acc.alb = sacc;
+        acc.rough = sacc + dv.nmats * 3;
+    }
+    const int64_t npix = (int64_t)sv.width * sv.height;
+    const float inv_spp = 1.f / (float)dv.spp;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dv.count; i += (int64_t)gridDim.x * blockDim.x) {
+        const int nvtx = ps.nrec[i];
+        const F3 L = f3(ps.L[i]);
+        if (nvtx == 0 || !valid(L)) continue;
+        const int64_t pixel = (dv.first + i) % npix;
+        const int k = (int)ps.pix[i].x;
+        const int64_t tp = (pixel / sv.width + k / 2) * sv.width + (pixel % sv.width + k % 2);
+        const F3 delta = f3(dv.dimg[3 * tp], dv.dimg[3 * tp + 1], dv.dimg[3 * tp + 2]) * inv_spp;
+        for (int j = 0; j < nvtx; j++) {
+            const size_t at = (size_t)j * dv.stride + i;
+            const float4 w4 = ps.rec_w[at];
+            const int flags = __float_as_int(w4.w);
+            const bool nee = (flags & kDiffShadow) && (flags & kDiffSeen);
+            if ((nee && (flags & kDiffEnvLight)) || (flags & kDiffEscape))
+                env_scatter(dv.env_e, f3(ps.rec_e[at]), delta * f3(w4), dv.g_env);
+            const bool cont = (flags & kDiffWeight) && j + 1 < nvtx;  // radiance collected after this vertex
+            if (!nee && !cont) continue;
+            const float4 ia4 = ps.rec_nrm[at], snap = ps.rec_wi[at];
+            const F3 ia = f3(ia4);
+            const int mat = __float_as_int(snap.w);
+            const bool alb = ia.x != 0.f || ia.y != 0.f || ia.z != 0.f;
+            if (nee) {
+                const float4 c4 = ps.rec_pos[at];
+                const F3 g = delta * f3(c4);
+                if (alb) add_alb(acc, mat, g * ia);
+                if (c4.w != 0.f) atomicAdd(acc.rough + mat, (double)((g.x + g.y + g.z) * c4.w));
+            }
+            if (cont) {
+                const F3 g = delta * (L - f3(snap));
+                if (alb) add_alb(acc, mat, g * ia);
+                if (ia4.w != 0.f) atomicAdd(acc.rough + mat, (double)((g.x + g.y + g.z) * ia4.w));
+            }
+        }
+    }
+    if (shared_acc) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < dv.nmats * 3; i += blockDim.x)
+            if (sacc[i] != 0.0) atomicAdd(dv.g_alb + i, sacc[i]);
+        for (int i = threadIdx.x; i < dv.nmats; i += blockDim.x)
+            if (sacc[dv.nmats * 3 + i] != 0.0) atomicAdd(dv.g_rough + i, sacc[dv.nmats * 3 + i]);
     }
 }
 
@@ -1835,77 +1922,6 @@ __global__ void k_diff_gather(const double* __restrict__ partial, int W, int H, 
                 for (int c = 0; c < 3; c++) v[c] += q[c];
             }
         for (int c = 0; c < 3; c++) img[p * 3 + c] = v[c] / (double)spp;
-    }
-}
-
-// Persistent warps over the samples (pixel-major within each sample index):
-// a lane whose path has ended takes the next sample from dv.next at once
-// (warp-aggregated atomicAdd), so short and long paths share the warp's
-// issue slots instead of each warp waiting for its longest path.
-__global__ void __launch_bounds__(kThreads) k_diff_adjoint(SceneView sv, DiffView dv) {
-    extern __shared__ double sacc[];  // [nmats*3 + nmats] when it fits
-    const bool shared_acc = dv.nmats * 4 * (int)sizeof(double) <= 32 * 1024;
-    DiffAcc acc;
-    if (shared_acc) {
-        for (int i = threadIdx.x; i < dv.nmats * 4; i += blockDim.x) sacc[i] = 0.0;
-        __syncthreads();
-        acc.alb = sacc;
-        acc.rough = sacc + dv.nmats * 3;
-    } else {
-        acc.alb = dv.g_alb;
-        acc.rough = dv.g_rough;
-    }
-    constexpr unsigned kFull = 0xFFFFFFFFu;
-    const int64_t npix = (int64_t)sv.width * sv.height;
-    const unsigned long long items = (unsigned long long)npix * (unsigned long long)dv.spp;
-    const F3 origin = f3(sv.cam.origin[0], sv.cam.origin[1], sv.cam.origin[2]);
-    const float inv_spp = 1.f / (float)dv.spp;
-    const int lane = threadIdx.x & 31;
-    DiffPath P;
-    DiffVertex vtx[kMaxDepthCap + 1];
-    bool active = false, exhausted = false;
-    for (;;) {
-        const bool need = !active && !exhausted;
-        const unsigned m = __ballot_sync(kFull, need);
-        if (m) {
-            const int leader = __ffs(m) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(dv.next, (unsigned long long)__popc(m));
-            base = __shfl_sync(kFull, base, leader);
-            if (need) {
-                const unsigned long long item = base + (unsigned long long)__popc(m & ((1u << lane) - 1u));
-                if (item < items) {
-                    const int64_t pixel = (int64_t)(item % (unsigned long long)npix);
-                    const int smp = (int)(item / (unsigned long long)npix);
-                    const int x = (int)(pixel % sv.width), y = (int)(pixel / sv.width);
-                    uint64_t rng;
-                    F3 dir;
-                    const int k = diff_camera(sv, dv, pixel, smp, rng, dir);
-                    if (k >= 0) {
-                        const int64_t tp = (int64_t)(y + k / 2) * sv.width + (x + k % 2);
-                        const F3 delta = f3(dv.dimg[3 * tp], dv.dimg[3 * tp + 1], dv.dimg[3 * tp + 2]) * inv_spp;
-                        if (delta.x != 0.f || delta.y != 0.f || delta.z != 0.f) {
-                            diff_begin(P, rng, origin, dir, delta);
-                            active = true;
-                        }
-                    }
-                } else {
-                    exhausted = true;
-                }
-            }
-        }
-        if (__all_sync(kFull, !active && exhausted)) break;
-        if (active && diff_step<true>(sv, dv, P, vtx)) {
-            diff_finish<true>(dv, P, vtx, acc);
-            active = false;
-        }
-    }
-    if (shared_acc) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < dv.nmats * 3; i += blockDim.x)
-            if (sacc[i] != 0.0) atomicAdd(dv.g_alb + i, sacc[i]);
-        for (int i = threadIdx.x; i < dv.nmats; i += blockDim.x)
-            if (sacc[dv.nmats * 3 + i] != 0.0) atomicAdd(dv.g_rough + i, sacc[dv.nmats * 3 + i]);
     }
 }
 
@@ -2497,6 +2513,7 @@ DiffView diff_view(pgx_ctx* ctx, RenderState* rs, int spp, uint64_t seed, int ma
     dv.seed = seed;
     dv.max_depth = max_depth;
     dv.nmats = ctx->nmats;
+    dv.Ts = rs->d_ts.as<float4>();  // reserved by the caller
     return dv;
 }
 
@@ -2514,6 +2531,29 @@ extern "C" int pgx_diff_set_params(pgx_ctx* ctx, const float* env_rgb, const flo
     return diff_params(ctx, state_of(ctx), env_rgb, albedo_offset, roughness);
 }
 
+// Traces one wave of differentiable samples, dv.first ... dv.first + dv.count:
+// camgen -> [trace -> classify -> shade] x (max_depth + 1) -> trace, as
+// enqueue_frame; the caller stores or emits.
+template <bool GRAD>
+static void diff_wave(const SceneView& sv, const PathState& ps, const DiffView& dv, cudaStream_t s) {
+    const unsigned g = grid_for(dv.count), pg = persistent_grid(dv.count);
+    const unsigned cg = grid_for((dv.count + kClassifyItems - 1) / kClassifyItems);
+    cudaMemsetAsync(ps.qcount, 0, sizeof(unsigned) * 4 * (kMaxDepthCap + 2), s);
+    cudaMemsetAsync(ps.ccount, 0, sizeof(unsigned) * kShadeClasses * (kMaxDepthCap + 2), s);
+    k_diff_camgen<GRAD><<<g, kThreads, 0, s>>>(sv, ps, dv);
+    auto seen = [&](int depth) { return GRAD && depth > 0 ? ps.rec_w + (size_t)(depth - 1) * dv.stride : nullptr; };
+    for (int depth = 0; depth <= dv.max_depth; depth++) {
+        k_trace_step<false><<<pg, kThreads, 0, s>>>(sv, ps, depth, true, depth > 0, nullptr, seen(depth));
+        k_classify<<<cg, kThreads, 0, s>>>(sv, ps, depth);
+        k_diff_shade<GRAD><<<g, kThreads, 0, s>>>(sv, ps, dv, depth);
+    }
+    k_trace_step<false><<<pg, kThreads, 0, s>>>(sv, ps, dv.max_depth + 1, false, true, nullptr, seen(dv.max_depth + 1));
+}
+
+// Paths per wave: the primal's state is about 220 bytes a path, the adjoint's
+// records add 80 bytes a path and depth (5.6 GB at 2^22 paths and depth 16).
+constexpr int64_t kDiffWave = 1 << 24, kDiffGradWave = 1 << 22;
+
 extern "C" int pgx_diff_render(pgx_ctx* ctx, int32_t spp, uint64_t seed, int32_t max_depth, double* image) {
     PGX_TRY(diff_check(ctx, "pgx_diff_render"));
     PGX_TRY(diff_args(ctx, spp, max_depth, "pgx_diff_render"));
@@ -2525,25 +2565,27 @@ extern "C" int pgx_diff_render(pgx_ctx* ctx, int32_t spp, uint64_t seed, int32_t
     PGX_CUDA_TRY(ctx, rs->d_img.reserve(sizeof(double) * 3 * npix));
     // sample values of up to 1 GiB at a time
     const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(spp, ((int64_t)1 << 30) / (16 * npix)));
+    const int64_t wave = std::min<int64_t>(npix * chunk, kDiffWave);
     PGX_CUDA_TRY(ctx, rs->d_samples.reserve(sizeof(float4) * (size_t)npix * chunk));
-    PGX_CUDA_TRY(ctx, rs->d_next.reserve(sizeof(unsigned long long)));
+    PGX_CUDA_TRY(ctx, rs->d_ts.reserve(sizeof(float4) * wave));
+    PGX_TRY(ensure_state(ctx, rs, wave, 0, 0));
     DiffView dv = diff_view(ctx, rs, spp, seed, max_depth);
     dv.partial = rs->d_partial.as<double>();
     dv.samples = rs->d_samples.as<float4>();
-    dv.next = rs->d_next.as<unsigned long long>();
     SceneView sv = scene_view(ctx);
+    PathState ps = path_view(rs);
     cudaStream_t s = ctx->stream;
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(dv.partial, 0, sizeof(double) * 12 * npix, s));
-    int per_sm = 0;
-    PGX_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_diff_primal, kThreads, 0));
     for (int s0 = 0; s0 < spp; s0 += chunk) {
-        dv.s0 = s0;
-        dv.ns = std::min(chunk, spp - s0);
-        const unsigned pg = (unsigned)std::max<int64_t>(
-            1, std::min<int64_t>((npix * dv.ns + kThreads - 1) / kThreads, (int64_t)pgx_num_sms() * std::max(per_sm, 1)));
-        PGX_CUDA_TRY(ctx, cudaMemsetAsync(dv.next, 0, sizeof(unsigned long long), s));
-        k_diff_primal<<<pg, kThreads, 0, s>>>(sv, dv);
-        k_diff_accumulate<<<grid_for(npix), kThreads, 0, s>>>(dv.samples, npix, dv.ns, dv.partial);
+        const int ns = std::min(chunk, spp - s0);
+        dv.chunk0 = npix * s0;
+        for (int64_t at = dv.chunk0; at < dv.chunk0 + npix * ns; at += wave) {
+            dv.first = at;
+            dv.count = std::min(wave, dv.chunk0 + npix * ns - at);
+            diff_wave<false>(sv, ps, dv, s);
+            k_diff_store<<<grid_for(dv.count), kThreads, 0, s>>>(ps, dv);
+        }
+        k_diff_accumulate<<<grid_for(npix), kThreads, 0, s>>>(dv.samples, npix, ns, dv.partial);
     }
     k_diff_gather<<<grid_for(npix), kThreads, 0, s>>>(dv.partial, ctx->width, ctx->height, spp, rs->d_img.as<double>());
     PGX_CUDA_TRY(ctx, cudaGetLastError());
@@ -2562,33 +2604,37 @@ extern "C" int pgx_diff_adjoint(pgx_ctx* ctx, int32_t spp, uint64_t seed, int32_
     const int64_t npix = (int64_t)ctx->width * ctx->height;
     const size_t ef = env_floats(ctx), nm = (size_t)ctx->nmats;
     cudaStream_t s = ctx->stream;
+    const int64_t wave = std::min<int64_t>(npix * spp, kDiffGradWave);
     PGX_CUDA_TRY(ctx, rs->d_dimg.reserve(sizeof(float) * 3 * npix));
     // Gradients are accumulated in double (millions of atomic additions
     // into the popular texels) and returned as float.
     PGX_CUDA_TRY(ctx, rs->d_genv.reserve(sizeof(double) * std::max<size_t>(ef, 1)));
     PGX_CUDA_TRY(ctx, rs->d_galb.reserve(sizeof(double) * std::max<size_t>(3 * nm, 1)));
     PGX_CUDA_TRY(ctx, rs->d_grough.reserve(sizeof(double) * std::max<size_t>(nm, 1)));
+    PGX_CUDA_TRY(ctx, rs->d_ts.reserve(sizeof(float4) * wave));
+    PGX_CUDA_TRY(ctx, rs->d_rec.reserve(5 * sizeof(float4) * (size_t)wave * (max_depth + 1)));
+    PGX_TRY(ensure_state(ctx, rs, wave, 0, 0));
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(rs->d_dimg.p, dloss_dimage, sizeof(float) * 3 * npix, cudaMemcpyHostToDevice, s));
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(rs->d_genv.p, 0, sizeof(double) * std::max<size_t>(ef, 1), s));
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(rs->d_galb.p, 0, sizeof(double) * std::max<size_t>(3 * nm, 1), s));
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(rs->d_grough.p, 0, sizeof(double) * std::max<size_t>(nm, 1), s));
-    PGX_CUDA_TRY(ctx, rs->d_next.reserve(sizeof(unsigned long long)));
-    PGX_CUDA_TRY(ctx, cudaMemsetAsync(rs->d_next.p, 0, sizeof(unsigned long long), s));
     DiffView dv = diff_view(ctx, rs, spp, seed, max_depth);
     dv.dimg = rs->d_dimg.as<float>();
     dv.g_env = ef ? rs->d_genv.as<double>() : nullptr;
     dv.g_alb = rs->d_galb.as<double>();
     dv.g_rough = rs->d_grough.as<double>();
-    dv.next = rs->d_next.as<unsigned long long>();
     const size_t sm = nm * 4 * sizeof(double) <= 32 * 1024 ? nm * 4 * sizeof(double) : 0;
     SceneView sv = scene_view(ctx);
-    // persistent: as many blocks as are resident at once
-    int per_sm = 0;
-    PGX_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_diff_adjoint, kThreads, sm));
-    const unsigned ag = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>((npix * (int64_t)spp + kThreads - 1) / kThreads,
-                             (int64_t)pgx_num_sms() * std::max(per_sm, 1)));
-    k_diff_adjoint<<<ag, kThreads, sm, s>>>(sv, dv);
+    PathState ps = path_view(rs);
+    dv.stride = wave;
+    float4** rec[5] = {&ps.rec_pos, &ps.rec_nrm, &ps.rec_wi, &ps.rec_w, &ps.rec_e};
+    for (int k = 0; k < 5; k++) *rec[k] = rs->d_rec.as<float4>() + (size_t)k * wave * (max_depth + 1);
+    for (int64_t at = 0; at < npix * spp; at += wave) {
+        dv.first = at;
+        dv.count = std::min(wave, npix * spp - at);
+        diff_wave<true>(sv, ps, dv, s);
+        k_diff_emit<<<grid_for(dv.count), kThreads, sm, s>>>(sv, ps, dv);
+    }
     PGX_CUDA_TRY(ctx, cudaGetLastError());
     std::vector<double> he(grad_env && ef ? ef : 0), ha(grad_albedo ? 3 * nm : 0), hr(grad_roughness ? nm : 0);
     if (!he.empty())
