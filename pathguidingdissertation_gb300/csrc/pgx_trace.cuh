@@ -326,7 +326,8 @@ __device__ __forceinline__ void lane_node(const BvhView& bvh, TraceLane& L, Stac
 // root ray i starts from (several trees can share the node and triangle
 // arrays).  `next` is a zeroed counter.  n_interior and n_tris get a counting
 // launch's visits.  Must be called by whole warps.
-template <TraceKind KIND, bool COUNT, class Load, class Store, class RootOf = SceneRoot, int SHORT = kShortStack>
+template <TraceKind KIND, bool COUNT, class Load, class Store, class RootOf = SceneRoot, int SHORT = kShortStack,
+          bool SPREAD = KIND == kTraceMixed>
 __device__ __forceinline__ void trace_persistent(const BvhView& bvh, unsigned n, unsigned* next, Load load,
                                                  Store store, unsigned long long& n_interior,
                                                  unsigned long long& n_tris, unsigned& status_or,
@@ -345,6 +346,16 @@ __device__ __forceinline__ void trace_persistent(const BvhView& bvh, unsigned n,
     constexpr int kTriSteps = 4;      // triangles per vote (a leaf of the builder's holds at most 4)
     constexpr int kLeafShare = 3;     // leaves step when at least 1 / kLeafShare of the busy lanes hold one
     const int lane = threadIdx.x & 31;
+    // SPREAD: with fewer rays than lanes, every warp takes its share instead
+    // of some warps 32: what remains is the longest rays' chain of steps, and
+    // a warp with fewer rays takes each step sooner (frames and adjoints
+    // 2-3 %).  Off in the kernels for long queues, where it costs 3 %.
+    int cap = 32, refill_below = kRefillBelow;
+    if (SPREAD) {
+        const unsigned warps = gridDim.x * (blockDim.x >> 5);
+        cap = (int)min(32u, max(1u, (n + warps - 1) / warps));
+        if (cap < 32) refill_below = max(1, cap * 3 / 4);
+    }
     __shared__ int2 s_stack[SHORT * kTraceMaxBlock];
     TraceStack<SHORT> stack;
     stack.sh = s_stack + threadIdx.x;
@@ -358,7 +369,7 @@ __device__ __forceinline__ void trace_persistent(const BvhView& bvh, unsigned n,
         // stretches run with many lanes (possibly several rounds when roots
         // are missed).
         for (;;) {
-            const bool idle = L.cnt < 0;
+            const bool idle = L.cnt < 0 && (!SPREAD || lane < cap);
             if (have && idle) {
                 status_or |= (unsigned)L.status;
                 if (COUNT) {
@@ -395,7 +406,7 @@ __device__ __forceinline__ void trace_persistent(const BvhView& bvh, unsigned n,
             const unsigned nodes = __ballot_sync(kFull, L.cnt == 0);
             const unsigned leaves = __ballot_sync(kFull, L.cnt > 0);
             const int busy = __popc(nodes | leaves);
-            if (busy < kRefillBelow && (!drained || busy == 0)) break;
+            if (busy < refill_below && (!drained || busy == 0)) break;
             if (kLeafShare * __popc(leaves) >= busy) {
 #pragma unroll
                 for (int x = 0; x < kTriSteps; x++)
