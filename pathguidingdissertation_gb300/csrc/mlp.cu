@@ -2,21 +2,23 @@
 // training (forward, loss, backward on tcgen05, Adam) and the C API
 // (pgx_mlp_*).  The network and its mixture are defined in pgx_mlp.cuh.
 //
-// Training kernel, per 128-row tile of samples and per CTA:
-//   forward: six MMAs chains as in inference, keeping every layer's input
+// Training kernel, per 128-row tile of samples and per CTA (512 threads, four
+// per row: each takes a quarter of the encoding, of every epilogue's columns
+// and of the mixture's lobes):
+//   forward: six MMA chains as in inference, keeping every layer's input
 //            tile X_l in shared memory (plus a constant-one feature column
 //            after its last feature, so the weight-gradient MMA also yields
 //            the bias gradient);
-//   loss:    each thread turns its row's 40 outputs into dLoss/dOutput
-//            (bf16, the tile dY);
+//   loss:    the row's 40 outputs become dLoss/dOutput (bf16, the tile dY);
 //   backward, l = 5..0:
+//            dX = dY W_l            (l > 0; W_l's image read MN-major)
 //            dW_l^T += X_l^T dY     (M = 128 input features incl. padding,
 //                                    N = 64 outputs, K = 128 rows; both
 //                                    operands read MN-major from the
 //                                    row-major tiles; accumulated in tensor
 //                                    memory across all tiles of the CTA)
-//            dX = dY W_l            (l > 0; W_l's image read MN-major)
-//            dY = dX * (X_l > 0)    (ReLU derivative, bf16)
+//            dY = dX * (X_l > 0)    (ReLU derivative, bf16; into the other of
+//                                    two dY tiles, so dW runs under it)
 // and finally each CTA adds its weight gradients to the global FP32
 // gradient with one atomic per entry.
 #include <cmath>
@@ -169,48 +171,63 @@ __global__ void __launch_bounds__(kThreads) k_query(const uint8_t* __restrict__ 
 }
 
 // ---- training -----------------------------------------------------------------------------
-// Shared memory: X_0 (11 chunks), X_1..X_5 (9 chunks each), dY (8 chunks),
-// weight images, biases.  The weight-gradient MMA reads 16 chunks from each
-// X_l; for X_5 the last 7 fall into dY, which is inside the allocation.
+// Shared memory: X_0 (11 chunks), X_1..X_5 (9 chunks each), dY twice (8 chunks
+// each), weight images, biases, the lobes' densities.  The weight-gradient MMA
+// reads 16 chunks from each X_l; for X_5 the last 7 fall into dY, which is
+// inside the allocation (their rows of the product are never read).
 constexpr int kX0Chunks = kIn / 8 + 1;
 constexpr int kXChunks = kHid / 8 + 1;
 __host__ __device__ constexpr int x_offset(int l) { return l == 0 ? 0 : (kX0Chunks + (l - 1) * kXChunks) * kChunk; }
 constexpr int kDyOffset = x_offset(kLayers);
-constexpr int kTrainWOffset = kDyOffset + (kHid / 8) * kChunk;
-constexpr int kTrainSmem = kTrainWOffset + kImageBytes + kBiasFloats * 4;
+constexpr int kDyBytes = (kHid / 8) * kChunk;
+constexpr int kTrainWOffset = kDyOffset + 2 * kDyBytes;
+constexpr int kTrainVOffset = kTrainWOffset + kImageBytes + kBiasFloats * 4;
+constexpr int kTrainSmem = kTrainVOffset + kRows * kLobes * 4;
 static_assert(x_offset(kLayers - 1) + 16 * kChunk <= kTrainWOffset, "weight-gradient reads stay in the tiles");
 static_assert(kTrainSmem <= 227 * 1024, "training tile fits in shared memory");
 constexpr uint32_t kTrainCols = 512;  // 64 (forward / dX) + 6 x 64 (dW^T)
+// Four threads per row.  With one (128 threads, a warp per scheduler) every
+// epilogue and the loss ran at the latency of one dependent chain: 278 us per
+// 262,144 samples.
+constexpr int kTrainParts = 4;
+constexpr int kTrainThreads = kRows * kTrainParts;
+constexpr int kPartCols = kHid / kTrainParts;
+constexpr int kPartLobes = kLobes / kTrainParts;
 
 // Sample record: position, normal, wo, wi, weight (13 floats).
 constexpr int kSampleFloats = 13;
 
-__global__ void __launch_bounds__(kThreads, 1) k_train(const uint8_t* __restrict__ image, Bounds bnd,
-                                                       const float* __restrict__ samples, int64_t n,
-                                                       const double* __restrict__ wsum, float* __restrict__ grad,
-                                                       double* __restrict__ loss_out, int* status) {
+// Makes the CTA's shared-memory writes visible to the tensor core and orders
+// them before the MMA issue; true when any thread's last wait ran out.
+__device__ __forceinline__ bool publish_all(bool failed) {
+    tc::fence_async_smem();
+    tc::fence_before_sync();
+    failed = __syncthreads_or(failed ? 1 : 0) != 0;
+    tc::fence_after_sync();
+    return failed;
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1) k_train(const uint8_t* __restrict__ image, Bounds bnd,
+                                                            const float* __restrict__ samples, int64_t n,
+                                                            const double* __restrict__ wsum, float* __restrict__ grad,
+                                                            double* __restrict__ loss_out, int* status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tslot;
-    __shared__ int flag;
-    const int t = threadIdx.x, warp = t >> 5;
+    const int t = threadIdx.x, row = t & (kRows - 1), part = t / kRows;  // uniform part per warp
+    const uint32_t lane0 = (uint32_t)((t >> 5) & 3) * 32;                // the warp's TMEM lanes
     FwdSmem s;
     s.w = smem + kTrainWOffset;
     s.bias = reinterpret_cast<float*>(smem + kTrainWOffset + kImageBytes);
-    s.act = smem + x_offset(0);
     s.mbar = &mbar;
-    s.flag = &flag;
-    s.bar = 1;
-    s.tg = t;
-    uint8_t* xs[kLayers];
-    for (int l = 0; l < kLayers; l++) xs[l] = smem + x_offset(l);
-    uint8_t* dy = smem + kDyOffset;
+    auto xs = [&](int l) { return smem + x_offset(l); };
+    float* dens = reinterpret_cast<float*>(smem + kTrainVOffset);  // [row][lobe]
     load_weights(image, s.w, s.bias);
     // constant-one feature after each tile's last feature (never read by the
     // forward MMAs, which stop at K)
-    for (int l = 0; l < kLayers; l++) {
+    for (int l = part; l < kLayers; l += kTrainParts) {
         float one[8] = {1.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        store_chunk(xs[l], t, layer_k(l) / 8, one);
+        store_chunk(xs(l), row, layer_k(l) / 8, one);
     }
     if (t == 0) tc::mbar_init(&mbar, 1);
     if (t < 32) {
@@ -225,52 +242,144 @@ __global__ void __launch_bounds__(kThreads, 1) k_train(const uint8_t* __restrict
     uint32_t phase = 0;
     bool first = true, failed = false;
     double loss_acc = 0.0;
+    auto wait = [&]() {
+        failed |= !tc::mbar_wait(&mbar, phase, kWaitPolls);
+        phase ^= 1u;
+        tc::fence_after_sync();
+    };
     const int64_t ntiles = (n + kRows - 1) / kRows;
-    for (int64_t tile = blockIdx.x; tile < ntiles && !failed; tile += gridDim.x) {
-        const int64_t r = tile * kRows + t;
+    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int64_t r = tile * kRows + row;
         const bool live = r < n;
-        F3 x = zero3(), nn = zero3(), wo = zero3(), wi = f3(0.f, 0.f, 1.f);
+        const float* sm = samples + r * kSampleFloats;
+        F3 wi = f3(0.f, 0.f, 1.f);
         float wgt = 0.f;
         if (live) {
-            const float* p = samples + r * kSampleFloats;
-            x = f3(p[0], p[1], p[2]);
-            nn = f3(p[3], p[4], p[5]);
-            wo = f3(p[6], p[7], p[8]);
-            wi = f3(p[9], p[10], p[11]);
-            wgt = p[12];
+            wi = f3(sm[9], sm[10], sm[11]);
+            wgt = sm[12];
         }
-        encode_row(s.act, t, bnd, x, nn, wo);
-        float raw[kOut];
-        if (!forward_tile(s, phase, raw, xs)) {
-            failed = true;
-            break;
+        if (part < 3) {
+            encode_axis(xs(0), row, part, bnd, live ? sm[part] : 0.f);
+        } else {
+            float tail[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (live)
+                for (int j = 0; j < 6; j++) tail[j] = sm[3 + j];
+            store_chunk(xs(0), row, 9, tail);
         }
-        float d[kOut];
-        float l = loss_grad(raw, wi, wgt * scale, d);
-        if (live) loss_acc += (double)l;
-        {
-            float v[8];
+        // ---- forward
+        for (int l = 0; l < kLayers; l++) {  // left by all threads together
+            if ((failed = publish_all(failed))) break;
+            if (t == 0) issue_layer(s, l, xs(l));
+            wait();
+            if (l == kLayers - 1) break;
+            uint32_t acc[kPartCols];
+            tc::tmem_ld16(tc::tmem_at(s.tmem, lane0, kPartCols * part), acc);
+            tc::tmem_ld_wait();
+            const float* b = s.bias + l * kHid + kPartCols * part;
 #pragma unroll
-            for (int c = 0; c < kHid / 8; c++) {
+            for (int c = 0; c < kPartCols / 8; c++) {
+                float v[8];
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    int f = 8 * c + j;
-                    v[j] = (live && f < kOut) ? d[f] : 0.f;
-                }
-                store_chunk(dy, t, c, v);
+                for (int j = 0; j < 8; j++) v[j] = fmaxf(__uint_as_float(acc[8 * c + j]) + b[8 * c + j], 0.f);
+                store_chunk(xs(l + 1), row, kPartCols / 8 * part + c, v);
             }
         }
-        for (int lay = kLayers - 1; lay >= 0; lay--) {
-            publish_smem(s.bar);
-            if (t == 0) {
-                // dW^T (+)= X^T dY
-                const uint32_t xa = tc::smem_addr(xs[lay]), ya = tc::smem_addr(dy);
-                const uint32_t id_w = tc::idesc_bf16(kRows, kHid, true, true);
-                for (int k = 0; k < kRows / 16; k++) {
-                    uint64_t ad = tc::smem_desc(xa + k * 256, 128, kChunk);
-                    uint64_t bd = tc::smem_desc(ya + k * 256, 128, kChunk);
-                    tc::mma_bf16(s.tmem + kHid + kHid * lay, ad, bd, id_w, !(first && k == 0));
+        // ---- loss: every thread computes the lobe weights, and its own two
+        // lobes' densities and gradients
+        float raw[kOut];
+        tc::tmem_ld32(tc::tmem_at(s.tmem, lane0, 0), raw);
+        {
+            uint32_t k8[8];
+            tc::tmem_ld8(tc::tmem_at(s.tmem, lane0, 32), k8);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; j++) raw[32 + j] = __uint_as_float(k8[j]);
+        }
+        const float* b = s.bias + (kLayers - 1) * kHid;
+        float w[kLobes];
+        float mx = -FLT_MAX, sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < kLobes; i++) {
+            w[i] = raw[i] + b[i];
+            mx = i == 0 ? w[0] : fmaxf(mx, w[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < kLobes; i++) {
+            w[i] = expf(w[i] - mx);
+            sum += w[i];
+        }
+        const float inv = 1.f / sum;
+#pragma unroll
+        for (int i = 0; i < kLobes; i++) w[i] *= inv;
+        float4 lobe[kPartLobes];
+        float len[kPartLobes], rk[kPartLobes], own[kPartLobes];
+#pragma unroll
+        for (int i = 0; i < kPartLobes; i++) {
+            const int f = 8 + 3 * (kPartLobes * part + i);
+            float a = 0.f, bb = 0.f, c = 0.f, kr = 0.f;
+#pragma unroll
+            for (int j = 0; j < kTrainParts; j++)  // constant indexes: raw stays in registers
+                if (j == part) {
+                    const int m = kPartLobes * j + i;
+                    a = raw[8 + 3 * m], bb = raw[9 + 3 * m], c = raw[10 + 3 * m], kr = raw[32 + m];
                 }
+            a += b[f], bb += b[f + 1], c += b[f + 2];
+            rk[i] = kr + b[32 + kPartLobes * part + i];
+            len[i] = sqrtf(a * a + bb * bb + c * c);
+            float il = len[i] > 1e-20f ? 1.f / len[i] : 0.f;
+            if (len[i] <= 1e-20f) c = 1.f, il = 1.f;
+            lobe[i] = make_float4(a * il, bb * il, c * il, softplus(rk[i]) + kKappaMin);
+            own[i] = vmf_pdf(lobe[i], wi);
+            dens[row * kLobes + kPartLobes * part + i] = own[i];
+        }
+        __syncthreads();
+        float q = 0.f;
+        {
+            const float4 v0 = *reinterpret_cast<const float4*>(dens + row * kLobes);
+            const float4 v1 = *reinterpret_cast<const float4*>(dens + row * kLobes + 4);
+            const float v[kLobes] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+            for (int i = 0; i < kLobes; i++) q += w[i] * v[i];
+        }
+        q = fmaxf(q, 1e-30f);
+        const float wl = wgt * scale;
+        if (live && part == 0) loss_acc += (double)(-wl * logf(q));
+        uint8_t* dy = smem + kDyOffset;
+        {
+            const float g = -wl / q;  // d loss / d q
+            float d[5 * kPartLobes];  // d loss / d (the lobes' logits, means, concentrations)
+#pragma unroll
+            for (int i = 0; i < kPartLobes; i++) {
+                float wi_w = 0.f;
+#pragma unroll
+                for (int j = 0; j < kTrainParts; j++)  // constant indexes: w stays in registers
+                    if (j == part) wi_w = w[kPartLobes * j + i];
+                const float k = lobe[i].w, vi = own[i];
+                const float cosv = lobe[i].x * wi.x + lobe[i].y * wi.y + lobe[i].z * wi.z;
+                const float sg = len[i] > 1e-20f ? g * wi_w * vi * k / len[i] : 0.f;
+                const float dlk = 1.f / k - 2.f / expm1f(2.f * k) + (cosv - 1.f);
+                const float sig = 1.f / (1.f + expf(-rk[i]));
+                d[i] = g * wi_w * (vi - q);
+                d[kPartLobes + 3 * i] = sg * (wi.x - cosv * lobe[i].x);
+                d[kPartLobes + 3 * i + 1] = sg * (wi.y - cosv * lobe[i].y);
+                d[kPartLobes + 3 * i + 2] = sg * (wi.z - cosv * lobe[i].z);
+                d[4 * kPartLobes + i] = g * wi_w * vi * dlk * sig;
+            }
+            auto put2 = [&](int f, float a, float c) {  // features f, f + 1 (f even)
+                *reinterpret_cast<uint32_t*>(dy + (f >> 3) * kChunk + row * 16 + (f & 7) * 2) =
+                    live ? pack_bf16x2(a, c) : 0u;
+            };
+            put2(kPartLobes * part, d[0], d[1]);
+#pragma unroll
+            for (int j = 0; j < 3; j++) put2(8 + 3 * kPartLobes * part + 2 * j, d[2 + 2 * j], d[3 + 2 * j]);
+            put2(32 + kPartLobes * part, d[8], d[9]);
+            if (part < 3) *reinterpret_cast<uint4*>(dy + (5 + part) * kChunk + row * 16) = make_uint4(0, 0, 0, 0);
+        }
+        // ---- backward
+        for (int lay = kLayers - 1; lay >= 0; lay--) {
+            if ((failed = publish_all(failed))) break;
+            if (t == 0) {
+                const uint32_t ya = tc::smem_addr(dy);
                 if (lay > 0) {
                     // dX = dY W
                     const uint32_t wa = tc::smem_addr(s.w + image_offset(lay));
@@ -280,60 +389,85 @@ __global__ void __launch_bounds__(kThreads, 1) k_train(const uint8_t* __restrict
                         uint64_t bd = tc::smem_desc(wa + k * 256, 128, kHid * 16);
                         tc::mma_bf16(s.tmem, ad, bd, id_x, k > 0);
                     }
+                    tc::mma_commit(&mbar);
                 }
-                tc::mma_commit(&mbar);
-            }
-            if (!group_wait(s, phase)) {
-                failed = true;
-                break;
-            }
-            if (lay > 0) {
-                float acc[64];
-                tc::tmem_ld32(tc::tmem_at(s.tmem, warp * 32, 0), acc);
-                tc::tmem_ld32(tc::tmem_at(s.tmem, warp * 32, 32), acc + 32);
-#pragma unroll
-                for (int c = 0; c < kHid / 8; c++) {
-                    float xv[8], v[8];
-                    load_chunk(xs[lay], t, c, xv);
-#pragma unroll
-                    for (int j = 0; j < 8; j++) v[j] = xv[j] > 0.f ? acc[8 * c + j] : 0.f;
-                    store_chunk(dy, t, c, v);
+                // dW^T (+)= X^T dY, under the next epilogue
+                const uint32_t xa = tc::smem_addr(xs(lay));
+                const uint32_t id_w = tc::idesc_bf16(kRows, kHid, true, true);
+                for (int k = 0; k < kRows / 16; k++) {
+                    uint64_t ad = tc::smem_desc(xa + k * 256, 128, kChunk);
+                    uint64_t bd = tc::smem_desc(ya + k * 256, 128, kChunk);
+                    tc::mma_bf16(s.tmem + kHid + kHid * lay, ad, bd, id_w, !(first && k == 0));
                 }
+                // layer 0 ends the tile: its inputs are overwritten next
+                if (lay == 0) tc::mma_commit(&mbar);
             }
-            tc::fence_before_sync();
+            wait();
+            if (lay == 0) break;
+            // The MMAs of the layer above, which read the other dY tile,
+            // precede this layer's dX and have completed with it.
+            uint8_t* dy_next = smem + kDyOffset + (dy == smem + kDyOffset ? kDyBytes : 0);
+            uint32_t acc[kPartCols];
+            tc::tmem_ld16(tc::tmem_at(s.tmem, lane0, kPartCols * part), acc);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < kPartCols / 8; c++) {
+                float xv[8], v[8];
+                load_chunk(xs(lay), row, kPartCols / 8 * part + c, xv);
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = xv[j] > 0.f ? __uint_as_float(acc[8 * c + j]) : 0.f;
+                store_chunk(dy_next, row, kPartCols / 8 * part + c, v);
+            }
+            dy = dy_next;
         }
+        failed = __syncthreads_or(failed ? 1 : 0) != 0;
+        if (failed) break;
         first = false;
     }
     if (failed) {
         if (t == 0) atomicAdd(status, 1);
     } else if (!first) {
-        // this CTA's weight gradients: row t of dW_l^T is input feature t
+        // this CTA's weight gradients: row r of dW_l^T is input feature r
         for (int lay = 0; lay < kLayers; lay++) {
             const int K = layer_k(lay), N = layer_n(lay);
-            float acc[64];
-            tc::tmem_ld32(tc::tmem_at(s.tmem + kHid + kHid * lay, warp * 32, 0), acc);
-            tc::tmem_ld32(tc::tmem_at(s.tmem + kHid + kHid * lay, warp * 32, 32), acc + 32);
-            if (t < K) {
-                for (int j = 0; j < N; j++) atomicAdd(&grad[param_w(lay) + j * K + t], acc[j]);
-            } else if (t == K) {
-                for (int j = 0; j < N; j++) atomicAdd(&grad[param_b(lay) + j], acc[j]);
+            uint32_t acc[kPartCols];
+            tc::tmem_ld16(tc::tmem_at(s.tmem + kHid + kHid * lay, lane0, kPartCols * part), acc);
+            tc::tmem_ld_wait();
+            const int j0 = kPartCols * part, j1 = min(N, j0 + kPartCols);
+#pragma unroll
+            for (int j = 0; j < kPartCols; j++) {
+                if (j0 + j >= j1) continue;
+                if (row < K)
+                    atomicAdd(&grad[param_w(lay) + (j0 + j) * K + row], __uint_as_float(acc[j]));
+                else if (row == K)
+                    atomicAdd(&grad[param_b(lay) + j0 + j], __uint_as_float(acc[j]));
             }
         }
     }
-    // loss: warp sums, one atomic per warp
-    for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
-    if ((t & 31) == 0) atomicAdd(loss_out, loss_acc);
+    // loss: warp sums of part 0, one atomic per warp
+    if (part == 0) {
+        for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
+        if ((t & 31) == 0) atomicAdd(loss_out, loss_acc);
+    }
     tc::fence_before_sync();
     __syncthreads();
     if (t < 32) tc::tmem_dealloc(s.tmem, kTrainCols);
 }
 
-__global__ void k_weight_sum(const float* __restrict__ samples, int64_t n, double* out) {
+// One atomic per block: one per warp put 8,192 of them on one address.
+__global__ void __launch_bounds__(512) k_weight_sum(const float* __restrict__ samples, int64_t n, double* out) {
+    __shared__ double s_sum[16];
     double acc = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         acc += (double)samples[i * kSampleFloats + 12];
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(out, acc);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        acc = s_sum[threadIdx.x];
+        for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffu, acc, o);
+        if (threadIdx.x == 0) atomicAdd(out, acc);
+    }
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master parameters.
@@ -410,11 +544,11 @@ int mlp_train_device(pgx_ctx* ctx, const float* samples, int64_t n, float lr, do
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(st->loss.p, 0, 2 * sizeof(double), s));
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(st->status.p, 0, sizeof(int), s));
     double* d_loss = st->loss.as<double>();
-    k_weight_sum<<<std::min<int64_t>(1024, (n + 255) / 256), 256, 0, s>>>(samples, n, d_loss + 1);
+    k_weight_sum<<<(unsigned)std::min<int64_t>(2 * st->sms, (n + 511) / 512), 512, 0, s>>>(samples, n, d_loss + 1);
     PGX_CUDA_TRY(ctx, cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem));
     const int64_t ntiles = (n + kRows - 1) / kRows;
     const int grid = (int)std::min<int64_t>(ntiles, st->sms);
-    k_train<<<grid, kThreads, kTrainSmem, s>>>(st->image.as<uint8_t>(), st->bounds, samples, n, d_loss + 1,
+    k_train<<<grid, kTrainThreads, kTrainSmem, s>>>(st->image.as<uint8_t>(), st->bounds, samples, n, d_loss + 1,
                                                st->grad.as<float>(), d_loss, st->status.as<int>());
     PGX_CUDA_TRY(ctx, cudaGetLastError());
     if (update) {

@@ -81,31 +81,34 @@ __device__ __forceinline__ void load_chunk(const uint8_t* tile, int r, int c, fl
     v[4] = bf16_lo(q.z), v[5] = bf16_hi(q.z), v[6] = bf16_lo(q.w), v[7] = bf16_hi(q.w);
 }
 
-// The 80 input features of one query, written as bf16 into row r of the
-// layer-0 tile.
-__device__ __forceinline__ void encode_row(uint8_t* tile, int r, const Bounds& b, F3 x, F3 n, F3 wo) {
-    float p[3] = {x.x, x.y, x.z};
+// The 24 features of one position coordinate (axis c), written as bf16 into
+// row r of the layer-0 tile.
+__device__ __forceinline__ void encode_axis(uint8_t* tile, int r, int c, const Bounds& b, float p) {
+    float t = (p - b.bmin[c]) * b.inv_ext[c];
+    t = fminf(fmaxf(t, 0.f), 1.f);
+    float v[24];
+    // sin/cos of 2^j pi t by the double-angle recurrence from j = 0
+    // (absolute error below 2^j ulp, far under the bf16 step of 2^-8)
+    float sn, cs;
+    sincospif(t, &sn, &cs);
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        float t = (p[c] - b.bmin[c]) * b.inv_ext[c];
-        t = fminf(fmaxf(t, 0.f), 1.f);
-        float v[24];
-        // sin/cos of 2^j pi t by the double-angle recurrence from j = 0
-        // (absolute error below 2^j ulp, far under the bf16 step of 2^-8)
-        float sn, cs;
-        sincospif(t, &sn, &cs);
-#pragma unroll
-        for (int j = 0; j < kFreq; j++) {
-            v[2 * j] = sn;
-            v[2 * j + 1] = cs;
-            float s2 = 2.f * sn * cs;
-            cs = (cs - sn) * (cs + sn);
-            sn = s2;
-        }
-        store_chunk(tile, r, 3 * c, v);
-        store_chunk(tile, r, 3 * c + 1, v + 8);
-        store_chunk(tile, r, 3 * c + 2, v + 16);
+    for (int j = 0; j < kFreq; j++) {
+        v[2 * j] = sn;
+        v[2 * j + 1] = cs;
+        float s2 = 2.f * sn * cs;
+        cs = (cs - sn) * (cs + sn);
+        sn = s2;
     }
+    store_chunk(tile, r, 3 * c, v);
+    store_chunk(tile, r, 3 * c + 1, v + 8);
+    store_chunk(tile, r, 3 * c + 2, v + 16);
+}
+
+// The 80 input features of one query.
+__device__ __forceinline__ void encode_row(uint8_t* tile, int r, const Bounds& b, F3 x, F3 n, F3 wo) {
+    encode_axis(tile, r, 0, b, x.x);
+    encode_axis(tile, r, 1, b, x.y);
+    encode_axis(tile, r, 2, b, x.z);
     float tail[8] = {n.x, n.y, n.z, wo.x, wo.y, wo.z, 0.f, 0.f};
     store_chunk(tile, r, 9, tail);
 }
@@ -248,42 +251,6 @@ __device__ __forceinline__ F3 packed_sample(const float4* __restrict__ g, float 
     return normalize(t * (sw * c) + bt * (sw * s) + mu * cw);
 }
 
-// Loss of one training sample, -weight * log q(wi), and its gradient with
-// respect to the 40 raw outputs (d[40]).
-__device__ __forceinline__ float loss_grad(const float* raw, F3 wi, float weight, float* d) {
-    Mixture m;
-    mixture_from_raw(raw, m);
-    float v[kLobes];
-    float q = 0.f;
-#pragma unroll
-    for (int i = 0; i < kLobes; i++) {
-        v[i] = vmf_pdf(m.lobe[i], wi);
-        q += m.w[i] * v[i];
-    }
-    q = fmaxf(q, 1e-30f);
-    float g = -weight / q;  // d loss / d q
-#pragma unroll
-    for (int i = 0; i < kLobes; i++) {
-        // softmax logits
-        d[i] = g * m.w[i] * (v[i] - q);
-        // mean direction: d v / d m = v kappa (wi - (mu.wi) mu) / |m|
-        float a = raw[8 + 3 * i], b = raw[9 + 3 * i], c = raw[10 + 3 * i];
-        float len = sqrtf(a * a + b * b + c * c);
-        float k = m.lobe[i].w;
-        float cosv = m.lobe[i].x * wi.x + m.lobe[i].y * wi.y + m.lobe[i].z * wi.z;
-        float s = len > 1e-20f ? g * m.w[i] * v[i] * k / len : 0.f;
-        d[8 + 3 * i] = s * (wi.x - cosv * m.lobe[i].x);
-        d[9 + 3 * i] = s * (wi.y - cosv * m.lobe[i].y);
-        d[10 + 3 * i] = s * (wi.z - cosv * m.lobe[i].z);
-        // concentration: d log v / d kappa = 1/kappa - 2/(e^{2 kappa} - 1) + cos - 1
-        float dlk = 1.f / k - 2.f / expm1f(2.f * k) + (cosv - 1.f);
-        float r = raw[32 + i];
-        float sig = 1.f / (1.f + expf(-r));
-        d[32 + i] = g * m.w[i] * v[i] * dlk * sig;
-    }
-    return -weight * logf(q);
-}
-
 // ---- one forward pass of a 128-row tile on the tensor cores ------------------------
 // A tile is processed by a group of 128 threads (4 warps; thread t of the
 // group owns row t, and its warp reads TMEM lanes 32 * (warp % 4) ..).  A CTA
@@ -343,17 +310,13 @@ __device__ __forceinline__ bool group_wait(const FwdSmem& s, uint32_t& phase) {
 // Runs the six layers on the tile already encoded in s.act; thread tg of
 // the group receives row tg's 40 raw outputs.  `phase` is the mbarrier
 // parity to wait for next (updated).  Returns false if an MMA did not
-// complete in time (uniform across the group).  When keep_acts is given,
-// layer l's input tile is s.act for l = 0 and keep_acts[l] for l > 0 (each
-// kIn/8 or kHid/8 + 1 chunks), and is left in place for a backward pass.
-__device__ __forceinline__ bool forward_tile(const FwdSmem& s, uint32_t& phase, float* out,
-                                             uint8_t* const* keep_acts = nullptr) {
+// complete in time (uniform across the group).
+__device__ __forceinline__ bool forward_tile(const FwdSmem& s, uint32_t& phase, float* out) {
     const int t = s.tg;
     const int warp = t >> 5;
     for (int l = 0; l < kLayers; l++) {
-        uint8_t* in = (l == 0 || !keep_acts) ? s.act : keep_acts[l];
         publish_smem(s.bar);
-        if (t == 0) issue_layer(s, l, in);
+        if (t == 0) issue_layer(s, l, s.act);
         if (!group_wait(s, phase)) return false;
         const float* b = s.bias + l * kHid;
         // two halves of 32 accumulator columns, to keep registers low
@@ -362,14 +325,13 @@ __device__ __forceinline__ bool forward_tile(const FwdSmem& s, uint32_t& phase, 
             float acc[32];
             tc::tmem_ld32(tc::tmem_at(s.tmem, warp * 32, 32 * half), acc);
             if (l < kLayers - 1) {
-                uint8_t* dst = keep_acts ? keep_acts[l + 1] : s.act;
                 // the MMA that read s.act has completed, so it may be overwritten
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     float v[8];
 #pragma unroll
                     for (int j = 0; j < 8; j++) v[j] = fmaxf(acc[8 * c + j] + b[32 * half + 8 * c + j], 0.f);
-                    store_chunk(dst, t, 4 * half + c, v);
+                    store_chunk(s.act, t, 4 * half + c, v);
                 }
             } else {
 #pragma unroll
