@@ -80,14 +80,43 @@ __device__ __forceinline__ int longest_axis(const pgx_cache_node& n) {
     return ax;
 }
 
-// Positions of the input records, each with its record index in w (at least
-// one block of 256 threads runs).
-__global__ void k_pos(const pgx_path_vertex* __restrict__ r, int64_t n, float4* __restrict__ pos,
-                      int* __restrict__ acc) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 6) acc[i] = i < 3 ? INT_MAX : INT_MIN;  // for k_root_bounds
-    if (i >= n) return;
-    pos[i] = make_float4(r[i].position[0], r[i].position[1], r[i].position[2], __int_as_float((int)i));
+__global__ void k_bounds_init(int* acc) {
+    if (threadIdx.x < 6) acc[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
+}
+
+// Positions of the input records, each with its record index in w, and their
+// bounds (ordered ints; one atomic per block and side).
+__global__ void __launch_bounds__(256) k_pos(const pgx_path_vertex* __restrict__ r, int64_t n, float4* __restrict__ pos,
+                                             int* __restrict__ acc) {
+    __shared__ int s_acc[6];
+    if (threadIdx.x < 6) s_acc[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
+    __syncthreads();
+    int a[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float4 p = *reinterpret_cast<const float4*>(r + i);  // 48-byte records: 16-byte aligned
+        pos[i] = make_float4(p.x, p.y, p.z, __int_as_float((int)i));
+        a[0] = min(a[0], f2o(p.x));
+        a[1] = min(a[1], f2o(p.y));
+        a[2] = min(a[2], f2o(p.z));
+        a[3] = max(a[3], f2o(p.x));
+        a[4] = max(a[4], f2o(p.y));
+        a[5] = max(a[5], f2o(p.z));
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        const int v = k < 3 ? __reduce_min_sync(0xFFFFFFFFu, a[k]) : __reduce_max_sync(0xFFFFFFFFu, a[k]);
+        if ((threadIdx.x & 31) == 0) {
+            if (k < 3)
+                atomicMin(&s_acc[k], v);
+            else
+                atomicMax(&s_acc[k], v);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3)
+        atomicMin(&acc[threadIdx.x], s_acc[threadIdx.x]);
+    else if (threadIdx.x < 6)
+        atomicMax(&acc[threadIdx.x], s_acc[threadIdx.x]);
 }
 
 // An item of the level-by-level phase, ready for its first select pass.
@@ -105,7 +134,7 @@ __device__ __forceinline__ void start_item(PItem& it, int node, int offset, int 
 }
 
 __global__ void k_root(int64_t n, PMisc* misc, pgx_cache_node* nodes, PItem* items, int2* small, int* acc) {
-    // acc: 6 ordered ints reduced by k_root_bounds
+    // acc: 6 ordered ints reduced by k_pos
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     pgx_cache_node& r = nodes[0];
     for (int k = 0; k < 3; k++) {
@@ -126,32 +155,6 @@ __global__ void k_root(int64_t n, PMisc* misc, pgx_cache_node* nodes, PItem* ite
         return;
     }
     start_item(items[0], 0, 0, (int)n, r);
-}
-
-__global__ void k_root_bounds(const float4* __restrict__ pos, int64_t n, int* acc) {
-    int a[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        float4 p = pos[i];
-        a[0] = min(a[0], f2o(p.x));
-        a[1] = min(a[1], f2o(p.y));
-        a[2] = min(a[2], f2o(p.z));
-        a[3] = max(a[3], f2o(p.x));
-        a[4] = max(a[4], f2o(p.y));
-        a[5] = max(a[5], f2o(p.z));
-    }
-    for (int k = 0; k < 6; k++) {
-        int v = a[k];
-        for (int o = 16; o > 0; o >>= 1) {
-            int w = __shfl_xor_sync(0xFFFFFFFFu, v, o);
-            v = k < 3 ? min(v, w) : max(v, w);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            if (k < 3)
-                atomicMin(&acc[k], v);
-            else
-                atomicMax(&acc[k], v);
-        }
-    }
 }
 
 // True in the block that finishes an item's last chunk: everything the other
@@ -401,11 +404,15 @@ __global__ void __launch_bounds__(kThreads) k_ppart(PItem* __restrict__ items, u
 // slot's upper half (used - used/2 <= S/2, so both always fit).  A slot whose
 // node is a leaf (at most 8 records) sorts too, which keeps the network
 // uniform, and keeps its records in its lower places.
-//   Bound: the network's shared-memory passes (about 276 compare steps for
-// 2,048 records); one thread per <= 256-record subtree with an in-place
-// quickselect took 5.1 ms for 0.9 M records.
+//   A thread holds four neighbouring places in registers: strides of 1 and 2
+// stay in the thread, 4 to 64 are shuffles, and only the 20 of 276 compare
+// steps with longer strides go through shared memory.
+//   Bound: issue of the network (0.9 M records: 0.33 ms with every step in
+// shared memory).  One thread per <= 256-record subtree with an in-place
+// quickselect took 5.1 ms.
 constexpr int kSubThreads = 512;
 constexpr int kSubSlots = kSmall / 8;  // slots of the deepest level
+constexpr int kSubEach = kSmall / kSubThreads;
 constexpr int kSubSmem = kSmall * (int)(sizeof(unsigned long long) + sizeof(float4));
 
 struct SubSlot {
@@ -414,14 +421,14 @@ struct SubSlot {
     int axis;   // -1: leaf or empty
 };
 
-__global__ void __launch_bounds__(kSubThreads) k_psubtree(const int2* __restrict__ small, PMisc* __restrict__ misc,
+__global__ void __launch_bounds__(kSubThreads, 3) k_psubtree(const int2* __restrict__ small, PMisc* __restrict__ misc,
                                                           const float4* __restrict__ pos0,
                                                           const float4* __restrict__ pos1, int* __restrict__ idx,
                                                           pgx_cache_node* __restrict__ nodes,
                                                           int2* __restrict__ regions, int* __restrict__ node_region,
                                                           int region_max) {
     extern __shared__ __align__(16) uint8_t s_dyn[];
-    unsigned long long* key = reinterpret_cast<unsigned long long*>(s_dyn);       // [kSmall] (coordinate, place)
+    unsigned long long* xchg = reinterpret_cast<unsigned long long*>(s_dyn);  // [kSmall]: long strides, then source places
     float4* rec = reinterpret_cast<float4*>(s_dyn + sizeof(unsigned long long) * kSmall);  // [kSmall]
     __shared__ SubSlot slot[2][kSubSlots];
     __shared__ int s_acc[kSubSlots][6];
@@ -465,38 +472,51 @@ __global__ void __launch_bounds__(kSubThreads) k_psubtree(const int2* __restrict
             s_rbase = s_nregion ? atomicAdd(&misc->nregions, s_nregion) : 0;
         }
         // Sort keys of the slots that split; the others keep their order.
-        for (int i = tid; i < P; i += kSubThreads) {
-            const SubSlot& sl = slot[cur][i / S];
-            const int r = i & (S - 1);
-            unsigned k = 0xFFFFFFFFu;
-            if (sl.axis >= 0)
-                k = r < sl.used ? key_of(axis_of(rec[i], sl.axis)) : 0xFFFFFFFFu;
-            else
-                k = 0u;
-            // place breaks ties, and puts records before the empty places
-            key[i] = ((unsigned long long)k << 32) | (unsigned)r;
+        unsigned long long key[kSubEach];
+#pragma unroll
+        for (int e = 0; e < kSubEach; e++) {
+            const int i = tid * kSubEach + e;
+            key[e] = ~0ull;
+            if (i < P) {
+                const SubSlot& sl = slot[cur][i / S];
+                const int r = i & (S - 1);
+                const unsigned k = sl.axis < 0 ? 0u : (r < sl.used ? key_of(axis_of(rec[i], sl.axis)) : 0xFFFFFFFFu);
+                // place breaks ties, and puts records before the empty places
+                key[e] = ((unsigned long long)k << 32) | (unsigned)r;
+            }
         }
-        __syncthreads();
-        bool wide = true;  // whether the previous step crossed warps
         for (int k2 = 2; k2 <= S; k2 <<= 1) {
             for (int j = k2 >> 1; j > 0; j >>= 1) {
-                const bool cross = j > 32;
-                if (cross || wide) __syncthreads();
-                else __syncwarp();
-                wide = cross;
-                for (int p = tid; p < (P >> 1); p += kSubThreads) {
-                    const int i = ((p & ~(j - 1)) << 1) | (p & (j - 1));
-                    const unsigned long long a = key[i], b = key[i + j];
+                unsigned long long other[kSubEach];
+                if (j >= 32 * kSubEach) {  // thread tid ^ (j / kSubEach), another warp
+                    __syncthreads();
+#pragma unroll
+                    for (int e = 0; e < kSubEach; e++) xchg[e * kSubThreads + tid] = key[e];
+                    __syncthreads();
+#pragma unroll
+                    for (int e = 0; e < kSubEach; e++) other[e] = xchg[e * kSubThreads + (tid ^ (j / kSubEach))];
+                } else if (j >= kSubEach) {
+#pragma unroll
+                    for (int e = 0; e < kSubEach; e++) other[e] = __shfl_xor_sync(0xFFFFFFFFu, key[e], j / kSubEach);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < kSubEach; e++) other[e] = j == 2 ? key[e ^ 2] : key[e ^ 1];
+                }
+#pragma unroll
+                for (int e = 0; e < kSubEach; e++) {
+                    const int i = tid * kSubEach + e;
                     // ascending blocks of k2 alternate within a slot; the
                     // slot-wide merge (k2 == S) always ascends
                     const bool up = k2 == S || (i & k2) == 0;
-                    if ((a > b) == up) {
-                        key[i] = b;
-                        key[i + j] = a;
-                    }
+                    const bool keep_min = ((i & j) == 0) == up;
+                    if ((other[e] < key[e]) == keep_min) key[e] = other[e];
                 }
             }
         }
+        int* from_place = reinterpret_cast<int*>(xchg);
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < kSubEach; e++) from_place[tid * kSubEach + e] = (int)(unsigned)key[e];
         __syncthreads();
         // Children into the slot halves: place q of a half takes the record
         // ranked q (left) or used/2 + q (right).
@@ -515,7 +535,7 @@ __global__ void __launch_bounds__(kSubThreads) k_psubtree(const int2* __restrict
                     from = r < half ? r : -1;
                 else
                     from = r - H < sl.used - half ? half + (r - H) : -1;
-                if (from >= 0) moved[m] = rec[(i & ~(S - 1)) + (int)(unsigned)key[(i & ~(S - 1)) + from]];
+                if (from >= 0) moved[m] = rec[(i & ~(S - 1)) + from_place[(i & ~(S - 1)) + from]];
             } else if (r < H) {
                 moved[m] = rec[i];  // a leaf (or an empty slot) stays in the lower half
             }
@@ -682,10 +702,25 @@ __global__ void k_regions(const int2* __restrict__ regions, int nreg, float4* __
     for (int i = threadIdx.x; i < g.y; i += blockDim.x) pos[g.x + i].w = __int_as_float(r);
 }
 
-__device__ __forceinline__ float warp_sum(float v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
+// A float sum with its rounding error carried along (Knuth's two-sum), so
+// that a cell's flux does not depend on the order of its records and the
+// refinement decisions are those of the exact sums.
+struct PairSum {
+    float s = 0.f, e = 0.f;
+    __device__ __forceinline__ void add(float w) {
+        const float t = s + w, z = t - s;
+        e += (s - (t - z)) + (w - z);
+        s = t;
+    }
+    __device__ __forceinline__ void warp_reduce() {
+        for (int o = 16; o > 0; o >>= 1) {
+            const float s2 = __shfl_xor_sync(0xFFFFFFFFu, s, o), e2 = __shfl_xor_sync(0xFFFFFFFFu, e, o);
+            add(s2);
+            e += e2;
+        }
+    }
+    __device__ __forceinline__ float value() const { return s + e; }
+};
 
 // One CTA builds one region's quadtree (pgx_guide.cuh).  The records are
 // sorted once by the Morton key of their cell at the depth limit (four
@@ -774,14 +809,21 @@ __global__ void __launch_bounds__(THREADS) k_quadtree(const int2* __restrict__ r
             lo = mid;
     }
     const float clamp = clamp_median > 0.f ? clamp_median * hi : FLT_MAX;
-    float total = 0.f;
-    for (int i = tid; i < n; i += THREADS) total += fminf(rw[i], clamp);
-    total = warp_sum(total);
+    PairSum sum;
+    for (int i = tid; i < n; i += THREADS) sum.add(fminf(rw[i], clamp));
+    sum.warp_reduce();
     __syncthreads();
-    if (lane == 0) s_f[warp] = total;
+    if (lane == 0) {
+        s_f[warp] = sum.s;
+        s_g[warp] = sum.e;
+    }
     __syncthreads();
-    total = 0.f;
-    for (int w = 0; w < kWarps; w++) total += s_f[w];
+    sum = PairSum{};
+    for (int w = 0; w < kWarps; w++) {
+        sum.add(s_f[w]);
+        sum.e += s_g[w];
+    }
+    const float total = sum.value();
     if (!(total > 0.f) || !isfinite(total)) {
         if (tid == 0) qroot[r] = -1;
         return;
@@ -876,14 +918,15 @@ __global__ void __launch_bounds__(THREADS) k_quadtree(const int2* __restrict__ r
         for (int i = warp; i < 4 * count; i += kWarps) {
             const int ni = i >> 2, c = i & 3;
             const int a = s_beg[ni][c], b = s_beg[ni][c + 1];
-            float f = 0.f;
+            PairSum cell;
             int some = 0;
             for (int k = a + lane; k < b; k += 32) {
                 const float w = wsrc[k];
-                f += w;
+                cell.add(w);
                 some += w > 0.f ? 1 : 0;
             }
-            f = warp_sum(f);
+            cell.warp_reduce();
+            const float f = cell.value();
             some = __reduce_add_sync(0xFFFFFFFFu, some);
             if (lane == 0) {
                 s_flux[ni][c] = f;
@@ -968,20 +1011,35 @@ __global__ void __launch_bounds__(THREADS) k_quadtree(const int2* __restrict__ r
     }
 }
 
-// k nearest records per query (ascending distance, ties to lower index).
-__global__ void k_knn(const CacheTravNode* __restrict__ nodes, const float4* __restrict__ pos, int nrec,
-                      const float* __restrict__ q, int64_t nq, int k, int* __restrict__ out_i,
-                      float* __restrict__ out_d) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nq) return;
-    float x = q[3 * t], y = q[3 * t + 1], z = q[3 * t + 2];
-    float bd[64];
-    int bi[64];
-    int cnt = 0;
-    for (int j = 0; j < k; j++) {
-        bd[j] = FLT_MAX;
-        bi[j] = -1;
+// k nearest records per query (ascending distance, ties to lower index), one
+// warp per query.  The best list lives in the lanes (entry e of lane l is rank
+// 32 e + l, kept sorted); a leaf's records are tested by one lane each and the
+// ones that improve the list are inserted in turn: every lane compares its
+// entries, the insertion point is a popcount, and the tail moves up one lane.
+// The visit order and the comparisons are those of one thread walking the tree
+// with a local list, which took 266 us for 16,384 queries of 8 among 0.9 M
+// records (128 blocks of dependent local-memory accesses).
+template <int E>
+__global__ void __launch_bounds__(128) k_knn(const CacheTravNode* __restrict__ nodes, const float4* __restrict__ pos,
+                                             int nrec, const float* __restrict__ q, int64_t nq, int k,
+                                             int* __restrict__ out_i, float* __restrict__ out_d) {
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    __shared__ int s_stack[4][64];
+    const int lane = threadIdx.x & 31;
+    int* stack = s_stack[threadIdx.x >> 5];
+    const int64_t t = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (t >= nq) return;  // whole warps
+    const float x = q[3 * t], y = q[3 * t + 1], z = q[3 * t + 2];
+    float bd[E];
+    int bi[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        bd[e] = FLT_MAX;
+        bi[e] = INT_MAX;
     }
+    int cnt = 0;
+    float worst_d = FLT_MAX;  // rank k - 1 once k records are known
+    int worst_i = INT_MAX;
     auto worse = [&](float d, int i, float d2, int i2) { return d > d2 || (d == d2 && i > i2); };
     auto box_d = [&](const CacheTravNode& c) {
         float dx = fmaxf(fmaxf(c.bmin.x - x, x - c.bmax.x), 0.f);
@@ -990,47 +1048,88 @@ __global__ void k_knn(const CacheTravNode* __restrict__ nodes, const float4* __r
         return dx * dx + dy * dy + dz * dz;
     };
     if (nrec > 0) {
-        int stack[64];
         int sp = 0;
-        stack[sp++] = 0;
+        if (lane == 0) stack[0] = 0;
+        sp = 1;
         while (sp > 0) {
-            int ni = stack[--sp];
-            CacheTravNode n = nodes[ni];
-            float lim = cnt < k ? FLT_MAX : bd[k - 1];
+            __syncwarp();
+            const int ni = stack[--sp];
+            const CacheTravNode n = nodes[ni];
+            const float lim = cnt < k ? FLT_MAX : worst_d;
             if (box_d(n) > lim) continue;
-            int l = __float_as_int(n.bmin.w), r = __float_as_int(n.bmax.w);
+            const int l = __float_as_int(n.bmin.w), r = __float_as_int(n.bmax.w);
             if (l < 0) {
-                int off = -l - 1;
-                for (int j = 0; j < r; j++) {
-                    float4 p = pos[off + j];
-                    float dx = p.x - x, dy = p.y - y, dz = p.z - z;
-                    float d = dx * dx + dy * dy + dz * dz;
-                    int id = off + j;
-                    if (cnt == k && !worse(bd[k - 1], bi[k - 1], d, id)) continue;
-                    int m = cnt < k ? cnt++ : k - 1;
-                    while (m > 0 && worse(bd[m - 1], bi[m - 1], d, id)) {
-                        bd[m] = bd[m - 1];
-                        bi[m] = bi[m - 1];
-                        m--;
+                const int off = -l - 1;
+                for (int j0 = 0; j0 < r; j0 += 32) {
+                    float d = 0.f;
+                    const int id = off + j0 + lane;
+                    const bool have = j0 + lane < r;
+                    if (have) {
+                        const float4 p = pos[id];
+                        const float dx = p.x - x, dy = p.y - y, dz = p.z - z;
+                        d = dx * dx + dy * dy + dz * dz;
                     }
-                    bd[m] = d;
-                    bi[m] = id;
+                    unsigned todo = __ballot_sync(kFull, have);
+                    while (todo) {
+                        const int src = __ffs(todo) - 1;
+                        todo &= todo - 1;
+                        const float cd = __shfl_sync(kFull, d, src);
+                        const int ci = off + j0 + src;
+                        if (cnt == k && !worse(worst_d, worst_i, cd, ci)) continue;
+                        if (cnt < k) cnt++;
+                        // entries that stay in front of the new one
+                        int at = 0;
+#pragma unroll
+                        for (int e = 0; e < E; e++)
+                            at += __popc(__ballot_sync(kFull, bi[e] != INT_MAX && !worse(bd[e], bi[e], cd, ci)));
+#pragma unroll
+                        for (int e = E - 1; e >= 0; e--) {
+                            float pd = __shfl_up_sync(kFull, bd[e], 1);
+                            int pi = __shfl_up_sync(kFull, bi[e], 1);
+                            if (e > 0) {  // rank 32 e takes over from the last lane of the entry before
+                                const float cd2 = __shfl_sync(kFull, bd[e > 0 ? e - 1 : 0], 31);
+                                const int ci2 = __shfl_sync(kFull, bi[e > 0 ? e - 1 : 0], 31);
+                                if (lane == 0) {
+                                    pd = cd2;
+                                    pi = ci2;
+                                }
+                            }
+                            const int rank = 32 * e + lane;
+                            if (rank == at) {
+                                bd[e] = cd;
+                                bi[e] = ci;
+                            } else if (rank > at) {
+                                bd[e] = pd;
+                                bi[e] = pi;
+                            }
+                        }
+                        if (cnt == k) {
+                            const int last = k - 1;
+                            worst_d = __shfl_sync(kFull, E > 1 && last >= 32 ? bd[E - 1] : bd[0], last & 31);
+                            worst_i = __shfl_sync(kFull, E > 1 && last >= 32 ? bi[E - 1] : bi[0], last & 31);
+                        }
+                    }
                 }
             } else if (sp + 2 <= 64) {
-                float da = box_d(nodes[l]), db = box_d(nodes[r]);
-                if (da < db) {
-                    stack[sp++] = r;
-                    stack[sp++] = l;
-                } else {
-                    stack[sp++] = l;
-                    stack[sp++] = r;
+                const float da = box_d(nodes[l]), db = box_d(nodes[r]);
+                const bool left_first = da < db;  // the one entered first is pushed last
+                __syncwarp();
+                if (lane == 0) {
+                    stack[sp] = left_first ? r : l;
+                    stack[sp + 1] = left_first ? l : r;
                 }
+                sp += 2;
             }
         }
     }
-    for (int j = 0; j < k; j++) {
-        out_i[t * k + j] = bi[j];
-        out_d[t * k + j] = bd[j] == FLT_MAX ? INFINITY : bd[j];
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        const int rank = 32 * e + lane;
+        if (rank < k) {
+            const bool have = rank < cnt;
+            out_i[t * k + rank] = have ? bi[e] : -1;
+            out_d[t * k + rank] = !have || bd[e] == FLT_MAX ? INFINITY : bd[e];
+        }
     }
 }
 
@@ -1208,8 +1307,9 @@ int cache_build_device(pgx_ctx* ctx, const pgx_path_vertex* d_records, int64_t n
     int* acc = reinterpret_cast<int*>(misc + 1);
     int2* regions = cs->regions.as<int2>();
 
-    k_pos<<<blocks_for(n, 256), 256, 0, s>>>(cs->recs_in.as<pgx_path_vertex>(), n, pos, acc);
-    k_root_bounds<<<std::min<unsigned>(blocks_for(n, 256), 4 * pgx_num_sms()), 256, 0, s>>>(pos, n, acc);
+    k_bounds_init<<<1, 32, 0, s>>>(acc);
+    k_pos<<<std::min<unsigned>(blocks_for(n, 256), 8 * pgx_num_sms()), 256, 0, s>>>(cs->recs_in.as<pgx_path_vertex>(), n,
+                                                                                    pos, acc);
     k_root<<<1, 32, 0, s>>>(n, misc, nodes, items, small, acc);
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(hist, 0, sizeof(int) * kDigits * item_cap, s));
     PGX_CUDA_TRY(ctx, cudaGetLastError());
@@ -1377,9 +1477,9 @@ extern "C" int pgx_cache_knn(pgx_ctx* ctx, const float* queries, int64_t nq, int
     PGX_CUDA_TRY(ctx, cs->knn_i.reserve(sizeof(int) * k * nq));
     PGX_CUDA_TRY(ctx, cs->knn_d.reserve(sizeof(float) * k * nq));
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(cs->knn_q.p, queries, sizeof(float) * 3 * nq, cudaMemcpyHostToDevice, s));
-    k_knn<<<blocks_for(nq, 128), 128, 0, s>>>(cs->trav.as<CacheTravNode>(), cs->pos.as<float4>(),
-                                              (int)cs->n_records, cs->knn_q.as<float>(), nq, k, cs->knn_i.as<int>(),
-                                              cs->knn_d.as<float>());
+    auto knn = k <= 32 ? k_knn<1> : k_knn<2>;
+    knn<<<blocks_for(nq, 4), 128, 0, s>>>(cs->trav.as<CacheTravNode>(), cs->pos.as<float4>(), (int)cs->n_records,
+                                          cs->knn_q.as<float>(), nq, k, cs->knn_i.as<int>(), cs->knn_d.as<float>());
     PGX_CUDA_TRY(ctx, cudaGetLastError());
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(idx, cs->knn_i.p, sizeof(int) * k * nq, cudaMemcpyDeviceToHost, s));
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(d2, cs->knn_d.p, sizeof(float) * k * nq, cudaMemcpyDeviceToHost, s));

@@ -1186,7 +1186,7 @@ __device__ __forceinline__ void finalize_path(const SceneView& sv, const PathSta
             size_t ri = (size_t)i * ps.capacity + p;
             float4 pos = ps.rec_pos[ri];
             if (collect && pos.w != 0.f && valid(li) && lum(li) > 0.f) {
-                unsigned slot = atomicAdd(ps.nvertices, 1u);
+                const unsigned slot = warp_aggregated_add(ps.nvertices, true);
                 if (slot < (unsigned)ps.vcapacity) {
                     float4 nr4 = ps.rec_nrm[ri], wi = ps.rec_wi[ri];
                     pgx_path_vertex v;
@@ -1232,7 +1232,7 @@ __device__ __forceinline__ void finalize_path(const SceneView& sv, const PathSta
                     if (u >= fp.train_keep) continue;
                     float wgt = lum(li * f3(ps.rec_f[ri]));
                     if (!(wgt > 0.f) || isinf(wgt)) continue;
-                    unsigned slot = atomicAdd(ps.ntrain, 1u);
+                    const unsigned slot = warp_aggregated_add(ps.ntrain, true);
                     if (slot >= (unsigned)ps.tcapacity) continue;
                     float4 nr4 = ps.rec_nrm[ri], wi = ps.rec_wi[ri], wo = ps.rec_wo[ri];
                     float* o = ps.train + (size_t)slot * 13;
@@ -1243,7 +1243,7 @@ __device__ __forceinline__ void finalize_path(const SceneView& sv, const PathSta
                     o[12] = wgt;
                     continue;
                 }
-                unsigned slot = atomicAdd(ps.nvertices, 1u);
+                const unsigned slot = warp_aggregated_add(ps.nvertices, true);
                 if (slot >= (unsigned)ps.vcapacity) continue;
                 float4 nr4 = ps.rec_nrm[ri], wi = ps.rec_wi[ri];
                 pgx_path_vertex v;

@@ -61,3 +61,24 @@ def test_tree_at_build_limits(ctx, n, ties, region):
         stack.append((int(nd["right"]), first + used // 2, used - used // 2, above))
     assert seen == len(nodes)
     assert sorted((int(r["first"]), int(r["count"]), int(r["node"])) for r in regions) == sorted(want_regions)
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (5, 8), (9, 31), (300, 32), (300, 33), (40, 64), (5000, 1), (5000, 64)])
+def test_knn_at_list_ends(ctx, n, k):
+    """Lists of one, a full warp, one more, and longer than the cache; equal
+    distances (duplicated records) keep the lower index first.  The distance
+    is the float32 expression of the brute force."""
+    recs = _records(n, n + k, ties=True)
+    recs["position"][n // 2:] = recs["position"][: n - n // 2]
+    ctx.cache_build(recs)
+    _, out = ctx.cache_export()
+    rng = np.random.default_rng(k)
+    q = np.concatenate([out["position"][rng.integers(0, n, 40)], rng.normal(size=(60, 3)) * 3]).astype(np.float32)
+    idx, d2 = ctx.cache_knn(q, k)
+    d = out["position"][None, :, :] - q[:, None, :]
+    ref = (d[..., 0] * d[..., 0] + d[..., 1] * d[..., 1]) + d[..., 2] * d[..., 2]
+    order = np.argsort(ref, axis=1, kind="stable")[:, :k]
+    m = min(n, k)
+    assert np.array_equal(idx[:, :m], order[:, :m])
+    assert np.array_equal(d2[:, :m], np.take_along_axis(ref, order[:, :m], 1))
+    assert np.all(idx[:, m:] == -1) and np.all(np.isinf(d2[:, m:]))
