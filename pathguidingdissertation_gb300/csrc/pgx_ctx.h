@@ -57,6 +57,8 @@ struct DevMaterial {
     float sigma;
     float emission[3];
     float alb_off[3];  // added to the sampled albedo (0 except in differentiable renders)
+    float alb[3];      // the texel of a 1x1 albedo texture (constant albedos), read instead of it
+    int constant;      // alb holds the texture
 };
 
 // Shading class of a surface (the wavefront shades one class per launch):

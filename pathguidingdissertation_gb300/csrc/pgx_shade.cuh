@@ -106,22 +106,28 @@ struct TexView {
     const float* texels;
 };
 __device__ __forceinline__ F3 texel(const float* p, long long i) { return f3(p[3 * i], p[3 * i + 1], p[3 * i + 2]); }
+// a % n with the reference's in-range values; texture coordinates in [0, 1]
+// (and the neighbour one past the edge) need no division.
 __device__ __forceinline__ int wrap_index(int a, int n) {
+    if ((unsigned)a < (unsigned)n) return a;
+    if (a >= n && a - n < n) return a - n;
     int r = a % n;
     return (r < 0 || r >= n) ? 0 : r;  // the reference relies on in-range values; keep reads in bounds
 }
-static __device__ F3 tex_sample_raw(const float* texels, long long offset, int W, int H, float tu, float tv) {
+// Bilinear weights of Texture::sample at (tu, tv), and the integer texel.
+__device__ __forceinline__ float4 tex_weights(int W, int H, float tu, float tv, int& x, int& y) {
     float u = fmaxf(0.f, fabsf(tu)) * (float)W;
     float v = fmaxf(0.f, fabsf(tv)) * (float)H;
     float fu = floorf(u), fv = floorf(v);
-    int x = (fu >= -2147483648.f && fu < 2147483648.f) ? (int)fu : 0;
-    int y = (fv >= -2147483648.f && fv < 2147483648.f) ? (int)fv : 0;
+    x = (fu >= -2147483648.f && fu < 2147483648.f) ? (int)fu : 0;
+    y = (fv >= -2147483648.f && fv < 2147483648.f) ? (int)fv : 0;
     float frac_u = u - (float)x;
     float frac_v = v - (float)y;
-    float w0 = (1.f - frac_u) * (1.f - frac_v);
-    float w1 = frac_u * (1.f - frac_v);
-    float w2 = (1.f - frac_u) * frac_v;
-    float w3 = frac_u * frac_v;
+    return make_float4((1.f - frac_u) * (1.f - frac_v), frac_u * (1.f - frac_v), (1.f - frac_u) * frac_v, frac_u * frac_v);
+}
+static __device__ F3 tex_sample_raw(const float* texels, long long offset, int W, int H, float tu, float tv) {
+    int x, y;
+    const float4 w = tex_weights(W, H, tu, tv, x, y);
     x = wrap_index(x, W);
     y = wrap_index(y, H);
     int x1 = wrap_index(x + 1, W), y1 = wrap_index(y + 1, H);
@@ -130,11 +136,23 @@ static __device__ F3 tex_sample_raw(const float* texels, long long offset, int W
     F3 s1 = texel(p, (long long)y * W + x1);
     F3 s2 = texel(p, (long long)y1 * W + x);
     F3 s3 = texel(p, (long long)y1 * W + x1);
-    return (((s0 * w0) + (s1 * w1)) + (s2 * w2)) + (s3 * w3);
+    return (((s0 * w.x) + (s1 * w.y)) + (s2 * w.z)) + (s3 * w.w);
 }
+// The albedo at a shading point.  A constant one is a 1x1 texture whose four
+// bilinear taps are one texel: it comes with the material (two dependent
+// gathers, 12 loads and four integer divisions less per evaluation), weighted
+// as the texture's taps are.
 __device__ __forceinline__ F3 albedo_of(const TexView& tv, const DevMaterial& m, const Shading& sd) {
-    DevTexture t = tv.info[m.tex];
-    F3 a = tex_sample_raw(tv.texels, t.offset, t.width, t.height, sd.tu, sd.tv);
+    F3 a;
+    if (m.constant) {
+        int x, y;
+        const float4 w = tex_weights(1, 1, sd.tu, sd.tv, x, y);
+        const F3 s = f3(m.alb[0], m.alb[1], m.alb[2]);
+        a = (((s * w.x) + (s * w.y)) + (s * w.z)) + (s * w.w);
+    } else {
+        DevTexture t = tv.info[m.tex];
+        a = tex_sample_raw(tv.texels, t.offset, t.width, t.height, sd.tu, sd.tv);
+    }
     return f3(a.x + m.alb_off[0], a.y + m.alb_off[1], a.z + m.alb_off[2]);
 }
 

@@ -296,7 +296,10 @@ extern "C" int pgx_scene_upload(pgx_ctx* ctx, const pgx_triangle* tris, int64_t 
             pool.push_back(m.albedo[1]);
             pool.push_back(m.albedo[2]);
         }
+        const DevTexture& tex = tex_info[(size_t)d.tex];
+        d.constant = tex.width == 1 && tex.height == 1 ? 1 : 0;
         for (int k = 0; k < 3; k++) {
+            if (d.constant) d.alb[k] = pool[(size_t)(3 * tex.offset) + k];
             d.eta[k] = m.eta[k];
             d.k[k] = m.k[k];
             d.emission[k] = m.emission[k];
