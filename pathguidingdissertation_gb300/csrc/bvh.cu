@@ -13,11 +13,12 @@
 // differ (the reference partitions in place by swapping).
 //
 // Phase A (nodes with more than kSmall triangles) runs level by level with two
-// launches a level and no host round trip: CTAs take 2048-triangle chunks of
+// launches a level and no host round trip: CTAs take 1024-triangle chunks of
 // the active nodes.  k_bin bins a chunk in shared memory, and the block that
-// finishes a node's last chunk sweeps the SAH; k_partition splits the chunk
-// into the other record buffer and reduces the children's boxes, and the
-// node's last block creates its children.  A triangle travels as one 48-byte
+// finishes a node's last chunk sweeps the SAH; k_partition splits the chunks
+// of such a node into the other record buffer and reduces the children's
+// boxes, and the node's last block creates its children.  A node of one chunk
+// is split by k_bin itself.  A triangle travels as one 48-byte
 // record (box, centroid, id), so every pass reads and writes runs.  Phase B
 // gives each node of at most kSmall triangles to one warp, which finishes its
 // subtree in shared memory.
@@ -34,10 +35,24 @@ namespace {
 constexpr int kBins = 16;          // BUILD_BINS, Geometry.h:20
 constexpr int kMaxLeaf = 4;        // MAXNODE_TRIANGLES, Geometry.h:17
 constexpr int kSmall = 128;        // phase-B threshold
-constexpr int kChunk = 2048;       // triangles per CTA chunk in phase A
 constexpr int kThreads = 256;
+// Triangles per CTA chunk in phase A (2,093,058 triangles, whole build: 3.99 ms
+// with 512, 3.48 with 1024, 3.50 with 2048, 4.04 with 4096: smaller ones merge
+// more bins, larger ones leave a nearly empty last wave).
+constexpr int kChunk = 1024;
 constexpr int kPerThread = kChunk / kThreads;
 constexpr int kBinInts = 3 * kBins * 7;
+// Bins of a node: count, box minimum and maximum, each for all (axis, bin).
+constexpr int kField = 3 * kBins;
+// Neighbouring triangles fall into the same bins, and updates of one bin by
+// one warp take turns, so neighbouring lanes use copies of their own, which
+// are merged before the sweep (2,093,058 triangles: k_bin 1213 us with one
+// copy, 3.40 / 3.22 / 3.15 / 3.14 / 3.21 ms of build with 1 / 2 / 4 / 8 / 16
+// copies; phase B 3.15 / 3.10 / 3.22 with 1 / 2 / 3, where more shared memory
+// costs warps).
+constexpr int kBinCopies = 4, kSmallCopies = 2;
+// (copies 8 banks apart: 2.91 ms; in the same banks 3.29, 16 apart 2.96)
+constexpr int kCopyInts = kBinInts + 8;
 constexpr int kMaxLevels = 200;
 
 struct BuildItem {
@@ -187,14 +202,13 @@ __global__ void k_root_init(pgx_bvh_node* nodes, int* node_rec, BuildItem* items
 }
 
 __device__ __forceinline__ void reset_bins(int* b, int i) {
-    const int f = i % 7;
-    b[i] = (f == 0) ? 0 : (f < 4 ? INT_MAX : INT_MIN);
+    b[i] = i < kField ? 0 : (i < 4 * kField ? INT_MAX : INT_MIN);
 }
 
 __global__ void k_bins_reset(int* bins, int64_t n) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
-        const int f = (int)(i % kBinInts) % 7;
+        const int f = (int)(i % kBinInts) / kField;
         bins[i] = (f == 0) ? 0 : (f < 4 ? INT_MAX : INT_MIN);
     }
 }
@@ -209,7 +223,7 @@ __device__ __forceinline__ void bin_add(int* bins, int ax, int bi, const int* lo
     __match_all_sync(0xFFFFFFFFu, bi, &same);
     if (same) {
         if (bi < 0) return;
-        int* b7 = bins + (ax * kBins + bi) * 7;
+        int* bn = bins + ax * kBins + bi;
         int v[6];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
@@ -218,20 +232,20 @@ __device__ __forceinline__ void bin_add(int* bins, int ax, int bi, const int* lo
         }
         const int lane = threadIdx.x & 31;
         if (lane == 0) {
-            atomicAdd(b7, 32);
+            atomicAdd(bn, 32);
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                atomicMin(b7 + 1 + k, v[k]);
-                atomicMax(b7 + 4 + k, v[3 + k]);
+                atomicMin(bn + (1 + k) * kField, v[k]);
+                atomicMax(bn + (4 + k) * kField, v[3 + k]);
             }
         }
     } else if (bi >= 0) {
-        int* b7 = bins + (ax * kBins + bi) * 7;
-        atomicAdd(b7, 1);
+        int* bn = bins + ax * kBins + bi;
+        atomicAdd(bn, 1);
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            atomicMin(b7 + 1 + k, lo[k]);
-            atomicMax(b7 + 4 + k, hi[k]);
+            atomicMin(bn + (1 + k) * kField, lo[k]);
+            atomicMax(bn + (4 + k) * kField, hi[k]);
         }
     }
 }
@@ -241,63 +255,71 @@ __device__ __forceinline__ int bin_of(float c, float lo, float scale) {
     return (bi < kBins - 1) ? bi : kBins - 1;
 }
 
-// Sweep of findBestSplitPlane (Geometry.h:325-362) by one warp: 16 lanes per
-// axis hold one bin each (axes 0 and 1 together, then axis 2), prefix and
-// suffix scans give every candidate's sides, and the smallest cost wins, the
-// first one in the reference's order (axis, then plane) on ties.  Returns the
-// axis (-1: none) with its plane and cost.  Minima and maxima commute, so the
-// result is the sequential sweep's.
+// Sweep of findBestSplitPlane (Geometry.h:325-362) by one warp, an axis at a
+// time: lanes 0-15 scan the bins upwards (the left sides), lanes 16-31
+// downwards (the right sides), each lane works out its side's cost term, and
+// one exchange per axis brings the terms of a plane together.  The smallest
+// cost wins, the first one in the reference's order (axis, then plane) on
+// ties.  Returns the axis (-1: none) with its plane and cost.  Minima and
+// maxima commute, so the result is the sequential sweep's.
+//   Shuffles bound it (one a cycle and SM): 87 a node.  Both scans in every
+// lane, two axes at once, took 126 and two more divisions.
+template <int COPIES>
 __device__ __forceinline__ int warp_sweep(const int* bins, const float* lo, const float* hi, float parent_area,
                                           float& best, float& pos) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31, b = lane & 15;
-    int axis = -1;
-    best = FLT_MAX;
-    pos = -FLT_MAX;
+    const int lane = threadIdx.x & 31, i = lane & 15;
+    const int b = lane < 16 ? i : 15 - i;
+    float cost[3];
+    int key[3];
 #pragma unroll
-    for (int half = 0; half < 2; half++) {
-        const int ax = half == 0 ? lane >> 4 : 2;
-        const float l = ax == 0 ? lo[0] : (ax == 1 ? lo[1] : lo[2]);
-        const float h = ax == 0 ? hi[0] : (ax == 1 ? hi[1] : hi[2]);
-        const int* b7 = bins + (ax * kBins + b) * 7;
-        int pc = b7[0], pm[6];
+    for (int ax = 0; ax < 3; ax++) {
+        cost[ax] = FLT_MAX;
+        key[ax] = INT_MAX;
+        if (lo[ax] == hi[ax]) continue;  // uniform
+        const int* bn = bins + ax * kBins + b;
+        int c = bn[0], m[6];
 #pragma unroll
-        for (int k = 0; k < 6; k++) pm[k] = b7[1 + k];
-        int sc = pc, sm[6];
+        for (int k = 0; k < 6; k++) m[k] = bn[(1 + k) * kField];
 #pragma unroll
-        for (int k = 0; k < 6; k++) sm[k] = pm[k];
+        for (int v = 1; v < COPIES; v++) {
+            const int* o = bn + v * kCopyInts;
+            c += o[0];
+#pragma unroll
+            for (int k = 0; k < 6; k++) m[k] = k < 3 ? min(m[k], o[(1 + k) * kField]) : max(m[k], o[(1 + k) * kField]);
+        }
 #pragma unroll
         for (int o = 1; o < 16; o <<= 1) {
-            int t = __shfl_up_sync(kFull, pc, o, 16);
-            if (b >= o) pc += t;
-            t = __shfl_down_sync(kFull, sc, o, 16);
-            if (b + o < 16) sc += t;
+            // (a lane without a source gets its own value: no change to a minimum)
+            const int t = __shfl_up_sync(kFull, c, o, 16);
+            if (i >= o) c += t;
 #pragma unroll
             for (int k = 0; k < 6; k++) {
-                t = __shfl_up_sync(kFull, pm[k], o, 16);
-                if (b >= o) pm[k] = k < 3 ? min(pm[k], t) : max(pm[k], t);
-                t = __shfl_down_sync(kFull, sm[k], o, 16);
-                if (b + o < 16) sm[k] = k < 3 ? min(sm[k], t) : max(sm[k], t);
+                const int v = __shfl_up_sync(kFull, m[k], o, 16);
+                m[k] = k < 3 ? min(m[k], v) : max(m[k], v);
             }
         }
-        // the right side of plane b starts at bin b + 1
-        sc = __shfl_down_sync(kFull, sc, 1, 16);
-#pragma unroll
-        for (int k = 0; k < 6; k++) sm[k] = __shfl_down_sync(kFull, sm[k], 1, 16);
-        const float la = pc > 0 ? area_x(o2f(pm[0]), o2f(pm[1]), o2f(pm[2]), o2f(pm[3]), o2f(pm[4]), o2f(pm[5])) : 0.f;
-        const float ra = sc > 0 ? area_x(o2f(sm[0]), o2f(sm[1]), o2f(sm[2]), o2f(sm[3]), o2f(sm[4]), o2f(sm[5])) : 0.f;
-        const float cost = x_add(x_add(1.f, x_mul(x_mul(x_div(la, parent_area), (float)pc), 1.5f)),
-                                 x_mul(x_mul(x_div(ra, parent_area), (float)sc), 1.5f));
-        const bool ok = b < kBins - 1 && !(l == h) && (half == 0 || lane < 16) && cost < best;
+        const float area = c > 0 ? area_x(o2f(m[0]), o2f(m[1]), o2f(m[2]), o2f(m[3]), o2f(m[4]), o2f(m[5])) : 0.f;
+        const float term = x_mul(x_mul(x_div(area, parent_area), (float)c), 1.5f);
+        // the right side of plane b starts at bin b + 1, in lane 30 - b
+        const float right = __shfl_sync(kFull, term, (30 - lane) & 31);
+        cost[ax] = x_add(x_add(1.f, term), right);
         // costs are ordered as ordered ints (a cost that is not below FLT_MAX, or NaN, is no candidate)
-        const int key = ok ? f2o(cost) : INT_MAX;
-        const int mn = __reduce_min_sync(kFull, key);
-        if (mn != INT_MAX) {
-            const int win = __ffs(__ballot_sync(kFull, key == mn)) - 1;
-            const float cand = x_add(l, x_mul(x_div(x_sub(h, l), (float)kBins), (float)(b + 1)));
-            best = __shfl_sync(kFull, cost, win);
-            pos = __shfl_sync(kFull, cand, win);
-            axis = __shfl_sync(kFull, ax, win);
+        if (lane < kBins - 1 && cost[ax] < FLT_MAX) key[ax] = f2o(cost[ax]);
+    }
+    best = FLT_MAX;
+    pos = -FLT_MAX;
+    const int mn = __reduce_min_sync(kFull, min(min(key[0], key[1]), key[2]));
+    if (mn == INT_MAX) return -1;
+    int axis = -1;
+#pragma unroll
+    for (int ax = 0; ax < 3; ax++) {
+        const unsigned who = __ballot_sync(kFull, key[ax] == mn);
+        if (axis < 0 && who) {
+            axis = ax;
+            const int win = __ffs(who) - 1;
+            best = __shfl_sync(kFull, cost[ax], win);
+            pos = x_add(lo[ax], x_mul(x_div(x_sub(hi[ax], lo[ax]), (float)kBins), (float)(win + 1)));
         }
     }
     return axis;
@@ -319,22 +341,207 @@ __device__ __forceinline__ bool last_chunk(BuildItem& it, unsigned nchunks, int*
     return last;
 }
 
+// Scratch of a block's partition pass.
+struct PartShared {
+    int warp_l[kThreads / 32], warp_r[kThreads / 32];
+    int base_l, base_r, flag;
+    int acc[24];
+};
+
+// Where a level's children go: the other record buffer, the next level's
+// items, the phase-B list, the nodes.
+struct BuildOut {
+    RecView rec;
+    int buf;
+    BuildItem* items;
+    int2* chunks;
+    int item_cap, chunk_cap, slot_cap;
+    int2* small;
+    int small_cap;
+    pgx_bvh_node* nodes;
+    int* node_rec;
+};
+
+// Partition of a chunk by centroid[axis] < pos (Geometry.h:384-391) into the
+// other record buffer, with the children's box and centroid bounds; the
+// block of the node's last chunk creates its children (Geometry.h:393-412).
+// SINGLE: the chunk is the whole node, so positions and boxes stay in the
+// block and no other block is waited for.  Whole blocks.
+//   Bound: 96 bytes moved a triangle, 30 us a level of 2,093,058; takes 51.  A
+// run of positions per thread instead of per warp (stores in pieces of 16
+// bytes) took 100.
+template <bool SINGLE>
+__device__ __forceinline__ void partition_chunk(BuildItem& it, int first, int axis, float pos, BuildMisc* misc, int level,
+                                                const RecView& rec, const BuildOut& out, PartShared& sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int start = it.start, count = it.count;
+    if (threadIdx.x < 24) sh.acc[threadIdx.x] = ((threadIdx.x % 6) < 3) ? INT_MAX : INT_MIN;
+    const int end = min(count, first + kChunk);
+    // Thread t reads positions first + k*kThreads + t; a warp's records go to
+    // one run per side, so that stores are as coalesced as loads.
+    unsigned left[kPerThread];
+    int wl = 0, wn = 0;
+#pragma unroll
+    for (int k = 0; k < kPerThread; k++) {
+        const int j = first + k * kThreads + threadIdx.x;
+        float cv = 0.f;
+        if (j < end) {
+            const float4 cc = rec.cent[start + j];
+            cv = axis == 0 ? cc.x : (axis == 1 ? cc.y : cc.z);
+        }
+        left[k] = __ballot_sync(0xFFFFFFFFu, j < end && cv < pos);
+        wl += __popc(left[k]);
+        wn += max(0, min(32, end - (j - lane)));
+    }
+    if (lane == 0) {
+        sh.warp_l[warp] = wl;
+        sh.warp_r[warp] = wn - wl;
+    }
+    __syncthreads();
+    int before_l = 0, before_r = 0, all_l = 0, all_r = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; w++) {
+        if (w == warp) before_l = all_l, before_r = all_r;
+        all_l += sh.warp_l[w];
+        all_r += sh.warp_r[w];
+    }
+    int base_l = 0, base_r = 0;
+    if (!SINGLE) {
+        if (threadIdx.x == 0) {
+            sh.base_l = atomicAdd(&it.lcur, all_l);
+            sh.base_r = atomicAdd(&it.rcur, all_r);
+        }
+        __syncthreads();
+        base_l = sh.base_l;
+        base_r = sh.base_r;
+    }
+    int offl = start + base_l + before_l;
+    int offr = start + count - 1 - (base_r + before_r);
+    int acc[2][12];
+#pragma unroll
+    for (int k = 0; k < 24; k++) acc[k / 12][k % 12] = ((k % 6) < 3) ? INT_MAX : INT_MIN;
+#pragma unroll
+    for (int k = 0; k < kPerThread; k++) {
+        const int j = first + k * kThreads + threadIdx.x;
+        const unsigned below = (1u << lane) - 1u;
+        if (j < end) {
+            const float4 a = rec.lo[start + j], b = rec.hi[start + j], cc = rec.cent[start + j];
+            const int side = (left[k] >> lane) & 1u ? 0 : 1;
+            const int to = side ? offr - __popc(~left[k] & below) : offl + __popc(left[k] & below);
+            out.rec.lo[to] = a;
+            out.rec.hi[to] = b;
+            out.rec.cent[to] = cc;
+            const int v[9] = {f2o(a.x), f2o(a.y), f2o(a.z), f2o(b.x), f2o(b.y), f2o(b.z), f2o(cc.x), f2o(cc.y), f2o(cc.z)};
+#pragma unroll
+            for (int s = 0; s < 2; s++)
+                if (s == side) {
+#pragma unroll
+                    for (int x = 0; x < 3; x++) {
+                        acc[s][x] = min(acc[s][x], v[x]);
+                        acc[s][3 + x] = max(acc[s][3 + x], v[3 + x]);
+                        acc[s][6 + x] = min(acc[s][6 + x], v[6 + x]);
+                        acc[s][9 + x] = max(acc[s][9 + x], v[6 + x]);
+                    }
+                }
+        }
+        const int nk = __popc(left[k]);
+        offl += nk;
+        offr -= max(0, min(32, end - (j - lane))) - nk;
+    }
+    if (first + warp * 32 < end) {  // a warp without triangles has nothing to add
+#pragma unroll
+        for (int k = 0; k < 24; k++) {
+            const bool is_min = (k % 6) < 3;
+            const int v = is_min ? __reduce_min_sync(0xFFFFFFFFu, acc[k / 12][k % 12])
+                                 : __reduce_max_sync(0xFFFFFFFFu, acc[k / 12][k % 12]);
+            if (lane == 0) {
+                if (is_min)
+                    atomicMin(&sh.acc[k], v);
+                else
+                    atomicMax(&sh.acc[k], v);
+            }
+        }
+    }
+    __syncthreads();
+    bool commit = true;
+    if (!SINGLE) {
+        if (threadIdx.x < 24) {
+            const int k = threadIdx.x;
+            int* dst = &it.acc[k / 12][k % 12];
+            if ((k % 6) < 3)
+                atomicMin(dst, sh.acc[k]);
+            else
+                atomicMax(dst, sh.acc[k]);
+        }
+        commit = last_chunk(it, (unsigned)((count + kChunk - 1) / kChunk), &sh.flag);
+        if (commit) {
+            if (threadIdx.x < 24) sh.acc[threadIdx.x] = __ldcg(&it.acc[threadIdx.x / 12][threadIdx.x % 12]);
+            __syncthreads();
+        }
+    }
+    // One lane per child: the two chains of list atomics run side by side.
+    if (commit && threadIdx.x < 2) {
+        const int side = threadIdx.x;
+        pgx_bvh_node& nd = out.nodes[it.node];
+        const int L = SINGLE ? all_l : __ldcg(&it.lcur);
+        const int from = out.buf ? kSmallBuf : 0;
+        if (L == 0 || L == count) {
+            if (side == 0) {
+                nd.left_first = start;
+                nd.used = count;
+                add_small(out.small, out.small_cap, misc, it.node, kSmallLeaf | from);
+            }
+        } else {
+            unsigned long long at = 0;
+            if (side == 0) at = atomicAdd(&misc->counts, 2ull | (1ull << 32));
+            at = __shfl_sync(3u, at, 0);
+            const int child = (int)(unsigned)at;
+            if (side == 0) {
+                out.node_rec[it.node] = (int)(at >> 32);
+                nd.left_first = child;
+                nd.used = 0;
+            }
+            const int cs = side ? start + L : start;
+            const int cn = side ? count - L : L;
+            const int* box = sh.acc + 12 * side;
+            pgx_bvh_node& cnd = out.nodes[child + side];
+            for (int k = 0; k < 3; k++) {
+                cnd.bmin[k] = o2f(box[k]);
+                cnd.bmax[k] = o2f(box[3 + k]);
+            }
+            cnd.left_first = cs;
+            cnd.used = cn;
+            out.node_rec[child + side] = -1;
+            if (cn <= kSmall)
+                add_small(out.small, out.small_cap, misc, child + side, from);
+            else
+                add_item(out.items, out.chunks, misc, level + 1, out.item_cap, out.chunk_cap, out.slot_cap, child + side,
+                         cs, cn, box + 6, box + 9);
+        }
+    }
+    __syncthreads();
+}
+
 // Bins of each chunk in shared memory, merged into the node's global bins
 // when it has several chunks; the last chunk's block decides the split
 // (subdivide, Geometry.h:367-381).  A node that stays a leaf goes to phase B
-// for its triangle ids.
+// for its triangle ids.  A node of one chunk is partitioned here as well,
+// while the block holds its split.
 __global__ void __launch_bounds__(kThreads) k_bin(BuildItem* __restrict__ items, const int2* __restrict__ chunks,
                                                   BuildMisc* __restrict__ misc, int level, RecView rec, int buf,
-                                                  int* __restrict__ gbins, pgx_bvh_node* __restrict__ nodes,
-                                                  int2* __restrict__ small, int small_cap) {
-    __shared__ int sb[kBinInts];
-    __shared__ int s_flag;
+                                                  int* __restrict__ gbins, BuildOut out) {
+    __shared__ int sb[kBinCopies * kCopyInts];
+    int* mine = sb + (threadIdx.x % kBinCopies) * kCopyInts;
+    __shared__ PartShared sh;
+    __shared__ int s_split, s_axis;
+    __shared__ float s_pos;
     const int nchunks = misc->nchunks[level];
     for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const int2 ch = chunks[c];
         BuildItem& it = items[ch.x];
         const int start = it.start, count = it.count;
-        for (int k = threadIdx.x; k < kBinInts; k += kThreads) reset_bins(sb, k);
+        for (int k = threadIdx.x; k < kBinInts; k += kThreads)
+            for (int v = 0; v < kBinCopies; v++) reset_bins(sb + v * kCopyInts, k);
         __syncthreads();
         float lo[3], hi[3], scale[3];
 #pragma unroll
@@ -357,7 +564,18 @@ __global__ void __launch_bounds__(kThreads) k_bin(BuildItem* __restrict__ items,
             }
 #pragma unroll
             for (int ax = 0; ax < 3; ax++)
-                if (!(lo[ax] == hi[ax])) bin_add(sb, ax, in ? bin_of(cv[ax], lo[ax], scale[ax]) : -1, l, h);
+                if (!(lo[ax] == hi[ax])) bin_add(mine, ax, in ? bin_of(cv[ax], lo[ax], scale[ax]) : -1, l, h);
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < kBinInts; k += kThreads) {
+            const int f = k / kField;
+            int r = sb[k];
+#pragma unroll
+            for (int v = 1; v < kBinCopies; v++) {
+                const int o = sb[v * kCopyInts + k];
+                r = f == 0 ? r + o : (f < 4 ? min(r, o) : max(r, o));
+            }
+            sb[k] = r;
         }
         __syncthreads();
         const unsigned nch = (unsigned)((count + kChunk - 1) / kChunk);
@@ -365,8 +583,8 @@ __global__ void __launch_bounds__(kThreads) k_bin(BuildItem* __restrict__ items,
         if (nch > 1) {
             int* g = gbins + (size_t)it.slot * kBinInts;
             for (int k = threadIdx.x; k < kBinInts; k += kThreads) {
-                if (sb[(k / 7) * 7] == 0) continue;
-                const int f = k % 7;
+                if (sb[k % kField] == 0) continue;
+                const int f = k / kField;
                 if (f == 0)
                     atomicAdd(g + k, sb[k]);
                 else if (f < 4)
@@ -374,7 +592,7 @@ __global__ void __launch_bounds__(kThreads) k_bin(BuildItem* __restrict__ items,
                 else
                     atomicMax(g + k, sb[k]);
             }
-            decide = last_chunk(it, nch, &s_flag);
+            decide = last_chunk(it, nch, &sh.flag);
             if (decide) {
                 for (int k = threadIdx.x; k < kBinInts; k += kThreads) {
                     sb[k] = __ldcg(g + k);
@@ -384,178 +602,46 @@ __global__ void __launch_bounds__(kThreads) k_bin(BuildItem* __restrict__ items,
             }
         }
         if (decide && threadIdx.x < 32) {
-            pgx_bvh_node& nd = nodes[it.node];
+            pgx_bvh_node& nd = out.nodes[it.node];
             const float parent_area = area_x(nd.bmin[0], nd.bmin[1], nd.bmin[2], nd.bmax[0], nd.bmax[1], nd.bmax[2]);
             float best, pos;
-            const int axis = warp_sweep(sb, lo, hi, parent_area, best, pos);
+            const int axis = warp_sweep<1>(sb, lo, hi, parent_area, best, pos);
             if (threadIdx.x == 0) {
                 const float no_split = x_mul((float)count, 1.5f);
+                s_split = 0;
                 if (best >= no_split || axis == -1) {
                     it.split = 0;
                     nd.left_first = start;
                     nd.used = count;
-                    add_small(small, small_cap, misc, it.node, kSmallLeaf | (buf ? kSmallBuf : 0));
-                } else {
+                    add_small(out.small, out.small_cap, misc, it.node, kSmallLeaf | (buf ? kSmallBuf : 0));
+                } else if (nch > 1) {
                     it.split = 1;
                     it.axis = axis;
                     it.pos = pos;
+                } else {
+                    s_split = 1;
+                    s_axis = axis;
+                    s_pos = pos;
                 }
             }
         }
         __syncthreads();  // the shared bins are reused
+        if (nch == 1 && s_split) partition_chunk<true>(it, 0, s_axis, s_pos, misc, level, rec, out, sh);
     }
 }
 
-// Partition of each chunk by centroid[axis] < pos (Geometry.h:384-391) into
-// the other record buffer, with the children's box and centroid bounds; the
-// node's last chunk's block creates its children (Geometry.h:393-412).
+// Partition of the chunks of the nodes that have several.
 __global__ void __launch_bounds__(kThreads) k_partition(BuildItem* __restrict__ items, const int2* __restrict__ chunks,
                                                         BuildMisc* __restrict__ misc, int level, RecView rec,
-                                                        RecView out, int out_buf, BuildItem* __restrict__ next,
-                                                        int2* __restrict__ next_chunks, int item_cap, int chunk_cap,
-                                                        int slot_cap, int2* __restrict__ small, int small_cap,
-                                                        pgx_bvh_node* __restrict__ nodes, int* __restrict__ node_rec) {
-    __shared__ int s_warp_l[kThreads / 32], s_warp_r[kThreads / 32];
-    __shared__ int s_base_l, s_base_r, s_flag;
-    __shared__ int s_acc[24];
+                                                        BuildOut out) {
+    __shared__ PartShared sh;
+    if (misc->nslots[level] == 0) return;  // no such node on this level
     const int nchunks = misc->nchunks[level];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const int2 ch = chunks[c];
         BuildItem& it = items[ch.x];
         if (!it.split) continue;  // uniform per block
-        const int start = it.start, count = it.count;
-        if (threadIdx.x < 24) s_acc[threadIdx.x] = ((threadIdx.x % 6) < 3) ? INT_MAX : INT_MIN;
-        const int axis = it.axis;
-        const float pos = it.pos;
-        const int end = min(count, ch.y + kChunk);
-        // Thread t owns positions ch.y + k*kThreads + t (coalesced reads).
-        unsigned sides = 0;
-        int nl = 0, nr = 0;
-#pragma unroll
-        for (int k = 0; k < kPerThread; k++) {
-            const int j = ch.y + k * kThreads + threadIdx.x;
-            if (j >= end) continue;
-            const float4 cc = rec.cent[start + j];
-            const float cv = axis == 0 ? cc.x : (axis == 1 ? cc.y : cc.z);
-            const int side = (cv < pos) ? 0 : 1;
-            sides |= (unsigned)side << k;
-            nl += 1 - side;
-            nr += side;
-        }
-        // Exclusive scan of nl / nr across the block.
-        int il = nl, ir = nr;
-        for (int o = 1; o < 32; o <<= 1) {
-            int tl = __shfl_up_sync(0xFFFFFFFFu, il, o);
-            int tr = __shfl_up_sync(0xFFFFFFFFu, ir, o);
-            if (lane >= o) {
-                il += tl;
-                ir += tr;
-            }
-        }
-        if (lane == 31) {
-            s_warp_l[warp] = il;
-            s_warp_r[warp] = ir;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int tl = 0, tr = 0;
-            for (int w = 0; w < kThreads / 32; w++) {
-                int a = s_warp_l[w], b = s_warp_r[w];
-                s_warp_l[w] = tl;
-                s_warp_r[w] = tr;
-                tl += a;
-                tr += b;
-            }
-            s_base_l = atomicAdd(&it.lcur, tl);
-            s_base_r = atomicAdd(&it.rcur, tr);
-        }
-        __syncthreads();
-        int offl = start + s_base_l + s_warp_l[warp] + il - nl;
-        int offr = start + count - 1 - (s_base_r + s_warp_r[warp] + ir - nr);
-        int acc[2][12];
-#pragma unroll
-        for (int k = 0; k < 24; k++) acc[k / 12][k % 12] = ((k % 6) < 3) ? INT_MAX : INT_MIN;
-        for (int k = 0; k < kPerThread; k++) {
-            const int j = ch.y + k * kThreads + threadIdx.x;
-            if (j >= end) continue;
-            const float4 a = rec.lo[start + j], b = rec.hi[start + j], cc = rec.cent[start + j];
-            const int side = (sides >> k) & 1;
-            const int to = side ? offr-- : offl++;
-            out.lo[to] = a;
-            out.hi[to] = b;
-            out.cent[to] = cc;
-            const int v[9] = {f2o(a.x), f2o(a.y), f2o(a.z), f2o(b.x), f2o(b.y), f2o(b.z), f2o(cc.x), f2o(cc.y), f2o(cc.z)};
-#pragma unroll
-            for (int s = 0; s < 2; s++)
-                if (s == side) {
-#pragma unroll
-                    for (int x = 0; x < 3; x++) {
-                        acc[s][x] = min(acc[s][x], v[x]);
-                        acc[s][3 + x] = max(acc[s][3 + x], v[3 + x]);
-                        acc[s][6 + x] = min(acc[s][6 + x], v[6 + x]);
-                        acc[s][9 + x] = max(acc[s][9 + x], v[6 + x]);
-                    }
-                }
-        }
-#pragma unroll
-        for (int k = 0; k < 24; k++) {
-            const bool is_min = (k % 6) < 3;
-            const int v = is_min ? __reduce_min_sync(0xFFFFFFFFu, acc[k / 12][k % 12])
-                                 : __reduce_max_sync(0xFFFFFFFFu, acc[k / 12][k % 12]);
-            if (lane == 0) {
-                if (is_min)
-                    atomicMin(&s_acc[k], v);
-                else
-                    atomicMax(&s_acc[k], v);
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x < 24) {
-            int k = threadIdx.x;
-            int* dst = &it.acc[k / 12][k % 12];
-            if ((k % 6) < 3)
-                atomicMin(dst, s_acc[k]);
-            else
-                atomicMax(dst, s_acc[k]);
-        }
-        const unsigned nch = (unsigned)((count + kChunk - 1) / kChunk);
-        if (last_chunk(it, nch, &s_flag) && threadIdx.x == 0) {
-            pgx_bvh_node& nd = nodes[it.node];
-            const int L = __ldcg(&it.lcur);
-            const int from = out_buf ? kSmallBuf : 0;
-            if (L == 0 || L == count) {
-                nd.left_first = start;
-                nd.used = count;
-                add_small(small, small_cap, misc, it.node, kSmallLeaf | from);
-            } else {
-                const unsigned long long at = atomicAdd(&misc->counts, 2ull | (1ull << 32));
-                const int child = (int)(unsigned)at;
-                node_rec[it.node] = (int)(at >> 32);
-                nd.left_first = child;
-                nd.used = 0;
-                for (int side = 0; side < 2; side++) {
-                    const int cs = side ? start + L : start;
-                    const int cn = side ? count - L : L;
-                    int box[12];
-                    for (int k = 0; k < 12; k++) box[k] = __ldcg(&it.acc[side][k]);
-                    pgx_bvh_node& cnd = nodes[child + side];
-                    for (int k = 0; k < 3; k++) {
-                        cnd.bmin[k] = o2f(box[k]);
-                        cnd.bmax[k] = o2f(box[3 + k]);
-                    }
-                    cnd.left_first = cs;
-                    cnd.used = cn;
-                    node_rec[child + side] = -1;
-                    if (cn <= kSmall)
-                        add_small(small, small_cap, misc, child + side, from);
-                    else
-                        add_item(next, next_chunks, misc, level + 1, item_cap, chunk_cap, slot_cap, child + side, cs, cn,
-                                 box + 6, box + 9);
-                }
-            }
-        }
-        __syncthreads();
+        partition_chunk<false>(it, ch.y, it.axis, it.pos, misc, level, rec, out, sh);
     }
 }
 
@@ -565,14 +651,14 @@ __global__ void __launch_bounds__(kThreads) k_partition(BuildItem* __restrict__ 
 // needs at most 2c - 2 of them, and those of the position range
 // [first, first + c) are scratch[2 first ...)), so that one atomic reserves a
 // contiguous run of nodes and traversal records per subtree.
-//   Bound: issue of dependent warp steps (about 450 instructions a node).  One
-// thread per subtree, with its bins in local memory and two atomics a node,
-// took 7.4 ms for 2,093,058 triangles.
+//   Bound: issue of dependent warp steps and the sweep's shuffles.  2,093,058
+// triangles: 0.82 ms; one thread per subtree, with its bins in local memory
+// and two atomics a node, took 7.4.
 constexpr int kSmallWarps = 4;
 struct SmallWarp {
     float v[9][kSmall];    // box min, box max, centroid
     int id[kSmall];
-    int bins[kBinInts];
+    int bins[kSmallCopies * kCopyInts];
     int2 stack[kSmall];    // (first | count << 8 | scratch node << 16, parent area)
     unsigned char perm[kSmall];
 };
@@ -639,7 +725,13 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(const int2* __restri
                         scale[x] = x_div((float)kBins, x_sub(hi[x], lo[x]));
                     }
                 }
-                for (int k = lane; k < kBinInts; k += 32) reset_bins(W.bins, k);
+#pragma unroll
+                for (int r = 0; r < (kBinInts + 31) / 32; r++) {
+                    const int k = r * 32 + lane;
+                    if (k >= kBinInts) break;
+#pragma unroll
+                    for (int v = 0; v < kSmallCopies; v++) reset_bins(W.bins + v * kCopyInts, k);
+                }
                 __syncwarp();
 #pragma unroll
                 for (int k = 0; k < kSmall / 32; k++) {
@@ -653,18 +745,19 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(const int2* __restri
 #pragma unroll
                     for (int ax = 0; ax < 3; ax++) {
                         if (lo[ax] == hi[ax]) continue;
-                        int* b7 = W.bins + (ax * kBins + bin_of(W.v[6 + ax][p[k]], lo[ax], scale[ax])) * 7;
-                        atomicAdd(b7, 1);
+                        int* bn = W.bins + (lane % kSmallCopies) * kCopyInts + ax * kBins +
+                                  bin_of(W.v[6 + ax][p[k]], lo[ax], scale[ax]);
+                        atomicAdd(bn, 1);
 #pragma unroll
                         for (int x = 0; x < 3; x++) {
-                            atomicMin(b7 + 1 + x, l[x]);
-                            atomicMax(b7 + 4 + x, h[x]);
+                            atomicMin(bn + (1 + x) * kField, l[x]);
+                            atomicMax(bn + (4 + x) * kField, h[x]);
                         }
                     }
                 }
                 __syncwarp();
                 float best, pos;
-                const int axis = warp_sweep(W.bins, lo, hi, area, best, pos);
+                const int axis = warp_sweep<kSmallCopies>(W.bins, lo, hi, area, best, pos);
                 split = !(best >= x_mul((float)cnt, 1.5f) || axis == -1);
                 int L = 0;
                 unsigned left[kSmall / 32];
@@ -934,11 +1027,10 @@ int bvh_build_gpu(pgx_ctx* ctx) {
     for (int level = 0; n > kSmall;) {
         for (const int stop = level + ahead; level < stop && level < kMaxLevels; level++) {
             const int a = level & 1, b = a ^ 1;
-            k_bin<<<grid, kThreads, 0, s>>>(items[a], chunks[a], misc, level, recs[a], a, bins, nodes, small,
-                                            (int)small_cap);
-            k_partition<<<grid, kThreads, 0, s>>>(items[a], chunks[a], misc, level, recs[a], recs[b], b, items[b],
-                                                  chunks[b], (int)item_cap, (int)chunk_cap, (int)slot_cap, small,
-                                                  (int)small_cap, nodes, node_rec);
+            const BuildOut out{recs[b], b, items[b], chunks[b], (int)item_cap, (int)chunk_cap, (int)slot_cap,
+                               small, (int)small_cap, nodes, node_rec};
+            k_bin<<<grid, kThreads, 0, s>>>(items[a], chunks[a], misc, level, recs[a], a, bins, out);
+            k_partition<<<grid, kThreads, 0, s>>>(items[a], chunks[a], misc, level, recs[a], out);
         }
         PGX_CUDA_TRY(ctx, cudaGetLastError());
         int left = 0, bad = 0;

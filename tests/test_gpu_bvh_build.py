@@ -45,7 +45,7 @@ def _soup(n, kind):
 
 
 @pytest.mark.parametrize("kind", ["soup", "coincident", "scales", "flat"])
-@pytest.mark.parametrize("n", [1, 4, 5, 31, 33, 127, 128, 129, 257, 2047, 2048, 2049, 4097, 9001])
+@pytest.mark.parametrize("n", [1, 4, 5, 31, 33, 127, 128, 129, 257, 1023, 1024, 1025, 2047, 2048, 2049, 4097, 9001])
 def test_build_matches_oracle_at_limits(ctx, oracle, n, kind):
     desc = _soup(n, kind)
     ctx.upload(desc)
