@@ -99,6 +99,7 @@ __device__ __forceinline__ float area_x(float mnx, float mny, float mnz, float m
 // bounds (one set of 12 atomics per block).
 __global__ void __launch_bounds__(kThreads) k_prep(const pgx_triangle* __restrict__ tris, int64_t n, RecView out,
                                                    BuildMisc* misc) {
+    grid_begin();
     __shared__ int s_acc[12];
     if (threadIdx.x < 12) s_acc[threadIdx.x] = ((threadIdx.x % 6) < 3) ? INT_MAX : INT_MIN;
     __syncthreads();
@@ -184,6 +185,7 @@ __device__ __forceinline__ void add_small(int2* small, int small_cap, BuildMisc*
 
 __global__ void k_root_init(pgx_bvh_node* nodes, int* node_rec, BuildItem* items, int2* chunks, int2* small,
                             BuildMisc* misc, int64_t n, int item_cap, int chunk_cap, int slot_cap, int small_cap) {
+    grid_begin();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     pgx_bvh_node& r = nodes[0];
     for (int k = 0; k < 3; k++) {
@@ -206,6 +208,7 @@ __device__ __forceinline__ void reset_bins(int* b, int i) {
 }
 
 __global__ void k_bins_reset(int* bins, int64_t n) {
+    grid_begin();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         const int f = (int)(i % kBinInts) / kField;
@@ -530,6 +533,7 @@ __device__ __forceinline__ void partition_chunk(BuildItem& it, int first, int ax
 __global__ void __launch_bounds__(kThreads) k_bin(BuildItem* __restrict__ items, const int2* __restrict__ chunks,
                                                   BuildMisc* __restrict__ misc, int level, RecView rec, int buf,
                                                   int* __restrict__ gbins, BuildOut out) {
+    grid_begin();
     __shared__ int sb[kBinCopies * kCopyInts];
     int* mine = sb + (threadIdx.x % kBinCopies) * kCopyInts;
     __shared__ PartShared sh;
@@ -634,6 +638,7 @@ __global__ void __launch_bounds__(kThreads) k_bin(BuildItem* __restrict__ items,
 __global__ void __launch_bounds__(kThreads) k_partition(BuildItem* __restrict__ items, const int2* __restrict__ chunks,
                                                         BuildMisc* __restrict__ misc, int level, RecView rec,
                                                         BuildOut out) {
+    grid_begin();
     __shared__ PartShared sh;
     if (misc->nslots[level] == 0) return;  // no such node on this level
     const int nchunks = misc->nchunks[level];
@@ -668,6 +673,7 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(const int2* __restri
                                                             int* __restrict__ idx, pgx_bvh_node* __restrict__ nodes,
                                                             int* __restrict__ node_rec,
                                                             pgx_bvh_node* __restrict__ scratch) {
+    grid_begin();
     extern __shared__ __align__(16) uint8_t s_dyn[];
     constexpr unsigned kFull = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
@@ -1013,11 +1019,11 @@ int bvh_build_gpu(pgx_ctx* ctx) {
     for (int k = 0; k < 12; k++) hm.root_acc[k] = ((k % 6) < 3) ? INT_MAX : INT_MIN;
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(misc, &hm, sizeof(hm), cudaMemcpyHostToDevice, s));
     const unsigned wide = 8 * pgx_num_sms();
-    k_prep<<<std::min<unsigned>(blocks_for(n, kThreads), wide), kThreads, 0, s>>>(ctx->tris_in.as<pgx_triangle>(), n,
-                                                                                  recs[0], misc);
-    k_bins_reset<<<blocks_for(kBinInts * slot_cap, 256), 256, 0, s>>>(bins, kBinInts * slot_cap);
-    k_root_init<<<1, 32, 0, s>>>(nodes, node_rec, items[0], chunks[0], small, misc, n, (int)item_cap, (int)chunk_cap,
-                                 (int)slot_cap, (int)small_cap);
+    launch_behind(k_prep, std::min<unsigned>(blocks_for(n, kThreads), wide), kThreads, 0, s,
+                  ctx->tris_in.as<pgx_triangle>(), n, recs[0], misc);
+    launch_behind(k_bins_reset, blocks_for(kBinInts * slot_cap, 256), 256, 0, s, bins, kBinInts * slot_cap);
+    launch_behind(k_root_init, 1, 32, 0, s, nodes, node_rec, items[0], chunks[0], small, misc, n, (int)item_cap,
+                  (int)chunk_cap, (int)slot_cap, (int)small_cap);
     // A level's work list is on the device, so levels are enqueued ahead: the
     // fewest there can be (splits in halves) at once, then two at a time until
     // the list is empty.
@@ -1029,8 +1035,8 @@ int bvh_build_gpu(pgx_ctx* ctx) {
             const int a = level & 1, b = a ^ 1;
             const BuildOut out{recs[b], b, items[b], chunks[b], (int)item_cap, (int)chunk_cap, (int)slot_cap,
                                small, (int)small_cap, nodes, node_rec};
-            k_bin<<<grid, kThreads, 0, s>>>(items[a], chunks[a], misc, level, recs[a], a, bins, out);
-            k_partition<<<grid, kThreads, 0, s>>>(items[a], chunks[a], misc, level, recs[a], out);
+            launch_behind(k_bin, grid, kThreads, 0, s, items[a], chunks[a], misc, level, recs[a], a, bins, out);
+            launch_behind(k_partition, grid, kThreads, 0, s, items[a], chunks[a], misc, level, recs[a], out);
         }
         PGX_CUDA_TRY(ctx, cudaGetLastError());
         int left = 0, bad = 0;
@@ -1048,8 +1054,8 @@ int bvh_build_gpu(pgx_ctx* ctx) {
     PGX_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small, 32 * kSmallWarps, kSmallSmem));
     // about two triangles a leaf at least: no more warps than subtrees of 8 triangles
     const int64_t small_blocks = std::min<int64_t>(n / (8 * kSmallWarps) + 1, (int64_t)pgx_num_sms() * std::max(per_sm, 1));
-    k_small<<<(unsigned)small_blocks, 32 * kSmallWarps, kSmallSmem, s>>>(small, misc, recs[0], recs[1], idx, nodes,
-                                                                         node_rec, ctx->b_tmp.as<pgx_bvh_node>());
+    launch_behind(k_small, (unsigned)small_blocks, 32 * kSmallWarps, kSmallSmem, s, small, misc, recs[0], recs[1],
+                  idx, nodes, node_rec, ctx->b_tmp.as<pgx_bvh_node>());
     PGX_CUDA_TRY(ctx, cudaGetLastError());
     BuildMisc fin{};
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&fin, misc, offsetof(BuildMisc, root_acc), cudaMemcpyDeviceToHost, s));

@@ -81,6 +81,7 @@ __device__ __forceinline__ int longest_axis(const pgx_cache_node& n) {
 }
 
 __global__ void k_bounds_init(int* acc) {
+    grid_begin();
     if (threadIdx.x < 6) acc[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
 }
 
@@ -88,6 +89,7 @@ __global__ void k_bounds_init(int* acc) {
 // bounds (ordered ints; one atomic per block and side).
 __global__ void __launch_bounds__(256) k_pos(const pgx_path_vertex* __restrict__ r, int64_t n, float4* __restrict__ pos,
                                              int* __restrict__ acc) {
+    grid_begin();
     __shared__ int s_acc[6];
     if (threadIdx.x < 6) s_acc[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
     __syncthreads();
@@ -134,6 +136,7 @@ __device__ __forceinline__ void start_item(PItem& it, int node, int offset, int 
 }
 
 __global__ void k_root(int64_t n, PMisc* misc, pgx_cache_node* nodes, PItem* items, int2* small, int* acc) {
+    grid_begin();
     // acc: 6 ordered ints reduced by k_pos
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     pgx_cache_node& r = nodes[0];
@@ -182,6 +185,7 @@ __device__ __forceinline__ bool last_chunk(PItem& it, unsigned nchunks, int* fla
 __global__ void __launch_bounds__(kThreads) k_pselect(PItem* __restrict__ items, unsigned per_item,
                                                       const float4* __restrict__ pos, int* __restrict__ hist,
                                                       int pass) {
+    grid_begin();
     __shared__ int sh[kDigits];
     __shared__ int s_warp[kThreads / 32];
     __shared__ int s_flag;
@@ -257,6 +261,7 @@ __global__ void __launch_bounds__(kThreads) k_ppart(PItem* __restrict__ items, u
                                                     pgx_cache_node* __restrict__ nodes, int2* __restrict__ regions,
                                                     int* __restrict__ node_region, PMisc* __restrict__ misc,
                                                     int region_max) {
+    grid_begin();
     __shared__ int s_wl[kThreads / 32], s_wr[kThreads / 32];
     __shared__ int s_bl, s_br, s_flag;
     __shared__ int s_acc[12];
@@ -427,6 +432,7 @@ __global__ void __launch_bounds__(kSubThreads, 3) k_psubtree(const int2* __restr
                                                           pgx_cache_node* __restrict__ nodes,
                                                           int2* __restrict__ regions, int* __restrict__ node_region,
                                                           int region_max) {
+    grid_begin();
     extern __shared__ __align__(16) uint8_t s_dyn[];
     unsigned long long* xchg = reinterpret_cast<unsigned long long*>(s_dyn);  // [kSmall]: long strides, then source places
     float4* rec = reinterpret_cast<float4*>(s_dyn + sizeof(unsigned long long) * kSmall);  // [kSmall]
@@ -657,6 +663,7 @@ __device__ __forceinline__ unsigned spread_bits(unsigned x) {  // bit i -> bit 2
 __global__ void k_gather(const pgx_path_vertex* __restrict__ in, const float* __restrict__ w_in,
                          const int* __restrict__ idx, int64_t n, pgx_path_vertex* __restrict__ out,
                          float* __restrict__ w_out, float4* __restrict__ pos, unsigned* __restrict__ key_out, int pss) {
+    grid_begin();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int j = idx[i];
@@ -685,6 +692,7 @@ __global__ void k_gather(const pgx_path_vertex* __restrict__ in, const float* __
 }
 
 __global__ void k_trav(const pgx_cache_node* __restrict__ nodes, int64_t nn, CacheTravNode* __restrict__ out) {
+    grid_begin();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nn) return;
     const pgx_cache_node& n = nodes[i];
@@ -696,6 +704,7 @@ __global__ void k_trav(const pgx_cache_node* __restrict__ nodes, int64_t nn, Cac
 }
 
 __global__ void k_regions(const int2* __restrict__ regions, int nreg, float4* __restrict__ pos) {
+    grid_begin();
     int r = blockIdx.x;
     if (r >= nreg) return;
     int2 g = regions[r];
@@ -738,6 +747,7 @@ __global__ void __launch_bounds__(THREADS) k_quadtree(const int2* __restrict__ r
                                                       const unsigned* keys, const float* wts, unsigned* kbuf,
                                                       float* wbuf, int64_t n_all, int* __restrict__ qroot,
                                                       QuadNode* __restrict__ qnodes, int pss, float clamp_median, float refine, float compensate) {
+    grid_begin();
     constexpr int kWarps = THREADS / 32;
     __shared__ int s_cnt[kWarps][32];
     __shared__ float s_f[kWarps], s_g[kWarps];
@@ -1023,6 +1033,7 @@ template <int E>
 __global__ void __launch_bounds__(128) k_knn(const CacheTravNode* __restrict__ nodes, const float4* __restrict__ pos,
                                              int nrec, const float* __restrict__ q, int64_t nq, int k,
                                              int* __restrict__ out_i, float* __restrict__ out_d) {
+    grid_begin();
     constexpr unsigned kFull = 0xFFFFFFFFu;
     __shared__ int s_stack[4][64];
     const int lane = threadIdx.x & 31;
@@ -1307,10 +1318,10 @@ int cache_build_device(pgx_ctx* ctx, const pgx_path_vertex* d_records, int64_t n
     int* acc = reinterpret_cast<int*>(misc + 1);
     int2* regions = cs->regions.as<int2>();
 
-    k_bounds_init<<<1, 32, 0, s>>>(acc);
-    k_pos<<<std::min<unsigned>(blocks_for(n, 256), 8 * pgx_num_sms()), 256, 0, s>>>(cs->recs_in.as<pgx_path_vertex>(), n,
-                                                                                    pos, acc);
-    k_root<<<1, 32, 0, s>>>(n, misc, nodes, items, small, acc);
+    launch_behind(k_bounds_init, 1, 32, 0, s, acc);
+    launch_behind(k_pos, std::min<unsigned>(blocks_for(n, 256), 8 * pgx_num_sms()), 256, 0, s,
+                  cs->recs_in.as<pgx_path_vertex>(), n, pos, acc);
+    launch_behind(k_root, 1, 32, 0, s, n, misc, nodes, items, small, acc);
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(hist, 0, sizeof(int) * kDigits * item_cap, s));
     PGX_CUDA_TRY(ctx, cudaGetLastError());
     float4 *src = pos, *dst = pos2;
@@ -1321,17 +1332,16 @@ int cache_build_device(pgx_ctx* ctx, const pgx_path_vertex* d_records, int64_t n
         const unsigned grid = (unsigned)(per_item * lv.items);
         PGX_CUDA_TRY(ctx, cudaMemsetAsync(&misc->nitems_next, 0, sizeof(int), s));
         for (int pass = 0; pass < kPasses; pass++)
-            k_pselect<<<grid, kThreads, 0, s>>>(items, (unsigned)per_item, src, hist, pass);
-        k_ppart<<<grid, kThreads, 0, s>>>(items, (unsigned)per_item, src, dst, items2, (int)item_cap, small,
-                                          (int)nsmall, dst_buf, nodes, regions, cs->node_region.as<int>(), misc,
-                                          region_max);
+            launch_behind(k_pselect, grid, kThreads, 0, s, items, (unsigned)per_item, src, hist, pass);
+        launch_behind(k_ppart, grid, kThreads, 0, s, items, (unsigned)per_item, src, dst, items2, (int)item_cap,
+                      small, (int)nsmall, dst_buf, nodes, regions, cs->node_region.as<int>(), misc, region_max);
         std::swap(items, items2);
         std::swap(src, dst);
         dst_buf ^= 1;
     }
     PGX_CUDA_TRY(ctx, cudaFuncSetAttribute(k_psubtree, cudaFuncAttributeMaxDynamicSharedMemorySize, kSubSmem));
-    k_psubtree<<<(unsigned)nsmall, kSubThreads, kSubSmem, s>>>(small, misc, pos, pos2, idx, nodes, regions,
-                                                               cs->node_region.as<int>(), region_max);
+    launch_behind(k_psubtree, (unsigned)nsmall, kSubThreads, kSubSmem, s, small, misc, pos, pos2, idx, nodes, regions,
+                  cs->node_region.as<int>(), region_max);
     PGX_CUDA_TRY(ctx, cudaGetLastError());
     cs->n_nodes = total_nodes;
     cs->n_regions = (int)nregions;
@@ -1344,19 +1354,19 @@ int cache_build_device(pgx_ctx* ctx, const pgx_path_vertex* d_records, int64_t n
     // the keys in leaf order start in the buffer that the sort's second pass
     // overwrites, once its first pass has read them
     unsigned* keys = qkey + n;
-    k_gather<<<blocks_for(n, 256), 256, 0, s>>>(cs->recs_in.as<pgx_path_vertex>(),
-                                                d_weights ? cs->wts_in.as<float>() : nullptr, idx, n, recs,
-                                                cs->wts.as<float>(), pos, keys, pss ? 1 : 0);
-    k_trav<<<blocks_for(cs->n_nodes, 256), 256, 0, s>>>(nodes, cs->n_nodes, cs->trav.as<CacheTravNode>());
+    launch_behind(k_gather, blocks_for(n, 256), 256, 0, s, cs->recs_in.as<pgx_path_vertex>(),
+                  d_weights ? cs->wts_in.as<float>() : nullptr, idx, n, recs, cs->wts.as<float>(), pos, keys,
+                  pss ? 1 : 0);
+    launch_behind(k_trav, blocks_for(cs->n_nodes, 256), 256, 0, s, nodes, cs->n_nodes, cs->trav.as<CacheTravNode>());
     // Records carry their region id; leaves below regions are inside them.
-    k_regions<<<(unsigned)nregions, 128, 0, s>>>(regions, cs->n_regions, pos);
+    launch_behind(k_regions, (unsigned)nregions, 128, 0, s, regions, cs->n_regions, pos);
     float* wbuf = reinterpret_cast<float*>(qkey + 2 * n);
     // 512 threads keep a region's serial passes short; small regions are many
     // and need no more than 128 (1,024 records: 8 a thread).
     auto quad = region_max <= 2048 ? k_quadtree<128> : k_quadtree<512>;
-    quad<<<(unsigned)nregions, region_max <= 2048 ? 128 : 512, 0, s>>>(
-        regions, keys, cs->wts.as<float>(), qkey, wbuf, n, cs->qroot.as<int>(), cs->qnodes.as<QuadNode>(), pss ? 1 : 0,
-        clamp_median, refine, compensate);
+    launch_behind(quad, (unsigned)nregions, region_max <= 2048 ? 128 : 512, 0, s, regions, keys, cs->wts.as<float>(),
+                  qkey, wbuf, n, cs->qroot.as<int>(), cs->qnodes.as<QuadNode>(), pss ? 1 : 0, clamp_median, refine,
+                  compensate);
     PGX_CUDA_TRY(ctx, cudaGetLastError());
     PMisc hm{};
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(&hm, misc, sizeof(hm), cudaMemcpyDeviceToHost, s));
@@ -1478,8 +1488,8 @@ extern "C" int pgx_cache_knn(pgx_ctx* ctx, const float* queries, int64_t nq, int
     PGX_CUDA_TRY(ctx, cs->knn_d.reserve(sizeof(float) * k * nq));
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(cs->knn_q.p, queries, sizeof(float) * 3 * nq, cudaMemcpyHostToDevice, s));
     auto knn = k <= 32 ? k_knn<1> : k_knn<2>;
-    knn<<<blocks_for(nq, 4), 128, 0, s>>>(cs->trav.as<CacheTravNode>(), cs->pos.as<float4>(), (int)cs->n_records,
-                                          cs->knn_q.as<float>(), nq, k, cs->knn_i.as<int>(), cs->knn_d.as<float>());
+    launch_behind(knn, blocks_for(nq, 4), 128, 0, s, cs->trav.as<CacheTravNode>(), cs->pos.as<float4>(),
+                  (int)cs->n_records, cs->knn_q.as<float>(), nq, k, cs->knn_i.as<int>(), cs->knn_d.as<float>());
     PGX_CUDA_TRY(ctx, cudaGetLastError());
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(idx, cs->knn_i.p, sizeof(int) * k * nq, cudaMemcpyDeviceToHost, s));
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(d2, cs->knn_d.p, sizeof(float) * k * nq, cudaMemcpyDeviceToHost, s));

@@ -53,6 +53,10 @@ __device__ __forceinline__ xv3 x_cross(xv3 a, xv3 b) {
 }
 __device__ __forceinline__ float comp(xv3 a, int ax) { return ax == 0 ? a.x : (ax == 1 ? a.y : a.z); }
 
+// Where a kernel that launch_behind launches starts: the kernel in front of it
+// on the stream has completed, and its writes are visible.
+__device__ __forceinline__ void grid_begin() { cudaGridDependencySynchronize(); }
+
 // Ordered-int encoding of floats so atomicMin/atomicMax order them like
 // floats (non-NaN inputs).
 __device__ __forceinline__ int f2o(float f) {

@@ -384,6 +384,7 @@ __global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_trace_step
                                                                                 bool with_ext, bool with_shadow,
                                                                                 const BatchInfo* binfo = nullptr,
                                                                                 float4* seen = nullptr) {
+    grid_begin();
     const unsigned n_ext = with_ext ? ps.qcount[ext] : 0u;
     const unsigned n_sh = with_shadow ? ps.scount[ext - 1] : 0u;
     const QueueRays rays{ps, ps.queue[ext & 1]};
@@ -469,8 +470,8 @@ struct LightView {
 // K is the material kind when the launch shades one kind (else -1); INL
 // inlines the environment sampler as well.
 template <int K, bool INL>
-__device__ __forceinline__ bool next_event_t(const SceneView& sv, const LightView& lv, const DevMaterial& m, const Shading& sd, uint64_t& rng,
-                                             float4& so, float4& sdir, F3& contrib, const GuideView& gv, int qroot,
+__device__ __forceinline__ bool next_event_t(const SceneView& sv, const LightView& lv, const DevMaterial& m,
+                                             const Shading& sd, uint64_t& rng, float4& so, float4& sdir, F3& contrib, const GuideView& gv, int qroot,
                                              float frac, const float4* __restrict__ mix) {
     if (bsdf_pure_specular_k<K>(m)) return false;
     if (lv.nlights == 0) return false;
@@ -536,8 +537,8 @@ __device__ __forceinline__ bool next_event_t(const SceneView& sv, const LightVie
     sdir = make_float4(dv.x, dv.y, dv.z, 0.f);
     return true;
 }
-__device__ __noinline__ bool next_event(const SceneView& sv, const LightView& lv, const DevMaterial& m, const Shading& sd, uint64_t& rng,
-                                        float4& so, float4& sdir, F3& contrib, const GuideView& gv, int qroot, float frac,
+__device__ __noinline__ bool next_event(const SceneView& sv, const LightView& lv, const DevMaterial& m,
+                                        const Shading& sd, uint64_t& rng, float4& so, float4& sdir, F3& contrib, const GuideView& gv, int qroot, float frac,
                                         const float4* __restrict__ mix) {
     return next_event_t<-1, false>(sv, lv, m, sd, rng, so, sdir, contrib, gv, qroot, frac, mix);
 }
@@ -612,6 +613,7 @@ constexpr uint32_t kInferCols = 256;  // >= 64 per group, a power of two
 __global__ void __launch_bounds__(128 * kInferGroups, 2) k_guide_infer(SceneView sv, PathState ps, int depth, MlpView mv,
                                                                    int* status, GuideView gv, const int* region_count,
                                                                    int fallback_min) {
+    grid_begin();
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar[kInferGroups];
     __shared__ int flag[kInferGroups];
@@ -724,6 +726,7 @@ constexpr int kClassifyItems = 8;
 constexpr unsigned kClassifyTile = kThreads * kClassifyItems;
 
 __global__ void __launch_bounds__(kThreads) k_classify(SceneView sv, PathState ps, int depth) {
+    grid_begin();
     __shared__ unsigned s_count[kShadeClasses];
     __shared__ unsigned s_base[kShadeClasses];
     const unsigned n = ps.qcount[depth];
@@ -1072,8 +1075,11 @@ struct ClassTiles {
 // and a tail each: five of six bins of a depth are often empty or small (empty
 // launches alone were 20-25 us a depth).
 template <int MODE, bool BATCH>
-__global__ void __launch_bounds__(kThreads, kShadeBlocksPerSM) k_shade(const __grid_constant__ SceneView sv, PathState ps, FrameParams fp, int depth,
-                                                                       const __grid_constant__ GuideView gv, const BatchInfo* binfo = nullptr) {
+__global__ void __launch_bounds__(kThreads, kShadeBlocksPerSM) k_shade(const __grid_constant__ SceneView sv,
+                                                                       PathState ps, FrameParams fp, int depth,
+                                                                       const __grid_constant__ GuideView gv,
+                                                                       const BatchInfo* binfo = nullptr) {
+    grid_begin();
     const ClassTiles tiles(ps, depth);
     int cls;
     unsigned i, n;
@@ -1283,6 +1289,7 @@ __device__ __forceinline__ void finalize_path(const SceneView& sv, const PathSta
 template <int MODE>
 __global__ void __launch_bounds__(kThreads) k_finalize(SceneView sv, PathState ps, FrameParams fp, float* film,
                                                        float* film2) {
+    grid_begin();
     const int64_t npix = (int64_t)sv.width * sv.height;
     const int64_t n = npix * fp.batch;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x)
@@ -1298,8 +1305,9 @@ __global__ void __launch_bounds__(kThreads) k_finalize(SceneView sv, PathState p
 // waiting for each other.  The vertices are shade_path's generic ones, on the
 // same state, so a path's draws, decisions and sums are the wavefront's.
 template <int MODE>
-__global__ void __launch_bounds__(32) k_path(const __grid_constant__ SceneView sv, PathState ps, FrameParams fp, const __grid_constant__ GuideView gv, int lanes, float* film,
-                                             float* film2) {
+__global__ void __launch_bounds__(32) k_path(const __grid_constant__ SceneView sv, PathState ps, FrameParams fp,
+                                              const __grid_constant__ GuideView gv, int lanes, float* film,
+                                              float* film2) {
     const int64_t npix = (int64_t)sv.width * sv.height;
     const int64_t n = npix * fp.batch;
     const int64_t p = (int64_t)blockIdx.x * lanes + threadIdx.x;
@@ -1706,6 +1714,7 @@ __device__ __forceinline__ int diff_camera(const SceneView& sv, const DiffView& 
 // traces only samples with a target and a non-zero adjoint there.
 template <bool GRAD>
 __global__ void __launch_bounds__(kThreads) k_diff_camgen(SceneView sv, PathState ps, DiffView dv) {
+    grid_begin();
     const int64_t npix = (int64_t)sv.width * sv.height;
     const int64_t rounds = (dv.count + (int64_t)gridDim.x * blockDim.x - 1) / ((int64_t)gridDim.x * blockDim.x);
     for (int64_t r = 0; r < rounds; r++) {  // whole warps reach the append
@@ -1799,7 +1808,9 @@ __device__ __forceinline__ void diff_vertex(const SceneView& sv, const DiffView&
 
 // Vertices of this depth, binned by surface class (the tiles of k_shade).
 template <bool GRAD>
-__global__ void __launch_bounds__(kThreads, kShadeBlocksPerSM) k_diff_shade(const __grid_constant__ SceneView sv, PathState ps, DiffView dv, int depth) {
+__global__ void __launch_bounds__(kThreads, kShadeBlocksPerSM) k_diff_shade(const __grid_constant__ SceneView sv,
+                                                                            PathState ps, DiffView dv, int depth) {
+    grid_begin();
     const ClassTiles tiles(ps, depth);
     int cls;
     unsigned i, n;
@@ -2141,29 +2152,27 @@ LaunchCount enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, 
         else if (!fused)
             k_extend<false><<<pg, kThreads, 0, s>>>(sv, ps, depth);
         else
-            k_trace_step<false><<<pg, kThreads, 0, s>>>(sv, ps, depth, true, shadows && depth > 0);
+            launch_behind(k_trace_step<false, kShortStack>, pg, kThreads, 0, s, sv, ps, depth, true, shadows && depth > 0,
+                          nullptr, nullptr);
         if (prof) cudaEventRecord(rs->prof[4 * depth + 1], s);
-        k_classify<<<grid_for((n + kClassifyItems - 1) / kClassifyItems), kThreads, 0, s>>>(sv, ps, depth);
+        launch_behind(k_classify, grid_for((n + kClassifyItems - 1) / kClassifyItems), kThreads, 0, s, sv, ps, depth);
         if (fp.mode == PGX_MODE_GUIDED_MLP && depth < fp.guide_depth) {
             const int64_t tiles = (n + mlp::kRows - 1) / mlp::kRows;
             const int64_t ctas = (tiles + kInferGroups - 1) / kInferGroups;
             const unsigned ig = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ctas, (int64_t)pgx_num_sms() * 2));
-            k_guide_infer<<<ig, 128 * kInferGroups, kInferSmem, s>>>(sv, ps, depth, mv, mlp_status, gv, fb_counts,
+            launch_behind(k_guide_infer, ig, 128 * kInferGroups, kInferSmem, s, sv, ps, depth, mv, mlp_status, gv, fb_counts,
                                                                       fb_min);
             launches++;
         }
+        const auto shade = [&](auto kernel) {
+            launch_behind(kernel, g, kThreads, 0, s, sv, ps, fp, depth, gv, nullptr);
+        };
         switch (fp.mode) {
-            case PGX_MODE_GUIDED_LI: k_shade<PGX_MODE_GUIDED_LI, false><<<g, kThreads, 0, s>>>(sv, ps, fp, depth, gv); break;
-            case PGX_MODE_GUIDED_QUADTREE:
-                k_shade<PGX_MODE_GUIDED_QUADTREE, false><<<g, kThreads, 0, s>>>(sv, ps, fp, depth, gv);
-                break;
-            case PGX_MODE_GUIDED_PSS:
-                k_shade<PGX_MODE_GUIDED_PSS, false><<<g, kThreads, 0, s>>>(sv, ps, fp, depth, gv);
-                break;
-            case PGX_MODE_GUIDED_MLP:
-                k_shade<PGX_MODE_GUIDED_MLP, false><<<g, kThreads, 0, s>>>(sv, ps, fp, depth, gv);
-                break;
-            default: k_shade<PGX_MODE_PLAIN, false><<<g, kThreads, 0, s>>>(sv, ps, fp, depth, gv); break;
+            case PGX_MODE_GUIDED_LI: shade(k_shade<PGX_MODE_GUIDED_LI, false>); break;
+            case PGX_MODE_GUIDED_QUADTREE: shade(k_shade<PGX_MODE_GUIDED_QUADTREE, false>); break;
+            case PGX_MODE_GUIDED_PSS: shade(k_shade<PGX_MODE_GUIDED_PSS, false>); break;
+            case PGX_MODE_GUIDED_MLP: shade(k_shade<PGX_MODE_GUIDED_MLP, false>); break;
+            default: shade(k_shade<PGX_MODE_PLAIN, false>); break;
         }
         launches += 3;
         if (prof) cudaEventRecord(rs->prof[4 * depth + 2], s);
@@ -2177,15 +2186,16 @@ LaunchCount enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, 
         if (prof) cudaEventRecord(rs->prof[4 * depth + 3], s);
     }
     if (fused && shadows) {
-        k_trace_step<false><<<pg, kThreads, 0, s>>>(sv, ps, fp.max_depth + 1, false, true);
+        launch_behind(k_trace_step<false, kShortStack>, pg, kThreads, 0, s, sv, ps, fp.max_depth + 1, false, true, nullptr,
+                      nullptr);
         launches++;
     }
     float* film = ctx->film.as<float>();
     float* film2 = ctx->film2.as<float>();
     if (fp.mode == PGX_MODE_GUIDED_LI)
-        k_finalize<PGX_MODE_GUIDED_LI><<<g, kThreads, 0, s>>>(sv, ps, fp, film, film2);
+        launch_behind(k_finalize<PGX_MODE_GUIDED_LI>, g, kThreads, 0, s, sv, ps, fp, film, film2);
     else
-        k_finalize<PGX_MODE_PLAIN><<<g, kThreads, 0, s>>>(sv, ps, fp, film, film2);
+        launch_behind(k_finalize<PGX_MODE_PLAIN>, g, kThreads, 0, s, sv, ps, fp, film, film2);
     return {launches + 1, fp.max_depth + 1};
 }
 
@@ -2547,11 +2557,13 @@ static void diff_wave(const SceneView& sv, const PathState& ps, const DiffView& 
     k_diff_camgen<GRAD><<<g, kThreads, 0, s>>>(sv, ps, dv);
     auto seen = [&](int depth) { return GRAD && depth > 0 ? ps.rec_w + (size_t)(depth - 1) * dv.stride : nullptr; };
     for (int depth = 0; depth <= dv.max_depth; depth++) {
-        k_trace_step<false><<<pg, kThreads, 0, s>>>(sv, ps, depth, true, depth > 0, nullptr, seen(depth));
-        k_classify<<<cg, kThreads, 0, s>>>(sv, ps, depth);
-        k_diff_shade<GRAD><<<g, kThreads, 0, s>>>(sv, ps, dv, depth);
+        launch_behind(k_trace_step<false, kShortStack>, pg, kThreads, 0, s, sv, ps, depth, true, depth > 0, nullptr,
+                      seen(depth));
+        launch_behind(k_classify, cg, kThreads, 0, s, sv, ps, depth);
+        launch_behind(k_diff_shade<GRAD>, g, kThreads, 0, s, sv, ps, dv, depth);
     }
-    k_trace_step<false><<<pg, kThreads, 0, s>>>(sv, ps, dv.max_depth + 1, false, true, nullptr, seen(dv.max_depth + 1));
+    launch_behind(k_trace_step<false, kShortStack>, pg, kThreads, 0, s, sv, ps, dv.max_depth + 1, false, true, nullptr,
+                  seen(dv.max_depth + 1));
 }
 
 // Paths per wave: the primal's state is about 220 bytes a path, the adjoint's
