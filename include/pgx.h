@@ -212,8 +212,10 @@ typedef struct pgx_render_config {
  * learned guide on the radiance samples that frame's paths produced
  * (pgx_mlp_configure). */
 #define PGX_RENDER_TRAIN_GUIDE 4
-/* Per-stage CUDA-event times only: the kernels are the ones a render without
- * flags runs. */
+/* Per-stage CUDA-event times only, without counting.  The stages are launches
+ * of their own; a render without flags has the same results and, in waves of
+ * up to 2^24 paths, traces extension and shadow rays in one launch (a whole
+ * path, in waves of up to 65,536). */
 #define PGX_RENDER_TIMING 8
 
 /* Statistics of the last pgx_render call.  The per-stage times are filled

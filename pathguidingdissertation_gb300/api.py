@@ -139,7 +139,7 @@ class Context:
                guide_fraction: float = 0.5, record_paths: int | bool = 0, profile: bool = False,
                mitchell: bool = False, train_guide: bool = False, guide_depth: int = 0, timing: bool = False) -> None:
         """profile: per-stage times and traversal counters (counting kernels);
-        timing: per-stage times only (the kernels of an unflagged render)."""
+        timing: per-stage times only, the stages as launches of their own."""
         flags = (abi.RENDER_PROFILE if profile else 0) | (abi.RENDER_FILTER_MITCHELL if mitchell else 0) | \
             (abi.RENDER_TRAIN_GUIDE if train_guide else 0) | (abi.RENDER_TIMING if timing else 0)
         cfg = abi.RenderConfig(mode, max_depth, seed, guide_fraction, int(record_paths), flags, guide_depth)

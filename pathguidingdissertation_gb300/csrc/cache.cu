@@ -412,8 +412,8 @@ __global__ void __launch_bounds__(kThreads) k_ppart(PItem* __restrict__ items, u
 //   A thread holds four neighbouring places in registers: strides of 1 and 2
 // stay in the thread, 4 to 64 are shuffles, and only the 20 of 276 compare
 // steps with longer strides go through shared memory.
-//   Bound: issue of the network (0.9 M records: 0.33 ms with every step in
-// shared memory).  One thread per <= 256-record subtree with an in-place
+//   Bound: issue of the network (0.9 M records: 0.26 ms, and 0.33 with every
+// step in shared memory).  One thread per <= 256-record subtree with an in-place
 // quickselect took 5.1 ms.
 constexpr int kSubThreads = 512;
 constexpr int kSubSlots = kSmall / 8;  // slots of the deepest level
@@ -1028,7 +1028,7 @@ __global__ void __launch_bounds__(THREADS) k_quadtree(const int2* __restrict__ r
 // entries, the insertion point is a popcount, and the tail moves up one lane.
 // The visit order and the comparisons are those of one thread walking the tree
 // with a local list, which took 266 us for 16,384 queries of 8 among 0.9 M
-// records (128 blocks of dependent local-memory accesses).
+// records (128 blocks of dependent local-memory accesses); this takes 140.
 template <int E>
 __global__ void __launch_bounds__(128) k_knn(const CacheTravNode* __restrict__ nodes, const float4* __restrict__ pos,
                                              int nrec, const float* __restrict__ q, int64_t nq, int k,

@@ -377,7 +377,8 @@ __global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_shadow(Sce
 // 40 % of its 5.6 ms; fused 4.64 -> 4.08 ms), and the short shadow rays, last
 // in the counter's order, fill the extension rays' tail.  A wave of 29.5 M
 // paths has nothing to gain from the tails and loses by warps that hold both
-// kinds (76.0 against 77.2 ms), a batch of 10.8 M gains (16.6 -> 16.2 ms).
+// kinds (76.0 against 77.2 ms); batches gain at 10.8 M (16.6 -> 16.2 ms) and at
+// 43 M paths in waves of 32 M (57.6 -> 56.3), and are always fused.
 constexpr int64_t kFusedTracePaths = 1 << 24;
 template <bool BATCH, int SHORT = kShortStack>
 __global__ void __launch_bounds__(kThreads, kPersistentBlocksPerSM) k_trace_step(SceneView sv, PathState ps, int ext,
@@ -774,9 +775,9 @@ __global__ void __launch_bounds__(kThreads) k_classify(SceneView sv, PathState p
 }
 
 // Resident blocks per SM the shading launches are compiled for (64
-// registers).  Measured on the interior workload: the inlined diffuse and
-// conductor kernels spill a little at this bound, and are still faster than
-// at 5-7 blocks per SM without spills or at 10-12 with more spills.
+// registers).  Shading of 1280x720 x 32 of the interior: 21.4 ms; with 5, 6
+// and 7 blocks, which spill less, 25.9, 22.6 and 23.7; with 10, which spill
+// more, 23.0.
 constexpr int kShadeBlocksPerSM = 8;
 
 // One path vertex: shades path p of this depth (whole warps; inactive lanes
@@ -1709,9 +1710,38 @@ __device__ __forceinline__ int diff_camera(const SceneView& sv, const DiffView& 
     return (by - y) * 2 + (bx - x);  // 0..3: which neighbour (right, down)
 }
 
-// Camera rays of one wave of differentiable samples.  The target neighbour of
-// the box filter (diff_camera; -1: outside) is kept with the path; the adjoint
-// traces only samples with a target and a non-zero adjoint there.
+// The camera ray of one differentiable sample.  The target neighbour of the
+// box filter (diff_camera; -1: outside) is kept with the path; the adjoint
+// traces only samples with a target and a non-zero adjoint there (true).
+template <bool GRAD>
+__device__ __forceinline__ bool diff_camgen_path(const SceneView& sv, const PathState& ps, const DiffView& dv,
+                                                 int64_t npix, int64_t i) {
+    const int64_t item = dv.first + i;
+    const int64_t pixel = item % npix;
+    uint64_t rng;
+    F3 dir;
+    const int k = diff_camera(sv, dv, pixel, (int)(item / npix), rng, dir);
+    bool trace = true;
+    if (GRAD) {
+        trace = false;
+        if (k >= 0) {
+            const int64_t tp = (pixel / sv.width + k / 2) * sv.width + (pixel % sv.width + k % 2);
+            trace = dv.dimg[3 * tp] != 0.f || dv.dimg[3 * tp + 1] != 0.f || dv.dimg[3 * tp + 2] != 0.f;
+        }
+    }
+    ps.o[i] = make_float4(sv.cam.origin[0], sv.cam.origin[1], sv.cam.origin[2], 0.f);
+    ps.d[i] = make_float4(dir.x, dir.y, dir.z, 0.f);
+    ps.T[i] = make_float4(1.f, 1.f, 1.f, 0.f);
+    dv.Ts[i] = make_float4(1.f, 1.f, 1.f, 0.f);
+    ps.L[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    ps.pix[i] = make_float2((float)k, 0.f);
+    ps.rng[i] = rng;
+    ps.flags[i] = 0;
+    ps.nrec[i] = 0;
+    return trace;
+}
+
+// Camera rays of one wave of differentiable samples.
 template <bool GRAD>
 __global__ void __launch_bounds__(kThreads) k_diff_camgen(SceneView sv, PathState ps, DiffView dv) {
     grid_begin();
@@ -1719,40 +1749,17 @@ __global__ void __launch_bounds__(kThreads) k_diff_camgen(SceneView sv, PathStat
     const int64_t rounds = (dv.count + (int64_t)gridDim.x * blockDim.x - 1) / ((int64_t)gridDim.x * blockDim.x);
     for (int64_t r = 0; r < rounds; r++) {  // whole warps reach the append
         const int64_t i = (r * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
-        bool trace = false;
-        if (i < dv.count) {
-            const int64_t item = dv.first + i;
-            const int64_t pixel = item % npix;
-            uint64_t rng;
-            F3 dir;
-            const int k = diff_camera(sv, dv, pixel, (int)(item / npix), rng, dir);
-            trace = true;
-            if (GRAD) {
-                trace = false;
-                if (k >= 0) {
-                    const int64_t tp = (pixel / sv.width + k / 2) * sv.width + (pixel % sv.width + k % 2);
-                    trace = dv.dimg[3 * tp] != 0.f || dv.dimg[3 * tp + 1] != 0.f || dv.dimg[3 * tp + 2] != 0.f;
-                }
-            }
-            ps.o[i] = make_float4(sv.cam.origin[0], sv.cam.origin[1], sv.cam.origin[2], 0.f);
-            ps.d[i] = make_float4(dir.x, dir.y, dir.z, 0.f);
-            ps.T[i] = make_float4(1.f, 1.f, 1.f, 0.f);
-            dv.Ts[i] = make_float4(1.f, 1.f, 1.f, 0.f);
-            ps.L[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            ps.pix[i] = make_float2((float)k, 0.f);
-            ps.rng[i] = rng;
-            ps.flags[i] = 0;
-            ps.nrec[i] = 0;
-        }
+        const bool trace = i < dv.count && diff_camgen_path<GRAD>(sv, ps, dv, npix, i);
         const unsigned slot = warp_aggregated_add(&ps.qcount[0], trace);
         if (trace) ps.queue[0][slot] = (int)i;
     }
 }
 
-// One path's vertex at this depth: state in, diff_shade, state, record, queues out.
-template <bool GRAD, int CLS>
+// One path's vertex at this depth: state in, diff_shade, state, record, queues
+// out (QUEUED) or the next rays to the caller.
+template <bool GRAD, int CLS, bool QUEUED = true>
 __device__ __forceinline__ void diff_vertex(const SceneView& sv, const DiffView& dv, PathState& ps, int depth, int p,
-                                            bool active) {
+                                            bool active, NextRays* next = nullptr) {
     DiffPath P;
     DiffVertex V;
     int out = 0;
@@ -1798,7 +1805,13 @@ __device__ __forceinline__ void diff_vertex(const SceneView& sv, const DiffView&
             ps.flags[p] = P.prev_spec ? 1 : 0;
         }
     }
-    if (CLS > 1) {
+    if (!QUEUED) {
+        next->shadow = CLS > 1 && (out & kDiffShadow);
+        next->cont = CLS > 1 && (out & kDiffContinue);
+        next->so = so;
+        next->sdir = make_float4(sdir.x, sdir.y, sdir.z, 0.f);
+        next->c = P.nee;
+    } else if (CLS > 1) {
         push_shadow(ps, depth, p, so, make_float4(sdir.x, sdir.y, sdir.z, 0.f), P.nee, active && (out & kDiffShadow));
         const bool cont = active && (out & kDiffContinue);
         const unsigned slot = warp_aggregated_add(&ps.qcount[depth + 1], cont);
@@ -1825,6 +1838,44 @@ __global__ void __launch_bounds__(kThreads, kShadeBlocksPerSM) k_diff_shade(cons
             case 4: diff_vertex<GRAD, 4>(sv, dv, ps, depth, p, active); break;
             default: diff_vertex<GRAD, 5>(sv, dv, ps, depth, p, active); break;
         }
+    }
+}
+
+// Small waves of differentiable samples: a thread takes its sample from the
+// camera ray to its last vertex, as k_path and for its reasons.
+template <bool GRAD>
+__global__ void __launch_bounds__(32) k_diff_path(const __grid_constant__ SceneView sv, PathState ps,
+                                                  const __grid_constant__ DiffView dv, int lanes) {
+    const int64_t npix = (int64_t)sv.width * sv.height;
+    const int64_t i = (int64_t)blockIdx.x * lanes + threadIdx.x;
+    if (threadIdx.x >= lanes || i >= dv.count || !diff_camgen_path<GRAD>(sv, ps, dv, npix, i)) return;
+    const int p = (int)i;
+    for (int depth = 0; depth <= dv.max_depth; depth++) {
+        const float4 o = ps.o[p], d = ps.d[p];
+        int id, status;
+        float t, u, v;
+        bvh_trace<false>(sv.bvh, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), FLT_MAX, id, t, u, v, status);
+        if (status) id = -1;
+        ps.hit[p] = make_float4(__int_as_float(id), t, u, v);
+        NextRays next;
+        const int cls = id >= 0 ? (int)sv.tri_class[id] : 0;
+        if (cls == 0)
+            diff_vertex<GRAD, 0, false>(sv, dv, ps, depth, p, true, &next);
+        else if (cls == 1)
+            diff_vertex<GRAD, 1, false>(sv, dv, ps, depth, p, true, &next);
+        else
+            diff_vertex<GRAD, 5, false>(sv, dv, ps, depth, p, true, &next);
+        if (next.shadow) {
+            const bool occluded =
+                bvh_trace<true>(sv.bvh, mk(next.so.x, next.so.y, next.so.z), mk(next.sdir.x, next.sdir.y, next.sdir.z),
+                                next.so.w, id, t, u, v, status);
+            if (!occluded && !status) {
+                if (GRAD) reinterpret_cast<int*>(ps.rec_w + (size_t)depth * dv.stride + p)[3] |= kDiffSeen;
+                const float4 l = ps.L[p];
+                ps.L[p] = make_float4(l.x + next.c.x, l.y + next.c.y, l.z + next.c.z, 0.f);
+            }
+        }
+        if (!next.cont) break;
     }
 }
 
@@ -2097,6 +2148,14 @@ SceneView scene_view(pgx_ctx* ctx) {
 // 1843 / 3118.
 constexpr int64_t kPathWave = 1 << 16;
 
+// Paths per warp in k_path and k_diff_path.
+int path_lanes(int64_t n) {
+    const int64_t warps = (int64_t)pgx_num_sms() * 8;  // two a scheduler (4 and 16: within 3 %, 32: up to 1.3x slower)
+    int lanes = 8;                                      // at least (4: 5 % slower, 1: 15 %)
+    while (lanes < 32 && lanes * warps < n) lanes *= 2;
+    return lanes;
+}
+
 // Stage times of one profiled batch (milliseconds).
 struct StageTimes {
     double extend = 0, shade = 0, shadow = 0;
@@ -2123,9 +2182,7 @@ LaunchCount enqueue_frame(pgx_ctx* ctx, RenderState* rs, const FrameParams& fp, 
     const bool cnt = fp.profile > 1;    // counting traversal kernels
     int launches = 0;
     if (!prof && n <= kPathWave && fp.mode != PGX_MODE_GUIDED_MLP) {
-        const int64_t warps = (int64_t)pgx_num_sms() * 8;  // two a scheduler (4 and 16: within 3 %, 32: up to 1.3x slower)
-        int lanes = 8;                                      // at least (4: 5 % slower, 1: 15 %)
-        while (lanes < 32 && lanes * warps < n) lanes *= 2;
+        const int lanes = path_lanes(n);
         const unsigned pb = (unsigned)((n + lanes - 1) / lanes);
         float *f1 = ctx->film.as<float>(), *f2 = ctx->film2.as<float>();
         switch (fp.mode) {
@@ -2545,6 +2602,13 @@ extern "C" int pgx_diff_set_params(pgx_ctx* ctx, const float* env_rgb, const flo
     return diff_params(ctx, state_of(ctx), env_rgb, albedo_offset, roughness);
 }
 
+// Waves of at most this many samples run in k_diff_path.  us per primal +
+// adjoint of depth 10 on fBm terrains (wavefront / k_diff_path): 8,192 samples
+// 1124 / 686, 32,768 1522 / 1078, 65,536 1236 / 934; beyond, it depends on the
+// scene: 131,072 1764 / 1504, 262,144 1905 / 1859 and, of depth 6 on 720,000
+// triangles, 2247 / 2662.
+constexpr int64_t kDiffPathWave = kPathWave;
+
 // Traces one wave of differentiable samples, dv.first ... dv.first + dv.count:
 // camgen -> [trace -> classify -> shade] x (max_depth + 1) -> trace, as
 // enqueue_frame; the caller stores or emits.
@@ -2552,6 +2616,11 @@ template <bool GRAD>
 static void diff_wave(const SceneView& sv, const PathState& ps, const DiffView& dv, cudaStream_t s) {
     const unsigned g = grid_for(dv.count), pg = persistent_grid(dv.count);
     const unsigned cg = grid_for((dv.count + kClassifyItems - 1) / kClassifyItems);
+    if (dv.count <= kDiffPathWave) {
+        const int lanes = path_lanes(dv.count);
+        k_diff_path<GRAD><<<(unsigned)((dv.count + lanes - 1) / lanes), 32, 0, s>>>(sv, ps, dv, lanes);
+        return;
+    }
     cudaMemsetAsync(ps.qcount, 0, sizeof(unsigned) * 4 * (kMaxDepthCap + 2), s);
     cudaMemsetAsync(ps.ccount, 0, sizeof(unsigned) * kShadeClasses * (kMaxDepthCap + 2), s);
     k_diff_camgen<GRAD><<<g, kThreads, 0, s>>>(sv, ps, dv);

@@ -1,5 +1,6 @@
-"""Differentiable renders at the sizes where the wavefront changes: one path,
-partial warps and tiles, one and several waves (2^24 paths of the primal, 2^22
+"""Differentiable renders at the sizes where their kernels change: one path,
+partial warps and tiles, the largest call of one thread per path (65,536) and
+the smallest wavefront, one and several waves (2^24 paths of the primal, 2^22
 of the adjoint), every depth limit end.  On a scene lit by its environment
 alone the image is linear in the texels, so for any adjoint image d:
 <d, image> = <gradient, texels>.  Both sides sum the same float32 terms of one
@@ -17,6 +18,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("size,spp,depth", [((1, 1), 1, 3), ((7, 5), 3, 0), ((33, 31), 5, 16), ((64, 48), 16, 8),
+                                            ((256, 256), 1, 6), ((257, 256), 1, 6),
                                             ((512, 512), 17, 4), ((512, 512), 65, 2)])
 def test_adjoint_is_the_transpose_of_the_primal(ctx, size, spp, depth):
     desc = scenes.terrain(grid=64, seed=4, width=size[0], height=size[1], env_width=64, env_height=32, sun_peak=20.0)
