@@ -188,7 +188,7 @@ static_assert(kTrainSmem <= 227 * 1024, "training tile fits in shared memory");
 constexpr uint32_t kTrainCols = 512;  // 64 (forward / dX) + 6 x 64 (dW^T)
 // Four threads per row.  With one (128 threads, a warp per scheduler) every
 // epilogue and the loss ran at the latency of one dependent chain: 278 us per
-// 262,144 samples, against 140 now.
+// 262,144 samples, against 168 now.
 constexpr int kTrainParts = 4;
 constexpr int kTrainThreads = kRows * kTrainParts;
 constexpr int kPartCols = kHid / kTrainParts;
