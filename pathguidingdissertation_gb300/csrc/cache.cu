@@ -923,7 +923,7 @@ __global__ void __launch_bounds__(THREADS) k_quadtree(const int2* __restrict__ r
             const int2 rg = s_range[node];
             s_beg[i / 5][c] = c == 0 ? rg.x : (c == 4 ? rg.y : lower(rg.x, rg.y, ((s_code[node] << 2) | (unsigned)c) << shift));
         }
-        if (tid < count) s_want[tid] = 0;
+        for (int i = tid; i < count; i += THREADS) s_want[i] = 0;  // a level can hold more nodes than THREADS
         __syncthreads();
         for (int i = warp; i < 4 * count; i += kWarps) {
             const int ni = i >> 2, c = i & 3;
