@@ -3034,7 +3034,8 @@ extern "C" int pgx_batch_render(pgx_batch* b, int32_t spp, uint64_t seed, int32_
     const bool replay = b->graph && b->g_spp == spp && b->g_depth == max_depth &&
                         b->g_tuning.wave_paths == b->tuning.wave_paths &&
                         b->g_tuning.trace_blocks_per_sm == b->tuning.trace_blocks_per_sm &&
-                        b->g_tuning.shade_blocks_per_sm == b->tuning.shade_blocks_per_sm;
+                        b->g_tuning.shade_blocks_per_sm == b->tuning.shade_blocks_per_sm &&
+                        b->g_tuning.stack_shared == b->tuning.stack_shared;
     if (!replay) {
         if (b->graph) cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
