@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "pgx_ctx.h"
@@ -95,6 +96,7 @@ struct PathState {
     int64_t tcapacity;
     int* scene;       // batched rendering: scene of each path
 };
+static_assert(std::has_unique_object_representations_v<PathState>, "compared bytewise");
 
 struct RenderState {
     DevBuf o, d, T, L, hit, pix, rng, flags, nrec, q0, q1, sh_path, sh_o, sh_d, sh_c;
@@ -2786,6 +2788,7 @@ struct pgx_batch {
     cudaGraphExec_t graph = nullptr;
     int g_spp = -1, g_depth = -1;
     pgx_batch_tuning g_tuning{};
+    PathState g_state{};            // the buffers the graph's kernels were given
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int sms = 0;
 };
@@ -3031,7 +3034,11 @@ extern "C" int pgx_batch_render(pgx_batch* b, int32_t spp, uint64_t seed, int32_
     PGX_TRY(batch_state(b, b->tuning));
     PGX_TRY(batch_tables(b, spp, nullptr));
     PGX_CUDA_TRY(h, cudaMemcpyAsync(b->d_seed.p, &seed, sizeof(uint64_t), cudaMemcpyHostToDevice, h->stream));
-    const bool replay = b->graph && b->g_spp == spp && b->g_depth == max_depth &&
+    // The graph holds the path state's addresses: a state that has been
+    // reallocated since (autotuning with larger waves) needs a new one.
+    const PathState state = path_view(state_of(h));
+    const bool replay = b->graph && std::memcmp(&b->g_state, &state, sizeof(state)) == 0 && b->g_spp == spp &&
+                        b->g_depth == max_depth &&
                         b->g_tuning.wave_paths == b->tuning.wave_paths &&
                         b->g_tuning.trace_blocks_per_sm == b->tuning.trace_blocks_per_sm &&
                         b->g_tuning.shade_blocks_per_sm == b->tuning.shade_blocks_per_sm &&
@@ -3054,6 +3061,7 @@ extern "C" int pgx_batch_render(pgx_batch* b, int32_t spp, uint64_t seed, int32_
         b->g_spp = spp;
         b->g_depth = max_depth;
         b->g_tuning = b->tuning;
+        b->g_state = state;
     }
     PGX_CUDA_TRY(h, cudaEventRecord(b->ev0, h->stream));
     PGX_CUDA_TRY(h, cudaGraphLaunch(b->graph, h->stream));
