@@ -34,6 +34,7 @@ struct DevBuf {
         cudaError_t e = cudaMalloc(&p, n);
         if (e != cudaSuccess) {
             p = nullptr;
+            cudaGetLastError();  // reported here, not by the next launch check
             return e;
         }
         bytes = n;

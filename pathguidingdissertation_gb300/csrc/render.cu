@@ -103,13 +103,9 @@ struct RenderState {
     DevBuf rec_pos, rec_nrm, rec_wi, rec_w, rec_e;
     DevBuf counters, vertices, vweight, cqueue, ccount;
     DevBuf guide, fallback, rec_wo, rec_f, train, scene;
-    int64_t capacity = 0;
-    int rec_depth = 0;
-    int64_t guide_capacity = 0;
-    int train_depth = 0;
-    int64_t tcapacity = 0;
+    // What the last ensure_state was asked for.
+    int64_t capacity = 0, vcapacity = 0, tcapacity = 0;
     int64_t train_last = 0;   // samples the previous batch produced
-    int64_t vcapacity = 0;
     int64_t nvertices_last = 0;
     bool vweight_valid = false;  // the last recording wrote flux weights (not guided-Li)
     // captured frame graph
@@ -2015,58 +2011,57 @@ RenderState* state_of(pgx_ctx* ctx) {
     return static_cast<RenderState*>(ctx->render_state);
 }
 
+// Reserves what one call needs: the state of waves of cap paths, with records
+// of rec_depth vertices a path (train_depth of them with the learned guide's
+// fields), vcap recorded vertices and tcap training samples.  Every buffer is
+// asked for its size on every call (a comparison where it is already large
+// enough), so that nothing but the buffers says what is held; when one
+// cannot be had, the wave's buffers are all given back.
 int ensure_state(pgx_ctx* ctx, RenderState* rs, int64_t cap, int rec_depth, int64_t vcap, bool guide = false,
                  int train_depth = 0, int64_t tcap = 0, bool batch = false) {
-    if (cap > rs->capacity) {
-        PGX_CUDA_TRY(ctx, rs->o.reserve(sizeof(float4) * cap));
-        PGX_CUDA_TRY(ctx, rs->d.reserve(sizeof(float4) * cap));
-        PGX_CUDA_TRY(ctx, rs->T.reserve(sizeof(float4) * cap));
-        PGX_CUDA_TRY(ctx, rs->L.reserve(sizeof(float4) * cap));
-        PGX_CUDA_TRY(ctx, rs->hit.reserve(sizeof(float4) * cap));
-        PGX_CUDA_TRY(ctx, rs->pix.reserve(sizeof(float2) * cap));
-        PGX_CUDA_TRY(ctx, rs->rng.reserve(sizeof(uint64_t) * cap));
-        PGX_CUDA_TRY(ctx, rs->flags.reserve(sizeof(int) * cap));
-        PGX_CUDA_TRY(ctx, rs->nrec.reserve(sizeof(int) * cap));
-        PGX_CUDA_TRY(ctx, rs->q0.reserve(sizeof(int) * cap));
-        PGX_CUDA_TRY(ctx, rs->q1.reserve(sizeof(int) * cap));
-        PGX_CUDA_TRY(ctx, rs->sh_path.reserve(sizeof(int) * cap));
-        PGX_CUDA_TRY(ctx, rs->sh_o.reserve(sizeof(float4) * cap));
-        PGX_CUDA_TRY(ctx, rs->sh_d.reserve(sizeof(float4) * cap));
-        PGX_CUDA_TRY(ctx, rs->sh_c.reserve(sizeof(float4) * cap));
-        rs->capacity = cap;
-        rs->rec_depth = 0;
+    const size_t n = (size_t)cap, nrec = (size_t)rec_depth * n, ntrain = (size_t)train_depth * n;
+    const std::pair<DevBuf*, size_t> wave[] = {
+        {&rs->o, sizeof(float4) * n},
+        {&rs->d, sizeof(float4) * n},
+        {&rs->T, sizeof(float4) * n},
+        {&rs->L, sizeof(float4) * n},
+        {&rs->hit, sizeof(float4) * n},
+        {&rs->pix, sizeof(float2) * n},
+        {&rs->rng, sizeof(uint64_t) * n},
+        {&rs->flags, sizeof(int) * n},
+        {&rs->nrec, sizeof(int) * n},
+        {&rs->q0, sizeof(int) * n},
+        {&rs->q1, sizeof(int) * n},
+        {&rs->sh_path, sizeof(int) * n},
+        {&rs->sh_o, sizeof(float4) * n},
+        {&rs->sh_d, sizeof(float4) * n},
+        {&rs->sh_c, sizeof(float4) * n},
+        {&rs->cqueue, sizeof(int) * kShadeClasses * n},
+        {&rs->rec_pos, sizeof(float4) * nrec},
+        {&rs->rec_nrm, sizeof(float4) * nrec},
+        {&rs->rec_wi, sizeof(float4) * nrec},
+        {&rs->rec_w, sizeof(float4) * nrec},
+        {&rs->rec_e, sizeof(float4) * nrec},
+        {&rs->guide, guide ? sizeof(float4) * mlp::kPacked * n : 0},
+        {&rs->fallback, guide ? sizeof(int) * n : 0},
+        {&rs->rec_wo, sizeof(float4) * ntrain},
+        {&rs->rec_f, sizeof(float4) * ntrain},
+        {&rs->train, sizeof(float) * 13 * (size_t)tcap},
+        {&rs->scene, batch ? sizeof(int) * n : 0},
+    };
+    rs->capacity = rs->vcapacity = rs->tcapacity = 0;
+    for (const auto& [buf, bytes] : wave) {
+        const cudaError_t e = bytes ? buf->reserve(bytes) : cudaSuccess;
+        if (e == cudaSuccess) continue;
+        for (const auto& w : wave) w.first->release();
+        return pgx_fail(ctx, PGX_ERR_CUDA, "path state of %lld paths: %s", (long long)cap, cudaGetErrorString(e));
     }
-    if (rec_depth > rs->rec_depth) {
-        size_t nrec = (size_t)rec_depth * rs->capacity;
-        PGX_CUDA_TRY(ctx, rs->rec_pos.reserve(sizeof(float4) * nrec));
-        PGX_CUDA_TRY(ctx, rs->rec_nrm.reserve(sizeof(float4) * nrec));
-        PGX_CUDA_TRY(ctx, rs->rec_wi.reserve(sizeof(float4) * nrec));
-        PGX_CUDA_TRY(ctx, rs->rec_w.reserve(sizeof(float4) * nrec));
-        PGX_CUDA_TRY(ctx, rs->rec_e.reserve(sizeof(float4) * nrec));
-        rs->rec_depth = rec_depth;
-    }
-    if (vcap > rs->vcapacity) {
+    if (sizeof(pgx_path_vertex) * (size_t)vcap > rs->vertices.bytes || sizeof(float) * (size_t)vcap > rs->vweight.bytes)
+        rs->nvertices_last = 0;  // the last recording's vertices go
+    if (vcap > 0) {
         PGX_CUDA_TRY(ctx, rs->vertices.reserve(sizeof(pgx_path_vertex) * vcap));
         PGX_CUDA_TRY(ctx, rs->vweight.reserve(sizeof(float) * vcap));
-        rs->vcapacity = vcap;
     }
-    if (guide && rs->guide_capacity < rs->capacity) {
-        PGX_CUDA_TRY(ctx, rs->guide.reserve(sizeof(float4) * mlp::kPacked * rs->capacity));
-        PGX_CUDA_TRY(ctx, rs->fallback.reserve(sizeof(int) * rs->capacity));
-        rs->guide_capacity = rs->capacity;
-    }
-    if (train_depth > 0 && (train_depth > rs->train_depth || rs->rec_wo.bytes < sizeof(float4) * train_depth * rs->capacity)) {
-        size_t nrec = (size_t)train_depth * rs->capacity;
-        PGX_CUDA_TRY(ctx, rs->rec_wo.reserve(sizeof(float4) * nrec));
-        PGX_CUDA_TRY(ctx, rs->rec_f.reserve(sizeof(float4) * nrec));
-        rs->train_depth = train_depth;
-    }
-    if (tcap > rs->tcapacity) {
-        PGX_CUDA_TRY(ctx, rs->train.reserve(sizeof(float) * 13 * tcap));
-        rs->tcapacity = tcap;
-    }
-    if (batch) PGX_CUDA_TRY(ctx, rs->scene.reserve(sizeof(int) * rs->capacity));
-    PGX_CUDA_TRY(ctx, rs->cqueue.reserve(sizeof(int) * kShadeClasses * rs->capacity));
     PGX_CUDA_TRY(ctx, rs->ccount.reserve(sizeof(unsigned) * kShadeClasses * (kMaxDepthCap + 2)));
     PGX_CUDA_TRY(ctx, rs->counters.reserve(sizeof(unsigned) * 4 * (kMaxDepthCap + 2) + sizeof(unsigned long long) * kStats +
                                            sizeof(unsigned) * 4));
@@ -2075,6 +2070,9 @@ int ensure_state(pgx_ctx* ctx, RenderState* rs, int64_t cap, int rec_depth, int6
         PGX_CUDA_TRY(ctx, cudaEventCreate(&rs->ev1));
         for (int i = 0; i < kProfEvents; i++) PGX_CUDA_TRY(ctx, cudaEventCreate(&rs->prof[i]));
     }
+    rs->capacity = cap;
+    rs->vcapacity = vcap;
+    rs->tcapacity = tcap;
     return PGX_OK;
 }
 
@@ -2272,7 +2270,7 @@ void stage_times(RenderState* rs, int max_depth, StageTimes& t) {
 
 int ensure_film(pgx_ctx* ctx) {
     size_t bytes = sizeof(float) * 3 * (size_t)ctx->width * ctx->height;
-    if (ctx->film.bytes < bytes || !ctx->film.p) {
+    if (ctx->film.bytes < bytes || ctx->film2.bytes < bytes) {
         PGX_CUDA_TRY(ctx, ctx->film.reserve(bytes));
         PGX_CUDA_TRY(ctx, ctx->film2.reserve(bytes));
         PGX_CUDA_TRY(ctx, cudaMemsetAsync(ctx->film.p, 0, bytes, ctx->stream));
@@ -2562,6 +2560,7 @@ int diff_params(pgx_ctx* ctx, RenderState* rs, const float* env_rgb, const float
         if (!(r >= 0.f)) return pgx_fail(ctx, PGX_ERR_INVALID_ARG, "pgx_diff_set_params: roughness must be >= 0");
         m[i].alpha = 1.62142f * sqrtf(r);
     }
+    rs->d_params = false;  // until all of them are in place
     PGX_CUDA_TRY(ctx, rs->d_mats.reserve(sizeof(DevMaterial) * std::max<size_t>(nm, 1)));
     if (nm)
         PGX_CUDA_TRY(ctx, cudaMemcpy(rs->d_mats.p, m.data(), sizeof(DevMaterial) * nm, cudaMemcpyHostToDevice));
