@@ -116,7 +116,7 @@ struct RenderState {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t prof[kProfEvents] = {};
     // differentiable rendering: evaluation parameters and scratch
-    DevBuf d_mats, d_env, d_partial, d_img, d_dimg, d_genv, d_galb, d_grough, d_samples, d_ts, d_rec;
+    DevBuf d_mats, d_env, d_partial, d_img, d_dimg, d_genv, d_galb, d_grough, d_samples, d_ts;
     bool d_params = false;
 };
 
@@ -2018,7 +2018,7 @@ RenderState* state_of(pgx_ctx* ctx) {
 // enough), so that nothing but the buffers says what is held; when one
 // cannot be had, the wave's buffers are all given back.
 int ensure_state(pgx_ctx* ctx, RenderState* rs, int64_t cap, int rec_depth, int64_t vcap, bool guide = false,
-                 int train_depth = 0, int64_t tcap = 0, bool batch = false) {
+                 int train_depth = 0, int64_t tcap = 0, bool batch = false, bool diff = false) {
     const size_t n = (size_t)cap, nrec = (size_t)rec_depth * n, ntrain = (size_t)train_depth * n;
     const std::pair<DevBuf*, size_t> wave[] = {
         {&rs->o, sizeof(float4) * n},
@@ -2048,6 +2048,7 @@ int ensure_state(pgx_ctx* ctx, RenderState* rs, int64_t cap, int rec_depth, int6
         {&rs->rec_f, sizeof(float4) * ntrain},
         {&rs->train, sizeof(float) * 13 * (size_t)tcap},
         {&rs->scene, batch ? sizeof(int) * n : 0},
+        {&rs->d_ts, diff ? sizeof(float4) * n : 0},
     };
     rs->capacity = rs->vcapacity = rs->tcapacity = 0;
     for (const auto& [buf, bytes] : wave) {
@@ -2585,7 +2586,7 @@ DiffView diff_view(pgx_ctx* ctx, RenderState* rs, int spp, uint64_t seed, int ma
     dv.seed = seed;
     dv.max_depth = max_depth;
     dv.nmats = ctx->nmats;
-    dv.Ts = rs->d_ts.as<float4>();  // reserved by the caller
+    dv.Ts = rs->d_ts.as<float4>();  // reserved by diff_state
     return dv;
 }
 
@@ -2636,9 +2637,25 @@ static void diff_wave(const SceneView& sv, const PathState& ps, const DiffView& 
                   seen(dv.max_depth + 1));
 }
 
-// Paths per wave: the primal's state is about 220 bytes a path, the adjoint's
+// Paths per wave: the state is about 200 bytes a path, and the adjoint's
 // records add 80 bytes a path and depth (5.6 GB at 2^22 paths and depth 16).
-constexpr int64_t kDiffWave = 1 << 24, kDiffGradWave = 1 << 22;
+// 512x512 x 64 of the 2,093,058-triangle terrain, depth 8, ms: primal in waves
+// of 2^20 / 22 / 23 / 24 30.0 / 18.6 / 16.8 / 16.0, adjoint in waves of
+// 2^18 / 20 / 21 / 22 82.8 / 36.0 / 27.7 / 23.6.
+constexpr int64_t kDiffWave = 1 << 24, kDiffGradWave = 1 << 22, kDiffLeastWave = 1 << 10;
+
+// Reserves the state of one wave, with vertex records of rec_depth depths:
+// `wave` paths, or half as many until it fits the memory there is.  The
+// results do not depend on the wave (the adjoint's only by the order of its
+// double sums).
+static int diff_state(pgx_ctx* ctx, RenderState* rs, int64_t& wave, int rec_depth) {
+    for (;;) {
+        const int rc = ensure_state(ctx, rs, wave, rec_depth, 0, false, 0, 0, false, true);
+        if (rc == PGX_OK || wave <= kDiffLeastWave) return rc;
+        wave = (wave + 1) / 2;
+        ctx->err.clear();
+    }
+}
 
 extern "C" int pgx_diff_render(pgx_ctx* ctx, int32_t spp, uint64_t seed, int32_t max_depth, double* image) {
     PGX_TRY(diff_check(ctx, "pgx_diff_render"));
@@ -2651,10 +2668,9 @@ extern "C" int pgx_diff_render(pgx_ctx* ctx, int32_t spp, uint64_t seed, int32_t
     PGX_CUDA_TRY(ctx, rs->d_img.reserve(sizeof(double) * 3 * npix));
     // sample values of up to 1 GiB at a time
     const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(spp, ((int64_t)1 << 30) / (16 * npix)));
-    const int64_t wave = std::min<int64_t>(npix * chunk, kDiffWave);
+    int64_t wave = std::min<int64_t>(npix * chunk, kDiffWave);
     PGX_CUDA_TRY(ctx, rs->d_samples.reserve(sizeof(float4) * (size_t)npix * chunk));
-    PGX_CUDA_TRY(ctx, rs->d_ts.reserve(sizeof(float4) * wave));
-    PGX_TRY(ensure_state(ctx, rs, wave, 0, 0));
+    PGX_TRY(diff_state(ctx, rs, wave, 0));
     DiffView dv = diff_view(ctx, rs, spp, seed, max_depth);
     dv.partial = rs->d_partial.as<double>();
     dv.samples = rs->d_samples.as<float4>();
@@ -2690,16 +2706,14 @@ extern "C" int pgx_diff_adjoint(pgx_ctx* ctx, int32_t spp, uint64_t seed, int32_
     const int64_t npix = (int64_t)ctx->width * ctx->height;
     const size_t ef = env_floats(ctx), nm = (size_t)ctx->nmats;
     cudaStream_t s = ctx->stream;
-    const int64_t wave = std::min<int64_t>(npix * spp, kDiffGradWave);
+    int64_t wave = std::min<int64_t>(npix * spp, kDiffGradWave);
     PGX_CUDA_TRY(ctx, rs->d_dimg.reserve(sizeof(float) * 3 * npix));
     // Gradients are accumulated in double (millions of atomic additions
     // into the popular texels) and returned as float.
     PGX_CUDA_TRY(ctx, rs->d_genv.reserve(sizeof(double) * std::max<size_t>(ef, 1)));
     PGX_CUDA_TRY(ctx, rs->d_galb.reserve(sizeof(double) * std::max<size_t>(3 * nm, 1)));
     PGX_CUDA_TRY(ctx, rs->d_grough.reserve(sizeof(double) * std::max<size_t>(nm, 1)));
-    PGX_CUDA_TRY(ctx, rs->d_ts.reserve(sizeof(float4) * wave));
-    PGX_CUDA_TRY(ctx, rs->d_rec.reserve(5 * sizeof(float4) * (size_t)wave * (max_depth + 1)));
-    PGX_TRY(ensure_state(ctx, rs, wave, 0, 0));
+    PGX_TRY(diff_state(ctx, rs, wave, max_depth + 1));
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(rs->d_dimg.p, dloss_dimage, sizeof(float) * 3 * npix, cudaMemcpyHostToDevice, s));
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(rs->d_genv.p, 0, sizeof(double) * std::max<size_t>(ef, 1), s));
     PGX_CUDA_TRY(ctx, cudaMemsetAsync(rs->d_galb.p, 0, sizeof(double) * std::max<size_t>(3 * nm, 1), s));
@@ -2713,8 +2727,6 @@ extern "C" int pgx_diff_adjoint(pgx_ctx* ctx, int32_t spp, uint64_t seed, int32_
     SceneView sv = scene_view(ctx);
     PathState ps = path_view(rs);
     dv.stride = wave;
-    float4** rec[5] = {&ps.rec_pos, &ps.rec_nrm, &ps.rec_wi, &ps.rec_w, &ps.rec_e};
-    for (int k = 0; k < 5; k++) *rec[k] = rs->d_rec.as<float4>() + (size_t)k * wave * (max_depth + 1);
     for (int64_t at = 0; at < npix * spp; at += wave) {
         dv.first = at;
         dv.count = std::min(wave, npix * spp - at);
