@@ -560,7 +560,8 @@ int pgx_mlp_set_fallback(pgx_ctx* ctx, int32_t min_samples);
  * the sampling held fixed is an unbiased estimate of the image's gradient. */
 
 /* Sets the evaluation parameters; NULL keeps the uploaded value (env W*H*3,
- * albedo_offset nmats*3 -- zero is the uploaded albedo -- roughness nmats). */
+ * albedo_offset nmats*3 -- zero is the uploaded albedo -- roughness nmats).
+ * They belong to the uploaded scene: the next upload starts from its own. */
 int pgx_diff_set_params(pgx_ctx* ctx, const float* env_rgb, const float* albedo_offset, const float* roughness);
 /* Mean of spp samples per pixel (seeds hash(seed, pixel, sample)) in double,
  * summed in a fixed order, so two calls differ only through the samples a

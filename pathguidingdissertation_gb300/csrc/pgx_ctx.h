@@ -148,6 +148,7 @@ struct pgx_ctx {
     pgx_camera host_camera{};
     SceneBoundsDev bounds{};
     bool has_scene = false;
+    uint64_t scene_generation = 0;  // counts uploads
 
     // environment map
     DevBuf env_texels, env_cond_func, env_cond_cdf, env_cond_int, env_marg_func, env_marg_cdf;

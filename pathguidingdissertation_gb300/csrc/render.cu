@@ -117,7 +117,7 @@ struct RenderState {
     cudaEvent_t prof[kProfEvents] = {};
     // differentiable rendering: evaluation parameters and scratch
     DevBuf d_mats, d_env, d_partial, d_img, d_dimg, d_genv, d_galb, d_grough, d_samples, d_ts;
-    bool d_params = false;
+    uint64_t d_scene = 0;  // upload the evaluation parameters belong to (0: none)
 };
 
 struct SceneView {
@@ -2561,7 +2561,7 @@ int diff_params(pgx_ctx* ctx, RenderState* rs, const float* env_rgb, const float
         if (!(r >= 0.f)) return pgx_fail(ctx, PGX_ERR_INVALID_ARG, "pgx_diff_set_params: roughness must be >= 0");
         m[i].alpha = 1.62142f * sqrtf(r);
     }
-    rs->d_params = false;  // until all of them are in place
+    rs->d_scene = 0;  // until all of them are in place
     PGX_CUDA_TRY(ctx, rs->d_mats.reserve(sizeof(DevMaterial) * std::max<size_t>(nm, 1)));
     if (nm)
         PGX_CUDA_TRY(ctx, cudaMemcpy(rs->d_mats.p, m.data(), sizeof(DevMaterial) * nm, cudaMemcpyHostToDevice));
@@ -2573,7 +2573,7 @@ int diff_params(pgx_ctx* ctx, RenderState* rs, const float* env_rgb, const float
         else
             PGX_CUDA_TRY(ctx, cudaMemcpy(rs->d_env.p, ctx->env.texels, sizeof(float) * ef, cudaMemcpyDeviceToDevice));
     }
-    rs->d_params = true;
+    rs->d_scene = ctx->scene_generation;
     return PGX_OK;
 }
 
@@ -2662,7 +2662,7 @@ extern "C" int pgx_diff_render(pgx_ctx* ctx, int32_t spp, uint64_t seed, int32_t
     PGX_TRY(diff_args(ctx, spp, max_depth, "pgx_diff_render"));
     if (!image) return pgx_fail(ctx, PGX_ERR_INVALID_ARG, "pgx_diff_render: null image");
     RenderState* rs = state_of(ctx);
-    if (!rs->d_params) PGX_TRY(diff_params(ctx, rs, nullptr, nullptr, nullptr));
+    if (rs->d_scene != ctx->scene_generation) PGX_TRY(diff_params(ctx, rs, nullptr, nullptr, nullptr));
     const int64_t npix = (int64_t)ctx->width * ctx->height;
     PGX_CUDA_TRY(ctx, rs->d_partial.reserve(sizeof(double) * 12 * npix));
     PGX_CUDA_TRY(ctx, rs->d_img.reserve(sizeof(double) * 3 * npix));
@@ -2702,7 +2702,7 @@ extern "C" int pgx_diff_adjoint(pgx_ctx* ctx, int32_t spp, uint64_t seed, int32_
     PGX_TRY(diff_args(ctx, spp, max_depth, "pgx_diff_adjoint"));
     if (!dloss_dimage) return pgx_fail(ctx, PGX_ERR_INVALID_ARG, "pgx_diff_adjoint: null dloss_dimage");
     RenderState* rs = state_of(ctx);
-    if (!rs->d_params) PGX_TRY(diff_params(ctx, rs, nullptr, nullptr, nullptr));
+    if (rs->d_scene != ctx->scene_generation) PGX_TRY(diff_params(ctx, rs, nullptr, nullptr, nullptr));
     const int64_t npix = (int64_t)ctx->width * ctx->height;
     const size_t ef = env_floats(ctx), nm = (size_t)ctx->nmats;
     cudaStream_t s = ctx->stream;

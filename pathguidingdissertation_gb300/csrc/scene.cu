@@ -268,6 +268,7 @@ extern "C" int pgx_scene_upload(pgx_ctx* ctx, const pgx_triangle* tris, int64_t 
     cudaStream_t s = ctx->stream;
     ctx->has_scene = false;
     ctx->has_bvh = false;
+    ctx->scene_generation++;
     ctx->ntris = ntris;
     ctx->nmats = nmats;
     ctx->host_mats.assign(mats, mats + nmats);
