@@ -1021,14 +1021,87 @@ __global__ void __launch_bounds__(THREADS) k_quadtree(const int2* __restrict__ r
     }
 }
 
-// k nearest records per query (ascending distance, ties to lower index), one
-// warp per query.  The best list lives in the lanes (entry e of lane l is rank
+// A warp per query shortens each query, a thread per query does more of them at
+// once.  Time with a warp over time with a thread, 1 M records on the faces
+// of a box, queries near them:
+//   queries    k = 1    4     8     12    16    24    32    64
+//     16,384   0.75  0.62  0.54  0.47  0.39  0.31  0.25  0.17
+//     65,536   1.40  1.13  0.99  0.82  0.71  0.55  0.42  0.22
+//    131,072   2.02  1.57  1.26  1.01  0.87  0.67  0.48  0.32
+//    262,144   2.31  1.75  1.42  1.15  0.99  0.70  0.60  0.31
+//  1,000,000   3.16  2.28  1.06  1.36  1.17  0.85  0.64  0.34
+// (records in the box's volume: 1.1 to 1.3 times these; 1,000, 100,000 and
+// 4 M records much the same).  The line runs where threads begin to win, and
+// leaves lists above 16 to warps.
+constexpr int kKnnThreadK = 16;
+inline bool knn_per_thread(int64_t nq, int k) { return k <= kKnnThreadK && nq >= 16384 + 6144 * (int64_t)k; }
+
+// The k nearest records of a query, ascending by distance, ties to the lower
+// index: (d, i) is behind (d2, i2).
+__device__ __forceinline__ bool knn_behind(float d, int i, float d2, int i2) { return d > d2 || (d == d2 && i > i2); }
+__device__ __forceinline__ float knn_box(const CacheTravNode& c, float x, float y, float z) {
+    const float dx = fmaxf(fmaxf(c.bmin.x - x, x - c.bmax.x), 0.f);
+    const float dy = fmaxf(fmaxf(c.bmin.y - y, y - c.bmax.y), 0.f);
+    const float dz = fmaxf(fmaxf(c.bmin.z - z, z - c.bmax.z), 0.f);
+    return dx * dx + dy * dy + dz * dz;
+}
+
+// Many queries of few neighbours: one thread per query with its list and
+// stack in local memory.
+__global__ void __launch_bounds__(128) k_knn_thread(const CacheTravNode* __restrict__ nodes,
+                                                    const float4* __restrict__ pos, int nrec,
+                                                    const float* __restrict__ q, int64_t nq, int k,
+                                                    int* __restrict__ out_i, float* __restrict__ out_d) {
+    grid_begin();
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nq) return;
+    const float x = q[3 * t], y = q[3 * t + 1], z = q[3 * t + 2];
+    float bd[kKnnThreadK];
+    int bi[kKnnThreadK];
+    int cnt = 0;
+    int stack[64];
+    int sp = 0;
+    if (nrec > 0) stack[sp++] = 0;
+    while (sp > 0) {
+        const CacheTravNode n = nodes[stack[--sp]];
+        const float lim = cnt < k ? FLT_MAX : bd[k - 1];
+        if (knn_box(n, x, y, z) > lim) continue;
+        const int l = __float_as_int(n.bmin.w), r = __float_as_int(n.bmax.w);
+        if (l < 0) {
+            const int off = -l - 1;
+            for (int id = off; id < off + r; id++) {
+                const float4 p = pos[id];
+                const float dx = p.x - x, dy = p.y - y, dz = p.z - z;
+                const float d = dx * dx + dy * dy + dz * dz;
+                if (cnt == k && !knn_behind(bd[k - 1], bi[k - 1], d, id)) continue;
+                int m = cnt < k ? cnt++ : k - 1;
+                for (; m > 0 && knn_behind(bd[m - 1], bi[m - 1], d, id); m--) {
+                    bd[m] = bd[m - 1];
+                    bi[m] = bi[m - 1];
+                }
+                bd[m] = d;
+                bi[m] = id;
+            }
+        } else if (sp + 2 <= 64) {
+            // the nearer child is pushed last and entered first
+            const bool left_first = knn_box(nodes[l], x, y, z) < knn_box(nodes[r], x, y, z);
+            stack[sp++] = left_first ? r : l;
+            stack[sp++] = left_first ? l : r;
+        }
+    }
+    for (int j = 0; j < k; j++) {
+        out_i[t * k + j] = j < cnt ? bi[j] : -1;
+        out_d[t * k + j] = j < cnt && bd[j] != FLT_MAX ? bd[j] : INFINITY;
+    }
+}
+
+// One warp per query.  The best list lives in the lanes (entry e of lane l is rank
 // 32 e + l, kept sorted); a leaf's records are tested by one lane each and the
 // ones that improve the list are inserted in turn: every lane compares its
 // entries, the insertion point is a popcount, and the tail moves up one lane.
-// The visit order and the comparisons are those of one thread walking the tree
-// with a local list, which took 266 us for 16,384 queries of 8 among 0.9 M
-// records (128 blocks of dependent local-memory accesses); this takes 140.
+// The visit order and the comparisons are those of k_knn_thread.  16,384
+// queries of 8 among 0.9 M records: 140 us, and 266 with a thread each (128
+// blocks of dependent local-memory accesses).
 template <int E>
 __global__ void __launch_bounds__(128) k_knn(const CacheTravNode* __restrict__ nodes, const float4* __restrict__ pos,
                                              int nrec, const float* __restrict__ q, int64_t nq, int k,
@@ -1051,13 +1124,6 @@ __global__ void __launch_bounds__(128) k_knn(const CacheTravNode* __restrict__ n
     int cnt = 0;
     float worst_d = FLT_MAX;  // rank k - 1 once k records are known
     int worst_i = INT_MAX;
-    auto worse = [&](float d, int i, float d2, int i2) { return d > d2 || (d == d2 && i > i2); };
-    auto box_d = [&](const CacheTravNode& c) {
-        float dx = fmaxf(fmaxf(c.bmin.x - x, x - c.bmax.x), 0.f);
-        float dy = fmaxf(fmaxf(c.bmin.y - y, y - c.bmax.y), 0.f);
-        float dz = fmaxf(fmaxf(c.bmin.z - z, z - c.bmax.z), 0.f);
-        return dx * dx + dy * dy + dz * dz;
-    };
     if (nrec > 0) {
         int sp = 0;
         if (lane == 0) stack[0] = 0;
@@ -1067,7 +1133,7 @@ __global__ void __launch_bounds__(128) k_knn(const CacheTravNode* __restrict__ n
             const int ni = stack[--sp];
             const CacheTravNode n = nodes[ni];
             const float lim = cnt < k ? FLT_MAX : worst_d;
-            if (box_d(n) > lim) continue;
+            if (knn_box(n, x, y, z) > lim) continue;
             const int l = __float_as_int(n.bmin.w), r = __float_as_int(n.bmax.w);
             if (l < 0) {
                 const int off = -l - 1;
@@ -1086,13 +1152,13 @@ __global__ void __launch_bounds__(128) k_knn(const CacheTravNode* __restrict__ n
                         todo &= todo - 1;
                         const float cd = __shfl_sync(kFull, d, src);
                         const int ci = off + j0 + src;
-                        if (cnt == k && !worse(worst_d, worst_i, cd, ci)) continue;
+                        if (cnt == k && !knn_behind(worst_d, worst_i, cd, ci)) continue;
                         if (cnt < k) cnt++;
                         // entries that stay in front of the new one
                         int at = 0;
 #pragma unroll
                         for (int e = 0; e < E; e++)
-                            at += __popc(__ballot_sync(kFull, bi[e] != INT_MAX && !worse(bd[e], bi[e], cd, ci)));
+                            at += __popc(__ballot_sync(kFull, bi[e] != INT_MAX && !knn_behind(bd[e], bi[e], cd, ci)));
 #pragma unroll
                         for (int e = E - 1; e >= 0; e--) {
                             float pd = __shfl_up_sync(kFull, bd[e], 1);
@@ -1122,7 +1188,7 @@ __global__ void __launch_bounds__(128) k_knn(const CacheTravNode* __restrict__ n
                     }
                 }
             } else if (sp + 2 <= 64) {
-                const float da = box_d(nodes[l]), db = box_d(nodes[r]);
+                const float da = knn_box(nodes[l], x, y, z), db = knn_box(nodes[r], x, y, z);
                 const bool left_first = da < db;  // the one entered first is pushed last
                 __syncwarp();
                 if (lane == 0) {
@@ -1487,8 +1553,9 @@ extern "C" int pgx_cache_knn(pgx_ctx* ctx, const float* queries, int64_t nq, int
     PGX_CUDA_TRY(ctx, cs->knn_i.reserve(sizeof(int) * k * nq));
     PGX_CUDA_TRY(ctx, cs->knn_d.reserve(sizeof(float) * k * nq));
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(cs->knn_q.p, queries, sizeof(float) * 3 * nq, cudaMemcpyHostToDevice, s));
-    auto knn = k <= 32 ? k_knn<1> : k_knn<2>;
-    launch_behind(knn, blocks_for(nq, 4), 128, 0, s, cs->trav.as<CacheTravNode>(), cs->pos.as<float4>(),
+    const bool per_thread = knn_per_thread(nq, k);
+    auto knn = per_thread ? k_knn_thread : (k <= 32 ? k_knn<1> : k_knn<2>);
+    launch_behind(knn, blocks_for(nq, per_thread ? 128 : 4), 128, 0, s, cs->trav.as<CacheTravNode>(), cs->pos.as<float4>(),
                   (int)cs->n_records, cs->knn_q.as<float>(), nq, k, cs->knn_i.as<int>(), cs->knn_d.as<float>());
     PGX_CUDA_TRY(ctx, cudaGetLastError());
     PGX_CUDA_TRY(ctx, cudaMemcpyAsync(idx, cs->knn_i.p, sizeof(int) * k * nq, cudaMemcpyDeviceToHost, s));
