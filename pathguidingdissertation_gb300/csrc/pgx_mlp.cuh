@@ -114,10 +114,8 @@ __device__ __forceinline__ void encode_row(uint8_t* tile, int r, const Bounds& b
 }
 
 // ---- the vMF mixture --------------------------------------------------------------
-// Per query the renderer keeps 10 float4: lobe i = (mu.xyz, kappa) for
-// i < 8, then the 8 lobe weights.
 struct Mixture {
-    float4 lobe[kLobes];
+    float4 lobe[kLobes];  // (mu.xyz, kappa)
     float w[kLobes];
 };
 
@@ -151,43 +149,6 @@ __device__ __forceinline__ float vmf_pdf(float4 l, F3 w) {
     float cosv = l.x * w.x + l.y * w.y + l.z * w.z;
     float norm = k / (2.f * 3.14159265f * (-expm1f(-2.f * k)));
     return norm * expf(k * (cosv - 1.f));
-}
-
-__device__ __forceinline__ float mixture_pdf(const Mixture& m, F3 w) {
-    float p = 0.f;
-#pragma unroll
-    for (int i = 0; i < kLobes; i++) p += m.w[i] * vmf_pdf(m.lobe[i], w);
-    return p;
-}
-
-// Lobe chosen by u0, then w = 1 + log(u1 + (1 - u1) e^{-2 kappa}) / kappa
-// about mu and a uniform azimuth 2 pi u2.
-__device__ __forceinline__ F3 mixture_sample(const Mixture& m, float u0, float u1, float u2) {
-    int pick = kLobes - 1;
-    float acc = 0.f;
-#pragma unroll
-    for (int i = 0; i < kLobes; i++) {
-        acc += m.w[i];
-        if (u0 < acc && pick == kLobes - 1 && i < kLobes - 1) pick = i;
-    }
-    float4 l = m.lobe[0];
-#pragma unroll
-    for (int i = 1; i < kLobes; i++)
-        if (i == pick) l = m.lobe[i];
-    float k = l.w;
-    float cw = 1.f + logf(u1 + (1.f - u1) * expf(-2.f * k)) / k;
-    cw = fminf(fmaxf(cw, -1.f), 1.f);
-    float sw = sqrtf(fmaxf(0.f, 1.f - cw * cw));
-    float s, c;
-    sincospif(2.f * u2, &s, &c);
-    F3 mu = f3(l.x, l.y, l.z);
-    // orthonormal basis about mu (Duff et al. 2017)
-    float sign = copysignf(1.f, mu.z);
-    float a = -1.f / (sign + mu.z);
-    float bb = mu.x * mu.y * a;
-    F3 t = f3(1.f + sign * mu.x * mu.x * a, sign * bb, -sign * mu.x);
-    F3 bt = f3(bb, sign + mu.y * mu.y * a, -mu.y);
-    return normalize(t * (sw * c) + bt * (sw * s) + mu * cw);
 }
 
 // ---- packed mixture, as the renderer keeps it per path ------------------------------

@@ -108,11 +108,6 @@ struct RenderState {
     int64_t train_last = 0;   // samples the previous batch produced
     int64_t nvertices_last = 0;
     bool vweight_valid = false;  // the last recording wrote flux weights (not guided-Li)
-    // captured frame graph
-    cudaGraphExec_t graph = nullptr;
-    int graph_mode = -1, graph_depth = -1, graph_batch = -1, graph_record = -1;
-    uint64_t graph_seed = 0;
-    int graph_spp0 = -1;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t prof[kProfEvents] = {};
     // differentiable rendering: evaluation parameters and scratch
@@ -2286,7 +2281,6 @@ int ensure_film(pgx_ctx* ctx) {
 void render_state_free(pgx_ctx* ctx) {
     RenderState* rs = static_cast<RenderState*>(ctx->render_state);
     if (!rs) return;
-    if (rs->graph) cudaGraphExecDestroy(rs->graph);
     if (rs->ev0) cudaEventDestroy(rs->ev0);
     if (rs->ev1) cudaEventDestroy(rs->ev1);
     for (int i = 0; i < kProfEvents; i++)
