@@ -213,9 +213,11 @@ typedef struct pgx_render_config {
  * (pgx_mlp_configure). */
 #define PGX_RENDER_TRAIN_GUIDE 4
 /* Per-stage CUDA-event times only, without counting.  The stages are launches
- * of their own; a render without flags has the same results and, in waves of
- * up to 2^24 paths, traces extension and shadow rays in one launch (a whole
- * path, in waves of up to 65,536). */
+ * of their own.  A render without flags traces the same paths, with the film's
+ * float sums in another order; in waves of up to 2^24 paths it traces
+ * extension and shadow rays in one launch, and in waves of up to 65,536, other
+ * than the learned guide's, whole paths.  The times are those of the separate
+ * launches and add up to more than such a render takes. */
 #define PGX_RENDER_TIMING 8
 
 /* Statistics of the last pgx_render call.  The per-stage times are filled
@@ -550,7 +552,7 @@ int pgx_mlp_set_fallback(pgx_ctx* ctx, int32_t min_samples);
 
 /* ---- differentiable rendering (extension; the reference renders forward only) ----
  * Plain path tracing with NEE + MIS (PGX_MODE_PLAIN's estimator, box
- * filter, one thread per pixel) whose sampling decisions -- directions,
+ * filter) whose sampling decisions -- directions,
  * pdfs, MIS weights, Russian roulette and the environment's sampling
  * tables -- use the uploaded scene, while radiance is evaluated with the
  * "evaluation parameters": environment texels, a per-material albedo

@@ -63,7 +63,7 @@ struct DevMaterial {
     int constant;      // alb holds the texture
 };
 
-// Shading class of a surface (the wavefront shades one class per launch):
+// Shading class of a surface (the wavefront shades a depth's paths class by class):
 // 1 emitter, 2 diffuse, 3 conductor, 4 glass, 5 other; 0 is a miss.
 __host__ __device__ inline unsigned char shade_class(const DevMaterial& m) {
     return m.is_light ? 1 : (m.kind == PGX_BSDF_DIFFUSE ? 2 : (m.kind == PGX_BSDF_CONDUCTOR ? 3 : (m.kind == PGX_BSDF_GLASS ? 4 : 5)));
@@ -211,13 +211,14 @@ int pgx_num_sms();
 // Launches a kernel that starts with grid_begin() behind the work in front of
 // it on the stream: its launch is prepared while a kernel in front still runs,
 // and its blocks start when that one has completed.  For chains of short
-// kernels, where each launch is about a microsecond that nothing else fills
-// (256x256x16 box 1192 -> 1114 us, a 1280x720 frame 3730 -> 3655, its learned
-// guide 3576 -> 3494, differentiable 256x256x16 3816 -> 3682).  Letting the
-// next kernel's blocks in early, to wait on the SMs, was no better (1121,
-// 3683, 3874, 3678).  Build of 2,093,058 triangles 2.93 -> 2.84 ms, a cache of
-// 900,001 records with its queries 1.50 -> 1.42.  A batch's captured graph gains nothing (15.89 / 15.96 ms)
-// and keeps plain launches.
+// kernels, where each launch is about a microsecond that nothing else fills.
+// Plain launches / these / these with the next kernel's blocks let in early,
+// to wait on the SMs, us in one run: 256x256x16 box 1192 / 1114 / 1121, a
+// 1280x720 frame 3730 / 3655 / 3683, its learned guide 3576 / 3494 / 3874,
+// differentiable 256x256x16 3816 / 3682 / 3678.  Plain launches / these: build
+// of 2,093,058 triangles 2.93 / 2.84 ms, a cache of 900,001 records with its
+// queries 1.50 / 1.42.  A batch's captured graph gains nothing (15.89 / 15.96
+// ms) and keeps plain launches.
 template <class... P, class... A>
 void launch_behind(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
     cudaLaunchAttribute at{};

@@ -9,18 +9,22 @@
 // One path per (pixel, sample); a wave holds up to 2^25 of them.  The
 // recursion of the reference becomes a loop over depth with queue-per-stage
 // kernels:
-//   camgen -> [trace -> classify -> (guide_infer) -> shade x 6 classes]
+//   camgen -> [trace -> classify -> (guide_infer) -> shade]
 //             x (max_depth + 1) -> trace -> finalize
 // `trace` (k_trace_step) holds the extension rays of a depth and the shadow
-// rays of the depth before it.
-// `classify` bins the depth's paths by surface class and `shade` runs once
-// per class with that class's code compiled in; it compacts surviving paths
+// rays of the depth before it; waves above 2^24 paths and renders with stage
+// times trace them in launches of their own (k_extend, k_shadow).
+// `classify` bins the depth's paths by surface class, and the blocks of
+// `shade` walk the bins class by class, each with that class's code compiled
+// in; it compacts surviving paths
 // into the next queue with warp-aggregated atomics (ballot + popc, one
 // atomicAdd per warp) and appends next-event shadow rays to a shadow queue;
 // their any-hit traversal adds the stored contribution of unoccluded rays to
 // the path's radiance.  Queue lengths live on the device,
 // so a wave needs no host round trip (batches replay their waves from a
-// captured CUDA graph).
+// captured CUDA graph).  Waves of up to 65,536 paths run in one launch, a
+// thread per path (k_path), except the learned guide's, whose network wants
+// tiles of paths.
 //
 // Each path owns a PCG32 stream keyed by (seed, pixel, sample) and draws
 // from it in the reference's order (jitter, light pick, light sample, RR,
@@ -48,7 +52,7 @@ constexpr int kCollectionSPP = 128 / 8;  // Renderer.h:721
 constexpr int kStats = 8;                 // 64-bit statistics counters
 constexpr int kProfEvents = 4 * (kMaxDepthCap + 2);
 // Shading classes: paths of one depth are binned by what they hit and shaded
-// one class per launch, so every SM runs one class's code path at a time.
+// bin after bin, so most SMs run one class's code path at a time.
 constexpr int kShadeClasses = 6;  // miss, emitter, diffuse, conductor, glass, other
 
 // Per-path state, structure of arrays.
@@ -86,7 +90,7 @@ struct PathState {
     unsigned* nvertices;
     int64_t capacity;
     int64_t vcapacity;
-    // learned guide: per-path mixture (10 float4), training records
+    // learned guide: per-path mixture (mlp::kPacked float4), training records
     float4* guide;
     int* fallback;    // per path: QuadTree root standing in for the network (-1: the network, -2: the BSDF)
     float4* rec_wo;   // wo
@@ -710,8 +714,8 @@ __device__ __forceinline__ void push_shadow(PathState& ps, int depth, int p, flo
     }
 }
 
-// Bins the paths of this depth by shading class (k_shade then runs once per
-// class on its bin).  Each block takes tiles of kClassifyTile queue entries,
+// Bins the paths of this depth by shading class (k_shade then walks the bins).
+// Each block takes tiles of kClassifyTile queue entries,
 // kClassifyItems per thread so the hit and class gathers overlap; entries are
 // ranked within their class by warp match + shared-memory counters and each
 // class bin is reserved with ONE global atomic per tile (a warp-level append
@@ -2840,8 +2844,8 @@ int batch_tables(pgx_batch* b, int spp, float* scratch) {
     return PGX_OK;
 }
 
-// Enqueues every wave of one call: camera rays, (extend, shade, shadow) per
-// depth, splat.
+// Enqueues every wave of one call: camera rays, (trace, classify, shade) per
+// depth, the last shadow rays, splat.
 int batch_enqueue(pgx_batch* b, int64_t total, int depth, const pgx_batch_tuning& tu) {
     pgx_ctx* h = b->host;
     RenderState* rs = state_of(h);
