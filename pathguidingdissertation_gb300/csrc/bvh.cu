@@ -85,13 +85,9 @@ struct RecView {
     float4* cent;
 };
 
-// Work for phase B: node and which record buffer holds its triangles.  A node
-// that stays a leaf in phase A only has its triangle ids copied, in pieces:
-// first position, and the piece's length above the flags.  (2,000,000
-// coincident triangles are one leaf: 15.4 ms with one warp for it, 0.30
-// with pieces.)
-constexpr int kSmallBuf = 1, kSmallLeaf = 2, kLeafShift = 2;
-constexpr int kLeafPiece = 1024;
+// Work for phase B: node, and which record buffer holds its triangles; a
+// leaf of one chunk only has its triangle ids copied.
+constexpr int kSmallBuf = 1, kSmallLeaf = 2;
 
 __device__ __forceinline__ float area_x(float mnx, float mny, float mnz, float mxx, float mxy, float mxz) {
     // AABB::area, Geometry.h:212-215
@@ -185,18 +181,6 @@ __device__ __forceinline__ void add_small(int2* small, int small_cap, BuildMisc*
         small[s] = make_int2(node, flags);
     else
         atomicExch(&misc->overflow, 1);
-}
-
-__device__ __forceinline__ void add_leaf(int2* small, int small_cap, BuildMisc* misc, int start, int count, int buf) {
-    const int pieces = (count + kLeafPiece - 1) / kLeafPiece;
-    const int s = atomicAdd(&misc->nsmall, pieces);
-    if (s + pieces > small_cap) {
-        atomicExch(&misc->overflow, 1);
-        return;
-    }
-    for (int p = 0; p < pieces; p++)
-        small[s + p] = make_int2(start + p * kLeafPiece,
-                                 (min(kLeafPiece, count - p * kLeafPiece) << kLeafShift) | kSmallLeaf | buf);
 }
 
 __global__ void k_root_init(pgx_bvh_node* nodes, int* node_rec, BuildItem* items, int2* chunks, int2* small,
@@ -508,7 +492,7 @@ __device__ __forceinline__ void partition_chunk(BuildItem& it, int first, int ax
             if (side == 0) {
                 nd.left_first = start;
                 nd.used = count;
-                add_leaf(out.small, out.small_cap, misc, start, count, from);
+                add_small(out.small, out.small_cap, misc, it.node, kSmallLeaf | from);
             }
         } else {
             unsigned long long at = 0;
@@ -633,7 +617,8 @@ __global__ void __launch_bounds__(kThreads) k_bin(BuildItem* __restrict__ items,
                     it.split = 0;
                     nd.left_first = start;
                     nd.used = count;
-                    add_leaf(out.small, out.small_cap, misc, start, count, buf ? kSmallBuf : 0);
+                    // (the chunks of a larger leaf: k_partition)
+                    if (nch == 1) add_small(out.small, out.small_cap, misc, it.node, kSmallLeaf | (buf ? kSmallBuf : 0));
                 } else if (nch > 1) {
                     it.split = 1;
                     it.axis = axis;
@@ -650,10 +635,14 @@ __global__ void __launch_bounds__(kThreads) k_bin(BuildItem* __restrict__ items,
     }
 }
 
-// Partition of the chunks of the nodes that have several.
+// Partition of the chunks of the nodes that have several; where such a node
+// stays a leaf (triangles no plane separates), the chunks' triangle ids go to
+// the leaf order here, by all its blocks: 2,000,000 coincident triangles are
+// one leaf, and the build takes 15.4 ms with one warp of k_small for it, 0.27
+// with these.
 __global__ void __launch_bounds__(kThreads) k_partition(BuildItem* __restrict__ items, const int2* __restrict__ chunks,
                                                         BuildMisc* __restrict__ misc, int level, RecView rec,
-                                                        BuildOut out) {
+                                                        int* __restrict__ idx, BuildOut out) {
     grid_begin();
     __shared__ PartShared sh;
     if (misc->nslots[level] == 0) return;  // no such node on this level
@@ -661,7 +650,11 @@ __global__ void __launch_bounds__(kThreads) k_partition(BuildItem* __restrict__ 
     for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const int2 ch = chunks[c];
         BuildItem& it = items[ch.x];
-        if (!it.split) continue;  // uniform per block
+        if (!it.split) {  // uniform per block
+            const int start = it.start, end = it.count > kChunk ? min(it.count, ch.y + kChunk) : 0;
+            for (int j = ch.y + threadIdx.x; j < end; j += kThreads) idx[start + j] = __float_as_int(rec.lo[start + j].w);
+            continue;
+        }
         partition_chunk<false>(it, ch.y, it.axis, it.pos, misc, level, rec, out, sh);
     }
 }
@@ -698,12 +691,10 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(const int2* __restri
     const int nsmall = misc->nsmall;
     for (int job = blockIdx.x * kSmallWarps + (threadIdx.x >> 5); job < nsmall; job += gridDim.x * kSmallWarps) {
         const int2 jb = small[job];
+        const pgx_bvh_node root = nodes[jb.x];
+        const int first = root.left_first, total = root.used;
         const RecView rec = (jb.y & kSmallBuf) ? rec1 : rec0;
-        const bool piece = (jb.y & kSmallLeaf) != 0;
-        pgx_bvh_node root{};
-        if (!piece) root = nodes[jb.x];
-        const int first = piece ? jb.x : root.left_first, total = piece ? jb.y >> kLeafShift : root.used;
-        if (piece || total <= kMaxLeaf) {
+        if ((jb.y & kSmallLeaf) || total <= kMaxLeaf) {
             for (int k = lane; k < total; k += 32) idx[first + k] = __float_as_int(rec.lo[first + k].w);
             continue;
         }
@@ -1054,7 +1045,7 @@ int bvh_build_gpu(pgx_ctx* ctx) {
             const BuildOut out{recs[b], b, items[b], chunks[b], (int)item_cap, (int)chunk_cap, (int)slot_cap,
                                small, (int)small_cap, nodes, node_rec};
             launch_behind(k_bin, grid, kThreads, 0, s, items[a], chunks[a], misc, level, recs[a], a, bins, out);
-            launch_behind(k_partition, grid, kThreads, 0, s, items[a], chunks[a], misc, level, recs[a], out);
+            launch_behind(k_partition, grid, kThreads, 0, s, items[a], chunks[a], misc, level, recs[a], idx, out);
         }
         PGX_CUDA_TRY(ctx, cudaGetLastError());
         int left = 0, bad = 0;
