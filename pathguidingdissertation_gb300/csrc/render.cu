@@ -115,7 +115,7 @@ struct RenderState {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t prof[kProfEvents] = {};
     // differentiable rendering: evaluation parameters and scratch
-    DevBuf d_mats, d_env, d_partial, d_img, d_dimg, d_genv, d_galb, d_grough, d_samples, d_ts;
+    DevBuf d_mats, d_env, d_partial, d_img, d_dimg, d_genv, d_galb, d_grough, d_samples, d_ts, d_rec;
     uint64_t d_scene = 0;  // upload the evaluation parameters belong to (0: none)
 };
 
@@ -2018,7 +2018,7 @@ RenderState* state_of(pgx_ctx* ctx) {
 // cannot be had, the wave's buffers are all given back.
 int ensure_state(pgx_ctx* ctx, RenderState* rs, int64_t cap, int rec_depth, int64_t vcap, bool guide = false,
                  int train_depth = 0, int64_t tcap = 0, bool batch = false, bool diff = false) {
-    const size_t n = (size_t)cap, nrec = (size_t)rec_depth * n, ntrain = (size_t)train_depth * n;
+    const size_t n = (size_t)cap, nrec = diff ? 0 : (size_t)rec_depth * n, ntrain = (size_t)train_depth * n;
     const std::pair<DevBuf*, size_t> wave[] = {
         {&rs->o, sizeof(float4) * n},
         {&rs->d, sizeof(float4) * n},
@@ -2048,6 +2048,7 @@ int ensure_state(pgx_ctx* ctx, RenderState* rs, int64_t cap, int rec_depth, int6
         {&rs->train, sizeof(float) * 13 * (size_t)tcap},
         {&rs->scene, batch ? sizeof(int) * n : 0},
         {&rs->d_ts, diff ? sizeof(float4) * n : 0},
+        {&rs->d_rec, diff ? 5 * sizeof(float4) * (size_t)rec_depth * n : 0},
     };
     rs->capacity = rs->vcapacity = rs->tcapacity = 0;
     for (const auto& [buf, bytes] : wave) {
@@ -2725,6 +2726,8 @@ extern "C" int pgx_diff_adjoint(pgx_ctx* ctx, int32_t spp, uint64_t seed, int32_
     SceneView sv = scene_view(ctx);
     PathState ps = path_view(rs);
     dv.stride = wave;
+    float4** rec[5] = {&ps.rec_pos, &ps.rec_nrm, &ps.rec_wi, &ps.rec_w, &ps.rec_e};
+    for (int k = 0; k < 5; k++) *rec[k] = rs->d_rec.as<float4>() + (size_t)k * wave * (max_depth + 1);
     for (int64_t at = 0; at < npix * spp; at += wave) {
         dv.first = at;
         dv.count = std::min(wave, npix * spp - at);
