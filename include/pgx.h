@@ -217,7 +217,7 @@ typedef struct pgx_render_config {
  * float sums in another order; in waves of up to 2^24 paths it traces
  * extension and shadow rays in one launch, and in waves of up to 65,536, other
  * than the learned guide's, whole paths.  The times are those of the separate
- * launches and add up to more than such a render takes. */
+ * launches, which in small waves add up to more than such a render takes. */
 #define PGX_RENDER_TIMING 8
 
 /* Statistics of the last pgx_render call.  The per-stage times are filled
